@@ -365,12 +365,10 @@ def run(state):
         _hold(state)
     if state["graphs"] is not None:
         return _decode(state)
-    entries = []
+    entries = _next(state) if state["held"] else []  # (the scheduler takes the running requests first)
     for i, ids in enumerate(state["prompts"]):
         r.add_request("p%d" % i)
         entries.append(state["entry"]("p%d" % i, ids, [len(ids) - 1]))
-    if state["held"]:
-        entries += _next(state)
     logits = r.step(entries)
     for i in range(len(state["prompts"])):
         r.end_request("p%d" % i)
@@ -931,7 +929,7 @@ def _forward(case, cfg, w, ids):
 def exact(case, seed):
     cfg = _config(case)
     prompts, held = _ids(case, seed)
-    seqs = prompts + [h[:n + 1] for h, n in zip(held, _held_lengths(case))]
+    seqs = [h[:n + 1] for h, n in zip(held, _held_lengths(case))] + prompts
     groups, rows = [], 0
     for s in sorted(range(len(seqs)), key=lambda i: len(seqs[i])):  # sequences of like lengths side by side
         if groups and len(groups[-1]) < 8 and len(seqs[s]) <= 1.3 * len(seqs[groups[-1][0]]):
