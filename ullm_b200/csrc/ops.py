@@ -135,7 +135,7 @@ class Kernels:
                 "ULLM_B200_FUSED_MLP_ROWS", "ULLM_B200_LT_ROWS", "ULLM_B200_FUSED_TAIL_ROWS",
                 "ULLM_B200_STREAM_ALL_ROWS", "ULLM_B200_CHAIN_NORMS", "ULLM_B200_GENERAL_ATTN_TC", "ULLM_B200_SSD_CHUNK",
                 "ULLM_B200_PAIR_BIASED_ROWS", "ULLM_B200_GLA_CHUNK",
-                "ULLM_B200_STATE_STEP")
+                "ULLM_B200_STATE_STEP", "ULLM_B200_PLAIN_ATTN")
 
     def apply_switches(self, env) -> None:
         """Sets every kernel choice from `env` (a mapping; the process environment at start-up): a switch that is
@@ -170,6 +170,8 @@ class Kernels:
         # rows from which a step with distance biases (heads of 128) takes the tcgen05 prompt kernel
         self.pair_biased_rows = int(get("ULLM_B200_PAIR_BIASED_ROWS", "128"))
         self.window_attention_tc = get("ULLM_B200_WINDOW_ATTN_TC", "1") != "0"
+        # attention of the 32-bit engine and of float16 by row tiles (csrc/attention_plain.cu); 0: the general kernel always
+        self.plain_attention_on = get("ULLM_B200_PLAIN_ATTN", "1") != "0"
         # the splits of a request's keys merge inside a thread-block cluster (at most 8 splits) instead of through
         # scratch arrays and a second kernel
         # ("auto": for steps of at most 8 rows; "1" / "0": always / never, with `decode_split_target` splits)
@@ -229,6 +231,8 @@ class Kernels:
             "ullm_qk_norm_rope_store": [I, P, I, I, I, I, P, P, F, P, P, I, I, P, P, P, P, LL, P, P],
             "ullm_qk_norm_in_place": [I, P, I, I, I, I, P, P, F, P, P],
             "ullm_paged_attention_generic": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, LL, P, P],
+            "ullm_attention_plain": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, LL, P, P],
+            "ullm_attention_plain_supported": [I, I, I, I],
             "ullm_decode_attention": [P, LL, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, I, LL, P, P],
             "ullm_decode_attention_balanced": [P, LL, P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, F, LL, P, P],
             "ullm_decode_attention_fused": [P, LL, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, I, LL, P, P, F, P, P, I,
@@ -2344,6 +2348,15 @@ class Kernels:
         if n_dec:
             raise KernelError("paged_attention: a step's decode rows were split off but no prompt kernel takes the rest")
         self.attention_path = "generic"
+        # 32-bit arithmetic at head sizes 64 and 128 (float32, float16): keys staged once for many rows; the kernel of one warp
+        # per row stays for every other size (per layer at Qwen3-0.6B sizes, prompts of 170 + 341 tokens: 76 against 749 us)
+        if self.plain_attention_on and self.lib.ullm_attention_plain_supported(_DT[qkv.dtype], head_dim, num_q, num_kv):
+            code = self.lib.ullm_attention_plain(
+                _DT[qkv.dtype], _ptr(qkv), qkv.stride(0), _ptr(out), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
+                block_table.shape[1], _ptr(req_slots), _ptr(cu_q), _ptr(kv_len), _ptr(token_req), T, cu_q.numel() - 1, num_q,
+                num_kv, head_dim, page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream())
+            if code != 4:  # (4: rows that do not start on the borders its reads need)
+                return self._check(code, f"attention_plain (head_dim {head_dim})")
         self._check(self.lib.ullm_paged_attention_generic(
             _DT[qkv.dtype], _ptr(qkv), qkv.stride(0), _ptr(out), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
             block_table.shape[1], _ptr(req_slots), _ptr(cu_q), _ptr(kv_len), _ptr(token_req), T, num_q, num_kv, head_dim, page_size,
