@@ -1,0 +1,85 @@
+"""The chunked matrix-memory recurrence (csrc/mlstm_chunk.cu) against the recurrence in 64 bits and against the token-by-token
+kernel: chunks that end early, several requests beside short ones, state carried from portion to portion, gates that forget at
+once and never, a maximum that stays and one that moves."""
+
+import pytest
+import torch
+
+from conftest import device
+from test_gpu_kernels import K
+
+pytestmark = [pytest.mark.gpu, pytest.mark.needs_cuda]
+
+
+def recurrence(q, k, v, gi, gf, S, n, m):
+    out = torch.zeros(q.shape[0], q.shape[1], v.shape[2], dtype=q.dtype, device=q.device)
+    for t in range(q.shape[0]):
+        m2 = torch.maximum(gf[t] + m, gi[t])
+        keep, take = torch.exp(gf[t] + m - m2), torch.exp(gi[t] - m2)
+        m = m2
+        S = keep[:, None, None] * S + take[:, None, None] * v[t][:, :, None] * k[t][:, None, :]
+        n = keep[:, None] * n + take[:, None] * k[t]
+        den = torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6
+        out[t] = (S * q[t][:, None, :]).sum(-1) / den[:, None]
+    return out, S, n, m
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 16, 16), (3, 128, 256), (1, 48, 144), (2, 256, 512)])
+@pytest.mark.parametrize("lens", [[64], [65, 3, 1, 130], [17, 16, 63, 200]])
+@pytest.mark.parametrize("forget", [-6.0, 0.0, 6.0])
+def test_chunks_match_the_recurrence(heads, dim, vdim, lens, forget):
+    from ullm_b200.engine import Workspace
+
+    kk, least, cap, scale = K(), 16, 15.0, dim ** -0.5
+    g = torch.Generator().manual_seed(3)
+    T, B = sum(lens), len(lens)
+    size = 2 * heads * dim + heads * vdim
+    qkv = torch.randn(T, size + 16, generator=g).bfloat16().to(device())
+    gates = (2.0 * torch.randn(T, 2 * heads, generator=g)).to(device())
+    bi, bf = torch.randn(heads, generator=g).to(device()), (forget + torch.randn(heads, generator=g)).to(device())
+    floats = heads * dim * (vdim + 1) + heads
+    stride = -(-floats // 4) * 4
+    state0 = torch.randn(B + 1, stride, generator=g).to(device())
+    slots = torch.randperm(B + 1, generator=g)[:B].int().to(device())
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=device())
+    req = torch.cat([torch.full((n,), r, dtype=torch.int32) for r, n in enumerate(lens)]).to(device())
+
+    def run(chunked):
+        state, out = state0.clone(), torch.full((T, heads * vdim), 5.0, device=device())
+        args = (qkv, 0, heads * dim, 2 * heads * dim, gates, bi, bf, state, cu, slots, req, out, B, heads, dim, vdim, scale, cap)
+        if chunked:
+            assert kk.mlstm_chunk(*args, Workspace(device(), T, B), least)
+            kk.mlstm_recurrence(*args, most_tokens=least)
+        else:
+            kk.mlstm_recurrence(*args)
+        kk.raise_on_status()
+        return out.double().cpu(), state.double().cpu()
+
+    got, state = run(True)
+    plain, state_p = run(False)
+    x = qkv.double().cpu()
+    q = x[:, :heads * dim].view(T, heads, dim) * scale
+    k = x[:, heads * dim:2 * heads * dim].view(T, heads, dim)
+    v = x[:, 2 * heads * dim:size].view(T, heads, vdim)
+    gd = gates.double().cpu()
+    gi = cap * torch.tanh((gd[:, :heads] + bi.double().cpu()) / cap)
+    gf = torch.nn.functional.logsigmoid(cap * torch.tanh((gd[:, heads:] + bf.double().cpu()) / cap))
+    ref, worst = torch.zeros(T, heads, vdim, dtype=torch.float64), 0.0
+    for r, n in enumerate(lens):
+        a, s = int(cu[r]), state0[int(slots[r])].double().cpu()
+        S, nn, m = s[:heads * dim * vdim].view(heads, vdim, dim), s[heads * dim * vdim:heads * dim * (vdim + 1)].view(heads, dim), \
+            s[heads * dim * (vdim + 1):floats]
+        ref[a:a + n], S, nn, m = recurrence(q[a:a + n], k[a:a + n], v[a:a + n], gi[a:a + n], gf[a:a + n], S, nn, m)
+        want = torch.cat([S.reshape(-1), nn.reshape(-1), m])
+        have = state[int(slots[r])][:floats]
+        worst = max(worst, float((have - want).norm() / want.norm()))
+    untouched = [i for i in range(B + 1) if i not in slots.tolist()]
+    assert torch.equal(state[untouched], state0.double().cpu()[untouched])
+
+    def err(o):
+        return float((o.view(T, heads, vdim) - ref).norm() / ref.norm())
+
+    print(f"chunks {err(got):.2e}, token by token {err(plain):.2e}, state {worst:.2e}")
+    # 32-bit sums: 1e-6 where nothing cancels.  Where the terms of the denominator cancel (long memories: up to 2e-5 here) the
+    # loss is the inputs' and the token-by-token kernel has it too: at most twice its distance
+    assert err(got) < 2.0 * err(plain) + 1e-6 and worst < 2e-6

@@ -43,7 +43,7 @@ mlstm_recurrence_kernel(const T* __restrict__ qkv, long long row_stride, int q_o
                         const float* __restrict__ bias_f, float* __restrict__ state, long long state_stride,
                         const int* __restrict__ cu_q, const int* __restrict__ req_slots,
                         const int* __restrict__ token_req, float* __restrict__ out, int heads, int dim, int vdim,
-                        int rs_arg, int chunk, float q_scale, float cap, int num_slots, int* status) {
+                        int rs_arg, int chunk, float q_scale, float cap, int num_slots, int* status, int most_tokens) {
   constexpr bool FULL = RS != 0;
   const int rs = FULL ? RS : rs_arg;
   // Threads 0 .. 127 run the recurrence; threads 128 .. 255 stage the next chunk of tokens (q, k, the tile's v,
@@ -60,7 +60,7 @@ mlstm_recurrence_kernel(const T* __restrict__ qkv, long long row_stride, int q_o
   const int col = blockIdx.x * cols_per_block + col_in_block * CPT;  // the thread's first column
   const bool col_ok = col < vdim;
   const int t0 = cu_q[req], t1 = cu_q[req + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || t1 - t0 > most_tokens) return;  // (longer portions are another kernel's)
   const bool padding = token_req[t0] < 0;  // a row that belongs to no request: zeros out, no state touched
   const int slot = req_slots[req];
   if (!padding && (slot < 0 || slot >= num_slots)) {
@@ -381,7 +381,7 @@ static int mlstm_launch(const void* qkv, long long row_stride, int q_off, int k_
                         const float* bias_i, const float* bias_f, float* state, long long state_stride,
                         const int* cu_q, const int* req_slots, const int* token_req, float* out, int requests,
                         int heads, int dim, int vdim, float q_scale, float cap, int num_slots, int* status,
-                        cudaStream_t st) {
+                        int most_tokens, cudaStream_t st) {
   const int rs = mlstm_rs(dim);
   // four (or two) columns per thread where that still leaves the SMs about two blocks each (fewer, fatter blocks: less
   // q / k staging, several multiply-add chains per row read: head size 256 x 512, one prompt of 2,048 tokens,
@@ -407,16 +407,16 @@ static int mlstm_launch(const void* qkv, long long row_stride, int q_off, int k_
       return ullm_launch_kernel(mlstm_recurrence_kernel<T, RPT_, RS_, 4>, grid, dim3(2 * MLSTM_THREADS), smem, st,     \
                                 (const T*)qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state,         \
                                 state_stride, cu_q, req_slots, token_req, out, heads, dim, vdim, rs, chunk, q_scale,   \
-                                cap, num_slots, status);                                                              \
+                                cap, num_slots, status, most_tokens);                                                              \
     if (cpt == 2)                                                                                                     \
       return ullm_launch_kernel(mlstm_recurrence_kernel<T, RPT_, RS_, 2>, grid, dim3(2 * MLSTM_THREADS), smem, st,     \
                                 (const T*)qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state,         \
                                 state_stride, cu_q, req_slots, token_req, out, heads, dim, vdim, rs, chunk, q_scale,   \
-                                cap, num_slots, status);                                                              \
+                                cap, num_slots, status, most_tokens);                                                              \
     return ullm_launch_kernel(mlstm_recurrence_kernel<T, RPT_, RS_, 1>, grid, dim3(2 * MLSTM_THREADS), smem, st,       \
                               (const T*)qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state,           \
                               state_stride, cu_q, req_slots, token_req, out, heads, dim, vdim, rs, chunk, q_scale,     \
-                              cap, num_slots, status);                                                                \
+                              cap, num_slots, status, most_tokens);                                                                \
   } while (0)
   if (dim == 64 && rs == 8) MLSTM_LAUNCH(8, 8);
   if (dim == 128 && rs == 16) MLSTM_LAUNCH(8, 16);
@@ -428,13 +428,13 @@ static int mlstm_launch(const void* qkv, long long row_stride, int q_off, int k_
 }
 
 // qkv: rows of `row_stride` elements that hold q [heads, dim] at q_off, k [heads, dim] at k_off and v [heads, vdim]
-// at v_off.  gates: [tokens, 2 heads] float32, the input-gate projections then the forget-gate projections (biases
+// at v_off; requests that bring more than `most_tokens` tokens are left alone.  gates: [tokens, 2 heads] float32, the input-gate projections then the forget-gate projections (biases
 // not yet added).  state: [num_slots, state_stride] float32.  out: [tokens, heads, vdim] float32.
 extern "C" int ullm_mlstm_recurrence(int dtype, const void* qkv, long long row_stride, int q_off, int k_off,
                                      int v_off, const float* gates, const float* bias_i, const float* bias_f,
                                      float* state, long long state_stride, const int* cu_q, const int* req_slots,
                                      const int* token_req, float* out, int requests, int heads, int dim, int vdim,
-                                     float q_scale, float cap, int num_slots, int* status, void* stream) {
+                                     float q_scale, float cap, int num_slots, int* status, void* stream, int most_tokens) {
   cudaStream_t st = (cudaStream_t)stream;
   if (requests < 0 || !ullm_mlstm_supported(heads, dim, vdim)) return ULLM_ERR_UNSUPPORTED;
   if (state_stride < ullm_mlstm_state_floats(heads, dim, vdim) || cap <= 0.f) return ULLM_ERR_BAD_SIZE;
@@ -443,15 +443,15 @@ extern "C" int ullm_mlstm_recurrence(int dtype, const void* qkv, long long row_s
   if (dtype == ULLM_DTYPE_F32)
     return mlstm_launch<float>(qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state, state_stride,
                                cu_q, req_slots, token_req, out, requests, heads, dim, vdim, q_scale, cap, num_slots,
-                               status, st);
+                               status, most_tokens, st);
   if (dtype == ULLM_DTYPE_BF16)
     return mlstm_launch<__nv_bfloat16>(qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state,
                                        state_stride, cu_q, req_slots, token_req, out, requests, heads, dim, vdim,
-                                       q_scale, cap, num_slots, status, st);
+                                       q_scale, cap, num_slots, status, most_tokens, st);
   if (dtype == ULLM_DTYPE_F16)
     return mlstm_launch<__half>(qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state, state_stride,
                                 cu_q, req_slots, token_req, out, requests, heads, dim, vdim, q_scale, cap, num_slots,
-                                status, st);
+                                status, most_tokens, st);
   return ULLM_ERR_BAD_DTYPE;
 }
 

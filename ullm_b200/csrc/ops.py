@@ -135,7 +135,8 @@ class Kernels:
                 "ULLM_B200_FUSED_MLP_ROWS", "ULLM_B200_LT_ROWS", "ULLM_B200_FUSED_TAIL_ROWS",
                 "ULLM_B200_STREAM_ALL_ROWS", "ULLM_B200_CHAIN_NORMS", "ULLM_B200_GENERAL_ATTN_TC", "ULLM_B200_SSD_CHUNK",
                 "ULLM_B200_PAIR_BIASED_ROWS", "ULLM_B200_GLA_CHUNK",
-                "ULLM_B200_STATE_STEP", "ULLM_B200_PLAIN_ATTN")
+                "ULLM_B200_STATE_STEP", "ULLM_B200_PLAIN_ATTN", "ULLM_B200_MOE_TCGEN05_ROWS",
+                "ULLM_B200_MLSTM_CHUNK", "ULLM_B200_LATENT_TCGEN05", "ULLM_B200_MOE_STREAM_TOKENS")
 
     def apply_switches(self, env) -> None:
         """Sets every kernel choice from `env` (a mapping; the process environment at start-up): a switch that is
@@ -176,6 +177,8 @@ class Kernels:
         # scratch arrays and a second kernel
         # ("auto": for steps of at most 8 rows; "1" / "0": always / never, with `decode_split_target` splits)
         mode = get("ULLM_B200_DECODE_CLUSTER", "auto")
+        # and for the matrix memory with exponential gates
+        self.mlstm_chunk_on = get("ULLM_B200_MLSTM_CHUNK", "1") != "0"
         self.decode_cluster_merge = {"1": True, "0": False}.get(mode, "auto")
         # decode steps: the per-request decode attention kernel applies the q/k norm and the rotation and writes the
         # new key and value itself (one launch less per layer)
@@ -265,7 +268,9 @@ class Kernels:
             "ullm_norm_scale_add_norm": [I, P, P, P, I, I, F, F, P, F, P, P],
             "ullm_rmsnorm_rows_f32": [I, P, P, P, P, I, I, I, F, P, P],
             "ullm_cast_rows_f32": [I, P, P, LL, P],
-            "ullm_mlstm_recurrence": [I, P, LL, I, I, I, P, P, P, P, LL, P, P, P, P, I, I, I, I, F, F, I, P, P],
+            "ullm_mlstm_recurrence": [I, P, LL, I, I, I, P, P, P, P, LL, P, P, P, P, I, I, I, I, F, F, I, P, P, I],
+            "ullm_mlstm_chunk": [P, LL, I, I, I, P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, F, F, I, I, P, P],
+            "ullm_mlstm_chunk_supported": [I, I, I],
             "ullm_mlstm_out_gate": [I, P, P, LL, P, P, I, I, I, F, P],
             "ullm_gated_add_f32": [I, P, P, P, LL, P, P, P, P, I, I, P],
             "ullm_side_gate_mul": [I, P, P, P, LL, I, P, I, I, I, P, P, P, P, P],
@@ -351,6 +356,8 @@ class Kernels:
         L.ullm_decode_attention_balanced_supported.restype = c_int
         L.ullm_decode_attention_balanced_scratch_floats.argtypes = [I, I]
         L.ullm_decode_attention_balanced_scratch_floats.restype = c_longlong
+        L.ullm_mlstm_chunk_floats.argtypes = [I, I, I, I, I, I]
+        L.ullm_mlstm_chunk_floats.restype = c_longlong
         L.ullm_decode_attention_tcgen05_supported.argtypes = [I, I, I, I, I]
         L.ullm_decode_attention_tcgen05_supported.restype = c_int
         L.ullm_decode_attention_tcgen05_scratch_floats.argtypes = [I]
@@ -1458,6 +1465,42 @@ class Kernels:
             raise KernelError("gla_recurrence: q, k or v lie outside the rows")
         if z_bias is not None and z_bias.numel() != heads * dim:
             raise KernelError("gla_recurrence: the decay bias has the wrong length")
+    def mlstm_chunk_applies(self, dtype, heads: int, dim: int, vdim: int) -> bool:
+        """True when `mlstm_chunk` takes these sizes (bfloat16; see csrc/mlstm_chunk.cu)."""
+        return bool(self.mlstm_chunk_on and dtype == torch.bfloat16 and self.lib.ullm_mlstm_chunk_supported(heads, dim, vdim))
+
+    @_timed("mlstm", skipped=True)
+    def mlstm_chunk(self, qkv, q_off, k_off, v_off, gates, bias_i, bias_f, state, cu_q, req_slots, token_req, out, requests,
+                    heads, dim, vdim, q_scale, cap, workspace, least: int) -> bool:
+        """`mlstm_recurrence` in its chunked form on the tensor cores, for the requests that bring MORE than `least` tokens (the
+        others are left alone).  False where the rows do not start on 16-byte borders (nothing has run then)."""
+        _need(qkv, "qkv", torch.bfloat16)
+        _need(gates, "gates", torch.float32)
+        _need(state, "state", torch.float32)
+        _need(out, "out", torch.float32)
+        for t_, n_ in ((bias_i, "input gate bias"), (bias_f, "forget gate bias")):
+            if t_ is not None:
+                _need(t_, n_, torch.float32)
+        for t_, n_ in ((cu_q, "cu_q"), (req_slots, "req_slots"), (token_req, "token_req")):
+            _need(t_, n_, torch.int32)
+        T = qkv.shape[0]
+        if gates.shape != (T, 2 * heads) or out.shape != (T, heads * vdim) or state.dim() != 2:
+            raise KernelError(f"mlstm_chunk: qkv {tuple(qkv.shape)}, gates {tuple(gates.shape)}, out {tuple(out.shape)}")
+        if max(q_off, k_off) + heads * dim > qkv.shape[1] or v_off + heads * vdim > qkv.shape[1]:
+            raise KernelError("mlstm_chunk: q, k or v lie outside the rows")
+        floats = self.lib.ullm_mlstm_chunk_floats
+        scratch = workspace.get("mlstm.chunks", 1, int(floats(max(T, workspace.max_tokens), max(requests, workspace.max_requests),
+                                                              heads, dim, vdim, int(least))), torch.float32)
+        code = self.lib.ullm_mlstm_chunk(
+            _ptr(qkv), qkv.stride(0), q_off, k_off, v_off, _ptr(gates), _ptr(bias_i), _ptr(bias_f), _ptr(scratch), _ptr(state),
+            state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req), _ptr(out), T, requests, heads, dim, vdim,
+            float(q_scale), float(cap), state.shape[0], int(least), _ptr(self.status), _stream())
+        if code == 4:
+            return False
+        self._check(code, f"mlstm_chunk (heads {heads}, dim {dim}, vdim {vdim})")
+        self.launches += 3
+        return True
+
         if single and self.state_step_on and T == requests:
             code = self.lib.ullm_gla_step(
                 _DT[qkv.dtype], _ptr(qkv), qkv.stride(0), q_off, k_off, v_off, _ptr(z), z.stride(0), _ptr(z_bias),

@@ -14,7 +14,8 @@ dtype; the gate projections are a product of their own with a 32-bit result.
 
 The state (S, n, m of every head, `Kernels.mlstm_state_floats` floats) is one row per request slot in the cache
 manager's state rows; it is zeroed when a slot is handed out and carried from step to step.  One kernel runs the
-recurrence over any mix of prompt portions and single tokens (csrc/mlstm.cu).
+recurrence over any mix of prompt portions and single tokens (csrc/mlstm.cu); portions of more than CHUNK_LEAST tokens
+in bfloat16 run in chunks on the tensor cores (csrc/mlstm_chunk.cu), whose results differ by 32-bit rounding.
 """
 
 from __future__ import annotations
@@ -24,6 +25,7 @@ import torch
 from ..csrc import kernels
 from .base import Mixer, ParamDecl, StateNeed
 from .linear import linear
+from .mamba2 import CHUNK_LEAST
 from .registry import register_mixer
 
 
@@ -100,9 +102,15 @@ class MLSTM(Mixer):
         gates = ws.tokens("mlstm.gates", T, 2 * Hn, torch.float32)
         K.linear_f32_out(x, self.w_if, gates)
         o = ws.tokens("mlstm.o", T, vs, torch.float32)
-        K.mlstm_recurrence(qkvg, 0, qk, 2 * qk, gates, self.tensors[n["i_bias"]], self.tensors[n["f_bias"]],
-                           cache.state, ctx.cu_q, ctx.req_slots, ctx.token_req, o, ctx.num_requests, Hn, d, dv,
-                           d ** -0.5, self.gate_cap)
+        args = (qkvg, 0, qk, 2 * qk, gates, self.tensors[n["i_bias"]], self.tensors[n["f_bias"]], cache.state, ctx.cu_q,
+                ctx.req_slots, ctx.token_req, o, ctx.num_requests, Hn, d, dv, d ** -0.5, self.gate_cap)
+        # prompt portions in chunks on the tensor cores (bfloat16, at the sizes that form takes), the rest token by token
+        chunked = (ctx.max_q_len > CHUNK_LEAST and x.is_cuda and K.mlstm_chunk_applies(x.dtype, Hn, d, dv)
+                   and K.mlstm_chunk(*args, ws, CHUNK_LEAST))
+        if not chunked:
+            K.mlstm_recurrence(*args)
+        elif ctx.num_requests > 1:
+            K.mlstm_recurrence(*args, most_tokens=CHUNK_LEAST)
         gated = ws.tokens("mlstm.gated", T, vs, x.dtype)
         K.mlstm_out_gate(o, qkvg[:, 2 * qk + vs:], self.tensors[n["norm"]], self.eps, gated, Hn, dv)
         out = ws.tokens("mixer.out", T, self.hidden_size, x.dtype)
