@@ -1,0 +1,80 @@
+"""The routed experts' grouped product on tcgen05 (csrc/moe_tcgen05.cu) against a 32-bit reference and the mma.sync kernel, where
+its tiles end: experts with no rows, one row, a row less and more than a tile; columns and k that fill no whole tile; choices that
+name no expert; weights on the input; every activation."""
+
+import pytest
+import torch
+
+from test_gpu_kernels import K, rnd
+
+pytestmark = [pytest.mark.gpu, pytest.mark.needs_cuda]
+
+
+def reference(x, w, choice, weight, top, from_pairs, gated, act, limit, alpha, rows_of):
+    out = {}
+    for p in range(choice.numel()):
+        e = int(choice.view(-1)[p])
+        if e >= w.shape[0]:
+            continue
+        out.setdefault(e, []).append(p)
+    n = w.shape[1] // 2 if gated else w.shape[1]
+    full = torch.zeros(choice.numel(), n, dtype=torch.float32, device=x.device)
+    for e, pairs in out.items():
+        p = torch.tensor(pairs, device=x.device)
+        v = (x[p // top] if from_pairs else x[rows_of[p]]).float() @ w[e].float().t()
+        if weight is not None:
+            v = v * weight.view(-1)[p][:, None]
+        if gated:
+            g, u = v[:, :n], v[:, n:]
+            if act == 2:
+                g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+                v = g * torch.sigmoid(alpha * g) * (u + 1)
+            else:
+                v = (torch.nn.functional.silu(g) if act == 0 else torch.nn.functional.gelu(g, approximate="tanh")) * u
+        elif act == 3:
+            v = v.clamp(min=0) ** 2
+        full[p] = v
+    return full
+
+
+@pytest.mark.parametrize("counts,top", [([0, 1, 127, 128, 129, 3], 1), ([257, 0, 0, 1], 2), ([5] * 40, 3), ([1, 0, 16, 0], 1), ([2], 1)])
+@pytest.mark.parametrize("n_out,k", [(128, 64), (264, 200), (72, 512), (520, 1032)])
+@pytest.mark.parametrize("gated,act,weighted", [(True, 0, True), (True, 1, False), (True, 2, False), (False, 3, False), (False, -1, True)])
+def test_grouped_product_matches_the_reference(counts, top, n_out, k, gated, act, weighted):
+    kk = K()
+    E = len(counts)
+    total = -(-sum(counts) // top) * top
+    flat = [e for e, n in enumerate(counts) for _ in range(n)] + [E + 1] * (total - sum(counts))  # (E + 1: no expert's)
+    g = torch.Generator().manual_seed(5)
+    choice = torch.tensor(flat, dtype=torch.int32)[torch.randperm(total, generator=g)].view(-1, top).contiguous().cuda()
+    T = total // top
+    offsets = torch.empty(E + 1, dtype=torch.int32, device="cuda")
+    order, place = torch.zeros(T, top, dtype=torch.int32, device="cuda"), torch.zeros(T, top, dtype=torch.int32, device="cuda")
+    kk.moe_arrange(choice, total, E, offsets, order, place)
+    w = rnd(E, (2 if gated else 1) * n_out, k, seed=6, dtype=torch.bfloat16, scale=k ** -0.5)
+    weight = (rnd(T, top, seed=7).abs() + 0.1) if weighted else None
+    for from_pairs in (True, False):
+        x = rnd(T if from_pairs else total, k, seed=8, dtype=torch.bfloat16)
+        out = torch.full((total, n_out), 9.0, dtype=torch.bfloat16, device="cuda")
+        old = kk.moe_tcgen05_rows
+        try:
+            kk.moe_tcgen05_rows = 0
+            gathered = torch.empty(total, k, dtype=torch.bfloat16, device="cuda") if from_pairs else None
+            kk.moe_grouped_linear(x, w, offsets, order, weight, out, top, from_pairs, gated, act, 3.0, 1.702, gathered=gathered)
+            other = torch.full_like(out, 9.0)
+            kk.moe_tcgen05_rows = 1 << 30
+            kk.moe_grouped_linear(x, w, offsets, order, weight, other, top, from_pairs, gated, act, 3.0, 1.702)
+        finally:
+            kk.moe_tcgen05_rows = old
+        kk.raise_on_status()
+        live = choice.view(-1).cpu() < E
+        at = place.view(-1).long()
+        ref = reference(x, w, choice.cpu(), weight, top, from_pairs, gated, act, 3.0, 1.702, at)
+        used = int(live.sum())
+        got, gen = out[at][live.cuda()].float(), other[at][live.cuda()].float()
+        ref = ref[live.cuda()]
+        s = ref.abs().max().item()
+        # one rounding to bfloat16 (2^-9 of the value) behind 32-bit sums of at most 1,032 products of order k^-1/2
+        assert (got - ref).abs().max().item() <= (2 ** -8 + 1e-4) * s
+        assert (got - gen).abs().max().item() <= (2 ** -7 + 1e-4) * s
+        assert (out[used:] == 9.0).all()  # (places that belong to no expert stay as they were)

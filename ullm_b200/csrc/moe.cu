@@ -25,6 +25,7 @@
 // The grouped product is a tiled kernel with 32-bit accumulation for float32 and 16-bit storage alike; a block
 // finds its (expert, row tile) from the offsets, so the grid depends only on the step's size.
 #include "common.cuh"
+#include "moe_act.cuh"
 
 #define MOE_MAX_TOP 32
 
@@ -173,24 +174,6 @@ __global__ void moe_arrange_kernel(const int* __restrict__ choice, int pairs, in
       place[p] = 0;  // (no expert's row: whoever combines must not find an index that was never written)
     }
   }
-}
-
-__device__ __forceinline__ float moe_gate_act(int act, float g, float u, float limit, float alpha) {
-  if (act == 2) {
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return g / (1.f + expf(-alpha * g)) * (u + 1.f);
-  }
-  return (act == 0 ? act_silu(g) : act_gelu_tanh(g)) * u;
-}
-
-// the activation of a product without gate rows
-__device__ __forceinline__ float moe_plain_act(int act, float v) {
-  if (act == 3) {
-    v = fmaxf(v, 0.f);
-    return v * v;
-  }
-  return v;
 }
 
 #define MOE_BM 32

@@ -115,6 +115,7 @@ class Kernels:
         self._lt_ws = None
         self._lt_tuned = set()
         self.timer = None  # a KernelGroupTimer while a profile is being taken
+        self._moe_plain = False
         # groups of kernels (the names `_timed` books them under) that are NOT launched: only for measuring what a
         # group costs inside a step, by the difference; the step's results are wrong while this is set
         self.skip_groups: frozenset = frozenset()
@@ -185,6 +186,8 @@ class Kernels:
         self.fuse_decode_rope = get("ULLM_B200_FUSE_DECODE_ROPE", "1") == "1"
         # a mixed step's leading one-token entries go to the decode attention kernel from this many on (0: never)
         self.mixed_decode_rows = int(get("ULLM_B200_MIXED_DECODE_ROWS", "4"))
+        # rows per expert, on average, from which the routed experts' products run on the tcgen05 kernel
+        self.moe_tcgen05_rows = int(get("ULLM_B200_MOE_TCGEN05_ROWS", "8"))
         # decode attention on the tcgen05 tensor cores (head size 128), the batch's keys cut evenly over the blocks
         self.use_tcgen05_decode = get("ULLM_B200_DECODE_TC", "0") == "1"
         # decode attention: the batch's keys cut evenly over the warps (True), every request split alike (False),
@@ -334,6 +337,7 @@ class Kernels:
         L.ullm_mlstm_state_floats.restype = c_longlong
         L.ullm_gla_supported.argtypes = [I, I, I]
         L.ullm_gla_supported.restype = c_int
+            "ullm_moe_grouped_tcgen05": [P, LL, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, P],
         L.ullm_gla_state_floats.argtypes = [I, I, I]
         L.ullm_gla_state_floats.restype = c_longlong
         L.ullm_gla_chunk_supported.argtypes = [I, I, I]
@@ -1928,10 +1932,11 @@ class Kernels:
 
     @_timed("moe", lambda x, weights, *r: weights.numel() * weights.element_size())
     def moe_grouped_linear(self, x, weights, offsets, sorted_pairs, pair_weight, out, top: int, rows_from_pairs: bool,
-                           gated: bool, act: int = 0, limit: float = 0.0, alpha: float = 1.0):
+                           gated: bool, act: int = 0, limit: float = 0.0, alpha: float = 1.0, gathered=None):
         """out[p] = W_e . x[row(p)] for every place p of every expert e (see csrc/moe.cu); weights
         [experts, (2 if gated) * n_out, k].  `act` 2: the clamped gate with `limit` and `alpha`; without gate rows 3:
-        max(v, 0)^2, anything else: no activation."""
+        max(v, 0)^2, anything else: no activation.  `gathered` ([pairs, k] of x's dtype, overwritten): room for the rows of
+        x in the order of their places, which the tcgen05 kernel wants when `rows_from_pairs`."""
         _need(x, "x")
         _need(weights, "expert weights", x.dtype)
         _need(out, "out", x.dtype)
@@ -2051,6 +2056,19 @@ class Kernels:
         if rotary_dim > 0:
             if cos is None or sin is None or cos.shape != sin.shape or cos.shape[1] != rotary_dim // 2:
                 raise KernelError("qk_norm_rope_store: cos/sin tables must be [positions, rotary_dim / 2]")
+        if gathered is not None:
+            _need(gathered, "gathered rows", x.dtype)
+            if gathered.numel() < pairs * K:
+                raise KernelError(f"moe_grouped_linear: gathered {tuple(gathered.shape)}")
+        if (x.dtype == torch.bfloat16 and not self._moe_plain and pairs >= self.moe_tcgen05_rows * E
+                and (not rows_from_pairs or gathered is not None)):
+            code = self.lib.ullm_moe_grouped_tcgen05(
+                _ptr(x), x.stride(0), _ptr(gathered) if rows_from_pairs else None, _ptr(weights), _ptr(offsets), _ptr(sorted_pairs), _ptr(pair_weight), _ptr(out),
+                pairs, E, top, int(rows_from_pairs), n_out, K, int(gated), act, float(limit), float(alpha), _ptr(self.status),
+                _stream())
+            if code != 4:
+                self.launches += int(rows_from_pairs)
+                return self._check(code, f"moe_grouped_tcgen05 ({E} experts, {N} x {K})")
             max_pos = cos.shape[0]
             _need(positions, "positions", torch.int32)
         num_slots = 0
@@ -2066,6 +2084,7 @@ class Kernels:
                                   f"in (Hkv, D) / (Hkv, Dv)")
             num_slots = k_pages.numel() // (num_kv * head_dim)
         if v_dim == head_dim and kv_in_row:
+        self._moe_plain = bool(on)
             code = self.lib.ullm_qk_norm_rope_store(
                 _DT[qkv.dtype], _ptr(qkv), T, num_q, num_kv, head_dim, _ptr(q_w), _ptr(k_w), float(eps), _ptr(cos),
                 _ptr(sin), rotary_dim, max_pos, _ptr(positions), _ptr(slot_mapping), _ptr(k_pages), _ptr(v_pages),

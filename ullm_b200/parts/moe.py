@@ -173,7 +173,7 @@ class RoutedExperts(FeedForward):
         on_input = self.weight_on == "input"
         # (a choice at or beyond E, an expert that passes its input, gets no place: `moe_arrange` skips it)
         K.moe_grouped_linear(x, self.w_gate_up[:E], offsets, order, weight if on_input else None, act, top, True, self.gated,
-                             self.act_code, self.limit, self.alpha)
+                             self.act_code, self.limit, self.alpha, **({"gathered": rows} if x.is_cuda else {}))
         K.moe_grouped_linear(act, self.w_down[:E], offsets, order, None, rows, top, False, False)
         shared = None
         if self.shared is not None and not always:
