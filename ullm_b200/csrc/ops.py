@@ -105,6 +105,7 @@ class Kernels:
         self.status = torch.zeros(4, dtype=torch.int32, device="cuda")
         self.sm_count = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
         self._f32_out_mm = None
+        self._moe_plain = False
         self._lin_ws = None  # partial sums and tile counters of the tcgen05 product, made at its first use
         self._lin_counters = None
         self.pdl = False
@@ -115,7 +116,6 @@ class Kernels:
         self._lt_ws = None
         self._lt_tuned = set()
         self.timer = None  # a KernelGroupTimer while a profile is being taken
-        self._moe_plain = False
         # groups of kernels (the names `_timed` books them under) that are NOT launched: only for measuring what a
         # group costs inside a step, by the difference; the step's results are wrong while this is set
         self.skip_groups: frozenset = frozenset()
@@ -167,27 +167,27 @@ class Kernels:
         self.ssd_chunk_on = get("ULLM_B200_SSD_CHUNK", "1") != "0"
         # the same for the recurrence with a decay per key channel
         self.gla_chunk_on = get("ULLM_B200_GLA_CHUNK", "1") != "0"
+        # and for the matrix memory with exponential gates
+        self.mlstm_chunk_on = get("ULLM_B200_MLSTM_CHUNK", "1") != "0"
         # steps of single tokens through a state: the kernel built around the state's stream; 0: the general recurrences
         self.state_step_on = get("ULLM_B200_STATE_STEP", "1") != "0"
         # rows from which a step with distance biases (heads of 128) takes the tcgen05 prompt kernel
         self.pair_biased_rows = int(get("ULLM_B200_PAIR_BIASED_ROWS", "128"))
         self.window_attention_tc = get("ULLM_B200_WINDOW_ATTN_TC", "1") != "0"
+        # rows per expert, on average, from which the routed experts' products run on the tcgen05 kernel
+        self.moe_tcgen05_rows = int(get("ULLM_B200_MOE_TCGEN05_ROWS", "8"))
         # attention of the 32-bit engine and of float16 by row tiles (csrc/attention_plain.cu); 0: the general kernel always
         self.plain_attention_on = get("ULLM_B200_PLAIN_ATTN", "1") != "0"
         # the splits of a request's keys merge inside a thread-block cluster (at most 8 splits) instead of through
         # scratch arrays and a second kernel
         # ("auto": for steps of at most 8 rows; "1" / "0": always / never, with `decode_split_target` splits)
         mode = get("ULLM_B200_DECODE_CLUSTER", "auto")
-        # and for the matrix memory with exponential gates
-        self.mlstm_chunk_on = get("ULLM_B200_MLSTM_CHUNK", "1") != "0"
         self.decode_cluster_merge = {"1": True, "0": False}.get(mode, "auto")
         # decode steps: the per-request decode attention kernel applies the q/k norm and the rotation and writes the
         # new key and value itself (one launch less per layer)
         self.fuse_decode_rope = get("ULLM_B200_FUSE_DECODE_ROPE", "1") == "1"
         # a mixed step's leading one-token entries go to the decode attention kernel from this many on (0: never)
         self.mixed_decode_rows = int(get("ULLM_B200_MIXED_DECODE_ROWS", "4"))
-        # rows per expert, on average, from which the routed experts' products run on the tcgen05 kernel
-        self.moe_tcgen05_rows = int(get("ULLM_B200_MOE_TCGEN05_ROWS", "8"))
         # decode attention on the tcgen05 tensor cores (head size 128), the batch's keys cut evenly over the blocks
         self.use_tcgen05_decode = get("ULLM_B200_DECODE_TC", "0") == "1"
         # decode attention: the batch's keys cut evenly over the warps (True), every request split alike (False),
@@ -318,6 +318,7 @@ class Kernels:
             "ullm_moe_route": [P, LL, P, P, P, I, I, I, I, I, I, I, F, I, P],
             "ullm_moe_arrange": [P, I, I, P, P, P, P],
             "ullm_moe_grouped_linear": [I, P, LL, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P],
+            "ullm_moe_grouped_tcgen05": [P, LL, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, P],
             "ullm_moe_combine": [I, P, P, P, P, I, I, I, P, I, P, LL, P, P, LL, P],
             "ullm_moe_combine_add_norm": [I, P, P, P, I, I, I, P, I, P, LL, P, P, LL, P, P, P, F, P, P, P, P, P, F],
             "ullm_argmax": [P, LL, I, I, P, P],
@@ -335,9 +336,10 @@ class Kernels:
         L.ullm_mlstm_supported.restype = c_int
         L.ullm_mlstm_state_floats.argtypes = [I, I, I]
         L.ullm_mlstm_state_floats.restype = c_longlong
+        L.ullm_mlstm_chunk_floats.argtypes = [I, I, I, I, I, I]
+        L.ullm_mlstm_chunk_floats.restype = c_longlong
         L.ullm_gla_supported.argtypes = [I, I, I]
         L.ullm_gla_supported.restype = c_int
-            "ullm_moe_grouped_tcgen05": [P, LL, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, P],
         L.ullm_gla_state_floats.argtypes = [I, I, I]
         L.ullm_gla_state_floats.restype = c_longlong
         L.ullm_gla_chunk_supported.argtypes = [I, I, I]
@@ -360,8 +362,6 @@ class Kernels:
         L.ullm_decode_attention_balanced_supported.restype = c_int
         L.ullm_decode_attention_balanced_scratch_floats.argtypes = [I, I]
         L.ullm_decode_attention_balanced_scratch_floats.restype = c_longlong
-        L.ullm_mlstm_chunk_floats.argtypes = [I, I, I, I, I, I]
-        L.ullm_mlstm_chunk_floats.restype = c_longlong
         L.ullm_decode_attention_tcgen05_supported.argtypes = [I, I, I, I, I]
         L.ullm_decode_attention_tcgen05_supported.restype = c_int
         L.ullm_decode_attention_tcgen05_scratch_floats.argtypes = [I]
@@ -1398,6 +1398,42 @@ class Kernels:
             vdim, float(q_scale), float(cap), state.shape[0], _ptr(self.status), _stream()),
             f"mlstm_recurrence (heads {heads}, dim {dim}, vdim {vdim})")
 
+    def mlstm_chunk_applies(self, dtype, heads: int, dim: int, vdim: int) -> bool:
+        """True when `mlstm_chunk` takes these sizes (bfloat16; see csrc/mlstm_chunk.cu)."""
+        return bool(self.mlstm_chunk_on and dtype == torch.bfloat16 and self.lib.ullm_mlstm_chunk_supported(heads, dim, vdim))
+
+    @_timed("mlstm", skipped=True)
+    def mlstm_chunk(self, qkv, q_off, k_off, v_off, gates, bias_i, bias_f, state, cu_q, req_slots, token_req, out, requests,
+                    heads, dim, vdim, q_scale, cap, workspace, least: int) -> bool:
+        """`mlstm_recurrence` in its chunked form on the tensor cores, for the requests that bring MORE than `least` tokens (the
+        others are left alone).  False where the rows do not start on 16-byte borders (nothing has run then)."""
+        _need(qkv, "qkv", torch.bfloat16)
+        _need(gates, "gates", torch.float32)
+        _need(state, "state", torch.float32)
+        _need(out, "out", torch.float32)
+        for t_, n_ in ((bias_i, "input gate bias"), (bias_f, "forget gate bias")):
+            if t_ is not None:
+                _need(t_, n_, torch.float32)
+        for t_, n_ in ((cu_q, "cu_q"), (req_slots, "req_slots"), (token_req, "token_req")):
+            _need(t_, n_, torch.int32)
+        T = qkv.shape[0]
+        if gates.shape != (T, 2 * heads) or out.shape != (T, heads * vdim) or state.dim() != 2:
+            raise KernelError(f"mlstm_chunk: qkv {tuple(qkv.shape)}, gates {tuple(gates.shape)}, out {tuple(out.shape)}")
+        if max(q_off, k_off) + heads * dim > qkv.shape[1] or v_off + heads * vdim > qkv.shape[1]:
+            raise KernelError("mlstm_chunk: q, k or v lie outside the rows")
+        floats = self.lib.ullm_mlstm_chunk_floats
+        scratch = workspace.get("mlstm.chunks", 1, int(floats(max(T, workspace.max_tokens), max(requests, workspace.max_requests),
+                                                              heads, dim, vdim, int(least))), torch.float32)
+        code = self.lib.ullm_mlstm_chunk(
+            _ptr(qkv), qkv.stride(0), q_off, k_off, v_off, _ptr(gates), _ptr(bias_i), _ptr(bias_f), _ptr(scratch), _ptr(state),
+            state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req), _ptr(out), T, requests, heads, dim, vdim,
+            float(q_scale), float(cap), state.shape[0], int(least), _ptr(self.status), _stream())
+        if code == 4:
+            return False
+        self._check(code, f"mlstm_chunk (heads {heads}, dim {dim}, vdim {vdim})")
+        self.launches += 3
+        return True
+
     @_timed("mlstm")
     def mlstm_out_gate(self, o, g, weight, eps, out, heads, vdim):
         """out = o / sqrt(mean over a head of o^2 + eps) * weight * sigmoid(g); o float32 [T, heads * vdim], g a
@@ -1469,42 +1505,6 @@ class Kernels:
             raise KernelError("gla_recurrence: q, k or v lie outside the rows")
         if z_bias is not None and z_bias.numel() != heads * dim:
             raise KernelError("gla_recurrence: the decay bias has the wrong length")
-    def mlstm_chunk_applies(self, dtype, heads: int, dim: int, vdim: int) -> bool:
-        """True when `mlstm_chunk` takes these sizes (bfloat16; see csrc/mlstm_chunk.cu)."""
-        return bool(self.mlstm_chunk_on and dtype == torch.bfloat16 and self.lib.ullm_mlstm_chunk_supported(heads, dim, vdim))
-
-    @_timed("mlstm", skipped=True)
-    def mlstm_chunk(self, qkv, q_off, k_off, v_off, gates, bias_i, bias_f, state, cu_q, req_slots, token_req, out, requests,
-                    heads, dim, vdim, q_scale, cap, workspace, least: int) -> bool:
-        """`mlstm_recurrence` in its chunked form on the tensor cores, for the requests that bring MORE than `least` tokens (the
-        others are left alone).  False where the rows do not start on 16-byte borders (nothing has run then)."""
-        _need(qkv, "qkv", torch.bfloat16)
-        _need(gates, "gates", torch.float32)
-        _need(state, "state", torch.float32)
-        _need(out, "out", torch.float32)
-        for t_, n_ in ((bias_i, "input gate bias"), (bias_f, "forget gate bias")):
-            if t_ is not None:
-                _need(t_, n_, torch.float32)
-        for t_, n_ in ((cu_q, "cu_q"), (req_slots, "req_slots"), (token_req, "token_req")):
-            _need(t_, n_, torch.int32)
-        T = qkv.shape[0]
-        if gates.shape != (T, 2 * heads) or out.shape != (T, heads * vdim) or state.dim() != 2:
-            raise KernelError(f"mlstm_chunk: qkv {tuple(qkv.shape)}, gates {tuple(gates.shape)}, out {tuple(out.shape)}")
-        if max(q_off, k_off) + heads * dim > qkv.shape[1] or v_off + heads * vdim > qkv.shape[1]:
-            raise KernelError("mlstm_chunk: q, k or v lie outside the rows")
-        floats = self.lib.ullm_mlstm_chunk_floats
-        scratch = workspace.get("mlstm.chunks", 1, int(floats(max(T, workspace.max_tokens), max(requests, workspace.max_requests),
-                                                              heads, dim, vdim, int(least))), torch.float32)
-        code = self.lib.ullm_mlstm_chunk(
-            _ptr(qkv), qkv.stride(0), q_off, k_off, v_off, _ptr(gates), _ptr(bias_i), _ptr(bias_f), _ptr(scratch), _ptr(state),
-            state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req), _ptr(out), T, requests, heads, dim, vdim,
-            float(q_scale), float(cap), state.shape[0], int(least), _ptr(self.status), _stream())
-        if code == 4:
-            return False
-        self._check(code, f"mlstm_chunk (heads {heads}, dim {dim}, vdim {vdim})")
-        self.launches += 3
-        return True
-
         if single and self.state_step_on and T == requests:
             code = self.lib.ullm_gla_step(
                 _DT[qkv.dtype], _ptr(qkv), qkv.stride(0), q_off, k_off, v_off, _ptr(z), z.stride(0), _ptr(z_bias),
@@ -1946,6 +1946,19 @@ class Kernels:
             raise KernelError(f"moe_grouped_linear: x {tuple(x.shape)}, weights {tuple(weights.shape)}, out {tuple(out.shape)}")
         if pair_weight is not None:
             _need(pair_weight, "pair weights", torch.float32)
+        if gathered is not None:
+            _need(gathered, "gathered rows", x.dtype)
+            if gathered.numel() < pairs * K:
+                raise KernelError(f"moe_grouped_linear: gathered {tuple(gathered.shape)}")
+        if (x.dtype == torch.bfloat16 and not self._moe_plain and pairs >= self.moe_tcgen05_rows * E
+                and (not rows_from_pairs or gathered is not None)):
+            code = self.lib.ullm_moe_grouped_tcgen05(
+                _ptr(x), x.stride(0), _ptr(gathered) if rows_from_pairs else None, _ptr(weights), _ptr(offsets), _ptr(sorted_pairs), _ptr(pair_weight), _ptr(out),
+                pairs, E, top, int(rows_from_pairs), n_out, K, int(gated), act, float(limit), float(alpha), _ptr(self.status),
+                _stream())
+            if code != 4:
+                self.launches += int(rows_from_pairs)
+                return self._check(code, f"moe_grouped_tcgen05 ({E} experts, {N} x {K})")
         self._check(self.lib.ullm_moe_grouped_linear(
             _DT[x.dtype], _ptr(x), x.stride(0), _ptr(weights), weights.stride(0), _ptr(offsets), _ptr(sorted_pairs),
             _ptr(pair_weight), _ptr(out), pairs, E, top, int(rows_from_pairs), n_out, K, int(gated), act, float(limit),
@@ -1955,6 +1968,7 @@ class Kernels:
     def moe_force_plain(self, on: bool) -> None:
         """True: the grouped product never takes its tensor-core kernel (tests compare the two)."""
         self.lib.ullm_moe_force_plain(1 if on else 0)
+        self._moe_plain = bool(on)
 
     @_timed("moe")
     def _combine_extras(self, what, rows, T, C, top, passing, shared):
@@ -2056,19 +2070,6 @@ class Kernels:
         if rotary_dim > 0:
             if cos is None or sin is None or cos.shape != sin.shape or cos.shape[1] != rotary_dim // 2:
                 raise KernelError("qk_norm_rope_store: cos/sin tables must be [positions, rotary_dim / 2]")
-        if gathered is not None:
-            _need(gathered, "gathered rows", x.dtype)
-            if gathered.numel() < pairs * K:
-                raise KernelError(f"moe_grouped_linear: gathered {tuple(gathered.shape)}")
-        if (x.dtype == torch.bfloat16 and not self._moe_plain and pairs >= self.moe_tcgen05_rows * E
-                and (not rows_from_pairs or gathered is not None)):
-            code = self.lib.ullm_moe_grouped_tcgen05(
-                _ptr(x), x.stride(0), _ptr(gathered) if rows_from_pairs else None, _ptr(weights), _ptr(offsets), _ptr(sorted_pairs), _ptr(pair_weight), _ptr(out),
-                pairs, E, top, int(rows_from_pairs), n_out, K, int(gated), act, float(limit), float(alpha), _ptr(self.status),
-                _stream())
-            if code != 4:
-                self.launches += int(rows_from_pairs)
-                return self._check(code, f"moe_grouped_tcgen05 ({E} experts, {N} x {K})")
             max_pos = cos.shape[0]
             _need(positions, "positions", torch.int32)
         num_slots = 0
@@ -2084,7 +2085,6 @@ class Kernels:
                                   f"in (Hkv, D) / (Hkv, Dv)")
             num_slots = k_pages.numel() // (num_kv * head_dim)
         if v_dim == head_dim and kv_in_row:
-        self._moe_plain = bool(on)
             code = self.lib.ullm_qk_norm_rope_store(
                 _DT[qkv.dtype], _ptr(qkv), T, num_q, num_kv, head_dim, _ptr(q_w), _ptr(k_w), float(eps), _ptr(cos),
                 _ptr(sin), rotary_dim, max_pos, _ptr(positions), _ptr(slot_mapping), _ptr(k_pages), _ptr(v_pages),
