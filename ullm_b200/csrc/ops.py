@@ -1375,9 +1375,10 @@ class Kernels:
 
     @_timed("mlstm")
     def mlstm_recurrence(self, qkv, q_off, k_off, v_off, gates, bias_i, bias_f, state, cu_q, req_slots, token_req, out,
-                         requests, heads, dim, vdim, q_scale, cap):
+                         requests, heads, dim, vdim, q_scale, cap, most_tokens: int = 1 << 30):
         """The recurrence of csrc/mlstm.cu over the step's tokens, from and into the requests' state rows.
-        qkv [T, *]: q, k, v at the given column offsets; gates [T, 2 heads] float32; out [T, heads * vdim] float32."""
+        qkv [T, *]: q, k, v at the given column offsets; gates [T, 2 heads] float32; out [T, heads * vdim] float32;
+        requests that bring more than `most_tokens` tokens are left alone."""
         _need(qkv, "qkv")
         _need(gates, "gates", torch.float32)
         _need(state, "state", torch.float32)
@@ -1395,7 +1396,7 @@ class Kernels:
         self._check(self.lib.ullm_mlstm_recurrence(
             _DT[qkv.dtype], _ptr(qkv), qkv.stride(0), q_off, k_off, v_off, _ptr(gates), _ptr(bias_i), _ptr(bias_f),
             _ptr(state), state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req), _ptr(out), requests, heads, dim,
-            vdim, float(q_scale), float(cap), state.shape[0], _ptr(self.status), _stream()),
+            vdim, float(q_scale), float(cap), state.shape[0], _ptr(self.status), _stream(), int(most_tokens)),
             f"mlstm_recurrence (heads {heads}, dim {dim}, vdim {vdim})")
 
     def mlstm_chunk_applies(self, dtype, heads: int, dim: int, vdim: int) -> bool:
