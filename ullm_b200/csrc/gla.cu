@@ -337,6 +337,16 @@ static int gla_launch(const void* qkv, long long row_stride, int q_off, int k_of
 #undef GLA_AS
 }
 
+// z [tokens, cols] 32-bit (rows `z_stride` apart) <- sigmoid(z + bias)^inv_tau, in place; `bias` [cols] or null.
+extern "C" int ullm_gla_decay(float* z, long long z_stride, const float* bias, float inv_tau, int tokens, int cols, void* stream) {
+  if (tokens < 0 || cols <= 0 || z_stride < cols) return ULLM_ERR_BAD_SIZE;
+  const long long total = (long long)tokens * cols, blocks = (total + 255) / 256;
+  if (blocks > 0x7fffffffLL) return ULLM_ERR_BAD_SIZE;
+  if (total == 0) return ULLM_OK;
+  return ullm_launch_kernel(gla_decay_kernel, dim3((int)blocks), dim3(256), 0, (cudaStream_t)stream, z, z_stride, bias, cols, total,
+                            inv_tau);
+}
+
 // qkv [tokens, *]: q and k (heads x dim) and v (heads x vdim) at the given column offsets of rows `row_stride`
 // apart; z [tokens, heads * dim] 32-bit (rows `z_stride` apart), `z_bias` [heads * dim] or null: the decay's
 // projection, REPLACED by the decays (`inv_tau` 0: z holds the decays already); `bonus` [heads * dim] or null; requests that bring more than

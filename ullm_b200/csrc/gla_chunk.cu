@@ -205,18 +205,20 @@ __global__ void gla_scan_kernel(float* __restrict__ fold, const float* __restric
   *st = s;
 }
 
-// A warp's 16 rows are two stretches, i0 and i0 + 1; its queries are weighted from the start of stretch i0 on.
+// A warp's 16 rows are two stretches, i0 and i0 + 1; its queries are weighted from the start of stretch i0 on.  A block owns
+// (chunk, head, v_tile value columns): see `gch_v_tile`.
 template <bool BONUS>
 __global__ void __launch_bounds__(GCH_THREADS, 3)
 gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int q_off, int k_off, int v_off,
                const float* __restrict__ decay, long long decay_stride, const float* __restrict__ bonus, float q_scale,
                const int* __restrict__ cu_q, const int* __restrict__ token_req, int requests, int least, int heads, int dim,
-               int vdim, const float* __restrict__ fold, float* __restrict__ out) {
+               int vdim, int v_tile, const float* __restrict__ fold, float* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char gch_smem[];
   pdl_launch_dependents();
   pdl_wait();
   int t0 = 0;
   const int tile = blockIdx.x, head = blockIdx.y;
+  const int v0 = blockIdx.z * v_tile, vn = min(v_tile, vdim - v0);  // the block's value columns
   const int cn = gch_find(tile, cu_q, requests, least, t0);
   if (cn == 0 || token_req[t0] < 0) return;
   const int ks = dim + 4, kb = dim + 8;
@@ -224,10 +226,10 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
   float* kq = rp + GCH_Q * ks;                                        // [GCH_Q][ks]: decays, then weighted k
   float* tot = kq + GCH_Q * ks;                                       // [GCH_SUBS][dim]
   float* diag = tot + GCH_SUBS * dim;                                 // [GCH_SUBS][8][10]: scores inside the stretches
-  __nv_bfloat16* v_s = reinterpret_cast<__nv_bfloat16*>(diag + GCH_SUBS * 80);  // [GCH_Q][vdim + 8]
-  __nv_bfloat16* k_s = v_s + GCH_Q * (vdim + 8);                      // [GCH_Q][kb]
+  __nv_bfloat16* v_s = reinterpret_cast<__nv_bfloat16*>(diag + GCH_SUBS * 80);  // [GCH_Q][vn + 8]
+  __nv_bfloat16* k_s = v_s + GCH_Q * (vn + 8);                      // [GCH_Q][kb]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  gch_load_v(v_s, qkv + (long long)t0 * row_stride + v_off + head * vdim, row_stride, vdim, cn);
+  gch_load_v(v_s, qkv + (long long)t0 * row_stride + v_off + head * vdim + v0, row_stride, vn, cn);
   {
     const int pieces = dim >> 3;
     for (int i = tid; i < GCH_Q * pieces; i += GCH_THREADS) {
@@ -394,10 +396,10 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
   }
   __syncwarp();
   // ---- outputs, 64 value columns at a time --------------------------------------------------------------------------
-  const float* st = fold + ((long long)tile * heads + head) * vdim * dim;
+  const float* st = fold + (((long long)tile * heads + head) * vdim + v0) * dim;
   const int mat = lane >> 3;
-  for (int n0 = 0; n0 < vdim; n0 += 64) {
-    const int nt = min(8, (vdim - n0) >> 3);
+  for (int n0 = 0; n0 < vn; n0 += 64) {
+    const int nt = min(8, (vn - n0) >> 3);
     float y[8][4];
 #pragma unroll
     for (int n = 0; n < 8; ++n) y[n][0] = y[n][1] = y[n][2] = y[n][3] = 0.f;
@@ -413,7 +415,7 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
         for (int n = 0; n < 8; n += 2) {
           if (n < nt) {
             unsigned b[4];
-            gch_ldsm4t(b, v_s + (s * 16 + (mat & 1) * 8 + (lane & 7)) * (vdim + 8) + n0 + n * 8 + (mat >> 1) * 8);
+            gch_ldsm4t(b, v_s + (s * 16 + (mat & 1) * 8 + (lane & 7)) * (vn + 8) + n0 + n * 8 + (mat >> 1) * 8);
             gch_mma(y[n], ah, b[0], b[1]);
             gch_mma(y[n + 1], ah, b[2], b[3]);
             gch_mma(y[n], al, b[0], b[1]);
@@ -451,7 +453,7 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
     for (int h = 0; h < 2; ++h) {
       const int row = warp * 16 + g + 8 * h;
       if (row >= cn) continue;
-      float* dst = out + ((long long)(t0 + row) * heads + head) * vdim + n0 + cp;
+      float* dst = out + ((long long)(t0 + row) * heads + head) * vdim + v0 + n0 + cp;
 #pragma unroll
       for (int n = 0; n < 8; ++n)
         if (n < nt) *reinterpret_cast<float2*>(dst + n * 8) = make_float2(y[n][2 * h], y[n][2 * h + 1]);
@@ -466,11 +468,26 @@ static size_t gch_out_smem(int dim, int vdim) {
   return (size_t)(2 * GCH_Q * (dim + 4) + GCH_SUBS * dim + GCH_SUBS * 80) * 4 + (size_t)GCH_Q * (vdim + 8) * 2 +
          (size_t)GCH_Q * (dim + 8) * 2;
 }
+// Value columns of a block of `gla_out`: all of them while that leaves room for three blocks per SM (dim 64, vdim 64: 51 KB);
+// else as many (a power of two times 64) as leave room for two, because one block of four warps per SM leaves the chip to its
+// latencies (dim 128, vdim 256: one tile needs 125 KB, two of 128 columns 109 KB each); else as many as fit at all.  The scores
+// are formed once per tile.  0: not even 16 columns fit.
+static int gch_v_tile(int dim, int vdim) {
+  if (gch_out_smem(dim, vdim) <= 75 * 1024) return vdim;
+  int most = 0;
+  for (int tile = 1024; tile >= 64; tile >>= 1) {
+    const int t = tile < vdim ? tile : vdim;
+    const size_t smem = gch_out_smem(dim, t);
+    if (smem <= 112 * 1024) return t;
+    if (smem <= 227 * 1024 && most == 0) most = t;
+  }
+  return most;
+}
 
 // Sizes the chunked form takes (bfloat16): key and value sizes that are multiples of 16, as far as the shared memory reaches.
 extern "C" int ullm_gla_chunk_supported(int heads, int dim, int vdim) {
   return heads > 0 && heads <= 65535 && dim > 0 && vdim > 0 && dim % 16 == 0 && vdim % 16 == 0 && dim <= GCH_MAX_DIM &&
-         gch_out_smem(dim, vdim) <= 227 * 1024;
+         gch_fold_smem(dim, vdim) <= 227 * 1024 && gch_v_tile(dim, vdim) > 0;
 }
 // Chunks a step of `tokens` tokens and `requests` requests has at most; floats of scratch per chunk.
 extern "C" int ullm_gla_chunk_tiles(int tokens, int requests) { return tokens / GCH_Q + requests; }
@@ -509,12 +526,13 @@ extern "C" int ullm_gla_chunk(const void* qkv, long long row_stride, int q_off, 
   float* fold = scratch;
   float* total = scratch + (long long)tiles * heads * dim * vdim;
   static size_t fold_smem = 48 * 1024, out_smem[2] = {48 * 1024, 48 * 1024};
-  const size_t fs = gch_fold_smem(dim, vdim), os = gch_out_smem(dim, vdim);
+  const int v_tile = gch_v_tile(dim, vdim);
+  const size_t fs = gch_fold_smem(dim, vdim), os = gch_out_smem(dim, v_tile);
   int rc = gch_allow(gla_fold_kernel, fs, &fold_smem);
   if (rc != ULLM_OK) return rc;
   rc = bonus != nullptr ? gch_allow(gla_out_kernel<true>, os, &out_smem[0]) : gch_allow(gla_out_kernel<false>, os, &out_smem[1]);
   if (rc != ULLM_OK) return rc;
-  const dim3 grid(tiles, heads), block(GCH_THREADS);
+  const dim3 grid(tiles, heads), out_grid(tiles, heads, (vdim + v_tile - 1) / v_tile), block(GCH_THREADS);
   rc = ullm_launch_kernel(gla_fold_kernel, grid, block, fs, st, (const __nv_bfloat16*)qkv, row_stride, k_off, v_off, decay,
                           decay_stride, cu_q, token_req, requests, least, heads, dim, vdim, fold, total);
   if (rc != ULLM_OK) return rc;
@@ -523,10 +541,10 @@ extern "C" int ullm_gla_chunk(const void* qkv, long long row_stride, int q_off, 
                           num_slots, status);
   if (rc != ULLM_OK) return rc;
   if (bonus != nullptr)
-    return ullm_launch_kernel(gla_out_kernel<true>, grid, block, os, st, (const __nv_bfloat16*)qkv, row_stride, q_off, k_off,
+    return ullm_launch_kernel(gla_out_kernel<true>, out_grid, block, os, st, (const __nv_bfloat16*)qkv, row_stride, q_off, k_off,
                               v_off, decay, decay_stride, bonus, q_scale, cu_q, token_req, requests, least, heads, dim, vdim,
-                              (const float*)fold, out);
-  return ullm_launch_kernel(gla_out_kernel<false>, grid, block, os, st, (const __nv_bfloat16*)qkv, row_stride, q_off, k_off,
+                              v_tile, (const float*)fold, out);
+  return ullm_launch_kernel(gla_out_kernel<false>, out_grid, block, os, st, (const __nv_bfloat16*)qkv, row_stride, q_off, k_off,
                             v_off, decay, decay_stride, bonus, q_scale, cu_q, token_req, requests, least, heads, dim, vdim,
-                            (const float*)fold, out);
+                            v_tile, (const float*)fold, out);
 }

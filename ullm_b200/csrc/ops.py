@@ -310,6 +310,7 @@ class Kernels:
             "ullm_gla_recurrence": [I, P, LL, I, I, I, P, LL, P, F, F, P, LL, P, P, P, P, I, I, I, I, I, I, P, P, P, I],
             "ullm_ssd_step": [I, P, LL, I, I, P, P, P, P, LL, P, P, P, I, I, I, I, I, I, P, P, LL, I],
             "ullm_gla_step": [I, P, LL, I, I, I, P, LL, P, F, F, P, LL, P, P, P, I, I, I, I, I, P, P, P],
+            "ullm_gla_decay": [P, LL, P, F, I, I, P],
             "ullm_gla_chunk": [P, LL, I, I, I, P, LL, P, F, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, P, P],
             "ullm_token_shift_mix": [I, P, LL, P, I, I, P, P, LL, I, P, P, P, I, I, P, P],
             "ullm_low_rank_decay": [I, P, LL, I, I, P, P, P, I, I, I, P],
@@ -1518,6 +1519,17 @@ class Kernels:
             float(inv_tau), float(q_scale), _ptr(state), state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req),
             _ptr(out), T, requests, heads, dim, vdim, state.shape[0], _ptr(self.status), _stream(), _ptr(bonus),
             int(most_tokens)), f"gla_recurrence (heads {heads}, dim {dim}, vdim {vdim})")
+
+    @_timed("gla")
+    def gla_decay(self, z, z_bias, inv_tau: float):
+        """z [T, n] float32 (a view with any row stride) <- sigmoid(z + z_bias)^inv_tau, in place; z_bias float32 [n] or None."""
+        _need(z, "z", torch.float32, contiguous=False)
+        if z_bias is not None:
+            _need(z_bias, "decay bias", torch.float32)
+        if z.dim() != 2 or z.stride(1) != 1 or (z_bias is not None and z_bias.numel() != z.shape[1]):
+            raise KernelError(f"gla_decay: z {tuple(z.shape)}")
+        self._check(self.lib.ullm_gla_decay(_ptr(z), z.stride(0), _ptr(z_bias), float(inv_tau), z.shape[0], z.shape[1], _stream()),
+                    "gla_decay")
 
     def gla_chunk_applies(self, dtype, heads: int, dim: int, vdim: int) -> bool:
         """True when `gla_chunk` takes these sizes (bfloat16; see csrc/gla_chunk.cu)."""

@@ -14,7 +14,8 @@ engine dtype; z is a product with a 32-bit result.
 
 The state (S of every head, `gla_state_floats` floats) is one row per request slot in the cache manager's state
 rows; it is zeroed when a slot is handed out and carried from step to step.  One kernel runs the recurrence over
-any mix of prompt portions and single tokens (csrc/gla.cu).
+any mix of prompt portions and single tokens (csrc/gla.cu); portions of more than CHUNK_LEAST tokens in bfloat16 run in
+chunks on the tensor cores (csrc/gla_chunk.cu).
 """
 
 from __future__ import annotations
@@ -24,6 +25,7 @@ import torch
 from ..csrc import kernels
 from .base import Mixer, ParamDecl, StateNeed
 from .linear import linear
+from .mamba2 import CHUNK_LEAST
 from .registry import register_mixer
 
 
@@ -95,9 +97,20 @@ class GatedLinearAttention(Mixer):
         z = ws.tokens("gla.z", T, qk, torch.float32)
         K.linear_f32_out(y[:, 2 * qk + 2 * vs:], self.tensors[n["a2"]], z)
         o = ws.tokens("gla.o", T, vs, torch.float32)
-        K.gla_recurrence(y, 0, qk, 2 * qk, z, self.tensors[n["a2_bias"]], 1.0 / self.tau, d ** -0.5, cache.state,
-                         ctx.cu_q, ctx.req_slots, ctx.token_req, o, ctx.num_requests, N, d, dv,
-                         single=ctx.max_q_len == 1)
+        # prompt portions in chunks on the tensor cores (bfloat16, at the sizes that form takes), the rest token by token
+        chunked = ctx.max_q_len > CHUNK_LEAST and x.is_cuda and y.stride(0) % 8 == 0 and K.gla_chunk_applies(x.dtype, N, d, dv)
+        if chunked:
+            K.gla_decay(z, self.tensors[n["a2_bias"]], 1.0 / self.tau)
+            scratch = K.gla_chunk_scratch(ws, T, ctx.num_requests, N, d, dv)
+            K.gla_chunk(y, 0, qk, 2 * qk, z, d ** -0.5, scratch, cache.state, ctx.cu_q, ctx.req_slots, ctx.token_req, o,
+                        ctx.num_requests, N, d, dv, CHUNK_LEAST)
+            if ctx.num_requests > 1:
+                K.gla_recurrence(y, 0, qk, 2 * qk, z, None, 0.0, d ** -0.5, cache.state, ctx.cu_q, ctx.req_slots,
+                                 ctx.token_req, o, ctx.num_requests, N, d, dv, most_tokens=CHUNK_LEAST)
+        else:
+            K.gla_recurrence(y, 0, qk, 2 * qk, z, self.tensors[n["a2_bias"]], 1.0 / self.tau, d ** -0.5, cache.state,
+                             ctx.cu_q, ctx.req_slots, ctx.token_req, o, ctx.num_requests, N, d, dv,
+                             single=ctx.max_q_len == 1)
         gated = ws.tokens("gla.gated", T, vs, x.dtype)
         K.head_norm_gate(o, y[:, 2 * qk + vs:2 * qk + 2 * vs], self.tensors[n["norm"]], self.eps, gated, N, dv, silu=True)
         out = ws.tokens("mixer.out", T, self.hidden_size, x.dtype)
