@@ -53,17 +53,24 @@ class Workspace:
         self.max_tokens = max_tokens
         self.max_requests = max_requests
         self.buffers: dict[tuple, torch.Tensor] = {}
+        # the view of each buffer that was asked for last: the layers of a step ask for the same rows one after the other, and
+        # making a view costs as much host time as launching a kernel
+        self._views: dict[tuple, torch.Tensor] = {}
         self.generation = 0
 
     def get(self, name: str, rows: int, cols: int, dtype: torch.dtype, reserve: int = 0) -> torch.Tensor:
         key = (name, cols, dtype)
+        view = self._views.get(key)
+        if view is not None and view.shape[0] == rows:
+            return view
         buf = self.buffers.get(key)
         if buf is None or buf.shape[0] < rows:
             cap = max(rows, reserve, 0 if buf is None else buf.shape[0], 1)
             buf = torch.empty((cap, cols), dtype=dtype, device=self.device)
             self.buffers[key] = buf
             self.generation += 1
-        return buf[:rows]
+        view = self._views[key] = buf[:rows]
+        return view
 
     def tokens(self, name: str, rows: int, cols: int, dtype: torch.dtype) -> torch.Tensor:
         """A buffer with a row per token of the step."""
