@@ -1,0 +1,76 @@
+"""Prompt attention over latent key rows on tcgen05 (csrc/attention_latent_tcgen05.cu) against a 32-bit reference and the mma.sync
+kernel: blocks that end early, key tiles that end in the middle of a page, windows and stretches that begin inside a tile, pages
+given back in front of the window, decoded tokens at the head of the step, garbage behind a request's last key."""
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from test_gpu_kernels import K, rnd
+
+pytestmark = [pytest.mark.gpu, pytest.mark.needs_cuda]
+
+
+def reference(q, kp, bt, slots, q_lens, kv_lens, H, dk, dv, page, window, scale):
+    out, t0 = [], 0
+    for r, (n, kv) in enumerate(zip(q_lens, kv_lens)):
+        rows = kp.view(-1, dk)[(bt[slots[r], torch.arange(kv) // page].long() * page + torch.arange(kv) % page).to(kp.device)]
+        for j in range(n):
+            pos = kv - n + j
+            lo = max(0, pos - window + 1) if window > 0 else (pos - pos % -window if window < 0 else 0)
+            k = rows[lo:pos + 1]
+            p = torch.softmax((q[t0 + j].view(H, dk) @ k.t()) * scale, -1)
+            out.append(p @ k[:, :dv])
+        t0 += n
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("H,dk,dv", [(16, 448, 384), (32, 448, 384), (8, 192, 128), (1, 64, 64), (128, 320, 320), (4, 448, 256)])
+@pytest.mark.parametrize("page,window", [(16, 0), (16, 100), (64, -128), (8, 0)])
+@pytest.mark.parametrize("q_lens,kv_lens", [([130], [130]), ([1, 1, 1, 1, 9, 33], [70, 129, 1, 64, 9, 200]), ([8, 7, 65], [64, 71, 321])])
+def test_latent_rows_match_the_reference(H, dk, dv, page, window, q_lens, kv_lens):
+    k, scale = K(), dk ** -0.5
+    T, B, dtype = sum(q_lens), len(q_lens), torch.bfloat16
+    g = torch.Generator().manual_seed(31)
+    pages = sum(-(-n // page) for n in kv_lens) + 2
+    perm, slots = torch.randperm(pages, generator=g), torch.randperm(B + 1, generator=g)[:B]
+    bt = torch.full((B + 1, max(-(-n // page) for n in kv_lens) + 1), -1, dtype=torch.int32)
+    used = 0
+    kp = rnd(pages, page, 1, dk, seed=32, dtype=dtype)
+    for r, kl in enumerate(kv_lens):
+        n = -(-kl // page)
+        bt[slots[r], :n] = perm[used:used + n].int()
+        if kl % page:
+            kp[int(perm[used + n - 1]), kl % page:] = float("nan")  # (slots behind the last key may hold anything)
+        used += n
+    ref_bt = bt.clone()
+    if window > 0:  # pages that lie wholly in front of every window have been given back
+        for r, (n, kl) in enumerate(zip(q_lens, kv_lens)):
+            bt[slots[r], :max(0, kl - n - window + 1) // page] = -1
+    q = rnd(T, H * dk + 8, seed=33, dtype=dtype)[:, :H * dk]
+    cu = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32).cuda()
+    req = torch.cat([torch.full((n,), r, dtype=torch.int32) for r, n in enumerate(q_lens)]).cuda()
+    ctx = SimpleNamespace(decode_only=False, num_requests=B, max_kv_len=max(kv_lens), cu_q_host=cu.tolist(), shared={},
+                          start_positions_host=[a - b for a, b in zip(kv_lens, q_lens)])
+
+    def run(on):
+        out = torch.full((T, H * dv), 3.0, dtype=dtype, device="cuda")
+        k.latent_attention_on = on
+        try:
+            k.windowed_attention(q, out, kp, None, bt.cuda(), slots.int().cuda(), cu, torch.tensor(kv_lens, dtype=torch.int32).cuda(),
+                                 req, H, 1, dk, dv, page, window, scale, num_requests=B, ctx=ctx)
+        finally:
+            k.latent_attention_on = True
+        k.raise_on_status()
+        return out
+
+    got, path = run(True), k.attention_path
+    ref = reference(q.float(), torch.nan_to_num(kp.float()), ref_bt, slots.tolist(), q_lens, kv_lens, H, dk, dv, page, window, scale)
+    # weights rounded to bfloat16 (2^-9 of each; they sum to one, the values are of order one) and one rounding of the result
+    err = (got.float().view(T, H, dv) - ref).abs().max().item()
+    assert err <= 2 ** -7 * max(1.0, ref.abs().max().item()), err
+    if len(q_lens) != 6:
+        assert path == "latent_tcgen05"
+    if page in (8, 16, 32, 64) and not (kp.isnan().any()):
+        assert (got.float() - run(False).float()).abs().max().item() <= 2 ** -6 * max(1.0, ref.abs().max().item())

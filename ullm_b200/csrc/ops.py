@@ -177,6 +177,8 @@ class Kernels:
         self.ssd_chunk_on = get("ULLM_B200_SSD_CHUNK", "1") != "0"
         # the same for the recurrence with a decay per key channel
         self.gla_chunk_on = get("ULLM_B200_GLA_CHUNK", "1") != "0"
+        # prompt attention over latent key rows on the tcgen05 kernel; 0: the mma.sync kernel always
+        self.latent_attention_on = get("ULLM_B200_LATENT_TCGEN05", "1") != "0"
         # and for the matrix memory with exponential gates
         self.mlstm_chunk_on = get("ULLM_B200_MLSTM_CHUNK", "1") != "0"
         # steps of single tokens through a state: the kernel built around the state's stream; 0: the general recurrences
@@ -295,6 +297,8 @@ class Kernels:
             "ullm_paged_attention_generic_ex2": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, LL, P, P, I, I,
                                                  F, P],
             "ullm_mix_heads": [I, P, P, P, I, I, I, I, P],
+            "ullm_latent_attention": [P, LL, P, LL, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, LL, P, P],
+            "ullm_latent_attention_supported": [I, I, I, I, I],
             "ullm_window_attention": [P, LL, P, LL, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, LL, P, P, P, I, P, P,
                                       P, I, LL, P, LL, F, I, P, I, P, I],
             "ullm_paged_attention_generic_ex3": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, LL, P, P, I, I,
@@ -1299,6 +1303,30 @@ class Kernels:
                 self.prefill_attention_kernel = "pair"
                 self.attention_path = "prefill_tcgen05"
                 return
+        if (ctx is not None and not ctx.decode_only and self.latent_attention_on and self.window_attention_tc
+                and self.use_tcgen05_attention and q.dtype == torch.bfloat16 and v_pages is None and not pool and slopes is None
+                and gate is None and dist_bias is None and out_scale == 1.0
+                and self.lib.ullm_latent_attention_supported(head_dim, v_dim, num_q, num_kv, page_size)):
+            # Prompt portions over latent rows.  The one-token entries at the step's head go to the kernel below, which cuts
+            # their keys into runs (a block of 128 rows for each of them would walk its keys alone, and be the step's tail).
+            # Few rows with many keys in sight stay there altogether: below half a block per SM its runs fill the chip,
+            # where this kernel's blocks would walk all keys one after the other (1.2 us per 64 keys).
+            n_dec, _ragged = self._decoded_head(ctx)
+            rows, keys = T - n_dec, min(ctx.max_kv_len, abs(window)) if window else ctx.max_kv_len
+            if 2 * -(-rows * num_q // 64) >= self.sm_count or keys <= 2048:
+                code = self.lib.ullm_latent_attention(
+                    _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(k_pages), _ptr(block_table), block_table.shape[1],
+                    _ptr(req_slots[n_dec:]), _ptr(cu_q[n_dec:]), _ptr(kv_len[n_dec:]), T, ctx.num_requests - n_dec, num_q, num_kv,
+                    head_dim, v_dim, page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream())
+                if code != 4:
+                    self._check(code, f"latent_attention (key rows {head_dim}, values {v_dim})")
+                    self.attention_path = "latent_tcgen05"
+                    if n_dec:
+                        self.windowed_attention(
+                            q[:n_dec], out[:n_dec], k_pages, None, block_table, req_slots[:n_dec], cu_q[:n_dec + 1],
+                            kv_len[:n_dec], token_req[:n_dec], num_q, num_kv, head_dim, v_dim, page_size, window, scale,
+                            num_requests=n_dec, workspace=workspace)
+                    return
         p_pages = pk.numel() // (page_size * num_kv * head_dim) if pk is not None else 0
         if (self.window_attention_tc and q.dtype == torch.bfloat16 and num_requests and q.stride(0) % 8 == 0
                 and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0 and q.data_ptr() % 16 == 0

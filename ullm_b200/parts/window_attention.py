@@ -307,7 +307,7 @@ class LatentAttention(Mixer):
         o_lat = ws.tokens("lat.o_lat", T, N * R, dt)
         K.windowed_attention(q_out, o_lat, cache.k_pages, None, g.block_table, g.req_slots, ctx.cu_q, g.kv_len,
                              ctx.token_req, N, 1, self.key_row, R, g.page_size, self.window or 0, self.scale,
-                             pool=self.pool, pooled=pooled, num_requests=ctx.num_requests, workspace=ws)
+                             pool=self.pool, pooled=pooled, num_requests=ctx.num_requests, workspace=ws, ctx=ctx)
         # each head's latent output through its value up-projection: [heads, T, rank] x [heads, rank, vdim]
         attn = ws.tokens("attn.out", T, N * dv, dt)
         batched_matmul(o_lat.view(T, N, R).transpose(0, 1), self.tensors[n["uv"]].view(N, dv, R).transpose(1, 2),
