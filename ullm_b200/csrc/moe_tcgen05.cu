@@ -9,8 +9,8 @@
 // N = 256, K = 16; one thread), warps 2..5 drain the accumulators; four stages of 48 KB; two accumulators in tensor memory, so
 // that a tile's activation and stores run behind the next tile's products.  What is different:
 //
-//   * a tile is 128 places of ONE expert x 256 rows of its matrix (gated: 128 gate rows and the same 128 rows of up, one
-//     three-dimensional box).  How many tiles there are only the device knows: every block forms the running count of row
+//   * a tile is 128 places of ONE expert x 256 rows of its matrix (gated: 128 gate rows and the same 128 rows of up, a
+//     box each).  How many tiles there are only the device knows: every block forms the running count of row
 //     tiles from `offsets` and takes the tiles blockIdx.x, blockIdx.x + gridDim.x, ...; the row tiles of one expert and column
 //     tile are neighbours, so that blocks that run together share the matrix rows in L2.
 //   * x lies in place order already: the first product's rows are gathered by `moe_gather_rows` in a launch of its own (17 MB
@@ -117,8 +117,7 @@ moe_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         int p0, rows, nt;
         mt_find(first_s, p.offsets, p.n_tiles, tile, e, p0, rows, nt);
-        int at = tile % p.k_blocks;  // (blocks that run side by side begin at different k: see above)
-        for (int kb = 0; kb < p.k_blocks; ++kb, at = at + 1 == p.k_blocks ? 0 : at + 1) {
+        for (int kb = 0; kb < p.k_blocks; ++kb) {
           if (!mbar_wait(&empty_bar[s], parity)) {
             ullm_report(p.status, ULLM_STATUS_TIMEOUT, 51, kb);
             ok = false;
@@ -126,15 +125,14 @@ moe_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
           }
           mbar_expect_tx(&full_bar[s], bytes);
           unsigned char* a = tiles + s * MT_STAGE_BYTES;
-          // (two boxes of 128 rows: one box over gate and up rows took twice as long as one over 256 neighbouring rows)
           if (p.gated) {
-            tma_load_3d(a + MT_A_BYTES, &map_w, &full_bar[s], at * MT_BK, nt * (MT_BN / 2), 2 * e);
-            tma_load_3d(a + MT_A_BYTES + MT_B_BYTES / 2, &map_w, &full_bar[s], at * MT_BK, nt * (MT_BN / 2), 2 * e + 1);
+            tma_load_3d(a + MT_A_BYTES, &map_w, &full_bar[s], kb * MT_BK, nt * (MT_BN / 2), 2 * e);
+            tma_load_3d(a + MT_A_BYTES + MT_B_BYTES / 2, &map_w, &full_bar[s], kb * MT_BK, nt * (MT_BN / 2), 2 * e + 1);
           } else {
-            tma_load_3d(a + MT_A_BYTES, &map_w, &full_bar[s], at * MT_BK, nt * MT_BN, e);
-            tma_load_3d(a + MT_A_BYTES + MT_B_BYTES / 2, &map_w, &full_bar[s], at * MT_BK, nt * MT_BN + MT_BN / 2, e);
+            tma_load_3d(a + MT_A_BYTES, &map_w, &full_bar[s], kb * MT_BK, nt * MT_BN, e);
+            tma_load_3d(a + MT_A_BYTES + MT_B_BYTES / 2, &map_w, &full_bar[s], kb * MT_BK, nt * MT_BN + MT_BN / 2, e);
           }
-          tma_load_2d(a, &map_x, &full_bar[s], at * MT_BK, p0);
+          tma_load_2d(a, &map_x, &full_bar[s], kb * MT_BK, p0);
           if (++s == MT_STAGES) s = 0, parity ^= 1;
         }
       }

@@ -186,8 +186,10 @@ class Kernels:
         # rows from which a step with distance biases (heads of 128) takes the tcgen05 prompt kernel
         self.pair_biased_rows = int(get("ULLM_B200_PAIR_BIASED_ROWS", "128"))
         self.window_attention_tc = get("ULLM_B200_WINDOW_ATTN_TC", "1") != "0"
-        # rows per expert, on average, from which the routed experts' products run on the tcgen05 kernel
-        self.moe_tcgen05_rows = int(get("ULLM_B200_MOE_TCGEN05_ROWS", "8"))
+        # rows per expert, on average, from which the routed experts' products run on the tcgen05 kernel (see _moe_tcgen05_pays)
+        self.moe_tcgen05_rows = int(get("ULLM_B200_MOE_TCGEN05_ROWS", "2"))
+        # tokens up to which those products stream the chosen experts' matrices (at most 16)
+        self.moe_stream_tokens = min(16, int(get("ULLM_B200_MOE_STREAM_TOKENS", "16")))
         # attention of the 32-bit engine and of float16 by row tiles (csrc/attention_plain.cu); 0: the general kernel always
         self.plain_attention_on = get("ULLM_B200_PLAIN_ATTN", "1") != "0"
         # the splits of a request's keys merge inside a thread-block cluster (at most 8 splits) instead of through
@@ -333,6 +335,7 @@ class Kernels:
             "ullm_moe_route": [P, LL, P, P, P, I, I, I, I, I, I, I, F, I, P],
             "ullm_moe_arrange": [P, I, I, P, P, P, P],
             "ullm_moe_grouped_linear": [I, P, LL, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P],
+            "ullm_moe_stream": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, P],
             "ullm_moe_grouped_tcgen05": [P, LL, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, P],
             "ullm_moe_combine": [I, P, P, P, P, I, I, I, P, I, P, LL, P, P, LL, P],
             "ullm_moe_combine_add_norm": [I, P, P, P, I, I, I, P, I, P, LL, P, P, LL, P, P, P, F, P, P, P, P, P, F],
@@ -1981,6 +1984,18 @@ class Kernels:
         self._check(self.lib.ullm_moe_arrange(_ptr(choice), pairs, experts, _ptr(offsets), _ptr(sorted_pairs), _ptr(place),
                                               _stream()), f"moe_arrange ({experts} experts)")
 
+    def _moe_tcgen05_pays(self, pairs: int, experts: int, n_out: int, gated: bool) -> bool:
+        """Whether a grouped product of more tokens than the streaming kernel takes runs on tcgen05 or on mma.sync, measured with
+        cold caches.  Products without gate rows: tcgen05 at 4 rows per expert already (2,048 x 1,024, 16 experts: 24.6 us for
+        33.7) and at every size above.  Gated ones too where the experts' matrices make several 128-column tiles per SM (32 experts
+        of 2,048 x 4,096: 186 us for 214 at 2 rows per expert); where they make one tile per SM at most (16 experts of
+        1,024 x 2,048) its loads have no second tile to run under, and mma.sync is the faster one as long as an expert's rows
+        fit one of its tiles of 64 (45 us for 63 at 16 rows, 61 for 64 at 64 rows, 88 for 50 at 96)."""
+        rows = self.moe_tcgen05_rows
+        if gated and rows and experts * -(-n_out // 128) <= 148:
+            rows = max(rows, 65)
+        return pairs >= rows * experts
+
     @_timed("moe", lambda x, weights, *r: weights.numel() * weights.element_size())
     def moe_grouped_linear(self, x, weights, offsets, sorted_pairs, pair_weight, out, top: int, rows_from_pairs: bool,
                            gated: bool, act: int = 0, limit: float = 0.0, alpha: float = 1.0, gathered=None):
@@ -2001,7 +2016,13 @@ class Kernels:
             _need(gathered, "gathered rows", x.dtype)
             if gathered.numel() < pairs * K:
                 raise KernelError(f"moe_grouped_linear: gathered {tuple(gathered.shape)}")
-        if (x.dtype == torch.bfloat16 and not self._moe_plain and pairs >= self.moe_tcgen05_rows * E
+        if x.dtype == torch.bfloat16 and not self._moe_plain and pairs <= self.moe_stream_tokens * top:
+            code = self.lib.ullm_moe_stream(
+                _ptr(x), _ptr(weights), _ptr(offsets), _ptr(sorted_pairs), _ptr(pair_weight), _ptr(out), pairs, E, top,
+                int(rows_from_pairs), n_out, K, int(gated), act, float(limit), float(alpha), _ptr(self.status), _stream())
+            if code != 4:
+                return self._check(code, f"moe_stream ({E} experts, {N} x {K})")
+        if (x.dtype == torch.bfloat16 and not self._moe_plain and self._moe_tcgen05_pays(pairs, E, n_out, gated)
                 and (not rows_from_pairs or gathered is not None)):
             code = self.lib.ullm_moe_grouped_tcgen05(
                 _ptr(x), x.stride(0), _ptr(gathered) if rows_from_pairs else None, _ptr(weights), _ptr(offsets), _ptr(sorted_pairs), _ptr(pair_weight), _ptr(out),
