@@ -101,6 +101,11 @@ def _timed(group: str, nbytes=None, skipped=None):
     return outer
 
 
+def _scratch_floats(workspace, name: str, floats: int, most: int) -> torch.Tensor:
+    """Scratch of at least `floats` float32 of the workspace, made at once for the `most` that its largest step takes."""
+    return workspace.get(name, max(1, -(-int(floats) // 1024)), 1024, torch.float32, reserve=-(-int(most) // 1024))
+
+
 def _weight_bytes(x, weight, *rest):
     return weight.numel() * weight.element_size()
 
@@ -312,7 +317,7 @@ class Kernels:
             "ullm_scale_f32": [P, LL, F, P],
             "ullm_ssd_prepare": [I, P, LL, I, I, I, I, P, I, P, P, P, P, LL, I, P, P, P, I, P, P, P, I, P, P],
             "ullm_ssd_recurrence": [I, P, LL, I, I, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, P, P, LL, I],
-            "ullm_ssd_chunk": [P, LL, I, I, P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, P, P, LL],
+            "ullm_ssd_chunk": [P, LL, I, I, P, P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, P, P, LL],
             "ullm_ssd_gate_norm": [I, P, P, LL, P, P, I, I, I, F, P, I],
             "ullm_norm_rows": [I, P, P, P, P, I, I, I, F, I, P, P, P, P],
             "ullm_xielu": [I, P, P, LL, P, P],
@@ -371,6 +376,8 @@ class Kernels:
         L.ullm_ssd_supported.restype = c_int
         L.ullm_ssd_chunk_supported.argtypes = [I, I, I, I]
         L.ullm_ssd_chunk_supported.restype = c_int
+        L.ullm_ssd_chunk_scratch.argtypes = [I, I, I, I, I, I]
+        L.ullm_ssd_chunk_scratch.restype = c_longlong
         L.ullm_ssd_chunk_tokens.argtypes = []
         L.ullm_ssd_chunk_tokens.restype = c_int
         L.ullm_wait_selftest.argtypes = [I, P, P, P]
@@ -1466,8 +1473,8 @@ class Kernels:
         if max(q_off, k_off) + heads * dim > qkv.shape[1] or v_off + heads * vdim > qkv.shape[1]:
             raise KernelError("mlstm_chunk: q, k or v lie outside the rows")
         floats = self.lib.ullm_mlstm_chunk_floats
-        scratch = workspace.get("mlstm.chunks", 1, int(floats(max(T, workspace.max_tokens), max(requests, workspace.max_requests),
-                                                              heads, dim, vdim, int(least))), torch.float32)
+        scratch = _scratch_floats(workspace, "mlstm.chunks", floats(T, requests, heads, dim, vdim, int(least)),
+                                  floats(workspace.max_tokens, workspace.max_requests, heads, dim, vdim, int(least)))
         code = self.lib.ullm_mlstm_chunk(
             _ptr(qkv), qkv.stride(0), q_off, k_off, v_off, _ptr(gates), _ptr(bias_i), _ptr(bias_f), _ptr(scratch), _ptr(state),
             state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req), _ptr(out), T, requests, heads, dim, vdim,
@@ -1817,9 +1824,10 @@ class Kernels:
 
     @_timed("ssd")
     def ssd_chunk(self, xbc, b_off: int, c_off: int, dt, log_decay, d_skip, scores, state, cu_q, req_slots, token_req, out,
-                  requests: int, heads: int, n_state: int, pdim: int, groups: int, least: int):
+                  requests: int, heads: int, n_state: int, pdim: int, groups: int, least: int, workspace=None):
         """`ssd_recurrence` in its chunked form on the tensor cores, for the requests that bring MORE than `least` tokens
-        (the others are left alone); `scores`: scratch (float32, `ssd_chunk_floats`)."""
+        (the others are left alone); `scores`: scratch (float32, `ssd_chunk_floats`).  The states between the chunks lie in
+        `workspace` (without one: in memory of the call's own)."""
         _need(xbc, "xbc", torch.bfloat16)
         _need(state, "state", torch.float32, contiguous=False)
         for t_, n_ in ((dt, "dt"), (log_decay, "log_decay"), (d_skip, "d_skip"), (out, "out"), (scores, "scores")):
@@ -1834,12 +1842,18 @@ class Kernels:
             raise KernelError(f"ssd_chunk: xbc {tuple(xbc.shape)}, out {tuple(out.shape)}, state {tuple(state.shape)}")
         if max(b_off, c_off) + groups * n_state > xbc.shape[1] or heads * pdim > xbc.shape[1]:
             raise KernelError("ssd_chunk: x, B or C lie outside the rows")
+        floats = self.lib.ullm_ssd_chunk_scratch
+        if workspace is None:
+            scratch = torch.empty(max(1, int(floats(T, requests, heads, n_state, pdim, int(least)))), device=xbc.device)
+        else:
+            scratch = _scratch_floats(workspace, "ssd.chunks", floats(T, requests, heads, n_state, pdim, int(least)),
+                                      floats(workspace.max_tokens, workspace.max_requests, heads, n_state, pdim, int(least)))
         self._check(self.lib.ullm_ssd_chunk(
-            _ptr(xbc), xbc.stride(0), b_off, c_off, _ptr(dt), _ptr(log_decay), _ptr(d_skip), _ptr(scores), _ptr(state),
-            state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req), _ptr(out), T, requests, heads, n_state, pdim,
-            groups, state.shape[0], int(least), _ptr(self.status), _stream(), heads if dt.shape[0] == T else 0),
+            _ptr(xbc), xbc.stride(0), b_off, c_off, _ptr(dt), _ptr(log_decay), _ptr(d_skip), _ptr(scores), _ptr(scratch),
+            _ptr(state), state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req), _ptr(out), T, requests, heads, n_state,
+            pdim, groups, state.shape[0], int(least), _ptr(self.status), _stream(), heads if dt.shape[0] == T else 0),
             f"ssd_chunk (heads {heads}, state {n_state}, columns {pdim})")
-        self.launches += 1  # the scores in front of it
+        self.launches += 2  # the scores in front of it, the outputs behind
 
     @_timed("ssd")
     def ssd_gate_norm(self, y, z, weight, parts: int, eps: float, out, gate_behind: bool = False):

@@ -73,8 +73,10 @@ class FixedDecayAttention(Mixer):
         return StateNeed((self.num_heads * self.value_dim * self.head_dim,), torch.float32)
 
     def activation_elems(self):
-        # the input product, o in 32-bit (two elements' worth), the gated o, the output, the chunked form's scores
-        return 2 * self.qk_size + 5 * self.v_size + self.hidden_size + 128 * self.num_heads
+        # the input product, o in 32-bit (two elements' worth), the gated o, the output, the chunked form's scores, sums and
+        # weights, and a 64th of its states
+        return (2 * self.qk_size + 5 * self.v_size + self.hidden_size + 134 * self.num_heads
+                + self.num_heads * self.head_dim * self.value_dim // 32)
 
     def operand_dtype(self):
         return self.w_in.dtype
@@ -95,7 +97,7 @@ class FixedDecayAttention(Mixer):
             K.act_rows("silu", u[:, :vs + 2 * qk], u[:, :vs + 2 * qk])
             scores = ws.tokens("ssd.scores", T, K.ssd_chunk_floats(1, N), torch.float32)
             K.ssd_chunk(u, vs, vs + qk, self.steps, self.log_decay, self.skip, scores, cache.state, ctx.cu_q, ctx.req_slots,
-                        ctx.token_req, o, ctx.num_requests, N, d, dv, N, CHUNK_LEAST)
+                        ctx.token_req, o, ctx.num_requests, N, d, dv, N, CHUNK_LEAST, ws)
         if not chunked or ctx.num_requests > 1:
             K.ssd_recurrence(u, vs, vs + qk, self.steps, self.log_decay, self.skip, cache.state, ctx.cu_q, ctx.req_slots,
                              ctx.token_req, o, ctx.num_requests, N, d, dv, N, CHUNK_LEAST if chunked else 1 << 30,

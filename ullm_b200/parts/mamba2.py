@@ -76,9 +76,9 @@ class Mamba2(Mixer, SharesInput):
 
     def activation_elems(self):
         # the input product, the convolved rows, steps and decays and y in 32-bit (two elements each), the gated y, the output
-        # ... and the chunked form's scores
-        return (self.input_width() + self.channels + 4 * self.num_heads + 3 * self.inner + self.hidden_size
-                + 128 * self.groups)
+        # ... and the chunked form's scores, sums and weights, and a 64th of its states (32-bit)
+        return (self.input_width() + self.channels + 10 * self.num_heads + 3 * self.inner + self.hidden_size
+                + 128 * self.groups + self.s_floats // 32)
 
     def output_projection(self):
         return self.tensors[self.names["o"]], None
@@ -108,7 +108,7 @@ class Mamba2(Mixer, SharesInput):
         if chunked:
             scores = ws.tokens("ssd.scores", T, K.ssd_chunk_floats(1, G), torch.float32)
             K.ssd_chunk(xbc, inner, inner + G * S, dt, log_decay, t[n["d"]], scores, cache.state, ctx.cu_q, ctx.req_slots,
-                        ctx.token_req, y, ctx.num_requests, N, S, P, G, CHUNK_LEAST)
+                        ctx.token_req, y, ctx.num_requests, N, S, P, G, CHUNK_LEAST, ws)
         if not chunked or ctx.num_requests > 1:
             K.ssd_recurrence(xbc, inner, inner + G * S, dt, log_decay, t[n["d"]], cache.state, ctx.cu_q, ctx.req_slots,
                              ctx.token_req, y, ctx.num_requests, N, S, P, G, CHUNK_LEAST if chunked else 1 << 30,

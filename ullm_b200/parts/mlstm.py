@@ -84,8 +84,10 @@ class MLSTM(Mixer):
         return StateNeed((mlstm_state_floats(self.num_heads, self.head_dim, self.value_dim),), torch.float32)
 
     def activation_elems(self):
-        # q | k | v | g, the gates, o in 32-bit (two elements' worth in a 16-bit engine), the gated o, the output
-        return 2 * self.qk_size + 2 * self.v_size + 2 * self.num_heads + 3 * self.v_size + self.hidden_size
+        # q | k | v | g, the gates, o in 32-bit (two elements' worth in a 16-bit engine), the gated o, the output, the chunked
+        # form's sums and weights and a 64th of its states
+        return (2 * self.qk_size + 2 * self.v_size + 16 * self.num_heads + 3 * self.v_size + self.hidden_size
+                + self.num_heads * self.head_dim * (self.value_dim + 1) // 32)
 
     def output_projection(self):
         return None
