@@ -1,0 +1,33 @@
+"""The clamped gate and xielu in 16-byte pieces against 32-bit references, where lengths or addresses allow pieces and where not."""
+
+import pytest
+import torch
+
+from test_gpu_kernels import K, rnd
+
+pytestmark = [pytest.mark.gpu, pytest.mark.needs_cuda]
+
+
+def apply(kind, z, pq):
+    if kind == "clamped":
+        g, u = z.chunk(2, -1)
+        g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
+        return g * torch.sigmoid(1.702 * g) * (u + 1)
+    a = torch.nn.functional.softplus(pq)
+    neg = z.clamp(max=0)
+    return torch.where(z > 0, a[0] * z * z + 0.5 * z, (0.5 + a[1]) * (torch.expm1(neg) - neg) + 0.5 * z)
+
+
+@pytest.mark.parametrize("dtype,limit", [(torch.float32, 2e-6), (torch.bfloat16, 2 ** -8), (torch.float16, 2 ** -10)])
+@pytest.mark.parametrize("rows,cols,shift", [(1, 8, 0), (3, 7, 0), (5, 96, 0), (2, 100, 0), (4, 64, 1)])
+def test_row_kernels_in_pieces(dtype, limit, rows, cols, shift):
+    kk, pq = K(), rnd(2, seed=54)
+    x = rnd(rows * 2 * cols + shift, seed=55, dtype=dtype)[shift:].view(rows, 2 * cols)  # (shift: off the 16-byte border)
+    out = torch.empty(rows, cols, dtype=dtype, device="cuda")
+    kk.act_mul_clamped(x, out, 1.5, 1.702)
+    ref = apply("clamped", x.float(), pq)
+    assert (out.float() - ref).abs().max().item() <= limit * max(1.0, ref.abs().max().item())
+    out = torch.empty_like(x)
+    kk.xielu(x, pq, out)
+    ref = apply("xielu", x.float(), pq)
+    assert (out.float() - ref).abs().max().item() <= limit * max(1.0, ref.abs().max().item())

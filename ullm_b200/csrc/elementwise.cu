@@ -2,6 +2,7 @@
 // activation, dtype casts.  Every kernel takes any row length; rows that can be
 // moved in 16-byte pieces are, others go element by element.
 #include "common.cuh"
+#include "moe_act.cuh"
 
 #include <type_traits>
 
@@ -392,20 +393,25 @@ extern "C" int ullm_cast_bf16_f32(const void* in, float* out, long long n, void*
 
 // ---------------------------------------------------------------------------
 // clamped gated activation: g' = min(g, limit), u' = clamp(u, -limit, limit),
-// out = g' * sigmoid(alpha * g') * (u' + 1), in 32-bit
+// out = g' * sigmoid(alpha * g') * (u' + 1), in 32-bit; VEC neighbouring columns
+// per thread and turn (2,048 x 8,192 in bfloat16, cold caches: 62 us one column at
+// a time, 31 us in 16-byte pieces; 101 MB are 15 us at the copy rate)
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void act_mul_clamped_kernel(const T* __restrict__ gu, T* __restrict__ out, long long rows, int inter,
+template <typename T, int VEC>
+__global__ void act_mul_clamped_kernel(const T* __restrict__ gu, T* __restrict__ out, long long pieces, int per_row,
                                        float limit, float alpha) {
   pdl_launch_dependents();
   pdl_wait();
-  const long long n = rows * inter;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / inter;
-    const int c = (int)(i - t * inter);
-    const float g = fminf(to_f32(gu[t * 2 * inter + c]), limit);
-    const float u = fminf(fmaxf(to_f32(gu[t * 2 * inter + inter + c]), -limit), limit);
-    out[i] = from_f32<T>(g / (1.f + expf(-alpha * g)) * (u + 1.f));
+  const long long inter = (long long)per_row * VEC;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < pieces; i += (long long)gridDim.x * blockDim.x) {
+    const long long t = i / per_row;
+    const int c = (int)(i - t * per_row) * VEC;
+    float g[VEC], u[VEC];
+    load_vec<T, VEC>(gu + t * 2 * inter + c, g);
+    load_vec<T, VEC>(gu + t * 2 * inter + inter + c, u);
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) g[k] = moe_gate_act(2, g[k], u[k], limit, alpha);
+    store_vec<T, VEC>(out + t * inter + c, g);
   }
 }
 
@@ -414,18 +420,28 @@ extern "C" int ullm_act_mul_clamped(int dtype, const void* gate_up, void* out, i
   cudaStream_t st = (cudaStream_t)stream;
   if (rows < 0 || inter <= 0) return ULLM_ERR_BAD_SIZE;
   if (rows == 0) return ULLM_OK;
-  const long long n = (long long)rows * inter;
-  long long blocks = (n + 255) / 256;
+  const int piece = dtype == ULLM_DTYPE_F32 ? 4 : 8;
+  const bool wide = inter % piece == 0 && (((uintptr_t)gate_up | (uintptr_t)out) & 15) == 0;
+  const int per_row = inter / (wide ? piece : 1);
+  const long long pieces = (long long)rows * per_row;
+  long long blocks = (pieces + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   const dim3 grid((int)blocks), block(256);
-  if (dtype == ULLM_DTYPE_F32)
-    return ullm_launch_kernel(act_mul_clamped_kernel<float>, grid, block, 0, st, (const float*)gate_up, (float*)out,
-                              (long long)rows, inter, limit, alpha);
-  if (dtype == ULLM_DTYPE_BF16)
-    return ullm_launch_kernel(act_mul_clamped_kernel<__nv_bfloat16>, grid, block, 0, st,
-                              (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, (long long)rows, inter, limit, alpha);
-  if (dtype == ULLM_DTYPE_F16)
-    return ullm_launch_kernel(act_mul_clamped_kernel<__half>, grid, block, 0, st, (const __half*)gate_up,
-                              (__half*)out, (long long)rows, inter, limit, alpha);
+#define AMC_GO(T, V)                                                                                                       \
+  return ullm_launch_kernel(act_mul_clamped_kernel<T, V>, grid, block, 0, st, (const T*)gate_up, (T*)out, pieces, per_row, \
+                            limit, alpha)
+  if (dtype == ULLM_DTYPE_F32) {
+    if (wide) AMC_GO(float, 4);
+    AMC_GO(float, 1);
+  }
+  if (dtype == ULLM_DTYPE_BF16) {
+    if (wide) AMC_GO(__nv_bfloat16, 8);
+    AMC_GO(__nv_bfloat16, 1);
+  }
+  if (dtype == ULLM_DTYPE_F16) {
+    if (wide) AMC_GO(__half, 8);
+    AMC_GO(__half, 1);
+  }
+#undef AMC_GO
   return ULLM_ERR_BAD_DTYPE;
 }

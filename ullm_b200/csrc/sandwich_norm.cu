@@ -232,16 +232,21 @@ __global__ void norm_rows_kernel(const float* __restrict__ stream, const int* __
 
 __device__ __forceinline__ float softplus_f32(float v) { return log1pf(expf(-fabsf(v))) + fmaxf(v, 0.f); }
 
-template <typename T>
+// VEC neighbouring elements per thread and turn: bound by the bytes moved (67 MB at 2,048 x 8,192: 43 us one element at a time,
+// 33 us in 16-byte pieces, with cold caches)
+template <typename T, int VEC>
 __global__ void xielu_kernel(const T* __restrict__ in, T* __restrict__ out, long long n,
                              const float* __restrict__ pq) {
   pdl_launch_dependents();
   pdl_wait();
   const float ap = softplus_f32(pq[0]), aq = 0.5f + softplus_f32(pq[1]);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float z = to_f32(in[i]);
-    const float y = z > 0.f ? ap * z * z + 0.5f * z : aq * (expm1f(z) - z) + 0.5f * z;
-    out[i] = from_f32<T>(y);
+  for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * VEC; i < n;
+       i += (long long)gridDim.x * blockDim.x * VEC) {
+    float v[VEC];
+    load_vec<T, VEC>(in + i, v);
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) v[k] = v[k] > 0.f ? ap * v[k] * v[k] + 0.5f * v[k] : aq * (expm1f(v[k]) - v[k]) + 0.5f * v[k];
+    store_vec<T, VEC>(out + i, v);
   }
 }
 
@@ -419,16 +424,25 @@ extern "C" int ullm_xielu(int dtype, const void* in, void* out, long long n, con
   cudaStream_t st = (cudaStream_t)stream_handle;
   if (n < 0 || pq == nullptr) return ULLM_ERR_BAD_SIZE;
   if (n == 0) return ULLM_OK;
-  long long blocks = (n + 255) / 256;
+  const int piece = dtype == ULLM_DTYPE_F32 ? 4 : 8;
+  const bool wide = n % piece == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+  long long blocks = (n / (wide ? piece : 1) + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   const dim3 grid((int)blocks), block(256);
-  if (dtype == ULLM_DTYPE_F32)
-    return ullm_launch_kernel(xielu_kernel<float>, grid, block, 0, st, (const float*)in, (float*)out, n, pq);
-  if (dtype == ULLM_DTYPE_BF16)
-    return ullm_launch_kernel(xielu_kernel<__nv_bfloat16>, grid, block, 0, st, (const __nv_bfloat16*)in,
-                              (__nv_bfloat16*)out, n, pq);
-  if (dtype == ULLM_DTYPE_F16)
-    return ullm_launch_kernel(xielu_kernel<__half>, grid, block, 0, st, (const __half*)in, (__half*)out, n, pq);
+#define XIELU_GO(T, V) return ullm_launch_kernel(xielu_kernel<T, V>, grid, block, 0, st, (const T*)in, (T*)out, n, pq)
+  if (dtype == ULLM_DTYPE_F32) {
+    if (wide) XIELU_GO(float, 4);
+    XIELU_GO(float, 1);
+  }
+  if (dtype == ULLM_DTYPE_BF16) {
+    if (wide) XIELU_GO(__nv_bfloat16, 8);
+    XIELU_GO(__nv_bfloat16, 1);
+  }
+  if (dtype == ULLM_DTYPE_F16) {
+    if (wide) XIELU_GO(__half, 8);
+    XIELU_GO(__half, 1);
+  }
+#undef XIELU_GO
   return ULLM_ERR_BAD_DTYPE;
 }
 
