@@ -195,6 +195,9 @@ class Kernels:
         self.moe_tcgen05_rows = int(get("ULLM_B200_MOE_TCGEN05_ROWS", "2"))
         # tokens up to which those products stream the chosen experts' matrices (at most 16)
         self.moe_stream_tokens = min(16, int(get("ULLM_B200_MOE_STREAM_TOKENS", "16")))
+        # float32 rows from which products run on the tensor cores in three bfloat16 terms per operand (csrc/linear_f32_split.cu)
+        self.f32_split_rows = int(get("ULLM_B200_F32_SPLIT_ROWS", "17"))
+        self.f32_split_results = 1 << 16  # ... and results, see linear_f32_split
         # attention of the 32-bit engine and of float16 by row tiles (csrc/attention_plain.cu); 0: the general kernel always
         self.plain_attention_on = get("ULLM_B200_PLAIN_ATTN", "1") != "0"
         # the splits of a request's keys merge inside a thread-block cluster (at most 8 splits) instead of through
@@ -279,6 +282,7 @@ class Kernels:
             "ullm_linear_stream": [P, P, P, P, P, I, I, I, I, I, P, P],
             "ullm_linear_stream_norm": [P, P, P, P, P, I, I, I, I, I, P, P, P, P, I, I, F, P, P],
             "ullm_layer_tail_fused": [P, P, P, P, P, P, P, P, F, I, I, I, I, I, P, P, P, P],
+            "ullm_linear_f32_split": [P, P, P, P, P, I, I, I, P, P],
             "ullm_linear_tcgen05_large": [P, P, P, P, I, I, I, I, I, I, P, P],
             "ullm_decode_attention_tcgen05": [P, LL, P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, F, LL, P, P],
             "ullm_lt_linear": [P, P, P, I, I, I, I, P, LL, I, P, LL, P],
@@ -386,6 +390,8 @@ class Kernels:
         L.ullm_decode_attention_supported.restype = c_int
         L.ullm_decode_attention_balanced_supported.argtypes = [I, I, I, I, I]
         L.ullm_decode_attention_balanced_supported.restype = c_int
+        L.ullm_linear_f32_split_terms.argtypes = [I, I]
+        L.ullm_linear_f32_split_terms.restype = c_longlong
         L.ullm_decode_attention_balanced_scratch_floats.argtypes = [I, I]
         L.ullm_decode_attention_balanced_scratch_floats.restype = c_longlong
         L.ullm_decode_attention_tcgen05_supported.argtypes = [I, I, I, I, I]
@@ -727,11 +733,37 @@ class Kernels:
             return out
         if bias is None and self._lt_takes(x.shape[0], weight) and self.lt_linear(x, weight, out):
             return out
+        if x.dtype == torch.float32 and self.linear_f32_split(x, weight, out, bias):
+            return out
         if bias is not None:
             torch.addmm(bias, x, weight.t(), out=out)
         else:
             torch.mm(x, weight.t(), out=out)
         return out
+
+    def linear_f32_split(self, x, weight, out, bias=None) -> bool:
+        """out = x @ weight.T (+ bias) in float32 on the tensor cores, every operand as three bfloat16 terms
+        (csrc/linear_f32_split.cu).  False for what the kernel does not take and where the library's product is as fast
+        (nothing has run): up to 16 rows, and fewer than 2^16 results, whose tiles leave most SMs idle (1,024 columns of
+        k 2,048: 32 rows 38 us for 26, 64 rows 38 for 57; 511 x 64 results 40 for 26, 2,048 x 64 44 for 58); very many columns
+        at few rows, where a tile's start is a fifth of its time (151,936 columns of k 1,024: 32 rows 278 us for 261, 48 rows
+        279 for 386)."""
+        M, K = x.shape
+        N = weight.shape[0]
+        if (M < self.f32_split_rows or M * N < self.f32_split_results or (M <= 32 and N > 32768)
+                or weight.dtype != torch.float32 or out.dtype != torch.float32 or not x.is_contiguous()
+                or not weight.is_contiguous() or not out.is_contiguous() or weight.shape[1] != K or out.shape != (M, N)
+                or (bias is not None and (bias.dtype != torch.float32 or bias.shape != (N,) or not bias.is_contiguous()))):
+            return False
+        # (of the caller's stream, not a kept buffer: products on two streams may run side by side)
+        terms = torch.empty(int(self.lib.ullm_linear_f32_split_terms(M, K)), dtype=torch.bfloat16, device=x.device)
+        code = self.lib.ullm_linear_f32_split(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), _ptr(terms), M, N, K, _ptr(self.status),
+                                              _stream())
+        if code == 4:
+            return False
+        self.launches += 1  # x in its three planes
+        self._check(code, f"linear_f32_split ({M}x{K} . {N}x{K})")
+        return True
 
     @_timed("linear_gate_up_act", _weight_bytes)
     def linear_act_mul(self, x, weight, out, gate_up, act: int = 0):
@@ -757,7 +789,8 @@ class Kernels:
         """out (float32) = x @ weight.T for x/weight in float32 or bfloat16."""
         _need(out, "out", torch.float32)
         if x.dtype == torch.float32:
-            torch.mm(x, weight.t(), out=out)
+            if not self.linear_f32_split(x, weight, out):
+                torch.mm(x, weight.t(), out=out)
             return out
         if self._own_linear(x, weight, out):
             return out
