@@ -2,7 +2,8 @@
 // generation tensor cores:  out[p] = f(W_e . (s_p * x[row(p)])) for every place p of every expert e.
 //
 // Bound by the tensor cores: at 2,048 tokens with 2 of 16 experts of 1,024 x 2,048 each (gated) the two products are 52 GFLOP,
-// 31 us at the card's rate.  The mma.sync kernel of moe.cu took 136 + 81 us there: tiles of 64 x 64 read both operands from
+// 31 us at the card's rate; measured with cold caches 69 + 37 us (512 tokens 46 + 25, bound by the 201 MB of matrices; 32 experts
+// of 2,048 x 4,096: 214 + 114).  The mma.sync kernel of moe.cu takes 140 + 88 us there: tiles of 64 x 64 read both operands from
 // shared memory once per 64 columns, and its warps spend their issue slots on ldmatrix.
 //
 // A persistent kernel, one block per SM, built as linear_tcgen05_large.cu: warp 0 loads, warp 1 issues the MMAs (M = 128,
@@ -54,6 +55,37 @@ __device__ __forceinline__ void mt_find(const int* first, const int* offsets, in
   const int lo = offsets[e], hi = offsets[e + 1];
   p0 = lo + (rem - nt * here) * MT_BM;
   rows = min(MT_BM, hi - p0);
+}
+
+// A thread's row of the tile out of tensor memory, activated, stored.  The gate without branches: with the division of
+// `moe_gate_act`, whose slow path keeps a thread's 128 elements in series, the last tile's end took 20 us more (63 for 44 us at 32
+// to 512 tokens, 87 for 69 at 2,048).
+template <int ACT, bool GATED>
+__device__ __forceinline__ void mt_store(const MtParams& p, uint32_t taddr, float sc, __nv_bfloat16* dst, int col0, bool on) {
+  constexpr int COLS = GATED ? MT_BN / 2 : MT_BN;
+#pragma unroll 1
+  for (int c = 0; c < COLS; c += 16) {
+    float v[16];
+    tmem_ld16(taddr + c, v);
+    if (GATED) {
+      float u[16];
+      tmem_ld16(taddr + MT_BN / 2 + c, u);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = moe_gate_act_flat<ACT>(v[i] * sc, u[i] * sc, p.limit, p.alpha);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = moe_plain_act(ACT, v[i] * sc);
+    }
+    if (on) {  // (n_out is a multiple of 8)
+      const int col = col0 + c;
+      uint4 w[2];
+      __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(w);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      if (col < p.n_out) *reinterpret_cast<uint4*>(dst + col) = w[0];
+      if (col + 8 < p.n_out) *reinterpret_cast<uint4*>(dst + col + 8) = w[1];
+    }
+  }
 }
 
 __global__ void __launch_bounds__(MT_THREADS, 1)
@@ -198,27 +230,16 @@ moe_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
       const uint32_t taddr = tmem_d + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * MT_BN);
       __nv_bfloat16* dst = p.out + (long long)(p0 + row) * p.n_out;
       const int cols = p.gated ? MT_BN / 2 : MT_BN;
-#pragma unroll 2
-      for (int c = 0; c < cols; c += 16) {
-        float v[16];
-        tmem_ld16(taddr + c, v);
-        if (p.gated) {
-          float u[16];
-          tmem_ld16(taddr + MT_BN / 2 + c, u);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = moe_gate_act(p.act, v[i] * sc, u[i] * sc, p.limit, p.alpha);
+      if (quarter * 32 < rows) {  // (a warp without places has nothing to read)
+        if (!p.gated) {
+          if (p.act == 3) mt_store<3, false>(p, taddr, sc, dst, nt * cols, on);
+          else mt_store<-1, false>(p, taddr, sc, dst, nt * cols, on);
+        } else if (p.act == 0) {
+          mt_store<0, true>(p, taddr, sc, dst, nt * cols, on);
+        } else if (p.act == 2) {
+          mt_store<2, true>(p, taddr, sc, dst, nt * cols, on);
         } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = moe_plain_act(p.act, v[i] * sc);
-        }
-        const int col = nt * cols + c;
-        if (on) {  // (n_out is a multiple of 8)
-          uint4 w[2];
-          __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(w);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-          if (col < p.n_out) *reinterpret_cast<uint4*>(dst + col) = w[0];
-          if (col + 8 < p.n_out) *reinterpret_cast<uint4*>(dst + col + 8) = w[1];
+          mt_store<1, true>(p, taddr, sc, dst, nt * cols, on);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -191,7 +191,9 @@ class Kernels:
         # rows from which a step with distance biases (heads of 128) takes the tcgen05 prompt kernel
         self.pair_biased_rows = int(get("ULLM_B200_PAIR_BIASED_ROWS", "128"))
         self.window_attention_tc = get("ULLM_B200_WINDOW_ATTN_TC", "1") != "0"
-        # rows per expert, on average, from which the routed experts' products run on the tcgen05 kernel (see _moe_tcgen05_pays)
+        # rows per expert, on average, from which the routed experts' products of more than 16 tokens run on the tcgen05 kernel: at
+        # 4 rows it takes 44 + 24 us for mma.sync's 45 + 34 (16 experts, gated 1,024 x 2,048), at 2 rows 162 + 90 for 213 + 132 (32
+        # experts of 2,048 x 4,096), and more rows only widen that
         self.moe_tcgen05_rows = int(get("ULLM_B200_MOE_TCGEN05_ROWS", "2"))
         # tokens up to which those products stream the chosen experts' matrices (at most 16)
         self.moe_stream_tokens = min(16, int(get("ULLM_B200_MOE_STREAM_TOKENS", "16")))
@@ -2064,18 +2066,6 @@ class Kernels:
         self._check(self.lib.ullm_moe_arrange(_ptr(choice), pairs, experts, _ptr(offsets), _ptr(sorted_pairs), _ptr(place),
                                               _stream()), f"moe_arrange ({experts} experts)")
 
-    def _moe_tcgen05_pays(self, pairs: int, experts: int, n_out: int, gated: bool) -> bool:
-        """Whether a grouped product of more tokens than the streaming kernel takes runs on tcgen05 or on mma.sync, measured with
-        cold caches.  Products without gate rows: tcgen05 at 4 rows per expert already (2,048 x 1,024, 16 experts: 24.6 us for
-        33.7) and at every size above.  Gated ones too where the experts' matrices make several 128-column tiles per SM (32 experts
-        of 2,048 x 4,096: 186 us for 214 at 2 rows per expert); where they make one tile per SM at most (16 experts of
-        1,024 x 2,048) its loads have no second tile to run under, and mma.sync is the faster one as long as an expert's rows
-        fit one of its tiles of 64 (45 us for 63 at 16 rows, 61 for 64 at 64 rows, 88 for 50 at 96)."""
-        rows = self.moe_tcgen05_rows
-        if gated and rows and experts * -(-n_out // 128) <= 148:
-            rows = max(rows, 65)
-        return pairs >= rows * experts
-
     @_timed("moe", lambda x, weights, *r: weights.numel() * weights.element_size())
     def moe_grouped_linear(self, x, weights, offsets, sorted_pairs, pair_weight, out, top: int, rows_from_pairs: bool,
                            gated: bool, act: int = 0, limit: float = 0.0, alpha: float = 1.0, gathered=None):
@@ -2102,7 +2092,7 @@ class Kernels:
                 int(rows_from_pairs), n_out, K, int(gated), act, float(limit), float(alpha), _ptr(self.status), _stream())
             if code != 4:
                 return self._check(code, f"moe_stream ({E} experts, {N} x {K})")
-        if (x.dtype == torch.bfloat16 and not self._moe_plain and self._moe_tcgen05_pays(pairs, E, n_out, gated)
+        if (x.dtype == torch.bfloat16 and not self._moe_plain and pairs >= self.moe_tcgen05_rows * E
                 and (not rows_from_pairs or gathered is not None)):
             code = self.lib.ullm_moe_grouped_tcgen05(
                 _ptr(x), x.stride(0), _ptr(gathered) if rows_from_pairs else None, _ptr(weights), _ptr(offsets), _ptr(sorted_pairs), _ptr(pair_weight), _ptr(out),
