@@ -1,4 +1,5 @@
-"""The clamped gate and xielu in 16-byte pieces against 32-bit references, where lengths or addresses allow pieces and where not."""
+"""The clamped gate, xielu and the gated add in 16-byte pieces against references, where lengths or addresses allow pieces and where
+not; the gated add with gates at infinities."""
 
 import pytest
 import torch
@@ -31,3 +32,20 @@ def test_row_kernels_in_pieces(dtype, limit, rows, cols, shift):
     kk.xielu(x, pq, out)
     ref = apply("xielu", x.float(), pq)
     assert (out.float() - ref).abs().max().item() <= limit * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("dtype,limit", [(torch.float32, 2e-6), (torch.bfloat16, 2 ** -8), (torch.float16, 2 ** -10)])
+@pytest.mark.parametrize("rows,cols,shift", [(1, 8, 0), (3, 7, 0), (5, 264, 0), (2, 100, 0), (4, 64, 1)])
+@pytest.mark.parametrize("both", [True, False])
+def test_gated_add(dtype, limit, rows, cols, shift, both):
+    a, f = (rnd(rows * cols + shift, seed=s, dtype=dtype)[shift:].view(rows, cols) for s in (61, 62))
+    n = 2 if both else 1
+    g, b1, b2 = 4 * rnd(rows, n * cols, seed=63), rnd(cols, seed=64), rnd(cols, seed=65)
+    stream, copy = rnd(rows, cols, seed=66), torch.empty(rows, cols, dtype=dtype, device="cuda")
+    g[0, 0], g[0, 1], g[0, 2], g[0, 3] = 200.0, -200.0, float("inf"), float("-inf")
+    ref = stream.double() + a.double() * torch.sigmoid(g[:, :cols].double() + b1.double())
+    if both:
+        ref += f.double() * torch.sigmoid(g[:, cols:].double() + b2.double())
+    K().gated_add_f32(a, f if both else None, g, b1, b2 if both else None, stream, copy)
+    assert (stream.double() - ref).abs().max().item() <= 1e-6 * max(1.0, ref.abs().max().item())
+    assert (copy.double() - ref).abs().max().item() <= limit * max(1.0, ref.abs().max().item())

@@ -92,6 +92,18 @@ __device__ __forceinline__ float act_gelu_tanh(float g) {
   return 0.5f * g * (1.f + tanhf(k * (g + 0.044715f * g * g * g)));
 }
 
+// g / (1 + e^-z) without a branch, so that a thread's elements run beside one another (a division's slow path keeps them in
+// series): a reciprocal and one step of Newton's method; from 2^126 on the denominator counts as infinite.  gelu_tanh is this with
+// z = 2 sqrt(2 / pi) (g + 0.044715 g^3), since (1 + tanh v) / 2 = 1 / (1 + e^-2v).
+__device__ __forceinline__ float gate_flat(float g, float z) {
+  const float y = 1.f + expf(-z), r = __fdividef(1.f, y), q = g * r;
+  const float s = fabsf(g) <= 3.4028234e38f ? fmaf(fmaf(-q, y, g), r, q) : q;
+  return y < 8.5e37f ? s : (y == y ? g * 0.f : y);
+}
+__device__ __forceinline__ float act_gelu_tanh_flat(float g) {
+  return gate_flat(g, 1.5957691216057308f * (g + 0.044715f * g * g * g));
+}
+
 // True when rows of `cols` elements of T starting at `p` can be moved in
 // 16-byte pieces.
 template <typename T>
