@@ -88,6 +88,89 @@ __global__ void norm_add_norm_kernel(const TA* __restrict__ a, float* __restrict
     out[base + c] = from_f32<TO>((row_s[c] - mean2) * rstd2 * w2[c]);
 }
 
+// The same with eight neighbouring columns per thread, in registers from the first load to the last store (rows of at most 8,192
+// columns in 16-byte pieces).  Bound by the bytes moved; everything a row needs is asked for at once, the weights in front of the
+// wait for the kernel before.  With cold caches, rows of 2,048 in bfloat16 with a norm on either side: 2,048 rows 34.9 us in shared
+// memory column by column, 18.6 here (50 MB: 7.5 at the copy rate); 8 rows 11.9 and 8.0 us.
+template <typename T>
+__device__ __forceinline__ void sn_load8(const T* p, float (&v)[8]) {
+  if constexpr (sizeof(T) == 4) load_vec32<8>(p, v);
+  else load_vec<T, 8>(p, v);
+}
+template <typename T>
+__device__ __forceinline__ void sn_store8(T* p, const float (&v)[8]) {
+  if constexpr (sizeof(T) == 4) store_vec32<8>(p, v);
+  else store_vec<T, 8>(p, v);
+}
+// as row_rstd, over the threads' own columns (`on`: the thread has some)
+__device__ __forceinline__ float piece_rstd(const float (&v)[8], bool on, int cols, bool center, float eps, float* scratch,
+                                            float* mean_out) {
+  float mean = 0.f, acc = 0.f;
+  if (center) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc += on ? v[i] : 0.f;
+    mean = block_sum(acc, scratch) / (float)cols;
+    acc = 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float d = v[i] - mean;
+    acc += on ? d * d : 0.f;
+  }
+  *mean_out = mean;
+  return 1.f / sqrtf(block_sum(acc, scratch) / (float)cols + eps);
+}
+
+template <typename TA, typename TO>
+__global__ void norm_add_norm_piece_kernel(const TA* __restrict__ a, float* __restrict__ stream, const float* __restrict__ w, int cols,
+                                           float eps, float mult, int center, const float* __restrict__ extra_rows,
+                                           const float* __restrict__ extra_vec, const float* __restrict__ w2, float eps2, int center2,
+                                           TO* __restrict__ out, const float* __restrict__ alpha2, const float* __restrict__ b2) {
+  __shared__ float scratch[33];
+  pdl_launch_dependents();
+  const int c0 = threadIdx.x * 8;
+  const bool on = c0 < cols;
+  const long long base = (long long)blockIdx.x * cols + c0;
+  float wv[8], w2v[8], s[8], v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) wv[i] = 1.f, w2v[i] = s[i] = v[i] = 0.f;
+  if (on && a != nullptr && w != nullptr) load_vec32<8>(w + c0, wv);
+  if (on && out != nullptr && center2 != 3) load_vec32<8>(w2 + c0, w2v);
+  pdl_wait();
+  if (on) load_vec32<8>(stream + base, s);
+  if (a != nullptr) {
+    if (on) sn_load8<TA>(a + base, v);
+    float rstd = 1.f, mean = 0.f;
+    if (center != 2) rstd = piece_rstd(v, on, cols, center != 0, eps, scratch, &mean);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] += mult * ((v[i] - mean) * rstd * wv[i]);
+  }
+  if (on && extra_rows != nullptr) {
+    load_vec32<8>(extra_rows + base, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] += v[i];
+  }
+  if (on && extra_vec != nullptr) {
+    load_vec32<8>(extra_vec + c0, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] += v[i];
+  }
+  if (on) store_vec32<8>(stream + base, s);
+  if (out == nullptr) return;
+  if (center2 == 2) {
+    const float al = *alpha2;
+    if (on) load_vec32<8>(b2 + c0, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = tanhf(al * s[i]) * w2v[i] + v[i];
+  } else if (center2 != 3) {
+    float mean2;
+    const float rstd2 = piece_rstd(s, on, cols, center2 != 0, eps2, scratch, &mean2);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = (s[i] - mean2) * rstd2 * w2v[i];
+  }
+  if (on) sn_store8<TO>(out + base, s);
+}
+
 // Two sub-layers' rows a and b, each divided by its own root mean square and weighted, their sum (times `mult`) added
 // to the stream; then the norm that reads the stream next.  One block per row; VEC neighbouring columns per thread and
 // turn (16-byte pieces where the rows allow), both sums of squares in one set of barriers.
@@ -307,6 +390,11 @@ static int norm_add_norm_launch(const void* a, float* stream, const float* w, in
                                 float mult, int center, const float* extra_rows, const float* extra_vec,
                                 const float* w2, float eps2, int center2, void* out, const float* alpha2,
                                 const float* b2, cudaStream_t st) {
+  const uintptr_t all = (uintptr_t)a | (uintptr_t)stream | (uintptr_t)w | (uintptr_t)extra_rows | (uintptr_t)extra_vec |
+                        (uintptr_t)w2 | (uintptr_t)out | (uintptr_t)b2;
+  if (cols % 8 == 0 && cols <= 8192 && (all & 15) == 0)
+    return ullm_launch_kernel(norm_add_norm_piece_kernel<TA, TO>, dim3(rows), dim3((cols / 8 + 31) / 32 * 32), 0, st, (const TA*)a,
+                              stream, w, cols, eps, mult, center, extra_rows, extra_vec, w2, eps2, center2, (TO*)out, alpha2, b2);
   const size_t smem = 2 * (size_t)cols * sizeof(float);
   if (smem > SN_MAX_SMEM) return ULLM_ERR_UNSUPPORTED;
   const int rc = sn_allow_smem(norm_add_norm_kernel<TA, TO>, smem);
