@@ -42,6 +42,8 @@ def test_value_tiles_match_the_recurrence(heads, dim, vdim, lens):
         kk.raise_on_status()
         outs.append(out.double())
         states.append(state.double())
-    # two bfloat16 terms keep 16 bits of every 32-bit operand: 2^-17 of each of the summed products
-    assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2e-5
-    assert float((states[0] - states[1]).norm() / states[1].norm()) < 2e-5
+    # three bfloat16 terms keep 24 bits of every 32-bit operand: both sides differ by the rounding of 32-bit sums and products (2^-24
+    # each): of up to 130 decays one after the other, of sums over up to 256 channels and 130 tokens, at most sqrt(130 + 256 + 130)
+    # roundings' worth when they are independent
+    assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2.0 ** -24 * 516 ** 0.5
+    assert float((states[0] - states[1]).norm() / states[1].norm()) < 2.0 ** -24 * 516 ** 0.5

@@ -17,7 +17,8 @@
 // product; the keys of its own stretch one by one in 32-bit, the product of decays carried from token to token.
 //
 // Precision: v is an exact bfloat16 operand; every 32-bit operand (weighted queries and keys, scores, the state) enters as
-// TWO bfloat16 terms, rounded value and rounded rest; accumulators, decays and states are 32-bit.
+// bfloat16 terms, rounded value, rounded rest and, without a bonus, the rest of that (24 bits: the outputs are then as near to 64
+// bits as the token-by-token kernel's; with a bonus two terms, 16 bits); accumulators, decays and states are 32-bit.
 //
 // mma.sync m16n8k16; a block of four warps owns (chunk, head), warp w the chunk's rows 16 w .. 16 w + 15.
 #include "common.cuh"
@@ -40,13 +41,6 @@ __device__ __forceinline__ void gch_mma(float (&c)[4], const unsigned (&a)[4], u
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void gch_split(float v0, float v1, unsigned& hi, unsigned& lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(v0 - __bfloat162float(h.x), v1 - __bfloat162float(h.y));
-  hi = *reinterpret_cast<const unsigned*>(&h);
-  lo = *reinterpret_cast<const unsigned*>(&l);
-}
-
 // Chunk `tile` of the step: its first token and its tokens (0: there is no such chunk).  Chunks are counted over the
 // requests that bring more than `least` tokens, from each request's first token of the step.
 __device__ __forceinline__ int gch_find(int tile, const int* cu_q, int requests, int least, int& t0) {
@@ -63,6 +57,38 @@ __device__ __forceinline__ int gch_find(int tile, const int* cu_q, int requests,
   return 0;
 }
 
+// (v0, v1) as N pairs of bfloat16: rounded values, rounded rests, ...
+template <int N>
+__device__ __forceinline__ void gch_terms(float v0, float v1, unsigned (&t)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+    v0 -= __bfloat162float(h.x);
+    v1 -= __bfloat162float(h.y);
+    t[i] = *reinterpret_cast<const unsigned*>(&h);
+  }
+}
+// c += a b for operands in N terms each (a[i]: the fragment of term i; M: terms of b): every product down to the first one's
+// 2^-8 N.  With three terms the products meet apart, smallest first, and are added by ordinary additions: the tensor core cuts
+// its sums instead of rounding them, which over a row of 128 channels came to 1.5e-6 of an output (token by token: 1e-7 to 4e-7).
+template <int N, int M>
+__device__ __forceinline__ void gch_mma_terms(float (&c)[4], const unsigned (&a)[N][4], const unsigned (&b0)[M], const unsigned (&b1)[M]) {
+  if (N == 2) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int j = 0; j < M && j < N - i; ++j) gch_mma(c, a[i], b0[j], b1[j]);
+  } else {
+    float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int order = N - 1; order >= 0; --order)
+#pragma unroll
+      for (int j = 0; j < M && j <= order; ++j) gch_mma(t, a[order - j], b0[j], b1[j]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[e] += t[e];
+  }
+}
+
 // v of the chunk, [GCH_Q][vdim + 8] bfloat16, rows past the chunk's end zero
 __device__ __forceinline__ void gch_load_v(__nv_bfloat16* v_s, const __nv_bfloat16* v, long long row_stride, int vdim, int cn) {
   const int pieces = vdim >> 3;
@@ -75,6 +101,7 @@ __device__ __forceinline__ void gch_load_v(__nv_bfloat16* v_s, const __nv_bfloat
 }
 
 // fold[(tile * heads + head)][vdim][dim] = sum_s v_s (W(s, Q) k_s)^T;  total[(tile * heads + head)][dim] = W(0, Q)
+template <int NT>
 __global__ void __launch_bounds__(GCH_THREADS)
 gla_fold_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int k_off, int v_off,
                 const float* __restrict__ decay, long long decay_stride, const int* __restrict__ cu_q,
@@ -128,14 +155,14 @@ gla_fold_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int
   const int mat = lane >> 3;
   for (int n0 = warp * 8; n0 < dim; n0 += 32) {  // eight key channels of the state
     const int ch = n0 + (lane >> 2);
-    unsigned bh[4][2], bl[4][2];
+    unsigned b[4][2][NT];
 #pragma unroll
     for (int s = 0; s < 4; ++s)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int r = s * 16 + h * 8 + (lane & 3) * 2;
         const float f = tot[(s * 2 + h) * dim + ch];
-        gch_split(kq[r * ks + ch] * f, kq[(r + 1) * ks + ch] * f, bh[s][h], bl[s][h]);
+        gch_terms<NT>(kq[r * ks + ch] * f, kq[(r + 1) * ks + ch] * f, b[s][h]);
       }
     for (int m0 = 0; m0 < vdim; m0 += 16) {
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -143,8 +170,16 @@ gla_fold_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int
       for (int s = 0; s < 4; ++s) {
         unsigned a[4];
         gch_ldsm4t(a, v_s + (s * 16 + (mat >> 1) * 8 + (lane & 7)) * (vdim + 8) + m0 + (mat & 1) * 8);
-        gch_mma(acc, a, bh[s][0], bh[s][1]);
-        gch_mma(acc, a, bl[s][0], bl[s][1]);
+        if (NT == 2) {
+#pragma unroll
+          for (int i = 0; i < NT; ++i) gch_mma(acc, a, b[s][0][i], b[s][1][i]);
+        } else {
+          float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int i = NT - 1; i >= 0; --i) gch_mma(t, a, b[s][0][i], b[s][1][i]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[e] += t[e];
+        }
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h)
@@ -154,8 +189,9 @@ gla_fold_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int
   }
 }
 
-// fold <- the state in front of every chunk, as pairs of key channels: (two rounded values, two rounded rests), the operands
-// that `gla_out` needs; state <- the state behind the last.  Two neighbouring key channels per thread.
+// fold <- the state in front of every chunk, as pairs of key channels: with PAIRS (two rounded values, two rounded rests), the
+// operands that `gla_out` needs in two terms, else as it is; state <- the state behind the last.  Two neighbouring key channels per thread.
+template <bool PAIRS>
 __global__ void gla_scan_kernel(float* __restrict__ fold, const float* __restrict__ total, float* __restrict__ state,
                                 long long state_stride, const int* __restrict__ cu_q, const int* __restrict__ req_slots,
                                 const int* __restrict__ token_req, int least, int heads, int dim, int vdim,
@@ -195,9 +231,13 @@ __global__ void gla_scan_kernel(float* __restrict__ fold, const float* __restric
 #pragma unroll
     for (int j = 0; j < U; ++j)
       if (c0 + j < chunks) {
-        uint2 terms;
-        gch_split(s.x, s.y, terms.x, terms.y);
-        *reinterpret_cast<uint2*>(f + (c0 + j) * step) = terms;
+        if (PAIRS) {
+          unsigned terms[2];
+          gch_terms<2>(s.x, s.y, terms);
+          *reinterpret_cast<uint2*>(f + (c0 + j) * step) = make_uint2(terms[0], terms[1]);
+        } else {
+          *reinterpret_cast<float2*>(f + (c0 + j) * step) = s;
+        }
         s.x = fmaf(a[j].x, s.x, d[j].x);
         s.y = fmaf(a[j].y, s.y, d[j].y);
       }
@@ -213,6 +253,7 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
                const float* __restrict__ decay, long long decay_stride, const float* __restrict__ bonus, float q_scale,
                const int* __restrict__ cu_q, const int* __restrict__ token_req, int requests, int least, int heads, int dim,
                int vdim, int v_tile, const float* __restrict__ fold, float* __restrict__ out) {
+  constexpr int NT = BONUS ? 2 : 3;  // terms of a 32-bit operand
   extern __shared__ __align__(16) unsigned char gch_smem[];
   pdl_launch_dependents();
   pdl_wait();
@@ -337,27 +378,34 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
     float* r_hi = r_lo + 8 * ks;                        // rows of stretch i0 + 1
     float2 q0 = *reinterpret_cast<const float2*>(r_lo), q1 = *reinterpret_cast<const float2*>(r_hi),
            q2 = *reinterpret_cast<const float2*>(r_lo + 8), q3 = *reinterpret_cast<const float2*>(r_hi + 8);
-    unsigned ah[4], al[4], bh[2], bl[2];
+    unsigned q[4][NT], qf[NT][4], b0[NT], b1[NT];  // the queries' four pairs, and as fragments
+    auto fragments = [&]() {
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) qf[i][e] = q[e][i];
+    };
     {
-      ah[0] = ah[2] = al[0] = al[2] = 0u;
-      gch_split(q1.x, q1.y, ah[1], al[1]);
-      gch_split(q3.x, q3.y, ah[3], al[3]);
+#pragma unroll
+      for (int i = 0; i < NT; ++i) q[0][i] = q[2][i] = 0u;
+      gch_terms<NT>(q1.x, q1.y, q[1]);
+      gch_terms<NT>(q3.x, q3.y, q[3]);
+      fragments();
       const float2 k0 = *reinterpret_cast<const float2*>(kq + (i0 * 8 + g) * ks + kk + cp);
       const float2 k1 = *reinterpret_cast<const float2*>(kq + (i0 * 8 + g) * ks + kk + cp + 8);
-      gch_split(k0.x, k0.y, bh[0], bl[0]);
-      gch_split(k1.x, k1.y, bh[1], bl[1]);
-      gch_mma(near, ah, bh[0], bh[1]);
-      gch_mma(near, ah, bl[0], bl[1]);
-      gch_mma(near, al, bh[0], bh[1]);
+      gch_terms<NT>(k0.x, k0.y, b0);
+      gch_terms<NT>(k1.x, k1.y, b1);
+      gch_mma_terms<NT, NT>(near, qf, b0, b1);
     }
     const float2 d0 = *reinterpret_cast<const float2*>(tot + i0 * dim + kk + cp);
     const float2 d1 = *reinterpret_cast<const float2*>(tot + i0 * dim + kk + cp + 8);
     q1.x *= d0.x, q1.y *= d0.y;
     q3.x *= d1.x, q3.y *= d1.y;
-    gch_split(q0.x, q0.y, ah[0], al[0]);
-    gch_split(q1.x, q1.y, ah[1], al[1]);
-    gch_split(q2.x, q2.y, ah[2], al[2]);
-    gch_split(q3.x, q3.y, ah[3], al[3]);
+    gch_terms<NT>(q0.x, q0.y, q[0]);
+    gch_terms<NT>(q1.x, q1.y, q[1]);
+    gch_terms<NT>(q2.x, q2.y, q[2]);
+    gch_terms<NT>(q3.x, q3.y, q[3]);
+    fragments();
     float2 f0 = make_float2(1.f, 1.f), f1 = f0;  // the decays between stretch j's end and stretch i0's start
 #pragma unroll
     for (int jj = 0; jj < GCH_SUBS - 2; ++jj) {
@@ -365,11 +413,9 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
       if (j < i0) {
         const float2 k0 = *reinterpret_cast<const float2*>(kq + (j * 8 + g) * ks + kk + cp);
         const float2 k1 = *reinterpret_cast<const float2*>(kq + (j * 8 + g) * ks + kk + cp + 8);
-        gch_split(k0.x * f0.x, k0.y * f0.y, bh[0], bl[0]);
-        gch_split(k1.x * f1.x, k1.y * f1.y, bh[1], bl[1]);
-        gch_mma(acc[j], ah, bh[0], bh[1]);
-        gch_mma(acc[j], ah, bl[0], bl[1]);
-        gch_mma(acc[j], al, bh[0], bh[1]);
+        gch_terms<NT>(k0.x * f0.x, k0.y * f0.y, b0);
+        gch_terms<NT>(k1.x * f1.x, k1.y * f1.y, b1);
+        gch_mma_terms<NT, NT>(acc[j], qf, b0, b1);
         const float2 e0 = *reinterpret_cast<const float2*>(tot + j * dim + kk + cp);
         const float2 e1 = *reinterpret_cast<const float2*>(tot + j * dim + kk + cp + 8);
         f0.x *= e0.x, f0.y *= e0.y;
@@ -406,20 +452,23 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
       if (s <= warp) {
-        unsigned ah[4], al[4];
-        gch_split(acc[2 * s][0], acc[2 * s][1], ah[0], al[0]);
-        gch_split(acc[2 * s][2], acc[2 * s][3], ah[1], al[1]);
-        gch_split(acc[2 * s + 1][0], acc[2 * s + 1][1], ah[2], al[2]);
-        gch_split(acc[2 * s + 1][2], acc[2 * s + 1][3], ah[3], al[3]);
+        unsigned p[4][NT], a[NT][4];
+        gch_terms<NT>(acc[2 * s][0], acc[2 * s][1], p[0]);
+        gch_terms<NT>(acc[2 * s][2], acc[2 * s][3], p[1]);
+        gch_terms<NT>(acc[2 * s + 1][0], acc[2 * s + 1][1], p[2]);
+        gch_terms<NT>(acc[2 * s + 1][2], acc[2 * s + 1][3], p[3]);
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[i][e] = p[e][i];
 #pragma unroll
         for (int n = 0; n < 8; n += 2) {
           if (n < nt) {
             unsigned b[4];
             gch_ldsm4t(b, v_s + (s * 16 + (mat & 1) * 8 + (lane & 7)) * (vn + 8) + n0 + n * 8 + (mat >> 1) * 8);
-            gch_mma(y[n], ah, b[0], b[1]);
-            gch_mma(y[n + 1], ah, b[2], b[3]);
-            gch_mma(y[n], al, b[0], b[1]);
-            gch_mma(y[n + 1], al, b[2], b[3]);
+            const unsigned l0[1] = {b[0]}, l1[1] = {b[1]}, r0[1] = {b[2]}, r1[1] = {b[3]};
+            gch_mma_terms<NT, 1>(y[n], a, l0, l1);
+            gch_mma_terms<NT, 1>(y[n + 1], a, r0, r1);
           }
         }
       }
@@ -428,8 +477,8 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
       const float* r_lo = rp + (warp * 16 + g) * ks + kk + cp;
       const float2 q0 = *reinterpret_cast<const float2*>(r_lo), q1 = *reinterpret_cast<const float2*>(r_lo + 8 * ks),
                    q2 = *reinterpret_cast<const float2*>(r_lo + 8), q3 = *reinterpret_cast<const float2*>(r_lo + 8 * ks + 8);
-      unsigned ah[4], al[4];
-      uint2 x0[8], x1[8];  // (rounded pair, pair of rests)
+      unsigned p[4][NT], a[NT][4];
+      uint2 x0[8], x1[8];  // two terms: (rounded pair, pair of rests); three: the pair itself
       const float* sp = st + (long long)(n0 + g) * dim + kk + cp;
 #pragma unroll
       for (int n = 0; n < 8; ++n)
@@ -437,16 +486,26 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
           x0[n] = *reinterpret_cast<const uint2*>(sp + (long long)n * 8 * dim);
           x1[n] = *reinterpret_cast<const uint2*>(sp + (long long)n * 8 * dim + 8);
         }
-      gch_split(q0.x, q0.y, ah[0], al[0]);
-      gch_split(q1.x, q1.y, ah[1], al[1]);
-      gch_split(q2.x, q2.y, ah[2], al[2]);
-      gch_split(q3.x, q3.y, ah[3], al[3]);
+      gch_terms<NT>(q0.x, q0.y, p[0]);
+      gch_terms<NT>(q1.x, q1.y, p[1]);
+      gch_terms<NT>(q2.x, q2.y, p[2]);
+      gch_terms<NT>(q3.x, q3.y, p[3]);
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a[i][e] = p[e][i];
 #pragma unroll
       for (int n = 0; n < 8; ++n)
         if (n < nt) {
-          gch_mma(y[n], ah, x0[n].x, x1[n].x);
-          gch_mma(y[n], ah, x0[n].y, x1[n].y);
-          gch_mma(y[n], al, x0[n].x, x1[n].x);
+          unsigned b0[NT], b1[NT];
+          if (NT == 2) {
+            b0[0] = x0[n].x, b0[1] = x0[n].y;
+            b1[0] = x1[n].x, b1[1] = x1[n].y;
+          } else {
+            gch_terms<NT>(__uint_as_float(x0[n].x), __uint_as_float(x0[n].y), b0);
+            gch_terms<NT>(__uint_as_float(x1[n].x), __uint_as_float(x1[n].y), b1);
+          }
+          gch_mma_terms<NT, NT>(y[n], a, b0, b1);
         }
     }
 #pragma unroll
@@ -525,26 +584,30 @@ extern "C" int ullm_gla_chunk(const void* qkv, long long row_stride, int q_off, 
   const int tiles = ullm_gla_chunk_tiles(tokens, requests);
   float* fold = scratch;
   float* total = scratch + (long long)tiles * heads * dim * vdim;
-  static size_t fold_smem = 48 * 1024, out_smem[2] = {48 * 1024, 48 * 1024};
+  static size_t fold_smem[2] = {48 * 1024, 48 * 1024}, out_smem[2] = {48 * 1024, 48 * 1024};
   const int v_tile = gch_v_tile(dim, vdim);
   const size_t fs = gch_fold_smem(dim, vdim), os = gch_out_smem(dim, v_tile);
-  int rc = gch_allow(gla_fold_kernel, fs, &fold_smem);
+  const bool two = bonus != nullptr;  // terms of a 32-bit operand, else three
+  int rc = two ? gch_allow(gla_fold_kernel<2>, fs, &fold_smem[0]) : gch_allow(gla_fold_kernel<3>, fs, &fold_smem[1]);
   if (rc != ULLM_OK) return rc;
-  rc = bonus != nullptr ? gch_allow(gla_out_kernel<true>, os, &out_smem[0]) : gch_allow(gla_out_kernel<false>, os, &out_smem[1]);
+  rc = two ? gch_allow(gla_out_kernel<true>, os, &out_smem[0]) : gch_allow(gla_out_kernel<false>, os, &out_smem[1]);
   if (rc != ULLM_OK) return rc;
   const dim3 grid(tiles, heads), out_grid(tiles, heads, (vdim + v_tile - 1) / v_tile), block(GCH_THREADS);
-  rc = ullm_launch_kernel(gla_fold_kernel, grid, block, fs, st, (const __nv_bfloat16*)qkv, row_stride, k_off, v_off, decay,
-                          decay_stride, cu_q, token_req, requests, least, heads, dim, vdim, fold, total);
-  if (rc != ULLM_OK) return rc;
-  rc = ullm_launch_kernel(gla_scan_kernel, dim3((dim * vdim / 2 + 127) / 128, heads, requests), dim3(128), 0, st, fold,
-                          (const float*)total, state, state_stride, cu_q, req_slots, token_req, least, heads, dim, vdim,
-                          num_slots, status);
-  if (rc != ULLM_OK) return rc;
-  if (bonus != nullptr)
-    return ullm_launch_kernel(gla_out_kernel<true>, out_grid, block, os, st, (const __nv_bfloat16*)qkv, row_stride, q_off, k_off,
-                              v_off, decay, decay_stride, bonus, q_scale, cu_q, token_req, requests, least, heads, dim, vdim,
-                              v_tile, (const float*)fold, out);
-  return ullm_launch_kernel(gla_out_kernel<false>, out_grid, block, os, st, (const __nv_bfloat16*)qkv, row_stride, q_off, k_off,
-                            v_off, decay, decay_stride, bonus, q_scale, cu_q, token_req, requests, least, heads, dim, vdim,
-                            v_tile, (const float*)fold, out);
+  const dim3 scan_grid((dim * vdim / 2 + 127) / 128, heads, requests);
+  const __nv_bfloat16* x = (const __nv_bfloat16*)qkv;
+#define GCH_GO(NT)                                                                                                             \
+  rc = ullm_launch_kernel(gla_fold_kernel<NT>, grid, block, fs, st, x, row_stride, k_off, v_off, decay, decay_stride, cu_q,     \
+                          token_req, requests, least, heads, dim, vdim, fold, total);                                           \
+  if (rc != ULLM_OK) return rc;                                                                                                 \
+  rc = ullm_launch_kernel(gla_scan_kernel<NT == 2>, scan_grid, dim3(128), 0, st, fold, (const float*)total, state,              \
+                          state_stride, cu_q, req_slots, token_req, least, heads, dim, vdim, num_slots, status);                \
+  if (rc != ULLM_OK) return rc;                                                                                                 \
+  return ullm_launch_kernel(gla_out_kernel<NT == 2>, out_grid, block, os, st, x, row_stride, q_off, k_off, v_off, decay,        \
+                            decay_stride, bonus, q_scale, cu_q, token_req, requests, least, heads, dim, vdim, v_tile,           \
+                            (const float*)fold, out)
+  if (two) {
+    GCH_GO(2);
+  }
+  GCH_GO(3);
+#undef GCH_GO
 }
