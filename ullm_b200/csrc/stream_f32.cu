@@ -272,7 +272,7 @@ __global__ void sigmoid_gate_kernel(T* __restrict__ a, const T* __restrict__ g, 
 // stream += sigmoid(g1 + b1) * a + sigmoid(g2 + b2) * f.  g1 | g2 are the columns of ONE 32-bit product
 // (row stride `g_stride`); f, g2 and b2 are absent for a layer without the second sub-layer.
 // VEC neighbouring columns per thread and turn (two sub-layers of 2,048 x 2,048 in bfloat16, 92 MB with cold caches: 40 us one
-// column at a time, 23 us in 16-byte pieces; in a step 29 and 13 us).
+// column at a time, 23 us in 16-byte pieces, in a step 29 and 13 us; 8 rows 12.4 and 8.2 us).
 template <typename T, int VEC>
 __global__ void gated_add_f32_kernel(const T* __restrict__ a, const T* __restrict__ f, const float* __restrict__ g,
                                      long long g_stride, const float* __restrict__ b1, const float* __restrict__ b2,
@@ -488,7 +488,8 @@ extern "C" int ullm_gated_add_f32(int dtype, const void* a, const void* f, const
   const uintptr_t floats = (uintptr_t)g | (uintptr_t)b1 | (uintptr_t)b2 | (uintptr_t)stream;
   const int piece = dtype == ULLM_DTYPE_F32 ? 4 : 8;
   const bool wide = cols % piece == 0 && g_stride % 4 == 0 && ((floats | (uintptr_t)a | (uintptr_t)f | (uintptr_t)copy) & 15) == 0;
-  const dim3 grid(rows), block(row_threads(wide ? cols / piece : cols));
+  const int pieces = (cols / piece + 31) / 32 * 32;  // a piece per thread: in a decode step a thread's pieces would follow one another
+  const dim3 grid(rows), block(wide ? (pieces < 512 ? pieces : 512) : row_threads(cols));
 #define GATED_GO(T, V)                                                                                                          \
   return ullm_launch_kernel(gated_add_f32_kernel<T, V>, grid, block, 0, st, (const T*)a, (const T*)f, g, g_stride, b1, b2, stream, \
                             (T*)copy, cols)
