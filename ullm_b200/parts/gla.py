@@ -81,9 +81,10 @@ class GatedLinearAttention(Mixer):
         return StateNeed((gla_state_floats(self.num_heads, self.head_dim, self.value_dim),), torch.float32)
 
     def activation_elems(self):
-        # the input product, z and o in 32-bit (two elements' worth each in a 16-bit engine), the gated o, the output
+        # the input product, z and o in 32-bit (two elements' worth each in a 16-bit engine), the gated o, the output, a 64th of
+        # the chunked form's states
         return (2 * self.qk_size + 2 * self.v_size + self.decay_rank + 2 * self.qk_size + 3 * self.v_size
-                + self.hidden_size)
+                + self.hidden_size + self.num_heads * self.head_dim * (self.value_dim + 1) // 32)
 
     def forward(self, x, ctx, cache):
         K = kernels()
