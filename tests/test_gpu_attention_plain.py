@@ -10,8 +10,8 @@ from test_gpu_kernels import K, attention_reference, close, rnd
 pytestmark = [pytest.mark.gpu, pytest.mark.needs_cuda]
 
 
-def case(dtype, Hq, Hkv, D, page, q_lens, kv_lens, pad=0):
-    B, T = len(q_lens), sum(q_lens)
+def case(dtype, Hq, Hkv, D, page, q_lens, kv_lens, pad=0, behind=0):
+    B, T = len(q_lens), sum(q_lens) + behind
     max_pages = max(-(-k // page) for k in kv_lens) + 1
     g = torch.Generator().manual_seed(21)
     pages = sum(-(-k // page) for k in kv_lens) + 2
@@ -26,7 +26,8 @@ def case(dtype, Hq, Hkv, D, page, q_lens, kv_lens, pad=0):
     kp, vp = rnd(pages, page, Hkv, D, seed=22, dtype=dtype), rnd(pages, page, Hkv, D, seed=23, dtype=dtype)
     qkv = rnd(T, (Hq + 2 * Hkv) * D + pad, seed=24, dtype=dtype)
     cu = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32).cuda()
-    req = torch.cat([torch.full((n,), r, dtype=torch.int32) for r, n in enumerate(q_lens)]).cuda()
+    req = torch.cat([torch.full((n,), r, dtype=torch.int32) for r, n in enumerate(q_lens)]
+                    + [torch.full((behind,), -1, dtype=torch.int32)]).cuda()
     return dict(qkv=qkv, kp=kp, vp=vp, bt=bt, slots=slots, cu=cu, req=req, q_lens=q_lens, kv_lens=kv_lens, T=T)
 
 
@@ -79,3 +80,25 @@ def test_padding_rows_are_zeros():
     c["req"][1] = -1
     out = run(c, 4, 2, 64, 16, 0, 0.125)
     assert torch.count_nonzero(out[1]) == 0 and torch.isfinite(out).all() and (out[[0, 2]] != 7.0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("Hq,Hkv,D", [(4, 2, 64), (16, 1, 128)])
+@pytest.mark.parametrize("q_lens,behind", [([0, 2], 0), ([0, 0, 2], 0), ([2, 0, 1], 0), ([1, 0, 0, 70], 0), ([1, 0], 1), ([1], 1), ([1, 1], 40),
+                                           ([33, 1], 3), ([32, 32], 32), ([0, 0], 2)])
+def test_requests_without_tokens_and_rows_behind_the_last(dtype, Hq, Hkv, D, q_lens, behind):
+    """A batch row may bring no token, whatever the rows and requests count, and rows behind the last request's are zeros: as the
+    general kernel has it."""
+    c = case(dtype, Hq, Hkv, D, 16, q_lens, [n + 19 for n in q_lens], behind=behind)
+    out, general = run(c, Hq, Hkv, D, 16, 0, D ** -0.5), run(c, Hq, Hkv, D, 16, 0, D ** -0.5, on=False)
+    # (as above: 32-bit sums in another order, a last place of float16)
+    assert (out.float() - general.float()).abs().max() < (4e-5 if dtype == torch.float32 else 4e-3)
+    assert torch.count_nonzero(out[c["T"] - behind:]) == 0
+
+
+def test_rows_of_a_portion_that_belong_to_no_request_or_lie_in_front_of_its_first_position():
+    """Rows marked as padding inside a portion, and rows whose position would be negative, are zeros in both kernels."""
+    c = case(torch.float32, 4, 2, 64, 16, [40, 12], [40, 12])
+    c["req"][3], c["req"][37], c["kv_lens"] = -1, -1, [40, 7]
+    out, general = run(c, 4, 2, 64, 16, 0, 0.125), run(c, 4, 2, 64, 16, 0, 0.125, on=False)
+    assert torch.count_nonzero(general[[3, 37, 40, 44]]) == 0 and (out - general).abs().max() < 4e-5

@@ -57,7 +57,7 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
                               const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                               const int* __restrict__ block_table, int max_pages, const int* __restrict__ req_slots,
                               const int* __restrict__ cu_q, const int* __restrict__ kv_len, const int* __restrict__ token_req,
-                              int requests, int num_q, int num_kv, int page_size, int window, float scale,
+                              int tokens, int requests, int num_q, int num_kv, int page_size, int window, float scale,
                               long long num_pages, int* status) {
   constexpr int ST = D + PT_PAD;
   constexpr int CV = D / 64;  // groups of four output columns a thread owns
@@ -70,7 +70,7 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
   pdl_launch_dependents();
   pdl_wait();
   const int gq = num_q / num_kv, per = PT_ROWS / gq;  // query heads per kv head; tokens of a row tile
-  // which request and which of its row tiles (requests of one token are the other kernel's)
+  // which request and which of its row tiles (requests of one token are the other kernel's, requests of none have no rows)
   int r = 0, tile = blockIdx.x, t0 = 0, n = 0;
   for (; r < requests; ++r) {
     t0 = cu_q[r];
@@ -83,13 +83,17 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
     }
     tile -= tiles;
   }
-  if (r >= requests) return;
   const int kh = blockIdx.y, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  if (r >= requests) {  // (at least one block is left over: rows behind the last request's are padding, and zeros)
+    const int spare = (int)gridDim.x - ((int)blockIdx.x - tile);
+    for (int t = cu_q[requests] + tile; t < tokens; t += spare)
+      for (int e = tid; e < gq * D; e += PT_THREADS) out[((long long)t * num_q + kh * gq) * D + e] = from_f32<T>(0.f);
+    return;
+  }
   const int row0 = tile * per, rows = min(per, n - row0) * gq;  // row i: token row0 + i / gq, query head i % gq
   const int kvl = kv_len[r];
-  const bool live = token_req[t0] >= 0 && kvl >= n;
   const int pos0 = kvl - n + row0;
-  if (!live) {
+  if (!__syncthreads_or(tid * gq < rows && token_req[t0 + row0 + tid] >= 0 && kvl > 0)) {
     for (int i = tid; i < rows * D; i += PT_THREADS) {
       const int row = i / D, e = i - row * D;
       out[(long long)(t0 + row0 + row / gq) * num_q * D + (long long)(kh * gq + row % gq) * D + e] = from_f32<T>(0.f);
@@ -121,7 +125,7 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
   const int* bt = block_table + (long long)req_slots[r] * max_pages;
   const long long kv_row = (long long)num_kv * D;
   const int last = pos0 + (rows - 1) / gq;
-  for (int base = first_seen(pos0, window); base <= last; base += PT_KEYS) {
+  for (int base = max(0, first_seen(pos0, window)); base <= last; base += PT_KEYS) {
     __syncthreads();  // (the tile before has been read; Q is in place)
     if (tid < PT_KEYS) {
       const int key = base + tid;
@@ -223,10 +227,12 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
     const int row = ty * 4 + i;
     if (row >= rows) continue;
     const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
+    const bool padding = token_req[t0 + row0 + row / gq] < 0;
     T* dst = out + (long long)(t0 + row0 + row / gq) * num_q * D + (long long)(kh * gq + row % gq) * D + tx * 4;
 #pragma unroll
     for (int c = 0; c < CV; ++c)
-      pl_store4(dst + c * 64, make_float4(o[i][c].x * inv, o[i][c].y * inv, o[i][c].z * inv, o[i][c].w * inv));
+      pl_store4(dst + c * 64, padding ? make_float4(0.f, 0.f, 0.f, 0.f)
+                                      : make_float4(o[i][c].x * inv, o[i][c].y * inv, o[i][c].z * inv, o[i][c].w * inv));
   }
 }
 
@@ -364,10 +370,10 @@ plain_attention_decode_kernel(const T* __restrict__ q, long long q_row_stride, T
 template <typename T, int D>
 static int plain_launch(const void* q, long long q_row_stride, void* out, const void* k_cache, const void* v_cache,
                         const int* block_table, int max_pages, const int* req_slots, const int* cu_q, const int* kv_len,
-                        const int* token_req, int tokens, int requests, int num_q, int num_kv, int page_size, int window,
-                        float scale, long long num_pages, int* status, cudaStream_t st) {
+                        const int* token_req, int tokens, int requests, int longest, int num_q, int num_kv, int page_size,
+                        int window, float scale, long long num_pages, int* status, cudaStream_t st) {
   const int gq = num_q / num_kv;
-  if (tokens > requests) {  // (some request brings more than one token)
+  if (longest != 1 || tokens != requests) {  // (as many rows as requests alone says nothing: a request may bring none)
     constexpr int ST = D + PT_PAD;
     constexpr size_t smem = ((size_t)(PT_ROWS + 2 * PT_KEYS) * ST + (size_t)PT_ROWS * PT_PS) * sizeof(float);
     static bool allowed = false;
@@ -380,13 +386,13 @@ static int plain_launch(const void* q, long long q_row_stride, void* out, const 
       allowed = true;
     }
     const int per = PT_ROWS / gq;
-    const long long tiles = tokens / per + requests;
+    const long long tiles = tokens / per + requests + 1;  // (one more than the requests' tiles can be)
     if (tiles > 0x7fffffffLL) return ULLM_ERR_BAD_SIZE;
     const int rc = ullm_launch_kernel(plain_attention_prompt_kernel<T, D>, dim3((int)tiles, num_kv), dim3(PT_THREADS), smem, st,
                                       (const T*)q, q_row_stride, (T*)out, (const T*)k_cache, (const T*)v_cache, block_table,
-                                      max_pages, req_slots, cu_q, kv_len, token_req, requests, num_q, num_kv, page_size, window,
-                                      scale, num_pages, status);
-    if (rc != ULLM_OK || requests == 1) return rc;
+                                      max_pages, req_slots, cu_q, kv_len, token_req, tokens, requests, num_q, num_kv, page_size,
+                                      window, scale, num_pages, status);
+    if (rc != ULLM_OK || requests == 0 || (requests == 1 && longest > 1)) return rc;
   }
 #define PD_GO(GQ)                                                                                                        \
   return ullm_launch_kernel(plain_attention_decode_kernel<T, D, GQ>, dim3(requests, num_kv, gq / GQ), dim3(PD_WARPS * 32), \
@@ -406,22 +412,23 @@ extern "C" int ullm_attention_plain_supported(int dtype, int head_dim, int num_q
          num_q % num_kv == 0 && num_q / num_kv >= 1 && num_q / num_kv <= PT_ROWS && num_kv <= 65535;
 }
 
-// Arguments as `ullm_paged_attention_generic`, and the number of requests (cu_q holds one more entry).  UNSUPPORTED where the
-// rows do not allow 16-byte (float16: 8-byte) reads.
+// Arguments as `ullm_paged_attention_generic`, the number of requests (cu_q holds one more entry) and how many tokens the longest
+// of them brings (0: not known; a step of which all requests are known to bring one token saves a launch).  UNSUPPORTED where
+// the rows do not allow 16-byte (float16: 8-byte) reads.
 extern "C" int ullm_attention_plain(int dtype, const void* q, long long q_row_stride, void* out, const void* k_cache,
                                     const void* v_cache, const int* block_table, int max_pages, const int* req_slots,
                                     const int* cu_q, const int* kv_len, const int* token_req, int tokens, int requests,
-                                    int num_q, int num_kv, int head_dim, int page_size, int window, float scale,
+                                    int longest, int num_q, int num_kv, int head_dim, int page_size, int window, float scale,
                                     long long num_pages, int* status, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
-  if (tokens < 0 || requests < 0 || page_size <= 0 || max_pages <= 0) return ULLM_ERR_BAD_SIZE;
+  if (tokens < 0 || requests < 0 || longest < 0 || page_size <= 0 || max_pages <= 0) return ULLM_ERR_BAD_SIZE;
   if (!ullm_attention_plain_supported(dtype, head_dim, num_q, num_kv) || q_row_stride % 4) return ULLM_ERR_UNSUPPORTED;
   const uintptr_t align = dtype == ULLM_DTYPE_F32 ? 15 : 7;
   if (((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_cache | (uintptr_t)v_cache) & align) return ULLM_ERR_UNSUPPORTED;
-  if (tokens == 0 || requests == 0) return ULLM_OK;
+  if (tokens == 0) return ULLM_OK;
 #define PL_GO(T, D)                                                                                                       \
   return plain_launch<T, D>(q, q_row_stride, out, k_cache, v_cache, block_table, max_pages, req_slots, cu_q, kv_len,       \
-                            token_req, tokens, requests, num_q, num_kv, page_size, window, scale, num_pages, status, st)
+                            token_req, tokens, requests, longest, num_q, num_kv, page_size, window, scale, num_pages, status, st)
   if (dtype == ULLM_DTYPE_F32) {
     if (head_dim == 64) PL_GO(float, 64);
     PL_GO(float, 128);

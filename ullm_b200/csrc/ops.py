@@ -261,7 +261,7 @@ class Kernels:
             "ullm_qk_norm_rope_store": [I, P, I, I, I, I, P, P, F, P, P, I, I, P, P, P, P, LL, P, P],
             "ullm_qk_norm_in_place": [I, P, I, I, I, I, P, P, F, P, P],
             "ullm_paged_attention_generic": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_attention_plain": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, F, LL, P, P],
+            "ullm_attention_plain": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, I, F, LL, P, P],
             "ullm_attention_plain_supported": [I, I, I, I],
             "ullm_decode_attention": [P, LL, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, I, LL, P, P],
             "ullm_decode_attention_balanced": [P, LL, P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, F, LL, P, P],
@@ -2568,8 +2568,8 @@ class Kernels:
         if self.plain_attention_on and self.lib.ullm_attention_plain_supported(_DT[qkv.dtype], head_dim, num_q, num_kv):
             code = self.lib.ullm_attention_plain(
                 _DT[qkv.dtype], _ptr(qkv), qkv.stride(0), _ptr(out), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
-                block_table.shape[1], _ptr(req_slots), _ptr(cu_q), _ptr(kv_len), _ptr(token_req), T, cu_q.numel() - 1, num_q,
-                num_kv, head_dim, page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream())
+                block_table.shape[1], _ptr(req_slots), _ptr(cu_q), _ptr(kv_len), _ptr(token_req), T, cu_q.numel() - 1,
+                0 if ctx is None else ctx.max_q_len, num_q, num_kv, head_dim, page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream())
             if code != 4:  # (4: rows that do not start on the borders its reads need)
                 return self._check(code, f"attention_plain (head_dim {head_dim})")
         self._check(self.lib.ullm_paged_attention_generic(
