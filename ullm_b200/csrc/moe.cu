@@ -29,10 +29,17 @@
 
 #define MOE_MAX_TOP 32
 
-// The choices of token t, by one warp: its logits `z`, `g_rank` the warp's ranks of the groups (only with groups).
-__device__ __forceinline__ void moe_route_token(const float* z, const float* correction, int* choice, float* weight, int t,
-                                                int lane, float* g_rank, int experts, int top, int softmax_scores,
-                                                int renormalize, int groups, int keep, float scale, int always) {
+__global__ void moe_route_kernel(const float* __restrict__ logits, long long logits_stride,
+                                 const float* __restrict__ correction, int* __restrict__ choice,
+                                 float* __restrict__ weight, int tokens, int experts, int top, int softmax_scores,
+                                 int renormalize, int groups, int keep, float scale, int always) {
+  extern __shared__ float rt_smem[];  // per warp: a rank per group (only with groups)
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (t >= tokens) return;
+  const float* z = logits + (long long)t * logits_stride;
   float zmax = -INFINITY, zsum = 0.f;
   if (softmax_scores) {
     for (int e = lane; e < experts; e += 32) zmax = fmaxf(zmax, z[e]);
@@ -42,6 +49,7 @@ __device__ __forceinline__ void moe_route_token(const float* z, const float* cor
   }
   auto score_of = [&](int e) { return softmax_scores ? expf(z[e] - zmax) / zsum : 1.f / (1.f + expf(-z[e])); };
   // A chosen group's rank becomes +infinity; experts of all others are out.
+  float* g_rank = rt_smem + (threadIdx.x >> 5) * groups;
   const int per = experts / groups;
   const bool grouped = keep < groups;
   if (grouped) {
@@ -131,22 +139,13 @@ __device__ __forceinline__ void moe_route_token(const float* z, const float* cor
   }
 }
 
-__global__ void moe_route_kernel(const float* __restrict__ logits, long long logits_stride,
-                                 const float* __restrict__ correction, int* __restrict__ choice,
-                                 float* __restrict__ weight, int tokens, int experts, int top, int softmax_scores,
-                                 int renormalize, int groups, int keep, float scale, int always) {
-  extern __shared__ float rt_smem[];  // per warp: a rank per group (only with groups)
+// One block.  counts in shared memory (experts <= 1024).
+__global__ void moe_arrange_kernel(const int* __restrict__ choice, int pairs, int experts, int* __restrict__ offsets,
+                                   int* __restrict__ sorted, int* __restrict__ place) {
+  __shared__ int count[1024];
+  __shared__ int cursor[1024];
   pdl_launch_dependents();
   pdl_wait();
-  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (t >= tokens) return;
-  moe_route_token(logits + (long long)t * logits_stride, correction, choice, weight, t, threadIdx.x & 31,
-                  rt_smem + (threadIdx.x >> 5) * groups, experts, top, softmax_scores, renormalize, groups, keep, scale, always);
-}
-
-// The pairs grouped by expert, by one block; `count` and `cursor`: a number per expert in shared memory.
-__device__ __forceinline__ void moe_arrange_block(const int* choice, int pairs, int experts, int* offsets, int* sorted,
-                                                  int* place, int* count, int* cursor) {
   for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
   __syncthreads();
   for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
@@ -175,82 +174,6 @@ __device__ __forceinline__ void moe_arrange_block(const int* choice, int pairs, 
       place[p] = 0;  // (no expert's row: whoever combines must not find an index that was never written)
     }
   }
-}
-
-// One block.  counts in shared memory (experts <= 1024).
-__global__ void moe_arrange_kernel(const int* __restrict__ choice, int pairs, int experts, int* __restrict__ offsets,
-                                   int* __restrict__ sorted, int* __restrict__ place) {
-  __shared__ int count[1024];
-  __shared__ int cursor[1024];
-  pdl_launch_dependents();
-  pdl_wait();
-  moe_arrange_block(choice, pairs, experts, offsets, sorted, place, count, cursor);
-}
-
-// Router product, choices and arrangement of a step of few tokens (bfloat16 rows) as ONE launch: a cluster of MRS_BLOCKS blocks
-// deals the router's rows over its warps, meets, and its first block routes and arranges.  Bound by latency: the three kernels
-// it replaces take 5 to 6 us each in a decode step, most of it launch, first loads and the way of their results to the next.
-// The router's rows (and the correction) are brought into L2 before the kernel in front has finished; behind that a block needs
-// the tokens' rows (32 to 131 KB, in shared memory) and one round over its router rows.
-#define MRS_BLOCKS 8
-#define MRS_THREADS 256
-#define MRS_MAX_TOKENS 16
-
-__global__ void __cluster_dims__(MRS_BLOCKS, 1, 1) __launch_bounds__(MRS_THREADS)
-moe_router_small_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, const __nv_bfloat16* __restrict__ w_router,
-                        int rows, int cols, float* logits, const float* __restrict__ correction, int* choice, float* weight,
-                        int tokens, int experts, int top, int softmax_scores, int renormalize, int groups, int keep,
-                        float scale, int always, int arranged, int* offsets, int* sorted, int* place) {
-  extern __shared__ __align__(16) unsigned char mrs_smem[];
-  __shared__ int count[1024];
-  __shared__ int cursor[1024];
-  pdl_launch_dependents();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = blockIdx.x;
-  constexpr int WARPS = MRS_THREADS / 32;
-  for (int r = warp * MRS_BLOCKS + rank; r < rows; r += WARPS * MRS_BLOCKS)
-    for (int c = lane * 64; c < cols; c += 32 * 64)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(w_router + (long long)r * cols + c));
-  pdl_wait();
-  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(mrs_smem);            // [tokens][cols]
-  float* ranks = reinterpret_cast<float*>(mrs_smem + (size_t)tokens * cols * 2);  // [WARPS][groups]
-  const int pieces = cols >> 3;
-  for (int i = tid; i < tokens * pieces; i += MRS_THREADS) {
-    const int t = i / pieces, c = (i - t * pieces) << 3;
-    *reinterpret_cast<uint4*>(xs + t * cols + c) = *reinterpret_cast<const uint4*>(x + (long long)t * x_stride + c);
-  }
-  __syncthreads();
-  for (int r = warp * MRS_BLOCKS + rank; r < rows; r += WARPS * MRS_BLOCKS) {
-    float acc[MRS_MAX_TOKENS];
-#pragma unroll
-    for (int t = 0; t < MRS_MAX_TOKENS; ++t) acc[t] = 0.f;
-    for (int p = lane; p < pieces; p += 32) {
-      float w[8];
-      load_vec<__nv_bfloat16, 8>(w_router + (long long)r * cols + p * 8, w);
-#pragma unroll
-      for (int t = 0; t < MRS_MAX_TOKENS; ++t) {
-        if (t < tokens) {
-          float v[8];
-          load_vec<__nv_bfloat16, 8>(xs + t * cols + p * 8, v);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) acc[t] = fmaf(w[i], v[i], acc[t]);
-        }
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < MRS_MAX_TOKENS; ++t) {
-      if (t < tokens) {
-        const float s = warp_sum(acc[t]);
-        if (lane == 0) logits[(long long)t * rows + r] = s;
-      }
-    }
-  }
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  if (rank != 0) return;
-  for (int t = warp; t < tokens; t += WARPS)
-    moe_route_token(logits + (long long)t * rows, correction, choice, weight, t, lane, ranks + warp * groups, experts, top,
-                    softmax_scores, renormalize, groups, keep, scale, always);
-  __syncthreads();
-  moe_arrange_block(choice, tokens * (top + always), arranged, offsets, sorted, place, count, cursor);
 }
 
 #define MOE_BM 32
@@ -714,35 +637,6 @@ extern "C" int ullm_moe_arrange(const int* choice, int pairs, int experts, int* 
   if (experts > 1024) return ULLM_ERR_UNSUPPORTED;
   return ullm_launch_kernel(moe_arrange_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, choice, pairs, experts,
                             offsets, sorted, place);
-}
-
-// `logits` [tokens, rows] 32-bit = x . w_router^T, and from its first `experts` columns the choices and arrangement of
-// `ullm_moe_route` and `ullm_moe_arrange` (over `arranged` experts) in one launch: at most 16 tokens in bfloat16, rows on 16-byte
-// borders.  UNSUPPORTED for anything else.
-extern "C" int ullm_moe_router_small(const void* x, long long x_stride, const void* w_router, int rows, int cols, float* logits,
-                                     const float* correction, int* choice, float* weight, int tokens, int experts, int top,
-                                     int softmax_scores, int renormalize, int groups, int keep, float scale, int always,
-                                     int arranged, int* offsets, int* sorted, int* place, void* stream) {
-  if (tokens < 0 || rows <= 0 || cols <= 0 || experts <= 0 || experts > rows || top <= 0 || arranged <= 0) return ULLM_ERR_BAD_SIZE;
-  if (groups < 1 || keep < 1 || keep > groups || experts % groups || always < 0 || always > 32) return ULLM_ERR_BAD_SIZE;
-  if (top > keep * (experts / groups) || top > MOE_MAX_TOP || arranged > 1024 || tokens > MRS_MAX_TOKENS || cols % 8 || x_stride % 8 ||
-      (((uintptr_t)x | (uintptr_t)w_router) & 15))
-    return ULLM_ERR_UNSUPPORTED;
-  const size_t smem = (size_t)tokens * cols * 2 + (size_t)(MRS_THREADS / 32) * groups * sizeof(float);
-  if (smem > 200 * 1024) return ULLM_ERR_UNSUPPORTED;
-  if (tokens == 0) return ULLM_OK;
-  static size_t have = 39 * 1024;  // (with the static arrays, what a kernel gets unasked)
-  if (smem > have) {
-    if (cudaFuncSetAttribute(moe_router_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      cudaGetLastError();
-      return ULLM_ERR_LAUNCH;
-    }
-    have = smem;
-  }
-  return ullm_launch_kernel(moe_router_small_kernel, dim3(MRS_BLOCKS), dim3(MRS_THREADS), smem, (cudaStream_t)stream,
-                            (const __nv_bfloat16*)x, x_stride, (const __nv_bfloat16*)w_router, rows, cols, logits, correction,
-                            choice, weight, tokens, experts, top, softmax_scores, renormalize, groups, keep, scale, always,
-                            arranged, offsets, sorted, place);
 }
 
 template <typename T>

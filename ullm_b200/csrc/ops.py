@@ -344,7 +344,6 @@ class Kernels:
             "ullm_linear_stream_grouped": [P, P, P, I, I, I, I, I, P, P],
             "ullm_head_norm_gate": [I, P, P, LL, P, P, I, I, I, F, I, I, P],
             "ullm_moe_route": [P, LL, P, P, P, I, I, I, I, I, I, I, F, I, P],
-            "ullm_moe_router_small": [P, LL, P, I, I, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P, P, P],
             "ullm_moe_arrange": [P, I, I, P, P, P, P],
             "ullm_moe_grouped_linear": [I, P, LL, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P],
             "ullm_moe_stream": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, P],
@@ -2024,38 +2023,6 @@ class Kernels:
                                             E, top, int(softmax_scores), int(renormalize), int(groups), int(keep),
                                             float(scale), int(always), _stream()),
                     f"moe_route ({E} experts, top {top})")
-
-    @_timed("moe", skipped=True)
-    def moe_router_small(self, x, w_router, logits, choice, weight, top: int, softmax_scores: bool, renormalize: bool,
-                         correction, experts: int, groups: int, keep: int, scale: float, always: int, arranged: int, offsets,
-                         sorted_pairs, place) -> bool:
-        """`linear_f32_out(x, w_router, logits)`, `moe_route` over the first `experts` columns and `moe_arrange` over `arranged`
-        experts as ONE launch for the steps whose products are all the weight-streaming kernel (bfloat16, at most 16 rows).
-        False for any other step (nothing has run)."""
-        T, H = x.shape
-        if (self.small_m_mode != "auto" or x.dtype != torch.bfloat16 or T > min(self.stream_all_rows, 16)
-                or w_router.dtype != torch.bfloat16 or not w_router.is_contiguous() or x.stride(1) != 1):
-            return False
-        _need(logits, "router logits", torch.float32)
-        _need(weight, "weight", torch.float32)
-        for t_, n_ in ((choice, "choice"), (offsets, "offsets"), (sorted_pairs, "sorted"), (place, "place")):
-            _need(t_, n_, torch.int32)
-        pairs = T * (top + always)
-        if (w_router.shape[1] != H or logits.shape != (T, w_router.shape[0]) or choice.numel() < pairs or weight.numel() < pairs
-                or offsets.numel() < arranged + 1 or sorted_pairs.numel() < pairs or place.numel() < pairs):
-            raise KernelError(f"moe_router_small: x {tuple(x.shape)}, router {tuple(w_router.shape)}, logits {tuple(logits.shape)}")
-        if correction is not None:
-            _need(correction, "correction", torch.float32)
-            if correction.numel() != experts:
-                raise KernelError(f"moe_router_small: {correction.numel()} corrections for {experts} router outputs")
-        code = self.lib.ullm_moe_router_small(
-            _ptr(x), x.stride(0), _ptr(w_router), w_router.shape[0], H, _ptr(logits), _ptr(correction), _ptr(choice), _ptr(weight),
-            T, experts, top, int(softmax_scores), int(renormalize), int(groups), int(keep), float(scale), int(always),
-            int(arranged), _ptr(offsets), _ptr(sorted_pairs), _ptr(place), _stream())
-        if code == 4:
-            return False
-        self._check(code, f"moe_router_small ({experts} experts, top {top})")
-        return True
 
     @_timed("moe")
     def moe_arrange(self, choice, pairs: int, experts: int, offsets, sorted_pairs, place):

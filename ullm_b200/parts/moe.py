@@ -158,19 +158,16 @@ class RoutedExperts(FeedForward):
         top, E = self.top + always, self.E + always
         ws = ctx.workspace
         logits = ws.tokens("moe.logits", T, self.w_router.shape[0], torch.float32)
+        K.linear_f32_out(x, self.w_router, logits)
         choice = ws.tokens("moe.choice", T, top, torch.int32)
         weight = ws.tokens("moe.weight", T, top, torch.float32)
+        K.moe_route(logits, choice, weight, self.top, self.scores == "softmax", self.renormalize,
+                    correction=self.w_correction, experts=self.R, groups=self.groups, keep=self.keep,
+                    scale=self.weight_scale, always=always)
         offsets = ws.get("moe.offsets", 1, E + 1, torch.int32)
         order = ws.tokens("moe.sorted", T, top, torch.int32)
         place = ws.tokens("moe.place", T, top, torch.int32)
-        if not (x.is_cuda and K.moe_router_small(x, self.w_router, logits, choice, weight, self.top, self.scores == "softmax",
-                                                 self.renormalize, self.w_correction, self.R, self.groups, self.keep,
-                                                 self.weight_scale, always, E, offsets, order, place)):
-            K.linear_f32_out(x, self.w_router, logits)
-            K.moe_route(logits, choice, weight, self.top, self.scores == "softmax", self.renormalize,
-                        correction=self.w_correction, experts=self.R, groups=self.groups, keep=self.keep,
-                        scale=self.weight_scale, always=always)
-            K.moe_arrange(choice, T * top, E, offsets, order, place)
+        K.moe_arrange(choice, T * top, E, offsets, order, place)
         act = ws.tokens("moe.act", T * top, self.I, x.dtype) if top == 1 else ws.get("moe.act", T * top, self.I, x.dtype, reserve=ws.max_tokens * top)
         rows = ws.tokens("moe.rows", T * top, self.H, x.dtype) if top == 1 else ws.get("moe.rows", T * top, self.H, x.dtype, reserve=ws.max_tokens * top)
         on_input = self.weight_on == "input"
