@@ -57,7 +57,7 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
                               const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                               const int* __restrict__ block_table, int max_pages, const int* __restrict__ req_slots,
                               const int* __restrict__ cu_q, const int* __restrict__ kv_len, const int* __restrict__ token_req,
-                              int tokens, int requests, int num_q, int num_kv, int page_size, int window, float scale,
+                              int requests, int num_q, int num_kv, int page_size, int window, float scale,
                               long long num_pages, int* status) {
   constexpr int ST = D + PT_PAD;
   constexpr int CV = D / 64;  // groups of four output columns a thread owns
@@ -83,13 +83,8 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
     }
     tile -= tiles;
   }
+  if (r >= requests) return;
   const int kh = blockIdx.y, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  if (r >= requests) {  // (at least one block is left over: rows behind the last request's are padding, and zeros)
-    const int spare = (int)gridDim.x - ((int)blockIdx.x - tile);
-    for (int t = cu_q[requests] + tile; t < tokens; t += spare)
-      for (int e = tid; e < gq * D; e += PT_THREADS) out[((long long)t * num_q + kh * gq) * D + e] = from_f32<T>(0.f);
-    return;
-  }
   const int row0 = tile * per, rows = min(per, n - row0) * gq;  // row i: token row0 + i / gq, query head i % gq
   const int kvl = kv_len[r];
   const int pos0 = kvl - n + row0;
@@ -246,8 +241,8 @@ plain_attention_decode_kernel(const T* __restrict__ q, long long q_row_stride, T
                               const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                               const int* __restrict__ block_table, int max_pages, const int* __restrict__ req_slots,
                               const int* __restrict__ cu_q, const int* __restrict__ kv_len, const int* __restrict__ token_req,
-                              int num_q, int num_kv, int page_size, int window, float scale, long long num_pages,
-                              int* status) {
+                              int tokens, int requests, int num_q, int num_kv, int page_size, int window, float scale,
+                              long long num_pages, int* status) {
   constexpr int P = D / 32;           // pieces of four channels a lane holds: 4 (lane % 8) + 32 i
   constexpr int U = GQ * P > 8 ? 1 : 2;  // keys of a group in flight, as far as the registers reach
   __shared__ float m_s[GQ][PD_GROUPS], l_s[GQ][PD_GROUPS];
@@ -255,6 +250,9 @@ plain_attention_decode_kernel(const T* __restrict__ q, long long q_row_stride, T
   pdl_launch_dependents();
   pdl_wait();
   const int r = blockIdx.x, kh = blockIdx.y, t = cu_q[r];
+  for (int x = cu_q[requests] + r; x < tokens; x += requests)  // (rows behind the last request's are padding, and zeros)
+    for (int e = threadIdx.x; e < GQ * D; e += PD_WARPS * 32)
+      out[((long long)x * num_q + kh * (num_q / num_kv) + blockIdx.z * GQ) * D + e] = from_f32<T>(0.f);
   if (cu_q[r + 1] - t != 1) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sub = lane & 7, group = tid >> 3;
   const int h0 = kh * (num_q / num_kv) + blockIdx.z * GQ;
@@ -386,19 +384,19 @@ static int plain_launch(const void* q, long long q_row_stride, void* out, const 
       allowed = true;
     }
     const int per = PT_ROWS / gq;
-    const long long tiles = tokens / per + requests + 1;  // (one more than the requests' tiles can be)
+    const long long tiles = tokens / per + requests;
     if (tiles > 0x7fffffffLL) return ULLM_ERR_BAD_SIZE;
     const int rc = ullm_launch_kernel(plain_attention_prompt_kernel<T, D>, dim3((int)tiles, num_kv), dim3(PT_THREADS), smem, st,
                                       (const T*)q, q_row_stride, (T*)out, (const T*)k_cache, (const T*)v_cache, block_table,
-                                      max_pages, req_slots, cu_q, kv_len, token_req, tokens, requests, num_q, num_kv, page_size,
-                                      window, scale, num_pages, status);
-    if (rc != ULLM_OK || requests == 0 || (requests == 1 && longest > 1)) return rc;
+                                      max_pages, req_slots, cu_q, kv_len, token_req, requests, num_q, num_kv, page_size, window,
+                                      scale, num_pages, status);
+    if (rc != ULLM_OK || (requests == 1 && longest > 1 && longest == tokens)) return rc;
   }
 #define PD_GO(GQ)                                                                                                        \
   return ullm_launch_kernel(plain_attention_decode_kernel<T, D, GQ>, dim3(requests, num_kv, gq / GQ), dim3(PD_WARPS * 32), \
                             0, st, (const T*)q, q_row_stride, (T*)out, (const T*)k_cache, (const T*)v_cache, block_table, \
-                            max_pages, req_slots, cu_q, kv_len, token_req, num_q, num_kv, page_size, window, scale,        \
-                            num_pages, status)
+                            max_pages, req_slots, cu_q, kv_len, token_req, tokens, requests, num_q, num_kv, page_size,     \
+                            window, scale, num_pages, status)
   if (gq % 4 == 0) PD_GO(4);
   if (gq % 2 == 0) PD_GO(2);
   PD_GO(1);
@@ -426,6 +424,9 @@ extern "C" int ullm_attention_plain(int dtype, const void* q, long long q_row_st
   const uintptr_t align = dtype == ULLM_DTYPE_F32 ? 15 : 7;
   if (((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_cache | (uintptr_t)v_cache) & align) return ULLM_ERR_UNSUPPORTED;
   if (tokens == 0) return ULLM_OK;
+  if (requests == 0)  // (all rows are padding)
+    return cudaMemsetAsync(out, 0, (size_t)tokens * num_q * head_dim * (dtype == ULLM_DTYPE_F32 ? 4 : 2), st) == cudaSuccess ? ULLM_OK
+                                                                                                                             : ULLM_ERR_LAUNCH;
 #define PL_GO(T, D)                                                                                                       \
   return plain_launch<T, D>(q, q_row_stride, out, k_cache, v_cache, block_table, max_pages, req_slots, cu_q, kv_len,       \
                             token_req, tokens, requests, longest, num_q, num_kv, page_size, window, scale, num_pages, status, st)
