@@ -102,3 +102,26 @@ def test_rows_of_a_portion_that_belong_to_no_request_or_lie_in_front_of_its_firs
     c["req"][3], c["req"][37], c["kv_lens"] = -1, -1, [40, 7]
     out, general = run(c, 4, 2, 64, 16, 0, 0.125), run(c, 4, 2, 64, 16, 0, 0.125, on=False)
     assert torch.count_nonzero(general[[3, 37, 40, 44]]) == 0 and (out - general).abs().max() < 4e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("window", [0, 33, -64])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_values_that_a_row_does_not_see_do_not_reach_it(dtype, window, value):
+    """An infinite or NaN value of a later token, or of one in front of a row's window, changes the rows that see it and no others."""
+    Hq, Hkv, D, q_lens, kv_lens = 4, 2, 64, [90, 1], [150, 140]
+    c = case(dtype, Hq, Hkv, D, 16, q_lens, kv_lens)
+    clean = run(c, Hq, Hkv, D, 16, window, D ** -0.5)
+    for at in (75, 90, 149):  # key positions of the first request, whose rows stand at 60 to 149
+        v = c["vp"].clone()
+        page = int(c["bt"][c["slots"][0], at // 16])
+        c["vp"][page, at % 16, 1, 3] = value
+        out, general = run(c, Hq, Hkv, D, 16, window, D ** -0.5), run(c, Hq, Hkv, D, 16, window, D ** -0.5, on=False)
+        pos = torch.arange(60, 150)
+        first = {0: 0 * pos, 33: (pos - 32).clamp(min=0), -64: pos - pos % 64}[window]
+        hit = torch.zeros(c["T"], Hq, D, dtype=torch.bool)
+        hit[:90, 2:, 3] = ((pos >= at) & (first <= at))[:, None]
+        hit = hit.view(c["T"], -1).cuda()
+        assert torch.equal(~torch.isfinite(out), hit) and torch.equal(~torch.isfinite(general), hit)
+        assert (out - clean)[~hit].abs().max() <= (2e-5 if dtype == torch.float32 else 2e-3)  # (sums in another order, see above)
+        c["vp"] = v

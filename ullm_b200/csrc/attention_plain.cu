@@ -51,6 +51,11 @@ __device__ __forceinline__ void pl_axpy(float p, const float4& v, float4& o) {
   o.w = fmaf(p, v.w, o.w);
 }
 
+// whether one of them is infinite or NaN
+__device__ __forceinline__ bool pl_odd(const float4& v) {
+  return fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, v.w * 0.f))) != 0.f;  // (a zero times either is NaN)
+}
+
 template <typename T, int D>
 __global__ void __launch_bounds__(PT_THREADS)
 plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T* __restrict__ out,
@@ -119,7 +124,7 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
   }
   const int* bt = block_table + (long long)req_slots[r] * max_pages;
   const long long kv_row = (long long)num_kv * D;
-  const int last = pos0 + (rows - 1) / gq;
+  const int last = pos0 + (rows - 1) / gq, first_last = first_seen(last, window);
   for (int base = max(0, first_seen(pos0, window)); base <= last; base += PT_KEYS) {
     __syncthreads();  // (the tile before has been read; Q is in place)
     if (tid < PT_KEYS) {
@@ -133,6 +138,10 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
       slot_s[tid] = slot;
     }
     __syncthreads();
+    // A weight of zero must not meet a value that a row does not see and that is infinite or NaN: tiles that some row sees a part
+    // of only are searched for such values as they are loaded.
+    const bool part = base + PT_KEYS - 1 > pos0 || base < first_last;
+    bool odd = false;
 #pragma unroll 4
     for (int i = tid; i < PT_KEYS * (D / 4); i += PT_THREADS) {
       const int key = i / (D / 4), e = (i - key * (D / 4)) * 4;
@@ -145,8 +154,10 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
       }
       *reinterpret_cast<float4*>(ks + key * ST + e) = a;
       *reinterpret_cast<float4*>(vs + key * ST + e) = b;
+      if (part) odd |= pl_odd(b);
     }
-    __syncthreads();
+    if (part) odd = __syncthreads_or(odd);
+    else __syncthreads();
     // scores of rows 4 ty .. + 3 against keys tx, tx + 16, tx + 32, tx + 48
     float s[4][4];
 #pragma unroll
@@ -196,6 +207,21 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
       for (int c = 0; c < CV; ++c) o[i][c].x *= keep, o[i][c].y *= keep, o[i][c].z *= keep, o[i][c].w *= keep;
     }
     __syncwarp();  // (a row's weights are written and read by the 16 lanes that own the row)
+    if (odd) {
+#pragma unroll 1
+      for (int key = 0; key < PT_KEYS; ++key) {
+        if (slot_s[key] < 0) continue;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (base + key < first[i] || base + key > pos[i]) continue;
+          const float p = ps[(ty * 4 + i) * PT_PS + key];
+#pragma unroll
+          for (int c = 0; c < CV; ++c) pl_axpy(p, *reinterpret_cast<const float4*>(vs + key * ST + c * 64 + tx * 4), o[i][c]);
+        }
+      }
+      __syncwarp();
+      continue;
+    }
 #pragma unroll 2
     for (int key = 0; key < PT_KEYS; key += 4) {
       float4 p[4];
