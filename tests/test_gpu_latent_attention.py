@@ -74,3 +74,34 @@ def test_latent_rows_match_the_reference(H, dk, dv, page, window, q_lens, kv_len
         assert path == "latent_tcgen05"
     if page in (8, 16, 32, 64) and not (kp.isnan().any()):
         assert (got.float() - run(False).float()).abs().max().item() <= 2 ** -6 * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("window", [0, 40, -64])
+def test_a_missing_page_is_reported_where_a_row_sees_it(window):
+    """A page that a row sees and the table does not hold is an error, as in the mma.sync kernel; one that only lies in a key tile
+    with seen keys is not."""
+    k, H, dk, dv, page, n, kv = K(), 16, 192, 128, 8, 20, 150  # positions 130 to 149; 40 positions: from 91 on, a stretch: from 128
+    first = {0: 0, 40: 91, -64: 128}[window]
+    kp, q = rnd(40, page, 1, dk, seed=42, dtype=torch.bfloat16), rnd(n, H * dk, seed=43, dtype=torch.bfloat16)
+    cu, lens, req = (torch.tensor(x, dtype=torch.int32).cuda() for x in ([0, n], [kv], [0] * n))
+    ctx = SimpleNamespace(decode_only=False, num_requests=1, max_kv_len=kv, cu_q_host=[0, n], shared={}, start_positions_host=[kv - n])
+
+    def run(gone, value, on):
+        bt = torch.arange(24, dtype=torch.int32).view(1, 24)
+        bt[0, gone] = value
+        k.latent_attention_on = on
+        try:
+            out = torch.zeros(n, H * dv, dtype=torch.bfloat16, device="cuda")
+            k.windowed_attention(q, out, kp, None, bt.cuda(), torch.zeros(1, dtype=torch.int32).cuda(), cu, lens, req, H, 1, dk, dv, page,
+                                 window, 0.07, num_requests=1, ctx=ctx)
+        finally:
+            k.latent_attention_on = True
+        k.raise_on_status()
+
+    for on in (True, False):
+        for value in (-1, 40):
+            for gone in {first // page, (first + 8) // page, 140 // page, (kv - 1) // page}:
+                with pytest.raises(Exception, match="page id out of range"):
+                    run(gone, value, on)
+            for gone in {max(0, first // page - 1)} if window else {}:
+                run(gone, value, on)

@@ -100,8 +100,9 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     }
     return;
   }
-  const int k_start = first_seen(p0, p.window) / LA_KEYS * LA_KEYS;
-  const int tiles = (p0 + ntok - 1 - k_start) / LA_KEYS + 1;
+  const int first_key = first_seen(p0, p.window), last_key = p0 + ntok - 1;  // what some row of the block sees
+  const int k_start = first_key / LA_KEYS * LA_KEYS;
+  const int tiles = (last_key - k_start) / LA_KEYS + 1;
   const int* bt = p.block_table + (long long)p.req_slots[r] * p.max_pages;
 
   if (tid == 0) {
@@ -135,10 +136,11 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       const int key = k_start + t * LA_KEYS + lane * p.page_size;
       int page = -1;
       if (lane < ppt && key < kvl) {
-        // (a tile may begin before the first key any row sees; pages there may have been given back: zero-filled and masked)
+        // A page that some row sees has to be there.  (A tile may begin before the first key any row sees; pages there may have
+        // been given back: zero-filled and masked.)
         page = bt[key / p.page_size];
-        if (page >= p.num_pages) {
-          ullm_report(p.status, ULLM_STATUS_PAGE, r, page);
+        if (page < 0 || page >= p.num_pages) {
+          if (key + p.page_size > first_key && key <= last_key) ullm_report(p.status, ULLM_STATUS_PAGE, r, page);
           page = -1;
         }
       }
