@@ -105,3 +105,27 @@ def test_a_missing_page_is_reported_where_a_row_sees_it(window):
                     run(gone, value, on)
             for gone in {max(0, first // page - 1)} if window else {}:
                 run(gone, value, on)
+
+
+def test_a_long_decoded_request_does_not_decide_the_kernel_of_a_short_portion():
+    """The kernel goes by the keys that the portions see, not by those of the decoded tokens in front of them."""
+    k, H, dk, dv, page = K(), 16, 192, 128, 16
+    q_lens, kv_lens = [1, 1, 1, 1, 24], [2500, 17, 900, 64, 40]
+    T, B = sum(q_lens), len(q_lens)
+    bt, used = torch.full((B, 160), -1, dtype=torch.int32), 0
+    for r, kl in enumerate(kv_lens):
+        n = -(-kl // page)
+        bt[r, :n] = torch.arange(used, used + n)
+        used += n
+    kp, q = rnd(used, page, 1, dk, seed=52, dtype=torch.bfloat16), rnd(T, H * dk, seed=53, dtype=torch.bfloat16)
+    cu = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32)
+    req = torch.cat([torch.full((n,), r, dtype=torch.int32) for r, n in enumerate(q_lens)]).cuda()
+    ctx = SimpleNamespace(decode_only=False, num_requests=B, max_kv_len=max(kv_lens), cu_q_host=cu.tolist(), shared={},
+                          start_positions_host=[a - b for a, b in zip(kv_lens, q_lens)])
+    out, launches = torch.zeros(T, H * dv, dtype=torch.bfloat16, device="cuda"), k.launches
+    k.windowed_attention(q, out, kp, None, bt.cuda(), torch.arange(B, dtype=torch.int32).cuda(), cu.cuda(),
+                         torch.tensor(kv_lens, dtype=torch.int32).cuda(), req, H, 1, dk, dv, page, 0, 0.07, num_requests=B, ctx=ctx)
+    k.raise_on_status()
+    assert k.launches == launches + 2  # (the portion's kernel, and the one of the decoded tokens)
+    ref = reference(q.float(), kp.float(), bt, list(range(B)), q_lens, kv_lens, H, dk, dv, page, 0, 0.07)
+    assert (out.float().view(T, H, dv) - ref).abs().max().item() <= 2 ** -7 * max(1.0, ref.abs().max().item())

@@ -1354,10 +1354,11 @@ class Kernels:
                 and self.lib.ullm_latent_attention_supported(head_dim, v_dim, num_q, num_kv, page_size)):
             # Prompt portions over latent rows.  The one-token entries at the step's head go to the kernel below, which cuts
             # their keys into runs (a block of 128 rows for each of them would walk its keys alone, and be the step's tail).
-            # Few rows with many keys in sight stay there altogether: below half a block per SM its runs fill the chip,
-            # where this kernel's blocks would walk all keys one after the other (1.2 us per 64 keys).
+            # Few rows with many keys in sight stay there altogether: below a block of 128 rows for every fourth SM its runs
+            # fill the chip, where this kernel's blocks would walk all keys one after the other (1.2 us per 64 keys).
             n_dec, _ragged = self._decoded_head(ctx)
-            rows, keys = T - n_dec, min(ctx.max_kv_len, abs(window)) if window else ctx.max_kv_len
+            longest = self._longest_behind(ctx, n_dec)
+            rows, keys = T - n_dec, min(longest, abs(window)) if window else longest
             if 2 * -(-rows * num_q // 64) >= self.sm_count or keys <= 2048:
                 code = self.lib.ullm_latent_attention(
                     _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(k_pages), _ptr(block_table), block_table.shape[1],
@@ -2368,6 +2369,19 @@ class Kernels:
         if shared is not None:
             shared["decoded_head"] = head
         return head
+
+    def _longest_behind(self, ctx, n: int) -> int:
+        """The longest context among the step's entries behind the first `n`, formed once per step."""
+        if n == 0:
+            return ctx.max_kv_len
+        shared = getattr(ctx, "shared", None)
+        if shared is not None and shared.get("longest_behind", (None,))[0] == n:
+            return shared["longest_behind"][1]
+        cq, held = ctx.cu_q_host, ctx.start_positions_host
+        longest = max(held[i] + cq[i + 1] - cq[i] for i in range(n, ctx.num_requests))
+        if shared is not None:
+            shared["longest_behind"] = (n, longest)
+        return longest
 
     @_timed("attention")
     def paged_attention(self, qkv, out, k_pages, v_pages, block_table, req_slots, cu_q, kv_len, token_req, num_q, num_kv,
