@@ -20,7 +20,8 @@
 // tiles would leave room for one only.  The reference point of a row's exponents moves only when its maximum grows by more than
 // 2^8, as in attention_prefill_pair.cu; O is rescaled in tensor memory then.
 //
-// Every wait on an mbarrier is bounded (ULLM_STATUS_TIMEOUT in the status word; the block then leaves).
+// Every wait on an mbarrier is bounded (ULLM_STATUS_TIMEOUT in the status word; the block then waits, bounded, for the copies that
+// it has in flight, and leaves).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -146,7 +147,7 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       }
       return page >= 0 ? page : (int)p.num_pages;  // (out of the map's range: the box is filled with zeros)
     };
-    int pages = page_of(0);
+    int pages = page_of(0), issued = 0;
     bool ok = true;
     for (int t = 0; t < tiles && ok; ++t) {
       const int next = t + 1 < tiles ? page_of(t + 1) : 0;
@@ -166,7 +167,13 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                     page);
       }
       pages = next;
+      issued = t + 1;
     }
+    if (lane == 0) {  // (a block in which a role gave up does not leave copies behind that are still on their way)
+      tp_mbar_wait(&q_full, 0);
+      for (int t = max(0, issued - 2); t < issued; ++t) tp_mbar_wait(&k_full[t & 1], (t >> 1) & 1);
+    }
+    __syncwarp();
   } else if (warp == 5) {
     if (lane == 0) {
       // ---- MMA --------------------------------------------------------------------------------------------------

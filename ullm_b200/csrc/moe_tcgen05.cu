@@ -20,7 +20,8 @@
 //   * a box of x is only as many rows high as the step has pairs (16, 32, 64 or 128): what the other rows of a stage hold is
 //     multiplied too, into rows of the accumulator that are never stored.
 //
-// Every wait on an mbarrier is bounded (ULLM_STATUS_TIMEOUT in the status word, then the block leaves).
+// Every wait on an mbarrier is bounded (ULLM_STATUS_TIMEOUT in the status word, then the block waits, bounded, for the copies that
+// it has in flight, and leaves).
 #include "moe_act.cuh"
 #include "tcgen05_util.cuh"
 
@@ -143,7 +144,7 @@ moe_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
     if (lane == 0) {
       // ---- loads -----------------------------------------------------------------------------------------------
       const uint32_t bytes = MT_B_BYTES + (uint32_t)p.box_rows * 128;
-      int s = 0, e = 0;
+      int s = 0, e = 0, issued = 0;
       uint32_t parity = 1;  // a fresh barrier passes a wait on parity 1
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -166,8 +167,11 @@ moe_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
           }
           tma_load_2d(a, &map_x, &full_bar[s], kb * MT_BK, p0);
           if (++s == MT_STAGES) s = 0, parity ^= 1;
+          ++issued;
         }
       }
+      // (a block in which a role gave up does not leave copies behind that are still on their way)
+      for (int i = issued > MT_STAGES ? issued - MT_STAGES : 0; i < issued; ++i) mbar_wait(&full_bar[i % MT_STAGES], (i / MT_STAGES) & 1);
     }
   } else if (warp == 1) {
     if (lane == 0) {
