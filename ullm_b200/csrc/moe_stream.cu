@@ -17,6 +17,10 @@
 //     only the results of the tokens that chose it are stored, at their places: no gathered copy of the rows.  In the second an
 //     expert's rows are neighbours: its box begins at its first place.
 //
+// A token may name an expert more than once (a router's choices never do; the product itself is defined for any).  In the first
+// product a result then goes to several places, found place by place; in the second an expert can have more rows than the tensor
+// instruction has columns, and its matrix is streamed once per 8 NT of them.
+//
 // Every wait on an mbarrier is bounded (ULLM_STATUS_TIMEOUT in the status word; a block that gives up waits, bounded, for the
 // copies it has in flight, and returns).
 #include "linear_stream_core.cuh"
@@ -24,6 +28,7 @@
 
 #define MS_MAX_TOKENS 16
 #define MS_MAX_EXPERTS 1024
+#define MS_MAX_PASSES 64  // of 8 NT places of one expert (16 tokens of 64 choices all at one expert)
 #define MS_SMEM_KB 100  // ring and partial sums of a block: two blocks per SM beside the static arrays
 
 struct MsParams {
@@ -37,6 +42,11 @@ struct MsParams {
   int* status;
 };
 
+__device__ __forceinline__ void ms_store(const MsParams& p, int at, int col, float r, float up, float sc) {
+  const float y = p.gated ? moe_gate_act(p.act, r * sc, up * sc, p.limit, p.alpha) : moe_plain_act(p.act, r * sc);
+  p.out[(size_t)at * p.n_out + col] = __float2bfloat16_rn(y);
+}
+
 template <int NT>
 __global__ void __launch_bounds__(LS_THREADS, 2)
 moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const MsParams p) {
@@ -44,8 +54,8 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
   constexpr int STAGE_BYTES = LS_W_STAGE_BYTES + 4 * X_BOX_BYTES;
   extern __shared__ unsigned char ms_smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[LS_MAX_STAGES], empty_bar[LS_MAX_STAGES];
-  __shared__ short live_s[MS_MAX_EXPERTS];  // the experts that have rows
-  __shared__ int count_s, abort_flag;
+  __shared__ unsigned short live_s[MS_MAX_EXPERTS + MS_MAX_PASSES];  // the experts that have rows (the low 10 bits), and the pass over their places
+  __shared__ int count_s, abort_flag, many_s;
   __shared__ int place_s[MS_MAX_TOKENS];    // where the unit's result of every token goes (-1: nowhere)
   __shared__ float scale_s[MS_MAX_TOKENS];
   pdl_launch_dependents();
@@ -66,10 +76,22 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
     int n = 0;
     for (int e0 = 0; e0 < p.experts; e0 += 32) {
       const int e = e0 + lane;
-      const bool live = e < p.experts && p.offsets[e + 1] > p.offsets[e];
-      const unsigned mask = __ballot_sync(0xffffffffu, live);
-      if (live) live_s[n + __popc(mask & ((1u << lane) - 1u))] = (short)e;
-      n += __popc(mask);
+      const int rows = e < p.experts ? p.offsets[e + 1] - p.offsets[e] : 0;
+      const int passes = p.from_tokens ? (rows > 0 ? 1 : 0) : (rows + 8 * NT - 1) / (8 * NT);
+      const unsigned mask = __ballot_sync(0xffffffffu, passes > 0);
+      int at = n + __popc(mask & ((1u << lane) - 1u)), all = __popc(mask);
+      if (__any_sync(0xffffffffu, passes > 1)) {
+        int sum = passes;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, sum, o);
+          if (lane >= o) sum += v;
+        }
+        at = n + sum - passes;
+        all = __shfl_sync(0xffffffffu, sum, 31);
+      }
+      for (int i = 0; i < passes; ++i) live_s[at + i] = (unsigned short)(e | i << 10);
+      n += all;
     }
     if (lane == 0) count_s = n;
   }
@@ -85,7 +107,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
       bool ok = true;
       for (int ui = 0; ui < my_units && ok; ++ui) {
         const int u = (int)blockIdx.x + ui * grid, a = u / p.units_per_expert, v = u - a * p.units_per_expert;
-        const int e = live_s[a], x_row = p.from_tokens ? 0 : p.offsets[e];
+        const int e = live_s[a] & 1023, x_row = p.from_tokens ? 0 : p.offsets[e] + (live_s[a] >> 10) * 8 * NT;
         for (int kb = 0; kb < p.k_blocks; ++kb) {
           if (round > 0 && !mbar_wait(&empty_bar[slot], (round - 1) & 1)) {
             ullm_report(p.status, ULLM_STATUS_TIMEOUT, 56, ui);
@@ -116,17 +138,23 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
     uint32_t parity = 0;
     for (int ui = 0; ui < my_units; ++ui) {
       const int u = (int)blockIdx.x + ui * grid, ea = u / p.units_per_expert, v = u - ea * p.units_per_expert;
-      const int e = live_s[ea], lo = p.offsets[e], n_e = p.offsets[e + 1] - lo;
+      const int e = live_s[ea] & 1023, lo = p.offsets[e] + (live_s[ea] >> 10) * 8 * NT;
+      const int n_e = p.from_tokens ? p.offsets[e + 1] - lo : min(p.offsets[e + 1] - lo, 8 * NT);
       if (warp == 0) {  // (read by the finishing warps behind the unit's barrier)
         if (lane < MS_MAX_TOKENS) place_s[lane] = -1, scale_s[lane] = 1.f;
         __syncwarp();
-        if (lane < n_e && lane < MS_MAX_TOKENS) {
-          const int pair = p.sorted[lo + lane], col = p.from_tokens ? pair / p.top : lane;
+        int col = 32 + lane;  // (no token's)
+        if (lane < n_e) {
+          const int pair = p.sorted[lo + lane];
+          col = p.from_tokens ? pair / p.top : lane;
           if (col < MS_MAX_TOKENS) {
             place_s[col] = lo + lane;
             if (p.pair_weight != nullptr) scale_s[col] = p.pair_weight[pair];
           }
         }
+        const bool twice = __popc(__match_any_sync(0xffffffffu, col)) > 1 || n_e > 32;
+        const bool many = __any_sync(0xffffffffu, twice);
+        if (lane == 0) many_s = many ? 1 : 0;  // (some token's result goes to several places)
       }
       float acc[NT][4];
 #pragma unroll
@@ -187,12 +215,17 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             // accumulator element i: weight row g + 8 (i >> 1), token 8 n + 2 t + (i & 1)
-            const int m = n * 8 + 2 * t + (i & 1), at = place_s[m];
+            const int m = n * 8 + 2 * t + (i & 1);
             const int col = p.gated ? v * 16 + g + 8 * (i >> 1) : v * 32 + mt * 16 + g + 8 * (i >> 1);
-            if (at < 0 || col >= p.n_out) continue;
-            const float sc = scale_s[m];
-            const float y = p.gated ? moe_gate_act(p.act, r[i] * sc, up[i] * sc, p.limit, p.alpha) : moe_plain_act(p.act, r[i] * sc);
-            p.out[(size_t)at * p.n_out + col] = __float2bfloat16_rn(y);
+            if (col >= p.n_out) continue;
+            if (many_s == 0) {
+              if (place_s[m] >= 0) ms_store(p, place_s[m], col, r[i], up[i], scale_s[m]);
+            } else {
+              for (int q = 0; q < n_e; ++q) {
+                const int pair = p.sorted[lo + q];
+                if (pair / p.top == m) ms_store(p, lo + q, col, r[i], up[i], p.pair_weight != nullptr ? p.pair_weight[pair] : 1.f);
+              }
+            }
           }
         }
       }
@@ -228,16 +261,15 @@ static int ms_launch(const CUtensorMap& w, const CUtensorMap& x, MsParams p, int
 }
 
 // Arguments as `ullm_moe_grouped_linear` in bfloat16 with the weights one after the other, and the status word; x contiguous,
-// pairs / top tokens (at most 16), each of which chose an expert at most once.  UNSUPPORTED for sizes and alignments that the
-// boxes cannot take.
+// pairs / top tokens (at most 16).  UNSUPPORTED for sizes and alignments that the boxes cannot take.
 extern "C" int ullm_moe_stream(const void* x, const void* weights, const int* offsets, const int* sorted,
                                const float* pair_weight, void* out, int pairs, int experts, int top, int rows_from_pairs,
                                int n_out, int k_dim, int gated, int act, float limit, float alpha, int* status, void* stream) {
   if (pairs < 0 || experts <= 0 || top <= 0 || n_out <= 0 || k_dim <= 0) return ULLM_ERR_BAD_SIZE;
   if (gated && (act < 0 || act > 2)) return ULLM_ERR_UNSUPPORTED;
   if (gated && act == 2 && !(limit > 0.f)) return ULLM_ERR_BAD_SIZE;
-  const int tokens = pairs / top;
-  if (pairs % top || tokens > MS_MAX_TOKENS || experts > MS_MAX_EXPERTS || k_dim % 64 || n_out % (gated ? 16 : 32) ||
+  const int tokens = pairs / top, NT = tokens <= 8 ? 1 : 2;
+  if (pairs % top || tokens > MS_MAX_TOKENS || pairs > MS_MAX_PASSES * 8 * NT || experts > MS_MAX_EXPERTS || k_dim % 64 || n_out % (gated ? 16 : 32) ||
       (((uintptr_t)x | (uintptr_t)weights) & 15))
     return ULLM_ERR_UNSUPPORTED;
   if (pairs == 0) return ULLM_OK;
@@ -249,7 +281,6 @@ extern "C" int ullm_moe_stream(const void* x, const void* weights, const int* of
       return ULLM_ERR_LAUNCH;
     }
   }
-  const int NT = tokens <= 8 ? 1 : 2;
   MsParams p = {};
   p.offsets = offsets;
   p.sorted = sorted;
