@@ -83,3 +83,45 @@ def test_chunks_match_the_recurrence(heads, dim, vdim, lens, forget):
     # 32-bit sums: 1e-6 where nothing cancels.  Where the terms of the denominator cancel (long memories: up to 2e-5 here) the
     # loss is the inputs' and the token-by-token kernel has it too: at most twice its distance
     assert err(got) < 2.0 * err(plain) + 1e-6 and worst < 2e-6
+
+
+def inputs(heads, dim, vdim, lens, seed=3, forget=2.0):
+    g = torch.Generator().manual_seed(seed)
+    T, B = sum(lens), len(lens)
+    qkv = torch.randn(T, 2 * heads * dim + heads * vdim, generator=g).bfloat16().to(device())
+    gates = (2.0 * torch.randn(T, 2 * heads, generator=g)).to(device())
+    bi, bf = torch.randn(heads, generator=g).to(device()), (forget + torch.randn(heads, generator=g)).to(device())
+    state = torch.randn(B, heads * dim * (vdim + 1) + heads, generator=g).to(device())
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=device())
+    req = torch.cat([torch.full((n,), r, dtype=torch.int32) for r, n in enumerate(lens)]).to(device())
+    return qkv, gates, bi, bf, state, torch.arange(B, dtype=torch.int32, device=device()), cu, req
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(8, 128, 256), (4, 256, 512), (2, 40, 300)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("lens", [[1] * 70, [300, 150, 40], [9, 2, 14] * 20, [120] * 6 + [3] * 12])
+def test_token_by_token_does_not_depend_on_the_other_requests(heads, dim, vdim, dtype, lens):
+    """More blocks than the chip holds at once: a block that starts behind others of its request and head that are done already
+    begins from the same state as they.  Every request alone gives the same bits."""
+    from ullm_b200.engine import Workspace
+
+    kk = K()
+    qkv, gates, bi, bf, state0, slots, cu, req = inputs(heads, dim, vdim, lens)
+    qkv = qkv.to(dtype)
+    T, B, ws = sum(lens), len(lens), Workspace(device(), sum(lens), len(lens))
+
+    def run(lo, hi, which, workspace):
+        n = len(which)
+        out, state = torch.empty(hi - lo, heads * vdim, device=device()), state0.clone()
+        kk.mlstm_recurrence(qkv[lo:hi], 0, heads * dim, 2 * heads * dim, gates[lo:hi], bi, bf, state, (cu[which[0]:which[-1] + 2] - lo),
+                            slots[which[0]:which[-1] + 1], req[lo:hi] - which[0], out, n, heads, dim, vdim, dim ** -0.5, 15.0,
+                            workspace=workspace)
+        kk.raise_on_status()
+        return out, state
+
+    for workspace in (ws, ws, None):  # (the counters are zeros again behind a launch)
+        out, state = run(0, T, list(range(B)), workspace)
+        for r in {0, 1, B // 2, B - 2, B - 1}:
+            a, b = int(cu[r]), int(cu[r + 1])
+            one, one_state = run(a, b, [r], None)
+            assert torch.equal(out[a:b], one) and torch.equal(state[r], one_state[r])

@@ -36,14 +36,23 @@ __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - l
 // (measured at dim 128: 2.5 times fewer instructions per token); RS == 0: any dim, lanes per column in `rs_arg`.
 // CPT: neighbouring value columns a thread holds (1 or 4): the k and q a thread reads from shared memory and its
 // share of n serve all of them, which is what the multiply-adds wait for otherwise.
+// Blocks per SM that the registers have to leave room for (left alone, the compiler's choice moves with every line).
 template <typename T, int RPT, int RS, int CPT>
-__global__ void __launch_bounds__(2 * MLSTM_THREADS)
+constexpr int mlstm_blocks() {
+  constexpr bool pieces = std::is_same<T, __nv_bfloat16>::value;  // 16-byte pieces in flight while tokens are staged
+  if (RPT == 8 && RS != 0) return pieces ? 2 : (CPT == 1 ? 4 : CPT == 2 ? 3 : 2);
+  if (RPT == 8) return pieces && CPT == 4 ? 1 : 2;
+  return CPT == 4 || (pieces && (CPT == 2 || RS == 0)) ? 1 : 2;
+}
+template <typename T, int RPT, int RS, int CPT>
+__global__ void __launch_bounds__(2 * MLSTM_THREADS, mlstm_blocks<T, RPT, RS, CPT>())
 mlstm_recurrence_kernel(const T* __restrict__ qkv, long long row_stride, int q_off, int k_off, int v_off,
                         const float* __restrict__ gates, const float* __restrict__ bias_i,
                         const float* __restrict__ bias_f, float* __restrict__ state, long long state_stride,
                         const int* __restrict__ cu_q, const int* __restrict__ req_slots,
                         const int* __restrict__ token_req, float* __restrict__ out, int heads, int dim, int vdim,
-                        int rs_arg, int chunk, float q_scale, float cap, int num_slots, int* status, int most_tokens) {
+                        int rs_arg, int chunk, float q_scale, float cap, int num_slots, int* status, int most_tokens,
+                        int* __restrict__ arrived) {
   constexpr bool FULL = RS != 0;
   const int rs = FULL ? RS : rs_arg;
   // Threads 0 .. 127 run the recurrence; threads 128 .. 255 stage the next chunk of tokens (q, k, the tile's v,
@@ -211,6 +220,14 @@ mlstm_recurrence_kernel(const T* __restrict__ qkv, long long row_stride, int q_o
     fill(0, t0, min(chunk, t1 - t0));
   }
   __syncthreads();
+  // n and m are read by all blocks of the (request, head) as they start, and are the same in all of them at the end: the block
+  // that is the last to have read them writes them.  (A block that starts late, behind others that are done already, must find
+  // them as they were.)  One of the staging threads asks now and looks at the answer behind the recurrence.
+  __shared__ int last_s;
+  int* count = arrived + (long long)req * heads + head;
+  int before = 0;
+  if (threadIdx.x == 2 * MLSTM_THREADS - 1)
+    asm volatile("atom.add.release.gpu.global.s32 %0, [%1], 1;" : "=r"(before) : "l"(count) : "memory");
 
   int which = 0;
   for (int c0 = t0; c0 < t1; c0 += chunk, which ^= 1) {
@@ -277,7 +294,20 @@ mlstm_recurrence_kernel(const T* __restrict__ qkv, long long row_stride, int q_o
     }
     __syncthreads();  // the next chunk is staged, this one used up
   }
-  if (loader) return;
+  if (loader) {
+    if (threadIdx.x >= 2 * MLSTM_THREADS - 32) {
+      if (threadIdx.x == 2 * MLSTM_THREADS - 1) {
+        last_s = before == (int)gridDim.x - 1 ? 1 : 0;
+        if (last_s) {
+          *count = 0;  // (for the next launch)
+          __threadfence();
+        }
+      }
+      __syncwarp();
+      asm volatile("bar.arrive 1, %0;" ::"n"(MLSTM_THREADS + 32) : "memory");
+    }
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < RPT; ++i) {
     const int r = lane_row + rs * i;
@@ -285,10 +315,16 @@ mlstm_recurrence_kernel(const T* __restrict__ qkv, long long row_stride, int q_o
 #pragma unroll
       for (int c = 0; c < CPT; ++c)
         if (col + c < vdim) st_S[(long long)c * dim + r] = S[i][c];
-      if (blockIdx.x == 0 && col_in_block == 0) st_n[r] = n[i];
     }
   }
-  if (blockIdx.x == 0 && tid == 0) *st_m = m;
+  asm volatile("bar.sync 1, %0;" ::"n"(MLSTM_THREADS + 32) : "memory");
+  if (last_s == 0) return;
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int r = lane_row + rs * i;
+    if (r < dim && col_in_block == 0) st_n[r] = n[i];
+  }
+  if (tid == 0) *st_m = m;
 }
 
 // out[t, h, :] = o[t, h, :] / sqrt(mean(o[t, h, :]^2) + eps) * w[h, :] * sigmoid(g[t, h, :]); one warp per (token, head).
@@ -381,7 +417,7 @@ static int mlstm_launch(const void* qkv, long long row_stride, int q_off, int k_
                         const float* bias_i, const float* bias_f, float* state, long long state_stride,
                         const int* cu_q, const int* req_slots, const int* token_req, float* out, int requests,
                         int heads, int dim, int vdim, float q_scale, float cap, int num_slots, int* status,
-                        int most_tokens, cudaStream_t st) {
+                        int most_tokens, int* arrived, cudaStream_t st) {
   const int rs = mlstm_rs(dim);
   // four (or two) columns per thread where that still leaves the SMs about two blocks each (fewer, fatter blocks: less
   // q / k staging, several multiply-add chains per row read: head size 256 x 512, one prompt of 2,048 tokens,
@@ -407,16 +443,16 @@ static int mlstm_launch(const void* qkv, long long row_stride, int q_off, int k_
       return ullm_launch_kernel(mlstm_recurrence_kernel<T, RPT_, RS_, 4>, grid, dim3(2 * MLSTM_THREADS), smem, st,     \
                                 (const T*)qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state,         \
                                 state_stride, cu_q, req_slots, token_req, out, heads, dim, vdim, rs, chunk, q_scale,   \
-                                cap, num_slots, status, most_tokens);                                                              \
+                                cap, num_slots, status, most_tokens, arrived);                                        \
     if (cpt == 2)                                                                                                     \
       return ullm_launch_kernel(mlstm_recurrence_kernel<T, RPT_, RS_, 2>, grid, dim3(2 * MLSTM_THREADS), smem, st,     \
                                 (const T*)qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state,         \
                                 state_stride, cu_q, req_slots, token_req, out, heads, dim, vdim, rs, chunk, q_scale,   \
-                                cap, num_slots, status, most_tokens);                                                              \
+                                cap, num_slots, status, most_tokens, arrived);                                        \
     return ullm_launch_kernel(mlstm_recurrence_kernel<T, RPT_, RS_, 1>, grid, dim3(2 * MLSTM_THREADS), smem, st,       \
                               (const T*)qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state,           \
                               state_stride, cu_q, req_slots, token_req, out, heads, dim, vdim, rs, chunk, q_scale,     \
-                              cap, num_slots, status, most_tokens);                                                                \
+                              cap, num_slots, status, most_tokens, arrived);                                          \
   } while (0)
   if (dim == 64 && rs == 8) MLSTM_LAUNCH(8, 8);
   if (dim == 128 && rs == 16) MLSTM_LAUNCH(8, 16);
@@ -428,30 +464,32 @@ static int mlstm_launch(const void* qkv, long long row_stride, int q_off, int k_
 }
 
 // qkv: rows of `row_stride` elements that hold q [heads, dim] at q_off, k [heads, dim] at k_off and v [heads, vdim]
-// at v_off; requests that bring more than `most_tokens` tokens are left alone.  gates: [tokens, 2 heads] float32, the input-gate projections then the forget-gate projections (biases
+// at v_off; requests that bring more than `most_tokens` tokens are left alone; `arrived` [requests, heads]: zeros, and zeros again
+// behind the launch (launches that may run at the same time need counters of their own).  gates: [tokens, 2 heads] float32, the input-gate projections then the forget-gate projections (biases
 // not yet added).  state: [num_slots, state_stride] float32.  out: [tokens, heads, vdim] float32.
 extern "C" int ullm_mlstm_recurrence(int dtype, const void* qkv, long long row_stride, int q_off, int k_off,
                                      int v_off, const float* gates, const float* bias_i, const float* bias_f,
                                      float* state, long long state_stride, const int* cu_q, const int* req_slots,
                                      const int* token_req, float* out, int requests, int heads, int dim, int vdim,
-                                     float q_scale, float cap, int num_slots, int* status, void* stream, int most_tokens) {
+                                     float q_scale, float cap, int num_slots, int* status, void* stream, int most_tokens,
+                                     int* arrived) {
   cudaStream_t st = (cudaStream_t)stream;
   if (requests < 0 || !ullm_mlstm_supported(heads, dim, vdim)) return ULLM_ERR_UNSUPPORTED;
-  if (state_stride < ullm_mlstm_state_floats(heads, dim, vdim) || cap <= 0.f) return ULLM_ERR_BAD_SIZE;
+  if (state_stride < ullm_mlstm_state_floats(heads, dim, vdim) || cap <= 0.f || arrived == nullptr) return ULLM_ERR_BAD_SIZE;
   if (requests == 0) return ULLM_OK;
   if (requests > 65535 || heads > 65535) return ULLM_ERR_BAD_SIZE;
   if (dtype == ULLM_DTYPE_F32)
     return mlstm_launch<float>(qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state, state_stride,
                                cu_q, req_slots, token_req, out, requests, heads, dim, vdim, q_scale, cap, num_slots,
-                               status, most_tokens, st);
+                               status, most_tokens, arrived, st);
   if (dtype == ULLM_DTYPE_BF16)
     return mlstm_launch<__nv_bfloat16>(qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state,
                                        state_stride, cu_q, req_slots, token_req, out, requests, heads, dim, vdim,
-                                       q_scale, cap, num_slots, status, most_tokens, st);
+                                       q_scale, cap, num_slots, status, most_tokens, arrived, st);
   if (dtype == ULLM_DTYPE_F16)
     return mlstm_launch<__half>(qkv, row_stride, q_off, k_off, v_off, gates, bias_i, bias_f, state, state_stride,
                                 cu_q, req_slots, token_req, out, requests, heads, dim, vdim, q_scale, cap, num_slots,
-                                status, most_tokens, st);
+                                status, most_tokens, arrived, st);
   return ULLM_ERR_BAD_DTYPE;
 }
 

@@ -106,6 +106,17 @@ def _scratch_floats(workspace, name: str, floats: int, most: int) -> torch.Tenso
     return workspace.get(name, max(1, -(-int(floats) // 1024)), 1024, torch.float32, reserve=-(-int(most) // 1024))
 
 
+def _arrivals(workspace, requests: int, heads: int, device) -> torch.Tensor:
+    """Counters that are zero between launches, [requests, heads]: of the workspace, cleared when they are made, or the call's own."""
+    if workspace is None:
+        return torch.zeros((max(1, requests), heads), dtype=torch.int32, device=device)
+    made = workspace.generation
+    counters = workspace.get("mlstm.arrived", max(1, requests), heads, torch.int32, reserve=workspace.max_requests)
+    if workspace.generation != made:
+        workspace.buffers[("mlstm.arrived", heads, torch.int32)].zero_()
+    return counters
+
+
 def _weight_bytes(x, weight, *rest):
     return weight.numel() * weight.element_size()
 
@@ -296,7 +307,7 @@ class Kernels:
             "ullm_norm_scale_add_norm": [I, P, P, P, I, I, F, F, P, F, P, P],
             "ullm_rmsnorm_rows_f32": [I, P, P, P, P, I, I, I, F, P, P],
             "ullm_cast_rows_f32": [I, P, P, LL, P],
-            "ullm_mlstm_recurrence": [I, P, LL, I, I, I, P, P, P, P, LL, P, P, P, P, I, I, I, I, F, F, I, P, P, I],
+            "ullm_mlstm_recurrence": [I, P, LL, I, I, I, P, P, P, P, LL, P, P, P, P, I, I, I, I, F, F, I, P, P, I, P],
             "ullm_mlstm_chunk": [P, LL, I, I, I, P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, F, F, I, I, P, P],
             "ullm_mlstm_chunk_supported": [I, I, I],
             "ullm_mlstm_out_gate": [I, P, P, LL, P, P, I, I, I, F, P],
@@ -1460,10 +1471,11 @@ class Kernels:
 
     @_timed("mlstm")
     def mlstm_recurrence(self, qkv, q_off, k_off, v_off, gates, bias_i, bias_f, state, cu_q, req_slots, token_req, out,
-                         requests, heads, dim, vdim, q_scale, cap, most_tokens: int = 1 << 30):
+                         requests, heads, dim, vdim, q_scale, cap, most_tokens: int = 1 << 30, workspace=None):
         """The recurrence of csrc/mlstm.cu over the step's tokens, from and into the requests' state rows.
         qkv [T, *]: q, k, v at the given column offsets; gates [T, 2 heads] float32; out [T, heads * vdim] float32;
-        requests that bring more than `most_tokens` tokens are left alone."""
+        requests that bring more than `most_tokens` tokens are left alone.  The counters of the blocks that are done lie in
+        `workspace` (without one: in memory of the call's own)."""
         _need(qkv, "qkv")
         _need(gates, "gates", torch.float32)
         _need(state, "state", torch.float32)
@@ -1481,7 +1493,8 @@ class Kernels:
         self._check(self.lib.ullm_mlstm_recurrence(
             _DT[qkv.dtype], _ptr(qkv), qkv.stride(0), q_off, k_off, v_off, _ptr(gates), _ptr(bias_i), _ptr(bias_f),
             _ptr(state), state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req), _ptr(out), requests, heads, dim,
-            vdim, float(q_scale), float(cap), state.shape[0], _ptr(self.status), _stream(), int(most_tokens)),
+            vdim, float(q_scale), float(cap), state.shape[0], _ptr(self.status), _stream(), int(most_tokens),
+            _ptr(_arrivals(workspace, requests, heads, qkv.device))),
             f"mlstm_recurrence (heads {heads}, dim {dim}, vdim {vdim})")
 
     def mlstm_chunk_applies(self, dtype, heads: int, dim: int, vdim: int) -> bool:

@@ -109,10 +109,11 @@ class MLSTM(Mixer):
         # prompt portions in chunks on the tensor cores (bfloat16, at the sizes that form takes), the rest token by token
         chunked = (ctx.max_q_len > CHUNK_LEAST and x.is_cuda and K.mlstm_chunk_applies(x.dtype, Hn, d, dv)
                    and K.mlstm_chunk(*args, ws, CHUNK_LEAST))
+        counters = {"workspace": ws} if x.is_cuda else {}
         if not chunked:
-            K.mlstm_recurrence(*args)
+            K.mlstm_recurrence(*args, **counters)
         elif ctx.num_requests > 1:
-            K.mlstm_recurrence(*args, most_tokens=CHUNK_LEAST)
+            K.mlstm_recurrence(*args, most_tokens=CHUNK_LEAST, **counters)
         gated = ws.tokens("mlstm.gated", T, vs, x.dtype)
         K.mlstm_out_gate(o, qkvg[:, 2 * qk + vs:], self.tensors[n["norm"]], self.eps, gated, Hn, dv)
         out = ws.tokens("mixer.out", T, self.hidden_size, x.dtype)
