@@ -125,3 +125,39 @@ def test_token_by_token_does_not_depend_on_the_other_requests(heads, dim, vdim, 
             a, b = int(cu[r]), int(cu[r + 1])
             one, one_state = run(a, b, [r], None)
             assert torch.equal(out[a:b], one) and torch.equal(state[r], one_state[r])
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(8, 128, 256), (4, 256, 512)])
+@pytest.mark.parametrize("lens", [[700], [500, 130]])
+def test_error_against_64_bits_is_not_above_the_token_by_token_kernels(heads, dim, vdim, lens):
+    """Long memories at the sizes of whole models: the typical error of an output row (a median, which the few rows whose denominator
+    cancels do not decide) is not above the one of ordinary 32-bit sums."""
+    from ullm_b200.engine import Workspace
+
+    kk = K()
+    for forget in (2.0, 6.0):
+        qkv, gates, bi, bf, state0, slots, cu, req = inputs(heads, dim, vdim, lens, forget=forget)
+        T, B, cap, scale = sum(lens), len(lens), 15.0, dim ** -0.5
+        x, gd = qkv.double(), gates.double()
+        q, k = (x[:, i * heads * dim:(i + 1) * heads * dim].view(T, heads, dim) for i in (0, 1))
+        v = x[:, 2 * heads * dim:].view(T, heads, vdim)
+        gi = cap * torch.tanh((gd[:, :heads] + bi.double()) / cap)
+        gf = torch.nn.functional.logsigmoid(cap * torch.tanh((gd[:, heads:] + bf.double()) / cap))
+        ref = torch.zeros(T, heads, vdim, dtype=torch.float64, device=device())
+        for r in range(B):
+            a, b, s = int(cu[r]), int(cu[r + 1]), state0[r].double()
+            parts = s[:heads * dim * vdim].view(heads, vdim, dim), s[heads * dim * vdim:-heads].view(heads, dim), s[-heads:]
+            ref[a:b] = recurrence(q[a:b] * scale, k[a:b], v[a:b], gi[a:b], gf[a:b], *parts)[0]
+        typical = []
+        for chunked in (True, False):
+            state, out = state0.clone(), torch.empty(T, heads * vdim, device=device())
+            args = (qkv, 0, heads * dim, 2 * heads * dim, gates, bi, bf, state, cu, slots, req, out, B, heads, dim, vdim, scale, cap)
+            if chunked:
+                assert kk.mlstm_chunk(*args, Workspace(device(), T, B), 16)
+            else:
+                kk.mlstm_recurrence(*args)
+            d = (out.double().view(T, heads, vdim) - ref).norm(dim=-1) / ref.norm(dim=-1)
+            typical.append(float(d.median()))
+        print(f"forget {forget}: chunks {typical[0]:.2e}, token by token {typical[1]:.2e}")
+        # (a tenth: the spread of the median between seeds)
+        assert typical[0] <= 1.1 * typical[1]
