@@ -161,3 +161,31 @@ def test_error_against_64_bits_is_not_above_the_token_by_token_kernels(heads, di
         print(f"forget {forget}: chunks {typical[0]:.2e}, token by token {typical[1]:.2e}")
         # (a tenth: the spread of the median between seeds)
         assert typical[0] <= 1.1 * typical[1]
+
+
+@pytest.mark.parametrize("where", ["v inf", "v nan", "k nan", "forget gate nan", "input gate nan"])
+@pytest.mark.parametrize("at", [20, 21, 63, 64, 75])
+def test_what_is_not_finite_does_not_reach_earlier_tokens(where, at):
+    from ullm_b200.engine import Workspace
+
+    kk, heads, dim, vdim, lens = K(), 2, 32, 48, [100]
+    qkv, gates, bi, bf, state0, slots, cu, req = inputs(heads, dim, vdim, lens)
+
+    def run():
+        out = torch.empty(100, heads * vdim, device=device())
+        assert kk.mlstm_chunk(qkv, 0, heads * dim, 2 * heads * dim, gates, bi, bf, state0.clone(), cu, slots, req, out, 1, heads, dim, vdim,
+                              dim ** -0.5, 15.0, Workspace(device(), 100, 1), 16)
+        return out.view(100, heads, vdim)
+
+    clean, value = run(), float("inf" if where == "v inf" else "nan")
+    if where[0] == "v":
+        qkv[at, 2 * heads * dim + vdim + 5] = value  # head 1, column 5
+    elif where[0] == "k":
+        qkv[at, heads * dim + dim + 5] = value
+    else:
+        gates[at, (heads if where[0] == "f" else 0) + 1] = value
+    out = run()
+    # (the sums of a chunk that holds such a value run in another order)
+    assert torch.isfinite(out[:at]).all() and float((out[:at] - clean[:at]).norm() / clean[:at].norm()) < 1e-5
+    assert torch.equal(out[:, 0], clean[:, 0]) or where[0] == "v" and torch.isfinite(out[:, 0]).all()
+    assert not torch.isfinite(out[at, 1, 5])

@@ -104,6 +104,17 @@ __device__ __forceinline__ float act_gelu_tanh_flat(float g) {
   return gate_flat(g, 1.5957691216057308f * (g + 0.044715f * g * g * g));
 }
 
+// Whether one of a thread's accumulators is infinite or NaN (a zero times either is NaN).
+template <int N>
+__device__ __forceinline__ bool any_odd(const float (&v)[N][4]) {
+  float z = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) z = fmaf(v[i][e], 0.f, z);
+  return z != 0.f;
+}
+
 // True when rows of `cols` elements of T starting at `p` can be moved in
 // 16-byte pieces.
 template <typename T>

@@ -165,8 +165,9 @@ mlstm_chunk_gates_kernel(const float* __restrict__ gates, const float* __restric
       const double v = __shfl_up_sync(0xffffffffu, sum, o);
       if (lane >= o) sum += v;
     }
+    const double in_front = __shfl_up_sync(0xffffffffu, sum, 1);
+    b[0] = (lane > 0 ? in_front : 0.0) + (double)gf[0];  // (not from the sum behind: a gate that is NaN reaches no token in front of it)
     b[1] = sum;
-    b[0] = sum - (double)gf[1];
     d[0] = (double)gi[0] - b[0];
     d[1] = (double)gi[1] - b[1];
   };
@@ -426,55 +427,82 @@ mlstm_chunk_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stri
   __syncthreads();
   for (int m0 = warp * 16; m0 < vdim; m0 += MCH_WARPS * 16) {
     float acc[8][4];
+    // A weight of zero must not meet an infinite or NaN value of a later token: where one shows, the columns again, the tokens'
+    // values without the tensor core, each by those that see it.
+    bool odd = false;
+#pragma unroll 1
+    for (;;) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    const float* sp = st + (long long)(m0 + g) * dim + cp;
-    const long long down = (long long)8 * dim;
-    float2 x[4], y[4];
-    x[0] = *reinterpret_cast<const float2*>(sp);
-    x[1] = *reinterpret_cast<const float2*>(sp + down);
-    x[2] = *reinterpret_cast<const float2*>(sp + 8);
-    x[3] = *reinterpret_cast<const float2*>(sp + down + 8);
-    for (int kk = 0; kk < dim; kk += 16) {
-      const int nx = kk + 16 < dim ? kk + 16 : kk;
-      y[0] = *reinterpret_cast<const float2*>(sp + nx);
-      y[1] = *reinterpret_cast<const float2*>(sp + down + nx);
-      y[2] = *reinterpret_cast<const float2*>(sp + nx + 8);
-      y[3] = *reinterpret_cast<const float2*>(sp + down + nx + 8);
-      unsigned a[3][4];
+      for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+      const float* sp = st + (long long)(m0 + g) * dim + cp;
+      const long long down = (long long)8 * dim;
+      float2 x[4], y[4];
+      x[0] = *reinterpret_cast<const float2*>(sp);
+      x[1] = *reinterpret_cast<const float2*>(sp + down);
+      x[2] = *reinterpret_cast<const float2*>(sp + 8);
+      x[3] = *reinterpret_cast<const float2*>(sp + down + 8);
+      for (int kk = 0; kk < dim; kk += 16) {
+        const int nx = kk + 16 < dim ? kk + 16 : kk;
+        y[0] = *reinterpret_cast<const float2*>(sp + nx);
+        y[1] = *reinterpret_cast<const float2*>(sp + down + nx);
+        y[2] = *reinterpret_cast<const float2*>(sp + nx + 8);
+        y[3] = *reinterpret_cast<const float2*>(sp + down + nx + 8);
+        unsigned a[3][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) mch_split(x[i].x, x[i].y, a[0][i], a[1][i], a[2][i]);
+        for (int i = 0; i < 4; ++i) mch_split(x[i].x, x[i].y, a[0][i], a[1][i], a[2][i]);
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        unsigned b[4];
-        mch_ldsm4(b, q_s + (j * 8 + (mat >> 1) * 8 + (lane & 7)) * kb + kk + (mat & 1) * 8);
-        mch_mma_a3(acc[j], a, b[0], b[1]);
-        mch_mma_a3(acc[j + 1], a, b[2], b[3]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = y[i];
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float f0 = from_s[j * 8 + cp], f1 = from_s[j * 8 + cp + 1];
-      acc[j][0] *= f0, acc[j][1] *= f1, acc[j][2] *= f0, acc[j][3] *= f1;
-    }
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      unsigned a[4];
-      mch_ldsm4t(a, v_s + (s * 16 + (mat >> 1) * 8 + (lane & 7)) * vb + m0 + (mat & 1) * 8);
-#pragma unroll
-      for (int j = 2 * s; j < 8; j += 2) {  // (earlier tokens do not see these keys)
-        unsigned b[4][3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          unsigned r[4];
-          mch_ldsm4(r, p_s + (i * MCH_Q + j * 8 + (mat >> 1) * 8 + (lane & 7)) * MCH_PS + s * 16 + (mat & 1) * 8);
-          b[0][i] = r[0], b[1][i] = r[1], b[2][i] = r[2], b[3][i] = r[3];
+        for (int j = 0; j < 8; j += 2) {
+          unsigned b[4];
+          mch_ldsm4(b, q_s + (j * 8 + (mat >> 1) * 8 + (lane & 7)) * kb + kk + (mat & 1) * 8);
+          mch_mma_a3(acc[j], a, b[0], b[1]);
+          mch_mma_a3(acc[j + 1], a, b[2], b[3]);
         }
-        mch_mma_b3(acc[j], a, b[0], b[1]);
-        mch_mma_b3(acc[j + 1], a, b[2], b[3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = y[i];
       }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float f0 = from_s[j * 8 + cp], f1 = from_s[j * 8 + cp + 1];
+        acc[j][0] *= f0, acc[j][1] *= f1, acc[j][2] *= f0, acc[j][3] *= f1;
+      }
+      if (odd) {
+#pragma unroll 1
+        for (int s = 0; s < cn; ++s) {
+          const __nv_bfloat16* vp = v_s + s * vb + m0 + g;
+          const float lo = __bfloat162float(vp[0]), hi = __bfloat162float(vp[8]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int x2 = 0; x2 < 2; ++x2) {
+              const int t = j * 8 + cp + x2;
+              if (s > t) continue;
+              const __nv_bfloat16* p = p_s + t * MCH_PS + s;
+              const float w = (__bfloat162float(p[2 * MCH_Q * MCH_PS]) + __bfloat162float(p[MCH_Q * MCH_PS])) + __bfloat162float(p[0]);
+              acc[j][x2] = fmaf(w, lo, acc[j][x2]);
+              acc[j][2 + x2] = fmaf(w, hi, acc[j][2 + x2]);
+            }
+        }
+        break;
+      }
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        unsigned a[4];
+        mch_ldsm4t(a, v_s + (s * 16 + (mat >> 1) * 8 + (lane & 7)) * vb + m0 + (mat & 1) * 8);
+#pragma unroll
+        for (int j = 2 * s; j < 8; j += 2) {  // (earlier tokens do not see these keys)
+          unsigned b[4][3];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            unsigned r[4];
+            mch_ldsm4(r, p_s + (i * MCH_Q + j * 8 + (mat >> 1) * 8 + (lane & 7)) * MCH_PS + s * 16 + (mat & 1) * 8);
+            b[0][i] = r[0], b[1][i] = r[1], b[2][i] = r[2], b[3][i] = r[3];
+          }
+          mch_mma_b3(acc[j], a, b[0], b[1]);
+          mch_mma_b3(acc[j + 1], a, b[2], b[3]);
+        }
+      }
+      if (!__any_sync(0xffffffffu, any_odd(acc))) break;
+      odd = true;
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j)
