@@ -47,3 +47,31 @@ def test_value_tiles_match_the_recurrence(heads, dim, vdim, lens):
     # roundings' worth when they are independent
     assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 2.0 ** -24 * 516 ** 0.5
     assert float((states[0] - states[1]).norm() / states[1].norm()) < 2.0 ** -24 * 516 ** 0.5
+
+
+@pytest.mark.parametrize("bonus", [False, True])
+@pytest.mark.parametrize("at,value", [(20, float("inf")), (21, float("nan")), (63, float("inf")), (64, float("nan")), (75, float("inf"))])
+def test_a_value_that_is_not_finite_does_not_reach_earlier_tokens(bonus, at, value):
+    from ullm_b200.engine import Workspace
+
+    kk, heads, dim, vdim, T = K(), 2, 32, 144, 100
+    g = torch.Generator().manual_seed(72)
+    y = torch.randn(T, 2 * heads * dim + heads * vdim, generator=g).bfloat16().to(device())
+    w = torch.sigmoid(2.0 + torch.randn(T, heads * dim, generator=g)).to(device())
+    u = torch.randn(heads * dim, generator=g).to(device()) if bonus else None
+    cu, req = torch.tensor([0, T], dtype=torch.int32, device=device()), torch.zeros(T, dtype=torch.int32, device=device())
+
+    def run():
+        out, state = torch.empty(T, heads * vdim, device=device()), torch.zeros(1, heads * dim * vdim, device=device())
+        kk.gla_chunk(y, 0, heads * dim, 2 * heads * dim, w, dim ** -0.5, kk.gla_chunk_scratch(Workspace(device(), T, 1), T, 1, heads, dim, vdim),
+                     state, cu, req[:1], req, out, 1, heads, dim, vdim, 16, bonus=u)
+        return out.view(T, heads, vdim)
+
+    clean = run()
+    y[at, 2 * heads * dim + vdim + 133] = value  # head 1, column 133
+    out = run()
+    # (the sums of a warp's own tokens run in another order; two terms of an operand with a bonus)
+    assert torch.isfinite(out[:at]).all() and float((out[:at] - clean[:at]).norm() / clean[:at].norm()) < (1e-4 if bonus else 1e-5)
+    other = torch.ones(heads, vdim, dtype=torch.bool)
+    other[1, 133] = False
+    assert torch.isfinite(out[:, other]).all() and not torch.isfinite(out[at:, 1, 133]).any()

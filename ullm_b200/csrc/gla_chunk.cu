@@ -447,31 +447,64 @@ gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int 
   for (int n0 = 0; n0 < vn; n0 += 64) {
     const int nt = min(8, (vn - n0) >> 3);
     float y[8][4];
+    bool odd = false;
+#pragma unroll 1
+    for (int last = warp; last >= warp - 1; --last) {
 #pragma unroll
-    for (int n = 0; n < 8; ++n) y[n][0] = y[n][1] = y[n][2] = y[n][3] = 0.f;
+      for (int n = 0; n < 8; ++n) y[n][0] = y[n][1] = y[n][2] = y[n][3] = 0.f;
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      if (s <= warp) {
-        unsigned p[4][NT], a[NT][4];
-        gch_terms<NT>(acc[2 * s][0], acc[2 * s][1], p[0]);
-        gch_terms<NT>(acc[2 * s][2], acc[2 * s][3], p[1]);
-        gch_terms<NT>(acc[2 * s + 1][0], acc[2 * s + 1][1], p[2]);
-        gch_terms<NT>(acc[2 * s + 1][2], acc[2 * s + 1][3], p[3]);
+      for (int s = 0; s < 4; ++s) {
+        if (s <= last) {
+          unsigned p[4][NT], a[NT][4];
+          gch_terms<NT>(acc[2 * s][0], acc[2 * s][1], p[0]);
+          gch_terms<NT>(acc[2 * s][2], acc[2 * s][3], p[1]);
+          gch_terms<NT>(acc[2 * s + 1][0], acc[2 * s + 1][1], p[2]);
+          gch_terms<NT>(acc[2 * s + 1][2], acc[2 * s + 1][3], p[3]);
 #pragma unroll
-        for (int i = 0; i < NT; ++i)
+          for (int i = 0; i < NT; ++i)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) a[i][e] = p[e][i];
+            for (int e = 0; e < 4; ++e) a[i][e] = p[e][i];
 #pragma unroll
-        for (int n = 0; n < 8; n += 2) {
-          if (n < nt) {
-            unsigned b[4];
-            gch_ldsm4t(b, v_s + (s * 16 + (mat & 1) * 8 + (lane & 7)) * (vn + 8) + n0 + n * 8 + (mat >> 1) * 8);
-            const unsigned l0[1] = {b[0]}, l1[1] = {b[1]}, r0[1] = {b[2]}, r1[1] = {b[3]};
-            gch_mma_terms<NT, 1>(y[n], a, l0, l1);
-            gch_mma_terms<NT, 1>(y[n + 1], a, r0, r1);
+          for (int n = 0; n < 8; n += 2) {
+            if (n < nt) {
+              unsigned b[4];
+              gch_ldsm4t(b, v_s + (s * 16 + (mat & 1) * 8 + (lane & 7)) * (vn + 8) + n0 + n * 8 + (mat >> 1) * 8);
+              const unsigned l0[1] = {b[0]}, l1[1] = {b[1]}, r0[1] = {b[2]}, r1[1] = {b[3]};
+              gch_mma_terms<NT, 1>(y[n], a, l0, l1);
+              gch_mma_terms<NT, 1>(y[n + 1], a, r0, r1);
+            }
           }
         }
       }
+      // A score of zero must not meet an infinite or NaN value of a later token: where one shows, the warp's own 16 tokens again
+      // without the tensor core, each by those that it sees.
+      if (odd || !__any_sync(0xffffffffu, any_odd(y))) break;
+      odd = true;
+    }
+    if (odd) {
+      // (lane 4 g + i of a group holds the scores of row g, and g + 8, against the tokens 2 i, 2 i + 1 of a stretch)
+      float own[8];
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (s == warp) own[e] = acc[2 * s + (e >> 2)][e & 3];
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int at = (x >> 1) * 8 + 2 * i + (x & 1), from = (lane & 28) | i;
+          const float lo = __shfl_sync(0xffffffffu, own[(x >> 1) * 4 + (x & 1)], from);
+          const float hi = __shfl_sync(0xffffffffu, own[(x >> 1) * 4 + 2 + (x & 1)], from);
+          const __nv_bfloat16* vp = v_s + (warp * 16 + at) * (vn + 8) + n0 + cp;
+#pragma unroll
+          for (int n = 0; n < 8; ++n)
+            if (n < nt) {
+              const float w0 = __bfloat162float(vp[n * 8]), w1 = __bfloat162float(vp[n * 8 + 1]);
+              if (at <= g) y[n][0] = fmaf(lo, w0, y[n][0]), y[n][1] = fmaf(lo, w1, y[n][1]);
+              if (at <= g + 8) y[n][2] = fmaf(hi, w0, y[n][2]), y[n][3] = fmaf(hi, w1, y[n][3]);
+            }
+        }
     }
     for (int kk = 0; kk < dim; kk += 16) {
       const float* r_lo = rp + (warp * 16 + g) * ks + kk + cp;
