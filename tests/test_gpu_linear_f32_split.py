@@ -63,3 +63,28 @@ def test_what_it_does_not_take():
     assert not kk.linear_f32_split(y, w, out)  # off the 16-byte border
     assert not kk.linear_f32_split(torch.randn(300, 128, device=device())[:, :64], w, out)  # rows with gaps
     assert not kk.linear_f32_split(torch.randn(200, 64, device=device()), w, out[:200])  # fewer than 2^16 results
+
+
+@pytest.mark.parametrize("low,other", [(-126, 0), (0, -126), (-126, 20), (20, -126), (-70, -50), (-112, 0), (-100, 60)])
+def test_operands_near_the_smallest_exponent_keep_24_bits(low, other):
+    """Operands down to 2^-126 keep all their bits: the errors are those of operands of order one, and the library's at most."""
+    M, N, k = 200, 512, 260
+    g = torch.Generator(device=device()).manual_seed(3)
+    x, w = (torch.randn(r, k, generator=g, device=device()).clamp(-8, 8) for r in (M, N))
+    x, w = (torch.where(v.abs() < 1, v.sign() + v, v).ldexp(torch.tensor(e, device=device())) for v, e in ((x, low), (w, other)))
+    got, ref = run(x, w).double(), x.double() @ w.double().t()
+    size = x.double().abs() @ w.double().abs().t()
+    # (as above, and half a unit of the smallest float)
+    assert ((got - ref).abs() <= 2.0 ** -24 * (72 + k / 64) * size + 2.0 ** -150).all()
+    lib = (x @ w.t()).double()
+    assert float((got - ref).norm()) <= 1.1 * float((lib - ref).norm()) + 1e-7 * float(ref.norm()) + 2.0 ** -149 * (M * N) ** 0.5
+
+
+def test_operands_and_sums_that_the_factor_takes_to_infinity():
+    """Operands from 2^104 on and sums from 2^80 on are formed by multiply-adds: finite where float32 is."""
+    x, w = torch.randn(140, 128, device=device()), torch.randn(600, 128, device=device())
+    x[1], x[2, 5], x[3], w[7], w[9, 0] = x[1] * 2.0 ** 60, 2.0 ** 110, x[3] * 2.0 ** 104, w[7] * 2.0 ** 22, -(2.0 ** 120)
+    got, ref = run(x, w).double(), x.double() @ w.double().t()
+    size = x.double().abs() @ w.double().abs().t()
+    fits = size < 2.0 ** 127
+    assert torch.isfinite(got[fits]).all() and ((got - ref).abs() <= 2.0 ** -24 * 200 * size)[fits].all()

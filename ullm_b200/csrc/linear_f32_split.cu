@@ -1,7 +1,8 @@
 // out[M, N] = x[M, K] . w[N, K]^T (+ bias) in float32 for many rows, on the 5th-generation tensor cores.
 //
-// Every float32 operand is the sum of three bfloat16 numbers, the rounded value, the rounded rest and the rest of that (24 bits:
-// nothing is lost but what lies under the smallest exponent).  Of the nine products of terms the six down to 2^-16 of the first are
+// Every float32 operand, times 2^24, is the sum of three bfloat16 numbers, the rounded value, the rounded rest and the rest of that.
+// The 24 bits of a number from 2^-126 on then lie at 2^-125 and above, so that none of them is lost under bfloat16's smallest
+// exponent (2^-133 without the factor: a number below 2^-110 would lose its last bits); the results are scaled back.  Of the nine products of terms the six down to 2^-16 of the first are
 // formed, h h + h m + m h + m m + h l + l h; what is left out is 2^-24 of a product, half a unit in its last place.  The sums of a
 // k block of 64 run in tensor memory, smallest products first, and are then added to float32 registers by ordinary rounded
 // additions: the tensor core's own additions do not round to nearest, and over a whole row of K that would show.
@@ -17,8 +18,8 @@
 // tiles; a thread of warp 0 asks for the planes of x; a thread of warp 16 issues the products; warps 8..15 add the block sums up, a
 // quarter of the rows and half of the columns each.  Two or three stages, two or four block sums in tensor memory.  BN from 32 to 128, so that the tiles fill the SMs.
 //
-// Infinities, NaN and values that bfloat16 rounds to infinity turn a sum into NaN that may not be NaN in float32: such a result is
-// formed again with multiply-adds from the rows themselves.
+// Infinities, NaN, operands from 2^104 on and sums from 2^80 on (which the factor takes to infinity) turn a sum into an infinity or
+// NaN that float32 may not show: such a result is formed again with multiply-adds from the rows themselves.
 //
 // Every wait on an mbarrier is bounded (ULLM_STATUS_TIMEOUT in the status word, then the role leaves, and the others after it).
 #include "tcgen05_util.cuh"
@@ -28,17 +29,33 @@
 #define FS_THREADS (17 * 32)
 #define FS_A_BYTES (FS_BM * 128)  // one term of x
 
+// two neighbouring floats in one 64-bit register, the low one first, for the instructions that work on both
+__device__ __forceinline__ unsigned long long fs_pair(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+// v as two bfloat16, and v without them
+__device__ __forceinline__ unsigned fs_term(unsigned long long& v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  const unsigned t = *reinterpret_cast<const unsigned*>(&h);
+  const unsigned long long taken = fs_pair(__uint_as_float(t << 16), __uint_as_float(t & 0xffff0000u)), minus = fs_pair(-1.f, -1.f);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v) : "l"(taken), "l"(minus));
+  return t;
+}
+#define FS_UP 0x1p24f
+#define FS_DOWN 0x1p-48f
 // four neighbouring values as three groups of four bfloat16
 __device__ __forceinline__ void fs_split(const float4& v, uint2& h, uint2& m, uint2& l) {
-  const __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
-  const float a = v.x - __bfloat162float(h0.x), b = v.y - __bfloat162float(h0.y);
-  const float c = v.z - __bfloat162float(h1.x), d = v.w - __bfloat162float(h1.y);
-  const __nv_bfloat162 m0 = __floats2bfloat162_rn(a, b), m1 = __floats2bfloat162_rn(c, d);
-  const __nv_bfloat162 l0 = __floats2bfloat162_rn(a - __bfloat162float(m0.x), b - __bfloat162float(m0.y));
-  const __nv_bfloat162 l1 = __floats2bfloat162_rn(c - __bfloat162float(m1.x), d - __bfloat162float(m1.y));
-  h = make_uint2(*reinterpret_cast<const unsigned*>(&h0), *reinterpret_cast<const unsigned*>(&h1));
-  m = make_uint2(*reinterpret_cast<const unsigned*>(&m0), *reinterpret_cast<const unsigned*>(&m1));
-  l = make_uint2(*reinterpret_cast<const unsigned*>(&l0), *reinterpret_cast<const unsigned*>(&l1));
+  unsigned long long a = fs_pair(v.x, v.y), b = fs_pair(v.z, v.w);
+  const unsigned long long up = fs_pair(FS_UP, FS_UP);
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(up));
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(b) : "l"(up));
+  h.x = fs_term(a), h.y = fs_term(b);
+  m.x = fs_term(a), m.y = fs_term(b);
+  l.x = fs_term(a), l.y = fs_term(b);
 }
 
 // x [M][K] as three planes of bfloat16 terms [3][M][stride]; four values per thread
@@ -267,8 +284,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1) linear_f32_split_kernel(const _
         float v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          v[i] = acc[c + i];
-          if (v[i] != v[i]) {
+          v[i] = acc[c + i] * FS_DOWN;
+          if (!(fabsf(acc[c + i]) <= 3.4028234e38f)) {
             const float* xr = p.x + (long long)row * p.K;
             const float* wr = p.w + (long long)(col + i) * p.K;
             float sum = 0.f;
