@@ -88,3 +88,12 @@ def test_operands_and_sums_that_the_factor_takes_to_infinity():
     size = x.double().abs() @ w.double().abs().t()
     fits = size < 2.0 ** 127
     assert torch.isfinite(got[fits]).all() and ((got - ref).abs() <= 2.0 ** -24 * 200 * size)[fits].all()
+
+
+def test_a_product_over_no_columns_is_the_bias():
+    kk, bias = K(), torch.randn(512, device=device())
+    out = torch.full((300, 512), 9.0, device=device())
+    kk.linear(torch.empty(300, 0, device=device()), torch.empty(512, 0, device=device()), out, bias)
+    assert torch.equal(out, bias.expand(300, 512))
+    kk.linear(torch.empty(300, 0, device=device()), torch.empty(512, 0, device=device()), out)
+    assert torch.count_nonzero(out) == 0

@@ -762,7 +762,7 @@ class Kernels:
         279 for 386)."""
         M, K = x.shape
         N = weight.shape[0]
-        if (M < self.f32_split_rows or M * N < self.f32_split_results or (M <= 32 and N > 32768)
+        if (M < self.f32_split_rows or M * N < self.f32_split_results or (M <= 32 and N > 32768) or K == 0
                 or weight.dtype != torch.float32 or out.dtype != torch.float32 or not x.is_contiguous()
                 or not weight.is_contiguous() or not out.is_contiguous() or weight.shape[1] != K or out.shape != (M, N)
                 or (bias is not None and (bias.dtype != torch.float32 or bias.shape != (N,) or not bias.is_contiguous()))):
