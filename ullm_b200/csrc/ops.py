@@ -1892,7 +1892,8 @@ class Kernels:
             raise KernelError("ssd_chunk: x, B or C lie outside the rows")
         floats = self.lib.ullm_ssd_chunk_scratch
         if workspace is None:
-            scratch = torch.empty(max(1, int(floats(T, requests, heads, n_state, pdim, int(least)))), device=xbc.device)
+            scratch = torch.empty(max(1, int(floats(T, requests, heads, n_state, pdim, int(least)))), dtype=torch.float32,
+                                  device=xbc.device)
         else:
             scratch = _scratch_floats(workspace, "ssd.chunks", floats(T, requests, heads, n_state, pdim, int(least)),
                                       floats(workspace.max_tokens, workspace.max_requests, heads, n_state, pdim, int(least)))
