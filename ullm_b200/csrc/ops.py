@@ -117,6 +117,11 @@ def _arrivals(workspace, requests: int, heads: int, device) -> torch.Tensor:
     return counters
 
 
+def _scratch_bytes(most: int) -> int:
+    """What `_scratch_floats` reserves."""
+    return -(-int(most) // 1024) * 4096
+
+
 def _weight_bytes(x, weight, *rest):
     return weight.numel() * weight.element_size()
 
@@ -1501,6 +1506,10 @@ class Kernels:
         """True when `mlstm_chunk` takes these sizes (bfloat16; see csrc/mlstm_chunk.cu)."""
         return bool(self.mlstm_chunk_on and dtype == torch.bfloat16 and self.lib.ullm_mlstm_chunk_supported(heads, dim, vdim))
 
+    def mlstm_chunk_bytes(self, max_tokens: int, max_requests: int, heads: int, dim: int, vdim: int, least: int) -> int:
+        """Bytes of scratch that `mlstm_chunk` reserves in a workspace for such steps."""
+        return _scratch_bytes(self.lib.ullm_mlstm_chunk_floats(max_tokens, max_requests, heads, dim, vdim, int(least)))
+
     @_timed("mlstm", skipped=True)
     def mlstm_chunk(self, qkv, q_off, k_off, v_off, gates, bias_i, bias_f, state, cu_q, req_slots, token_req, out, requests,
                     heads, dim, vdim, q_scale, cap, workspace, least: int) -> bool:
@@ -1631,6 +1640,10 @@ class Kernels:
     def gla_chunk_applies(self, dtype, heads: int, dim: int, vdim: int) -> bool:
         """True when `gla_chunk` takes these sizes (bfloat16; see csrc/gla_chunk.cu)."""
         return bool(self.gla_chunk_on and dtype == torch.bfloat16 and self.lib.ullm_gla_chunk_supported(heads, dim, vdim))
+
+    def gla_chunk_bytes(self, max_tokens: int, max_requests: int, heads: int, dim: int, vdim: int) -> int:
+        """Bytes of scratch that `gla_chunk_scratch` reserves in a workspace for such steps."""
+        return 4 * self.lib.ullm_gla_chunk_tiles(max_tokens, max_requests) * int(self.lib.ullm_gla_chunk_floats(heads, dim, vdim))
 
     def gla_chunk_scratch(self, workspace, tokens: int, requests: int, heads: int, dim: int, vdim: int):
         """Scratch rows of `gla_chunk` for a step of this size."""
@@ -1869,6 +1882,10 @@ class Kernels:
 
     def ssd_chunk_floats(self, tokens: int, groups: int) -> int:
         return tokens * groups * int(self.lib.ullm_ssd_chunk_tokens())
+
+    def ssd_chunk_bytes(self, max_tokens: int, max_requests: int, heads: int, n_state: int, pdim: int, least: int) -> int:
+        """Bytes of scratch that `ssd_chunk` reserves in a workspace for such steps."""
+        return _scratch_bytes(self.lib.ullm_ssd_chunk_scratch(max_tokens, max_requests, heads, n_state, pdim, int(least)))
 
     @_timed("ssd")
     def ssd_chunk(self, xbc, b_off: int, c_off: int, dt, log_decay, d_skip, scores, state, cu_q, req_slots, token_req, out,

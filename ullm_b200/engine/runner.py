@@ -138,13 +138,18 @@ class ModelRunner:
 
     def _activation_bytes(self) -> int:
         """Room for one step's work buffers: every part says how many elements per token it keeps in the
-        workspace (`Part.activation_elems`); layers reuse the buffers, so the widest layer counts."""
+        workspace (`Part.activation_elems`); layers reuse the buffers, so the widest layer counts.  Scratch that goes by
+        chunks or requests comes on top (`Part.step_scratch`), and in a 32-bit engine the three bfloat16 planes of a
+        product's rows (`Kernels.linear_f32_split`), once per length of such rows."""
         s = self.spec
         widest = max((b.activation_elems() for b in self.model.blocks), default=0)
         itemsize = torch.empty((), dtype=self.dtype).element_size()
         acts = self.max_step_tokens * (widest + 2 * s.hidden_size) * itemsize
         logits = self.max_requests * s.vocab_size * 4 * 2
-        return int(acts + logits + (512 << 20))
+        scratch = sum(self.model.step_scratch(self.max_step_tokens, self.max_requests).values())
+        if self.dtype == torch.float32:
+            scratch += 6 * self.max_step_tokens * sum({t.shape[-1] for t in self.model.all_tensors().values() if t.dim() >= 2})
+        return int(acts + logits + scratch + (512 << 20))
 
     # -- requests -----------------------------------------------------------------
     def add_request(self, request_id: str, tokens=None) -> RequestCache | None:

@@ -120,6 +120,16 @@ class Part:
         buffers from `ctx.workspace` says here how wide they are together."""
         return sum(p.activation_elems() for p in self.subparts().values())
 
+    def step_scratch(self, max_tokens: int, max_requests: int) -> dict[tuple, int]:
+        """Bytes of the workspace's buffers that this part (with its sub-parts) takes and that are not so many elements per token,
+        by buffer (name, and the size that tells buffers of one name apart): what the largest step reserves.  Parts that name the
+        same buffer share it.  Called when the parameters are in place."""
+        out: dict[tuple, int] = {}
+        for p in self.subparts().values():
+            for key, size in p.step_scratch(max_tokens, max_requests).items():
+                out[key] = max(out.get(key, 0), size)
+        return out
+
     # -- walking a tree of parts ------------------------------------------
     def all_decls(self, prefix: str = "") -> dict[str, ParamDecl]:
         out = {prefix + n: d for n, d in self.param_decls().items()}

@@ -81,10 +81,15 @@ class GatedLinearAttention(Mixer):
         return StateNeed((gla_state_floats(self.num_heads, self.head_dim, self.value_dim),), torch.float32)
 
     def activation_elems(self):
-        # the input product, z and o in 32-bit (two elements' worth each in a 16-bit engine), the gated o, the output, a 64th of
-        # the chunked form's states
+        # the input product, z and o in 32-bit (two elements' worth each in a 16-bit engine), the gated o, the output
         return (2 * self.qk_size + 2 * self.v_size + self.decay_rank + 2 * self.qk_size + 3 * self.v_size
-                + self.hidden_size + self.num_heads * self.head_dim * (self.value_dim + 1) // 32)
+                + self.hidden_size)
+
+    def step_scratch(self, max_tokens, max_requests):
+        K, sizes = kernels(), (self.num_heads, self.head_dim, self.value_dim)
+        if not K.gla_chunk_applies(self.w_in.dtype, *sizes):
+            return {}
+        return {("gla.chunks", *sizes): K.gla_chunk_bytes(max_tokens, max_requests, *sizes)}
 
     def forward(self, x, ctx, cache):
         K = kernels()

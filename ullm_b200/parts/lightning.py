@@ -73,10 +73,14 @@ class FixedDecayAttention(Mixer):
         return StateNeed((self.num_heads * self.value_dim * self.head_dim,), torch.float32)
 
     def activation_elems(self):
-        # the input product, o in 32-bit (two elements' worth), the gated o, the output, the chunked form's scores, sums and
-        # weights, and a 64th of its states
-        return (2 * self.qk_size + 5 * self.v_size + self.hidden_size + 134 * self.num_heads
-                + self.num_heads * self.head_dim * self.value_dim // 32)
+        # the input product, o in 32-bit (two elements' worth), the gated o, the output, the chunked form's scores
+        return 2 * self.qk_size + 5 * self.v_size + self.hidden_size + 128 * self.num_heads
+
+    def step_scratch(self, max_tokens, max_requests):
+        K, N, d, dv = kernels(), self.num_heads, self.head_dim, self.value_dim
+        if not K.ssd_chunk_applies(self.w_in.dtype, N, d, dv, N):
+            return {}
+        return {("ssd.chunks",): K.ssd_chunk_bytes(max_tokens, max_requests, N, d, dv, CHUNK_LEAST)}
 
     def operand_dtype(self):
         return self.w_in.dtype

@@ -76,9 +76,15 @@ class Mamba2(Mixer, SharesInput):
 
     def activation_elems(self):
         # the input product, the convolved rows, steps and decays and y in 32-bit (two elements each), the gated y, the output
-        # ... and the chunked form's scores, sums and weights, and a 64th of its states (32-bit)
-        return (self.input_width() + self.channels + 10 * self.num_heads + 3 * self.inner + self.hidden_size
-                + 128 * self.groups + self.s_floats // 32)
+        # ... and the chunked form's scores
+        return (self.input_width() + self.channels + 4 * self.num_heads + 3 * self.inner + self.hidden_size
+                + 128 * self.groups)
+
+    def step_scratch(self, max_tokens, max_requests):
+        K, N, S, P = kernels(), self.num_heads, self.state, self.value_dim
+        if not K.ssd_chunk_applies(self.tensors[self.names["in_proj"]].dtype, N, S, P, self.groups):
+            return {}
+        return {("ssd.chunks",): K.ssd_chunk_bytes(max_tokens, max_requests, N, S, P, CHUNK_LEAST)}
 
     def output_projection(self):
         return self.tensors[self.names["o"]], None

@@ -84,10 +84,14 @@ class MLSTM(Mixer):
         return StateNeed((mlstm_state_floats(self.num_heads, self.head_dim, self.value_dim),), torch.float32)
 
     def activation_elems(self):
-        # q | k | v | g, the gates, o in 32-bit (two elements' worth in a 16-bit engine), the gated o, the output, the chunked
-        # form's sums and weights and a 64th of its states
-        return (2 * self.qk_size + 2 * self.v_size + 16 * self.num_heads + 3 * self.v_size + self.hidden_size
-                + self.num_heads * self.head_dim * (self.value_dim + 1) // 32)
+        # q | k | v | g, the gates, o in 32-bit (two elements' worth in a 16-bit engine), the gated o, the output
+        return 2 * self.qk_size + 2 * self.v_size + 2 * self.num_heads + 3 * self.v_size + self.hidden_size
+
+    def step_scratch(self, max_tokens, max_requests):
+        K, sizes = kernels(), (self.num_heads, self.head_dim, self.value_dim)
+        if not K.mlstm_chunk_applies(self.w_if.dtype, *sizes):
+            return {}
+        return {("mlstm.chunks",): K.mlstm_chunk_bytes(max_tokens, max_requests, *sizes, CHUNK_LEAST)}
 
     def output_projection(self):
         return None

@@ -85,6 +85,12 @@ class TimeMixing(Mixer):
         # the mixes, the input products, decays and o in 32-bit (two elements each), the gated o, the output
         return 5 * self.hidden_size + 4 * self.size + self.rank_rows + 5 * self.size + self.hidden_size
 
+    def step_scratch(self, max_tokens, max_requests):
+        K, sizes = kernels(), (self.num_heads, self.head_dim, self.head_dim)
+        if not K.gla_chunk_applies(self.w_in.dtype, *sizes):
+            return {}
+        return {("gla.chunks", *sizes): K.gla_chunk_bytes(max_tokens, max_requests, *sizes)}
+
     def operand_dtype(self):
         return self.w_in.dtype
 
