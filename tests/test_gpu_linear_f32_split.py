@@ -25,6 +25,22 @@ def run(x, w, bias=None):
                                    (512, 4096, 1024), (257, 2052, 132), (1000, 32, 2048)])
 @pytest.mark.parametrize("spread", [0.0, 6.0])
 def test_error_against_64_bits(M, N, k, spread):
+    check_error(M, N, k, spread)
+
+
+# every width of a tile, with k blocks well past the ring's stages and the block sums in tensor memory, k and columns that end
+# inside a block and a tile (148 SMs, which the choice of the width goes by)
+WIDTHS = [(32, 511, 1028, 836), (64, 200, 4100, 1028), (96, 400, 6148, 900), (128, 300, 6148, 708)]
+
+
+@pytest.mark.parametrize("width,M,N,k", WIDTHS)
+def test_every_width_wraps_its_rings(width, M, N, k):
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert K().lib.ullm_linear_f32_split_columns(M, N) == width
+    check_error(M, N, k, 0.0)
+
+
+def check_error(M, N, k, spread):
     g = torch.Generator(device=device()).manual_seed(M + N)
     x, w = (torch.randn(r, k, generator=g, device=device()) * torch.exp(spread * torch.randn(r, k, generator=g, device=device()))
             for r in (M, N))
@@ -42,8 +58,10 @@ def test_error_against_64_bits(M, N, k, spread):
     assert err <= err_lib * 1.1 + 1e-7
 
 
-def test_infinities_and_nan_as_in_float32():
-    x, w = torch.randn(200, 256, device=device()), torch.randn(160, 256, device=device())
+@pytest.mark.parametrize("N", [160] + [n for _, _, n, _ in WIDTHS[1:]])
+def test_infinities_and_nan_as_in_float32(N):
+    M = {160: 200}.get(N) or next(m for _, m, n, _ in WIDTHS if n == N)
+    x, w = torch.randn(M, 256, device=device()), torch.randn(N, 256, device=device())
     x[3, 7], x[5, 9], x[199, 255], w[17, 3], w[20, 4] = float("inf"), float("nan"), 3.4e38, float("-inf"), 0.0
     x[8] = 0.0
     x[8, 4], x[9, 100] = float("inf"), -3.4028e38

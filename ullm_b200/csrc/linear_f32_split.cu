@@ -322,6 +322,26 @@ static int fs_go(const CUtensorMap& x_map, const FsParams& p, long long tiles, c
   return ullm_launch_kernel(linear_f32_split_kernel<BN>, dim3((unsigned)tiles), dim3(FS_THREADS), (size_t)smem, st, x_map, p);
 }
 
+// Columns per tile by (waves of tiles) x (ns of a k block, measured: 511 rows, 1,024 columns of k 3,072 in tiles of 32, 64, 96 and
+// 128: 54, 58, 79, 91 us in one wave each); the wider tile where both agree.  0: the device's SM count cannot be read.
+extern "C" int ullm_linear_f32_split_columns(int M, int N) {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      return 0;
+    sms = n;
+  }
+  const double ns[4] = {950., 1050., 1450., 1700.};
+  int best = 0;
+  double least = 0.;
+  for (int bn = 128; bn >= 32; bn -= 32) {
+    const long long tiles = (long long)((M + FS_BM - 1) / FS_BM) * ((N + bn - 1) / bn);
+    const double cost = (double)((tiles + sms - 1) / sms) * ns[bn / 32 - 1];
+    if (best == 0 || cost < least) best = bn, least = cost;
+  }
+  return best;
+}
 // bfloat16 numbers of the planes of x
 extern "C" long long ullm_linear_f32_split_terms(int M, int K) { return 3LL * M * ((K + 7) / 8 * 8); }
 
@@ -332,24 +352,9 @@ extern "C" int ullm_linear_f32_split(const float* x, const float* w, const float
   if (M < 0 || N <= 0 || K <= 0 || terms == nullptr) return ULLM_ERR_BAD_SIZE;
   if (N % 4 || K % 4 || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out | (uintptr_t)terms) & 15)) return ULLM_ERR_UNSUPPORTED;
   if (M == 0) return ULLM_OK;
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-      return ULLM_ERR_LAUNCH;
-    sms = n;
-  }
   const FsParams p = {x, w, bias, out, M, N, K, status};
-  // columns per tile by (waves of tiles) x (ns of a k block, measured: 511 rows, 1,024 columns of k 3,072 in tiles of 32, 64, 96 and
-  // 128: 54, 58, 79, 91 us in one wave each); the wider tile where both agree
-  const double ns[4] = {950., 1050., 1450., 1700.};
-  int best = 0;
-  double least = 0.;
-  for (int bn = 128; bn >= 32; bn -= 32) {
-    const long long tiles = (long long)((M + FS_BM - 1) / FS_BM) * ((N + bn - 1) / bn);
-    const double cost = (double)((tiles + sms - 1) / sms) * ns[bn / 32 - 1];
-    if (best == 0 || cost < least) best = bn, least = cost;
-  }
+  const int best = ullm_linear_f32_split_columns(M, N);
+  if (best == 0) return ULLM_ERR_LAUNCH;
   const long long tiles = (long long)((M + FS_BM - 1) / FS_BM) * ((N + best - 1) / best);
   if (tiles > 0x7fffffffLL) return ULLM_ERR_UNSUPPORTED;
   const int stride = (K + 7) / 8 * 8;
@@ -364,7 +369,7 @@ extern "C" int ullm_linear_f32_split(const float* x, const float* w, const float
     return ULLM_ERR_LAUNCH;
   cudaStream_t st = (cudaStream_t)stream;
   const long long pieces = ((long long)M * (K / 4) + 255) / 256;
-  const int rc = ullm_launch_kernel(f32_terms_kernel, dim3((unsigned)(pieces < 16LL * sms ? pieces : 16LL * sms)), dim3(256), 0, st, x,
+  const int rc = ullm_launch_kernel(f32_terms_kernel, dim3((unsigned)(pieces < 2368 ? pieces : 2368)), dim3(256), 0, st, x,
                                     (__nv_bfloat16*)terms, M, K, stride);
   if (rc != ULLM_OK) return rc;
   if (best == 128) return fs_go<128>(x_map, p, tiles, st);

@@ -407,6 +407,8 @@ class Kernels:
         L.ullm_decode_attention_supported.restype = c_int
         L.ullm_decode_attention_balanced_supported.argtypes = [I, I, I, I, I]
         L.ullm_decode_attention_balanced_supported.restype = c_int
+        L.ullm_linear_f32_split_columns.argtypes = [I, I]
+        L.ullm_linear_f32_split_columns.restype = c_int
         L.ullm_linear_f32_split_terms.argtypes = [I, I]
         L.ullm_linear_f32_split_terms.restype = c_longlong
         L.ullm_decode_attention_balanced_scratch_floats.argtypes = [I, I]
