@@ -78,3 +78,31 @@ def test_grouped_product_matches_the_reference(counts, top, n_out, k, gated, act
         assert (got - ref).abs().max().item() <= (2 ** -8 + 1e-4) * s
         assert (got - gen).abs().max().item() <= (2 ** -7 + 1e-4) * s
         assert (out[used:] == 9.0).all()  # (places that belong to no expert stay as they were)
+
+
+@pytest.mark.parametrize("gated,act", [(True, 0), (False, 3)])
+def test_blocks_with_many_tiles_use_their_accumulators_again(gated, act):
+    """More than four tiles per block (two accumulators in turn, each handed over several times), experts without places between
+    full ones."""
+    kk, n_out, k = K(), 2056 if gated else 4112, 136
+    counts = [260, 0, 256, 129, 0, 250, 270, 128, 1, 0, 255, 257, 300, 0, 264, 127]
+    tiles = sum(-(-c // 128) for c in counts) * -(-n_out // (128 if gated else 256))
+    assert tiles > 2.5 * torch.cuda.get_device_properties(0).multi_processor_count
+    E, total = len(counts), sum(counts)
+    g = torch.Generator().manual_seed(9)
+    flat = torch.tensor([e for e, n in enumerate(counts) for _ in range(n)], dtype=torch.int32)
+    choice = flat[torch.randperm(total, generator=g)].view(-1, 1).contiguous().cuda()
+    offsets = torch.empty(E + 1, dtype=torch.int32, device="cuda")
+    order, place = (torch.zeros(total, 1, dtype=torch.int32, device="cuda") for _ in range(2))
+    kk.moe_arrange(choice, total, E, offsets, order, place)
+    w = rnd(E, (2 if gated else 1) * n_out, k, seed=6, dtype=torch.bfloat16, scale=k ** -0.5)
+    x = rnd(total, k, seed=8, dtype=torch.bfloat16)
+    out, gathered = (torch.full((total, n), 9.0, dtype=torch.bfloat16, device="cuda") for n in (n_out, k))
+    launches = kk.launches
+    kk.moe_grouped_linear(x, w, offsets, order, None, out, 1, True, gated, act, gathered=gathered)
+    kk.raise_on_status()
+    assert kk.launches == launches + 2  # (the rows gathered, the product)
+    at = place.view(-1).long()
+    ref = reference(x, w, choice.cpu(), None, 1, True, gated, act, 0.0, 1.0, at)
+    # (one rounding to bfloat16 behind 32-bit sums of 136 products, as above)
+    assert (out[at].float() - ref).abs().max().item() <= (2 ** -8 + 1e-4) * ref.abs().max().item()
