@@ -168,7 +168,8 @@ class Kernels:
                 "ULLM_B200_STREAM_ALL_ROWS", "ULLM_B200_CHAIN_NORMS", "ULLM_B200_GENERAL_ATTN_TC", "ULLM_B200_SSD_CHUNK",
                 "ULLM_B200_PAIR_BIASED_ROWS", "ULLM_B200_GLA_CHUNK",
                 "ULLM_B200_STATE_STEP", "ULLM_B200_PLAIN_ATTN", "ULLM_B200_MOE_TCGEN05_ROWS",
-                "ULLM_B200_MLSTM_CHUNK", "ULLM_B200_LATENT_TCGEN05", "ULLM_B200_MOE_STREAM_TOKENS")
+                "ULLM_B200_MLSTM_CHUNK", "ULLM_B200_LATENT_TCGEN05", "ULLM_B200_MOE_STREAM_TOKENS",
+                "ULLM_B200_F32_SPLIT_ROWS")
 
     def apply_switches(self, env) -> None:
         """Sets every kernel choice from `env` (a mapping; the process environment at start-up): a switch that is

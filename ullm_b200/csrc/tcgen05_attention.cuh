@@ -1,5 +1,5 @@
 // Device helpers of the prompt attention kernels on tcgen05 (attention_prefill_pair.cu, attention_latent_tcgen05.cu): bounded
-// waits on mbarriers, TMA boxes of three and four dimensions, operand descriptors, tensor-memory loads and stores.
+// waits on mbarriers, TMA boxes of three and four dimensions, tensor-memory loads and stores.
 #pragma once
 
 #include <cuda.h>
@@ -75,41 +75,6 @@ __device__ __forceinline__ void tp_tma_4d(void* dst, const CUtensorMap* map, uin
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
       ::"r"(tp_smem(dst)), "l"(map), "r"(tp_smem(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
-      : "memory");
-}
-// K-major operand tile: rows of 128 bytes, 128-byte swizzle, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t tp_desc_kmajor(const void* tile) {
-  uint64_t d = (uint64_t)((tp_smem(tile) & 0x3FFFF) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// MN-major operand tile (V as B: N = head dim, K = keys): a row of 128 bytes holds 64 neighbouring N elements
-// of one key; 8-key groups 1024 bytes apart (stride offset); the next 64 N elements `lbo_bytes` further
-__device__ __forceinline__ uint64_t tp_desc_mnmajor(const void* tile, uint32_t lbo_bytes) {
-  uint64_t d = (uint64_t)((tp_smem(tile) & 0x3FFFF) >> 4);
-  d |= (uint64_t)(lbo_bytes >> 4) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// both operands from shared memory
-__device__ __forceinline__ void tp_mma_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// the A operand from tensor memory (row m in lane m, two bfloat16 per 32-bit column)
-__device__ __forceinline__ void tp_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void tp_commit(uint64_t* bar) {
