@@ -24,8 +24,21 @@ MODELS = {"one size": (lh, lambda: ludalix((2, 32, 48), (2, 32, 48))), "two size
           "ninelix": (nh, lambda: nh.weights_for("F", "bfloat16"))}
 
 
+@pytest.fixture
+def always_chunks():
+    """Every form with scratch at every size (steps as short as these take others)."""
+    from test_gpu_kernels import K
+
+    k = K()
+    old = k.mlstm_chunk_on, k.gla_chunk_on
+    k.mlstm_chunk_on, k.gla_chunk_on = 2, 2
+    yield
+    k.mlstm_chunk_on, k.gla_chunk_on = old
+
+
 @pytest.mark.parametrize("name", MODELS)
 @pytest.mark.parametrize("max_requests", [1, 3, 9])
+@pytest.mark.usefixtures("always_chunks")
 def test_prompt_steps_reserve_what_the_plan_holds(tmp_path, name, max_requests):
     helpers, make = MODELS[name]
     cfg, w, page = make()

@@ -576,6 +576,13 @@ static int gch_v_tile(int dim, int vdim) {
   return most;
 }
 
+extern "C" int ullm_gla_chunk_v_tile(int dim, int vdim) { return gch_v_tile(dim, vdim); }
+// blocks of `gla_out` that fit an SM
+extern "C" int ullm_gla_chunk_per_sm(int dim, int vdim) {
+  const size_t smem = gch_out_smem(dim, gch_v_tile(dim, vdim));
+  return smem <= 75 * 1024 ? 3 : (smem <= 112 * 1024 ? 2 : 1);
+}
+
 // Sizes the chunked form takes (bfloat16): key and value sizes that are multiples of 16, as far as the shared memory reaches.
 extern "C" int ullm_gla_chunk_supported(int heads, int dim, int vdim) {
   return heads > 0 && heads <= 65535 && dim > 0 && vdim > 0 && dim % 16 == 0 && vdim % 16 == 0 && dim <= GCH_MAX_DIM &&

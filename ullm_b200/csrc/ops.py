@@ -11,6 +11,7 @@ from __future__ import annotations
 import ctypes
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
+from typing import NamedTuple
 
 import torch
 
@@ -106,6 +107,21 @@ def _scratch_floats(workspace, name: str, floats: int, most: int) -> torch.Tenso
     return workspace.get(name, max(1, -(-int(floats) // 1024)), 1024, torch.float32, reserve=-(-int(most) // 1024))
 
 
+class Portions(NamedTuple):
+    """The portions of a step that are longer than some number of tokens: how many, their tokens together, the longest one's, and
+    their chunks of 64 together; the step's other requests."""
+
+    count: int
+    tokens: int
+    longest: int
+    chunks: int
+    others: int
+
+    def beside(self, size: int) -> float:
+        """us of the launch that takes the other requests, whose states of `size` numbers pass through memory."""
+        return 5 + 3.5e-6 * size * self.others if self.others else 0.0
+
+
 def _arrivals(workspace, requests: int, heads: int, device) -> torch.Tensor:
     """Counters that are zero between launches, [requests, heads]: of the workspace, cleared when they are made, or the call's own."""
     if workspace is None:
@@ -198,11 +214,12 @@ class Kernels:
         # token always
         self.ssd_chunk_on = get("ULLM_B200_SSD_CHUNK", "1") != "0"
         # the same for the recurrence with a decay per key channel
-        self.gla_chunk_on = get("ULLM_B200_GLA_CHUNK", "1") != "0"
+        # (without a bonus: 1 where it is the faster form, 2 always)
+        self.gla_chunk_on = {"0": 0, "2": 2}.get(get("ULLM_B200_GLA_CHUNK", "1"), 1)
         # prompt attention over latent key rows on the tcgen05 kernel; 0: the mma.sync kernel always
         self.latent_attention_on = get("ULLM_B200_LATENT_TCGEN05", "1") != "0"
-        # and for the matrix memory with exponential gates
-        self.mlstm_chunk_on = get("ULLM_B200_MLSTM_CHUNK", "1") != "0"
+        # and for the matrix memory with exponential gates (1 where it is the faster form, 2 always)
+        self.mlstm_chunk_on = {"0": 0, "2": 2}.get(get("ULLM_B200_MLSTM_CHUNK", "1"), 1)
         # steps of single tokens through a state: the kernel built around the state's stream; 0: the general recurrences
         self.state_step_on = get("ULLM_B200_STATE_STEP", "1") != "0"
         # rows from which a step with distance biases (heads of 128) takes the tcgen05 prompt kernel
@@ -388,6 +405,10 @@ class Kernels:
         L.ullm_gla_supported.restype = c_int
         L.ullm_gla_state_floats.argtypes = [I, I, I]
         L.ullm_gla_state_floats.restype = c_longlong
+        L.ullm_gla_chunk_v_tile.argtypes = [I, I]
+        L.ullm_gla_chunk_v_tile.restype = c_int
+        L.ullm_gla_chunk_per_sm.argtypes = [I, I]
+        L.ullm_gla_chunk_per_sm.restype = c_int
         L.ullm_gla_chunk_supported.argtypes = [I, I, I]
         L.ullm_gla_chunk_supported.restype = c_int
         L.ullm_gla_chunk_tiles.argtypes = [I, I]
@@ -1504,6 +1525,55 @@ class Kernels:
             vdim, float(q_scale), float(cap), state.shape[0], _ptr(self.status), _stream(), int(most_tokens),
             _ptr(_arrivals(workspace, requests, heads, qkv.device))),
             f"mlstm_recurrence (heads {heads}, dim {dim}, vdim {vdim})")
+
+    @staticmethod
+    def long_portions(ctx, least: int) -> Portions:
+        """The step's portions of more than `least` tokens, formed once per step."""
+        key = ("long_portions", least)
+        if key not in ctx.shared:
+            cq = ctx.cu_q_host
+            lens = [n for n in (cq[i + 1] - cq[i] for i in range(ctx.num_requests)) if n > least]
+            ctx.shared[key] = Portions(len(lens), sum(lens), max(lens, default=0), sum(-(-n // 64) for n in lens),
+                                       ctx.num_requests - len(lens))
+        return ctx.shared[key]
+
+    def chunk_pays(self, ctx, form: str, least: int, *sizes) -> bool:
+        """`mlstm_chunk_pays` or `gla_chunk_pays` of the step's portions of more than `least` tokens, formed once per step."""
+        key = (form, least, sizes)
+        if key not in ctx.shared:
+            ctx.shared[key] = getattr(self, form + "_pays")(self.long_portions(ctx, least), *sizes)
+        return ctx.shared[key]
+
+    def mlstm_chunk_pays(self, portions: Portions, heads: int, dim: int, vdim: int) -> bool:
+        """Whether `mlstm_chunk` is faster than the token-by-token kernel for a step's long portions, by models of both that
+        measured steps give (us; 8 heads of 128 x 256, one portion of 17 / 64 / 100 / 256 tokens: chunks 37 / 41 / 41 / 42, token
+        by token 13 / 30 / 44 / 101; 16 portions of 40: 83 and 126; 256 x 512, one of 64 / 100 / 150: 101 / 103 / 103 and 53 /
+        79 / 115).  Token by token: the longest portion's chain, or all portions' multiply-adds.  Chunks: the chain of the outputs'
+        kernel over the key channels, the states on their way through memory, and the other requests' launch."""
+        if self.mlstm_chunk_on == 2 or not portions.count:
+            return bool(portions.count)
+        size = heads * dim * vdim
+        rate = 0.3 + 0.0011 * (dim - 64) if dim in (64, 128, 256, 512) else 0.65  # (the sizes with loops of a fixed length)
+        token = 6 + max(rate * portions.longest, 6.8e-7 * size * portions.tokens)
+        chunk = 18 + 1.2 * -(-dim // 16) * -(-vdim // 128) + size * (5e-6 * portions.count + 3e-6 * portions.chunks)
+        return chunk + portions.beside(size) < token
+
+    def gla_chunk_pays(self, portions: Portions, heads: int, dim: int, vdim: int) -> bool:
+        """`mlstm_chunk_pays` for `gla_chunk` without a bonus (8 heads of 128 x 256, one portion of 17 / 100 / 256 / 400 tokens: chunks
+        63 / 71 / 72 / 74, token by token 10 / 32 / 73 / 110; 16 of 100: 183 and 170; 256 x 512, one of 256 / 400 / 800: 210 / 214 /
+        375 and 136 / 208 / 410).  Chunks: the outputs' kernel, which forms scores inside stretches one by one, in waves of its
+        blocks."""
+        if self.gla_chunk_on == 2 or not portions.count:
+            return bool(portions.count)
+        size = heads * dim * vdim
+        chain, work = (0.08 + 0.00166 * dim) * portions.longest, 4e-7 * size * portions.tokens
+        # (a portion that outlasts the others runs on alone)
+        alone = 1 - portions.tokens / (portions.count * portions.longest)
+        token = 6 + max(chain, work) + 0.35 * alone * min(chain, work)
+        tile = self.lib.ullm_gla_chunk_v_tile(dim, vdim)
+        waves = -(-portions.chunks * heads * -(-vdim // tile) // (self.sm_count * self.lib.ullm_gla_chunk_per_sm(dim, vdim)))
+        chunk = (6 + 0.2 * dim + 0.0024 * dim * tile) * (0.25 + 0.75 * waves) + size * (1e-5 * portions.count + 1.5e-6 * portions.chunks)
+        return chunk + portions.beside(size) < token
 
     def mlstm_chunk_applies(self, dtype, heads: int, dim: int, vdim: int) -> bool:
         """True when `mlstm_chunk` takes these sizes (bfloat16; see csrc/mlstm_chunk.cu)."""

@@ -103,8 +103,9 @@ class GatedLinearAttention(Mixer):
         z = ws.tokens("gla.z", T, qk, torch.float32)
         K.linear_f32_out(y[:, 2 * qk + 2 * vs:], self.tensors[n["a2"]], z)
         o = ws.tokens("gla.o", T, vs, torch.float32)
-        # prompt portions in chunks on the tensor cores (bfloat16, at the sizes that form takes), the rest token by token
-        chunked = ctx.max_q_len > CHUNK_LEAST and x.is_cuda and y.stride(0) % 8 == 0 and K.gla_chunk_applies(x.dtype, N, d, dv)
+        # prompt portions in chunks on the tensor cores (bfloat16, where that is the faster form), the rest token by token
+        chunked = (ctx.max_q_len > CHUNK_LEAST and x.is_cuda and y.stride(0) % 8 == 0 and K.gla_chunk_applies(x.dtype, N, d, dv)
+                   and K.chunk_pays(ctx, "gla_chunk", CHUNK_LEAST, N, d, dv))
         if chunked:
             K.gla_decay(z, self.tensors[n["a2_bias"]], 1.0 / self.tau)
             scratch = K.gla_chunk_scratch(ws, T, ctx.num_requests, N, d, dv)

@@ -110,9 +110,9 @@ class MLSTM(Mixer):
         o = ws.tokens("mlstm.o", T, vs, torch.float32)
         args = (qkvg, 0, qk, 2 * qk, gates, self.tensors[n["i_bias"]], self.tensors[n["f_bias"]], cache.state, ctx.cu_q,
                 ctx.req_slots, ctx.token_req, o, ctx.num_requests, Hn, d, dv, d ** -0.5, self.gate_cap)
-        # prompt portions in chunks on the tensor cores (bfloat16, at the sizes that form takes), the rest token by token
+        # prompt portions in chunks on the tensor cores (bfloat16, where that is the faster form), the rest token by token
         chunked = (ctx.max_q_len > CHUNK_LEAST and x.is_cuda and K.mlstm_chunk_applies(x.dtype, Hn, d, dv)
-                   and K.mlstm_chunk(*args, ws, CHUNK_LEAST))
+                   and K.chunk_pays(ctx, "mlstm_chunk", CHUNK_LEAST, Hn, d, dv) and K.mlstm_chunk(*args, ws, CHUNK_LEAST))
         counters = {"workspace": ws} if x.is_cuda else {}
         if not chunked:
             K.mlstm_recurrence(*args, **counters)
