@@ -30,10 +30,10 @@ def always_chunks():
     from test_gpu_kernels import K
 
     k = K()
-    old = k.mlstm_chunk_on, k.gla_chunk_on
-    k.mlstm_chunk_on, k.gla_chunk_on = 2, 2
+    old = k.mlstm_chunk_on, k.gla_chunk_on, k.lib.ullm_ssd_chunk_short_pays
+    k.mlstm_chunk_on, k.gla_chunk_on, k.lib.ullm_ssd_chunk_short_pays = 2, 2, lambda *a: 0
     yield
-    k.mlstm_chunk_on, k.gla_chunk_on = old
+    k.mlstm_chunk_on, k.gla_chunk_on, k.lib.ullm_ssd_chunk_short_pays = old
 
 
 @pytest.mark.parametrize("name", MODELS)

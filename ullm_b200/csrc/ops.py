@@ -358,6 +358,7 @@ class Kernels:
             "ullm_ssd_prepare": [I, P, LL, I, I, I, I, P, I, P, P, P, P, LL, I, P, P, P, I, P, P, P, I, P, P],
             "ullm_ssd_recurrence": [I, P, LL, I, I, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, P, P, LL, I],
             "ullm_ssd_chunk": [P, LL, I, I, P, P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, P, P, LL],
+            "ullm_ssd_chunk_short": [P, LL, I, I, P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, P, P, LL],
             "ullm_ssd_gate_norm": [I, P, P, LL, P, P, I, I, I, F, P, I],
             "ullm_norm_rows": [I, P, P, P, P, I, I, I, F, I, P, P, P, P],
             "ullm_xielu": [I, P, P, LL, P, P],
@@ -419,6 +420,8 @@ class Kernels:
         L.ullm_ssd_supported.restype = c_int
         L.ullm_ssd_chunk_supported.argtypes = [I, I, I, I]
         L.ullm_ssd_chunk_supported.restype = c_int
+        L.ullm_ssd_chunk_short_pays.argtypes = [I, I, I, I, I, I]
+        L.ullm_ssd_chunk_short_pays.restype = c_int
         L.ullm_ssd_chunk_scratch.argtypes = [I, I, I, I, I, I]
         L.ullm_ssd_chunk_scratch.restype = c_longlong
         L.ullm_ssd_chunk_tokens.argtypes = []
@@ -1962,10 +1965,11 @@ class Kernels:
 
     @_timed("ssd")
     def ssd_chunk(self, xbc, b_off: int, c_off: int, dt, log_decay, d_skip, scores, state, cu_q, req_slots, token_req, out,
-                  requests: int, heads: int, n_state: int, pdim: int, groups: int, least: int, workspace=None):
+                  requests: int, heads: int, n_state: int, pdim: int, groups: int, least: int, workspace=None, portions=None):
         """`ssd_recurrence` in its chunked form on the tensor cores, for the requests that bring MORE than `least` tokens
         (the others are left alone); `scores`: scratch (float32, `ssd_chunk_floats`).  The states between the chunks lie in
-        `workspace` (without one: in memory of the call's own)."""
+        `workspace` (without one: in memory of the call's own).  `portions` (what `long_portions` gives for `least`): steps of
+        few chunks take the form that keeps the states in registers (csrc/ssd_chunk_short.cu)."""
         _need(xbc, "xbc", torch.bfloat16)
         _need(state, "state", torch.float32, contiguous=False)
         for t_, n_ in ((dt, "dt"), (log_decay, "log_decay"), (d_skip, "d_skip"), (out, "out"), (scores, "scores")):
@@ -1980,6 +1984,15 @@ class Kernels:
             raise KernelError(f"ssd_chunk: xbc {tuple(xbc.shape)}, out {tuple(out.shape)}, state {tuple(state.shape)}")
         if max(b_off, c_off) + groups * n_state > xbc.shape[1] or heads * pdim > xbc.shape[1]:
             raise KernelError("ssd_chunk: x, B or C lie outside the rows")
+        if portions is not None and portions.count and self.lib.ullm_ssd_chunk_short_pays(
+                heads, n_state, pdim, portions.count, -(-portions.longest // 64), portions.chunks):
+            self._check(self.lib.ullm_ssd_chunk_short(
+                _ptr(xbc), xbc.stride(0), b_off, c_off, _ptr(dt), _ptr(log_decay), _ptr(d_skip), _ptr(scores), _ptr(state),
+                state.stride(0), _ptr(cu_q), _ptr(req_slots), _ptr(token_req), _ptr(out), T, requests, heads, n_state, pdim,
+                groups, state.shape[0], int(least), _ptr(self.status), _stream(), heads if dt.shape[0] == T else 0),
+                f"ssd_chunk_short (heads {heads}, state {n_state}, columns {pdim})")
+            self.launches += 1  # the scores in front of it
+            return
         floats = self.lib.ullm_ssd_chunk_scratch
         if workspace is None:
             scratch = torch.empty(max(1, int(floats(T, requests, heads, n_state, pdim, int(least)))), dtype=torch.float32,

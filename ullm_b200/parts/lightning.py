@@ -101,7 +101,8 @@ class FixedDecayAttention(Mixer):
             K.act_rows("silu", u[:, :vs + 2 * qk], u[:, :vs + 2 * qk])
             scores = ws.tokens("ssd.scores", T, K.ssd_chunk_floats(1, N), torch.float32)
             K.ssd_chunk(u, vs, vs + qk, self.steps, self.log_decay, self.skip, scores, cache.state, ctx.cu_q, ctx.req_slots,
-                        ctx.token_req, o, ctx.num_requests, N, d, dv, N, CHUNK_LEAST, ws)
+                        ctx.token_req, o, ctx.num_requests, N, d, dv, N, CHUNK_LEAST, ws,
+                        K.long_portions(ctx, CHUNK_LEAST) if x.is_cuda else None)
         if not chunked or ctx.num_requests > 1:
             K.ssd_recurrence(u, vs, vs + qk, self.steps, self.log_decay, self.skip, cache.state, ctx.cu_q, ctx.req_slots,
                              ctx.token_req, o, ctx.num_requests, N, d, dv, N, CHUNK_LEAST if chunked else 1 << 30,

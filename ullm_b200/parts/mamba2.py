@@ -114,7 +114,8 @@ class Mamba2(Mixer, SharesInput):
         if chunked:
             scores = ws.tokens("ssd.scores", T, K.ssd_chunk_floats(1, G), torch.float32)
             K.ssd_chunk(xbc, inner, inner + G * S, dt, log_decay, t[n["d"]], scores, cache.state, ctx.cu_q, ctx.req_slots,
-                        ctx.token_req, y, ctx.num_requests, N, S, P, G, CHUNK_LEAST, ws)
+                        ctx.token_req, y, ctx.num_requests, N, S, P, G, CHUNK_LEAST, ws,
+                        K.long_portions(ctx, CHUNK_LEAST) if x.is_cuda else None)
         if not chunked or ctx.num_requests > 1:
             K.ssd_recurrence(xbc, inner, inner + G * S, dt, log_decay, t[n["d"]], cache.state, ctx.cu_q, ctx.req_slots,
                              ctx.token_req, y, ctx.num_requests, N, S, P, G, CHUNK_LEAST if chunked else 1 << 30,
