@@ -70,3 +70,39 @@ def test_short_and_long_walks_agree(heads, n_state, pdim, groups, lens, single_r
     # both keep 16 bits of every 32-bit operand, in other orders: 2^-16 of the values each
     for a, b in zip(*outs):
         assert float((a - b).norm() / b.norm()) < 2.0 ** -15
+
+
+def paged(q_lens, kv_lens, page=16):
+    """Block table, page count and the step's arrays of requests that hold `kv_lens` tokens behind `q_lens` new ones."""
+    per, bt, used = [-(-n // page) for n in kv_lens], torch.full((len(q_lens), max(-(-n // page) for n in kv_lens) + 1), -1, dtype=torch.int32), 0
+    for r, n in enumerate(per):
+        bt[r, :n] = torch.arange(used, used + n)
+        used += n
+    cu = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32)
+    req = torch.cat([torch.full((n,), r, dtype=torch.int32) for r, n in enumerate(q_lens)])
+    ctx = SimpleNamespace(decode_only=False, num_requests=len(q_lens), max_q_len=max(q_lens), max_kv_len=max(kv_lens), cu_q_host=cu.tolist(),
+                          shared={}, start_positions_host=[b - a for a, b in zip(q_lens, kv_lens)])
+    i = dict(dtype=torch.int32, device="cuda")
+    return bt.cuda(), used, torch.arange(len(q_lens), **i), cu.cuda(), torch.tensor(kv_lens, **i), req.cuda(), ctx
+
+
+@pytest.mark.parametrize("H,dk,dv,n,kv,window,path", [
+    (16, 448, 384, 17, 17, 0, "latent_tcgen05"), (16, 448, 384, 17, 2000, 0, "window_mma"), (16, 448, 384, 64, 2000, 0, "window_mma"),
+    (16, 448, 384, 200, 2000, 0, "latent_tcgen05"), (16, 448, 384, 600, 600, 0, "latent_tcgen05"), (8, 192, 128, 200, 2000, 1024, "window_mma"),
+    (8, 192, 128, 400, 2000, 1024, "latent_tcgen05"), (32, 448, 384, 64, 2000, 1024, "window_mma")])
+def test_latent_attention_by_rows_and_keys_in_sight(H, dk, dv, n, kv, window, path):
+    k, outs = K(), []
+    bt, pages, slots, cu, lens, req, ctx = paged([n], [kv])
+    g = torch.Generator().manual_seed(95)
+    kp, q = (torch.randn(*s, generator=g).bfloat16().cuda() for s in ((pages, 16, 1, dk), (n, H * dk)))
+    for on in (True, False):
+        k.latent_attention_on = on
+        outs.append(torch.zeros(n, H * dv, dtype=torch.bfloat16, device="cuda"))
+        try:
+            k.windowed_attention(q, outs[-1], kp, None, bt, slots, cu, lens, req, H, 1, dk, dv, 16, window, dk ** -0.5, num_requests=1, ctx=ctx)
+        finally:
+            k.latent_attention_on = True
+        assert k.attention_path == (path if on else "window_mma")
+    k.raise_on_status()
+    # (weights rounded to bfloat16 and one rounding of values of order one, on either side)
+    assert (outs[0].float() - outs[1].float()).abs().max().item() <= 2.0 ** -6

@@ -1397,12 +1397,18 @@ class Kernels:
                 and self.lib.ullm_latent_attention_supported(head_dim, v_dim, num_q, num_kv, page_size)):
             # Prompt portions over latent rows.  The one-token entries at the step's head go to the kernel below, which cuts
             # their keys into runs (a block of 128 rows for each of them would walk its keys alone, and be the step's tail).
-            # Few rows with many keys in sight stay there altogether: below a block of 128 rows for every fourth SM its runs
-            # fill the chip, where this kernel's blocks would walk all keys one after the other (1.2 us per 64 keys).
+            # Few rows with many keys in sight stay there altogether: its runs fill the chip, where a block of this kernel walks
+            # all keys one after the other.  In us, with blocks of 64 rows there: tiles of 64 keys * (1.15 + 0.0021 * dk) here
+            # (behind a window more, the longer the rows are), tiles * blocks * 0.0175 * dk / SMs there, whose start takes 12
+            # more.  16 heads of 448 / 384, 2,000 keys: 17 / 64 / 200 tokens 83 / 77 / 78 here, 38 / 49 / 99 there; 1,024 keys of
+            # 8,000: 57 / 55 / 59 and 25 / 40 / 77; 8 heads of 192 / 128, 1,024 keys: 200 / 400 tokens 38 / 33 and 26 / 44.
             n_dec, _ragged = self._decoded_head(ctx)
             longest = self._longest_behind(ctx, n_dec)
             rows, keys = T - n_dec, min(longest, abs(window)) if window else longest
-            if 2 * -(-rows * num_q // 64) >= self.sm_count or keys <= 2048:
+            tiles, here = -(-keys // 64) + (1 if window else 0), 1.15 + 0.0021 * head_dim
+            if window:
+                here *= 1 + 0.001 * max(0, head_dim - 192)
+            if tiles * (here - 0.0175 * head_dim * -(-rows * num_q // 64) / self.sm_count) <= 12:
                 code = self.lib.ullm_latent_attention(
                     _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(k_pages), _ptr(block_table), block_table.shape[1],
                     _ptr(req_slots[n_dec:]), _ptr(cu_q[n_dec:]), _ptr(kv_len[n_dec:]), T, ctx.num_requests - n_dec, num_q, num_kv,
