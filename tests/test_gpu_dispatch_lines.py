@@ -106,3 +106,23 @@ def test_latent_attention_by_rows_and_keys_in_sight(H, dk, dv, n, kv, window, pa
     k.raise_on_status()
     # (weights rounded to bfloat16 and one rounding of values of order one, on either side)
     assert (outs[0].float() - outs[1].float()).abs().max().item() <= 2.0 ** -6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("q_lens,kv_lens,tiles", [([2], [2], False), ([8, 16], [8, 16], False), ([17], [17], True), ([8], [300], True), ([1, 1], [5, 9], True)])
+def test_32_bit_attention_of_a_few_keys_stays_with_the_general_kernel(dtype, q_lens, kv_lens, tiles):
+    k, calls, outs = K(), [], []
+    bt, pages, slots, cu, lens, req, ctx = paged(q_lens, kv_lens)
+    g = torch.Generator().manual_seed(96)
+    kp, vp, qkv = (torch.randn(*s, generator=g).to(dtype).cuda() for s in ((pages, 16, 2, 64), (pages, 16, 2, 64), (sum(q_lens), 8 * 64)))
+    real = k.lib.ullm_attention_plain
+    for on in (True, False):
+        outs.append(torch.zeros(sum(q_lens), 4 * 64, dtype=dtype, device="cuda"))
+        k.lib.ullm_attention_plain, k.plain_attention_on = (lambda *a: calls.append(0) or real(*a)), on
+        try:
+            k.paged_attention(qkv, outs[-1], kp, vp, bt, slots, cu, lens, req, 4, 2, 64, 16, 0, 0.125, ctx=ctx)
+        finally:
+            k.lib.ullm_attention_plain, k.plain_attention_on = real, True
+    assert bool(calls) is tiles
+    # (32-bit sums in another order, a last place of float16)
+    assert (outs[0].float() - outs[1].float()).abs().max() < (4e-5 if dtype == torch.float32 else 4e-3)
