@@ -35,6 +35,14 @@ def test_recurrences_run_in_chunks_where_that_was_faster(lens, sizes, matrix, de
     assert k.mlstm_chunk_pays(p, *sizes) is matrix and k.gla_chunk_pays(p, *sizes) is decays
 
 
+def test_float32_products_that_stay_with_the_library():
+    k = K()
+    for (M, N, K_), split in (((511, 4096, 1024), True), ((17, 4096, 1024), True), ((17, 32768, 1024), False), ((17, 4096, 768), False),
+                              ((48, 6144, 1024), True), ((300, 256, 64), False), ((256, 1024, 256), False), ((1024, 1024, 256), True)):
+        x, w = torch.empty(M, K_, device="meta"), torch.empty(N, K_, device="meta")
+        assert k._split_pays(x, w) is split, (M, N, K_)
+
+
 @pytest.mark.parametrize("heads,n_state,pdim,groups", [(4, 128, 64, 1), (8, 64, 48, 2), (2, 256, 32, 1), (3, 32, 16, 3), (32, 128, 64, 1)])
 @pytest.mark.parametrize("lens", [[17], [64], [65, 3, 200], [150, 16, 1], [40] * 5])
 @pytest.mark.parametrize("single_row", [False, True])

@@ -777,13 +777,27 @@ class Kernels:
             return out
         if bias is None and self._lt_takes(x.shape[0], weight) and self.lt_linear(x, weight, out):
             return out
-        if x.dtype == torch.float32 and self.linear_f32_split(x, weight, out, bias):
+        if x.dtype == torch.float32 and self._split_pays(x, weight) and self.linear_f32_split(x, weight, out, bias):
             return out
         if bias is not None:
             torch.addmm(bias, x, weight.t(), out=out)
         else:
             torch.mm(x, weight.t(), out=out)
         return out
+
+    @staticmethod
+    def _split_pays(x, weight) -> bool:
+        """Where `linear_f32_split` takes a product and the library's is faster (weights from memory, us): short rows, where the
+        splitting of x and a tile's start are most of its time (k 64: at every size; k 256: 256 x 1,024 8.9 for 8.1, 1,024 x
+        1,024 faster; k 512: 1,024 x 256 12.7 for 11.9), and few rows over many columns (17 rows, 32,768 columns of k 1,024: 68.6
+        for 58.4; 4,096 of k 768: 23.0 for 21.3)."""
+        M, K = x.shape
+        N = weight.shape[0]
+        if K < 128 or (M <= 32 and (N > 16384 or (N >= 4096 and K < 1024))):
+            return False
+        if K < 512:
+            return M >= 128 and M * N > 1 << 19
+        return K >= 1024 or M * N > 1 << 18
 
     def linear_f32_split(self, x, weight, out, bias=None) -> bool:
         """out = x @ weight.T (+ bias) in float32 on the tensor cores, every operand as three bfloat16 terms
@@ -833,7 +847,7 @@ class Kernels:
         """out (float32) = x @ weight.T for x/weight in float32 or bfloat16."""
         _need(out, "out", torch.float32)
         if x.dtype == torch.float32:
-            if not self.linear_f32_split(x, weight, out):
+            if not (self._split_pays(x, weight) and self.linear_f32_split(x, weight, out)):
                 torch.mm(x, weight.t(), out=out)
             return out
         if self._own_linear(x, weight, out):
