@@ -134,3 +134,18 @@ def test_32_bit_attention_of_a_few_keys_stays_with_the_general_kernel(dtype, q_l
     assert bool(calls) is tiles
     # (32-bit sums in another order, a last place of float16)
     assert (outs[0].float() - outs[1].float()).abs().max() < (4e-5 if dtype == torch.float32 else 4e-3)
+
+
+@pytest.mark.parametrize("k_dim,n_out,launches", [(128, 256, 1), (256, 512, 1), (512, 512, 2), (1024, 256, 2)])
+def test_small_experts_stay_with_mma_sync(k_dim, n_out, launches):
+    kk, E, T = K(), 4, 40
+    x, w = torch.randn(T, k_dim, device="cuda").bfloat16(), (torch.randn(E, n_out, k_dim, device="cuda") * k_dim ** -0.5).bfloat16()
+    choice = (torch.arange(T, device="cuda") % E).int().view(T, 1)
+    offsets, order, place = (torch.zeros(n, dtype=torch.int32, device="cuda") for n in (E + 1, T, T))
+    kk.moe_arrange(choice, T, E, offsets, order, place)
+    out, gathered, before = torch.zeros(T, n_out, dtype=torch.bfloat16, device="cuda"), torch.zeros_like(x), kk.launches
+    kk.moe_grouped_linear(x, w, offsets, order, None, out, 1, True, False, gathered=gathered)
+    assert kk.launches - before == launches
+    ref = torch.stack([x[t].float() @ w[t % E].float().t() for t in range(T)])
+    # (one rounding to bfloat16 behind 32-bit sums)
+    assert (out[place.long()].float() - ref).abs().max() <= 2.0 ** -7 * ref.abs().max()
