@@ -15,7 +15,7 @@ engine dtype; z is a product with a 32-bit result.
 The state (S of every head, `gla_state_floats` floats) is one row per request slot in the cache manager's state
 rows; it is zeroed when a slot is handed out and carried from step to step.  One kernel runs the recurrence over
 any mix of prompt portions and single tokens (csrc/gla.cu); portions of more than CHUNK_LEAST tokens in bfloat16 run in
-chunks on the tensor cores (csrc/gla_chunk.cu).
+chunks on the tensor cores (csrc/gla_chunk.cu) in the steps where that is the faster form.
 """
 
 from __future__ import annotations

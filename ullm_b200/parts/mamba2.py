@@ -24,7 +24,7 @@ from .linear import linear
 from .registry import register_mixer
 
 
-CHUNK_LEAST = 16  # requests that bring more tokens than this take the chunked form
+CHUNK_LEAST = 16  # requests that bring more tokens than this may take a chunked form
 
 
 def _up4(n: int) -> int:

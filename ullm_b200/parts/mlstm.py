@@ -15,7 +15,8 @@ dtype; the gate projections are a product of their own with a 32-bit result.
 The state (S, n, m of every head, `Kernels.mlstm_state_floats` floats) is one row per request slot in the cache
 manager's state rows; it is zeroed when a slot is handed out and carried from step to step.  One kernel runs the
 recurrence over any mix of prompt portions and single tokens (csrc/mlstm.cu); portions of more than CHUNK_LEAST tokens
-in bfloat16 run in chunks on the tensor cores (csrc/mlstm_chunk.cu), whose results differ by 32-bit rounding.
+in bfloat16 run in chunks on the tensor cores (csrc/mlstm_chunk.cu), whose results differ by 32-bit rounding, in the steps where
+that is the faster form.
 """
 
 from __future__ import annotations
