@@ -115,133 +115,140 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
   }
   float m[4], l[4];
   float4 o[4][CV];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    m[i] = -INFINITY;
-    l[i] = 0.f;
-#pragma unroll
-    for (int c = 0; c < CV; ++c) o[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
   const int* bt = block_table + (long long)req_slots[r] * max_pages;
   const long long kv_row = (long long)num_kv * D;
-  const int last = pos0 + (rows - 1) / gq, first_last = first_seen(last, window);
-  for (int base = max(0, first_seen(pos0, window)); base <= last; base += PT_KEYS) {
-    __syncthreads();  // (the tile before has been read; Q is in place)
-    if (tid < PT_KEYS) {
-      const int key = base + tid;
-      long long slot = -1;
-      if (key <= last) {
-        const int page = bt[key / page_size];
-        if (page < 0 || page >= num_pages) ullm_report(status, ULLM_STATUS_PAGE, t0 + row0, page);
-        else slot = (long long)page * page_size + key % page_size;
-      }
-      slot_s[tid] = slot;
+  const int last = pos0 + (rows - 1) / gq;
+  // A weight of zero must not meet a value that a row does not see and that is infinite or NaN: where an output is not finite, the
+  // tile's rows run once more, and each adds up only what it sees.
+  bool odd = false;
+#pragma unroll 1
+  for (;;) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      m[i] = -INFINITY;
+      l[i] = 0.f;
+#pragma unroll
+      for (int c = 0; c < CV; ++c) o[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    __syncthreads();
-    // A weight of zero must not meet a value that a row does not see and that is infinite or NaN: tiles that some row sees a part
-    // of only are searched for such values as they are loaded.
-    const bool part = base + PT_KEYS - 1 > pos0 || base < first_last;
-    bool odd = false;
-#pragma unroll 4
-    for (int i = tid; i < PT_KEYS * (D / 4); i += PT_THREADS) {
-      const int key = i / (D / 4), e = (i - key * (D / 4)) * 4;
-      const long long slot = slot_s[key];
-      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-      if (slot >= 0) {
-        const long long at = slot * kv_row + (long long)kh * D + e;
-        a = pl_load4(k_cache + at);
-        b = pl_load4(v_cache + at);
+    for (int base = max(0, first_seen(pos0, window)); base <= last; base += PT_KEYS) {
+      __syncthreads();  // (the tile before has been read; Q is in place)
+      if (tid < PT_KEYS) {
+        const int key = base + tid;
+        long long slot = -1;
+        if (key <= last) {
+          const int page = bt[key / page_size];
+          if (page < 0 || page >= num_pages) ullm_report(status, ULLM_STATUS_PAGE, t0 + row0, page);
+          else slot = (long long)page * page_size + key % page_size;
+        }
+        slot_s[tid] = slot;
       }
-      *reinterpret_cast<float4*>(ks + key * ST + e) = a;
-      *reinterpret_cast<float4*>(vs + key * ST + e) = b;
-      if (part) odd |= pl_odd(b);
-    }
-    if (part) odd = __syncthreads_or(odd);
-    else __syncthreads();
-    // scores of rows 4 ty .. + 3 against keys tx, tx + 16, tx + 32, tx + 48
-    float s[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+      __syncthreads();
 #pragma unroll 4
-    for (int e = 0; e < D; e += 4) {
-      float4 a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(qs + (ty * 4 + i) * ST + e);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * ST + e);
+      for (int i = tid; i < PT_KEYS * (D / 4); i += PT_THREADS) {
+        const int key = i / (D / 4), e = (i - key * (D / 4)) * 4;
+        const long long slot = slot_s[key];
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (slot >= 0) {
+          const long long at = slot * kv_row + (long long)kh * D + e;
+          a = pl_load4(k_cache + at);
+          b = pl_load4(v_cache + at);
+        }
+        *reinterpret_cast<float4*>(ks + key * ST + e) = a;
+        *reinterpret_cast<float4*>(vs + key * ST + e) = b;
+      }
+      __syncthreads();
+      // scores of rows 4 ty .. + 3 against keys tx, tx + 16, tx + 32, tx + 48
+      float s[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s[i][j] = pl_dot(a[i], b[j], s[i][j]);
-    }
-    bool there[4];
+        for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 4
+      for (int e = 0; e < D; e += 4) {
+        float4 a[4], b[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) there[j] = slot_s[tx + 16 * j] >= 0;
+        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(qs + (ty * 4 + i) * ST + e);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float top = -INFINITY;
+        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * ST + e);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int key = base + tx + 16 * j;
-        s[i][j] = (there[j] && key >= first[i] && key <= pos[i]) ? s[i][j] * scale : -INFINITY;
-        top = fmaxf(top, s[i][j]);
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s[i][j] = pl_dot(a[i], b[j], s[i][j]);
       }
+      bool there[4];
 #pragma unroll
-      for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
-      const float m2 = fmaxf(m[i], top);
-      const float keep = m2 == -INFINITY ? 1.f : expf(m[i] - m2);  // (no key seen yet: nothing to rescale)
-      float sum = 0.f;
+      for (int j = 0; j < 4; ++j) there[j] = slot_s[tx + 16 * j] >= 0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float p = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m2);
-        ps[(ty * 4 + i) * PT_PS + tx + 16 * j] = p;
-        sum += p;
+      for (int i = 0; i < 4; ++i) {
+        float top = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int key = base + tx + 16 * j;
+          s[i][j] = (there[j] && key >= first[i] && key <= pos[i]) ? s[i][j] * scale : -INFINITY;
+          top = fmaxf(top, s[i][j]);
+        }
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
+        const float m2 = fmaxf(m[i], top);
+        const float keep = m2 == -INFINITY ? 1.f : expf(m[i] - m2);  // (no key seen yet: nothing to rescale)
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float p = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m2);
+          ps[(ty * 4 + i) * PT_PS + tx + 16 * j] = p;
+          sum += p;
+        }
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+        l[i] = l[i] * keep + sum;
+        m[i] = m2;
+#pragma unroll
+        for (int c = 0; c < CV; ++c) o[i][c].x *= keep, o[i][c].y *= keep, o[i][c].z *= keep, o[i][c].w *= keep;
       }
-#pragma unroll
-      for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-      l[i] = l[i] * keep + sum;
-      m[i] = m2;
-#pragma unroll
-      for (int c = 0; c < CV; ++c) o[i][c].x *= keep, o[i][c].y *= keep, o[i][c].z *= keep, o[i][c].w *= keep;
-    }
-    __syncwarp();  // (a row's weights are written and read by the 16 lanes that own the row)
-    if (odd) {
+      __syncwarp();  // (a row's weights are written and read by the 16 lanes that own the row)
+      if (odd) {  // each row adds up the keys that it sees
 #pragma unroll 1
-      for (int key = 0; key < PT_KEYS; ++key) {
-        if (slot_s[key] < 0) continue;
+        for (int key = 0; key < PT_KEYS; ++key) {
+          if (slot_s[key] < 0) continue;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (base + key < first[i] || base + key > pos[i]) continue;
-          const float p = ps[(ty * 4 + i) * PT_PS + key];
+          for (int i = 0; i < 4; ++i) {
+            if (base + key < first[i] || base + key > pos[i]) continue;
+            const float p = ps[(ty * 4 + i) * PT_PS + key];
 #pragma unroll
-          for (int c = 0; c < CV; ++c) pl_axpy(p, *reinterpret_cast<const float4*>(vs + key * ST + c * 64 + tx * 4), o[i][c]);
+            for (int c = 0; c < CV; ++c) pl_axpy(p, *reinterpret_cast<const float4*>(vs + key * ST + c * 64 + tx * 4), o[i][c]);
+          }
+        }
+        __syncwarp();
+        continue;
+      }
+#pragma unroll 2
+      for (int key = 0; key < PT_KEYS; key += 4) {
+        float4 p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(ps + (ty * 4 + i) * PT_PS + key);
+#pragma unroll
+        for (int c = 0; c < CV; ++c) {
+          const float* vp = vs + key * ST + c * 64 + tx * 4;
+          const float4 v0 = *reinterpret_cast<const float4*>(vp), v1 = *reinterpret_cast<const float4*>(vp + ST),
+                       v2 = *reinterpret_cast<const float4*>(vp + 2 * ST), v3 = *reinterpret_cast<const float4*>(vp + 3 * ST);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            pl_axpy(p[i].x, v0, o[i][c]);
+            pl_axpy(p[i].y, v1, o[i][c]);
+            pl_axpy(p[i].z, v2, o[i][c]);
+            pl_axpy(p[i].w, v3, o[i][c]);
+          }
         }
       }
       __syncwarp();
-      continue;
     }
-#pragma unroll 2
-    for (int key = 0; key < PT_KEYS; key += 4) {
-      float4 p[4];
+    bool bad = false;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(ps + (ty * 4 + i) * PT_PS + key);
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int c = 0; c < CV; ++c) {
-        const float* vp = vs + key * ST + c * 64 + tx * 4;
-        const float4 v0 = *reinterpret_cast<const float4*>(vp), v1 = *reinterpret_cast<const float4*>(vp + ST),
-                     v2 = *reinterpret_cast<const float4*>(vp + 2 * ST), v3 = *reinterpret_cast<const float4*>(vp + 3 * ST);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          pl_axpy(p[i].x, v0, o[i][c]);
-          pl_axpy(p[i].y, v1, o[i][c]);
-          pl_axpy(p[i].z, v2, o[i][c]);
-          pl_axpy(p[i].w, v3, o[i][c]);
-        }
-      }
-    }
-    __syncwarp();
+      for (int c = 0; c < CV; ++c) bad |= pl_odd(o[i][c]);
+    if (odd || !__syncthreads_or(bad)) break;
+    odd = true;
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
