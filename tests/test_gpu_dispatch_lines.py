@@ -117,7 +117,7 @@ def test_latent_attention_by_rows_and_keys_in_sight(H, dk, dv, n, kv, window, pa
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
-@pytest.mark.parametrize("q_lens,kv_lens,tiles", [([2], [2], False), ([8, 16], [8, 16], False), ([17], [17], True), ([8], [300], True), ([1, 1], [5, 9], True)])
+@pytest.mark.parametrize("q_lens,kv_lens,tiles", [([2], [2], False), ([8, 16], [8, 16], False), ([16] * 33, [16] * 33, True), ([17], [17], True), ([8], [300], True), ([1, 1], [5, 9], True)])
 def test_32_bit_attention_of_a_few_keys_stays_with_the_general_kernel(dtype, q_lens, kv_lens, tiles):
     k, calls, outs = K(), [], []
     bt, pages, slots, cu, lens, req, ctx = paged(q_lens, kv_lens)

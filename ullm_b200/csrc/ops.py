@@ -2685,9 +2685,10 @@ class Kernels:
         self.attention_path = "generic"
         # 32-bit arithmetic at head sizes 64 and 128 (float32, float16): keys staged once for many rows; the kernel of one warp
         # per row stays for every other size (per layer at Qwen3-0.6B sizes, prompts of 170 + 341 tokens: 76 against 749 us)
-        # (prompts of up to 16 tokens stay with that kernel: 2 / 8 / 17 tokens, 16 query heads of 128: 6.9 / 9.6 / 13.7 us there, 13.5
-        # / 14.0 / 15.0 by tiles of 64 keys)
-        short = ctx is not None and ctx.max_q_len > 1 and ctx.max_kv_len <= 16
+        # (prompts of up to 16 tokens stay with that kernel while its warps, one per row, fit the chip: 2 / 8 / 17 tokens, 16 query heads
+        # of 128: 6.9 / 9.6 / 13.7 us there, 13.5 / 14.0 / 15.0 by tiles of 64 keys; 16 prompts of 8 tokens, 16 / 32 heads: 14.4 /
+        # 24.0 and 19.8 / 19.9)
+        short = ctx is not None and ctx.max_q_len > 1 and ctx.max_kv_len <= 16 and T * num_q <= 2048
         if (self.plain_attention_on and not short
                 and self.lib.ullm_attention_plain_supported(_DT[qkv.dtype], head_dim, num_q, num_kv)):
             code = self.lib.ullm_attention_plain(
