@@ -106,3 +106,31 @@ def test_blocks_with_many_tiles_use_their_accumulators_again(gated, act):
     ref = reference(x, w, choice.cpu(), None, 1, True, gated, act, 0.0, 1.0, at)
     # (one rounding to bfloat16 behind 32-bit sums of 136 products, as above)
     assert (out[at].float() - ref).abs().max().item() <= (2 ** -8 + 1e-4) * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("act", [0, 2])
+def test_gates_that_are_almost_shut(act):
+    """Denominators 1 + e^-z up to the largest 32-bit number: silu(-88) is -5.3e-37 and no zero, as in the mma.sync kernel."""
+    kk, n_out, k, rows = K(), 64, 64, 20
+    z = torch.tensor([-86.0, -87.0, -87.5, -88.0, -88.5, -90.0, -1.0, 3.0]).repeat(n_out // 8)  # (bfloat16 holds them)
+    w = torch.zeros(1, 2 * n_out, k)
+    w[0, :n_out, 0], w[0, n_out:, 0] = z, 1024.0
+    w, x = w.to(torch.bfloat16).cuda(), torch.zeros(rows, k, dtype=torch.bfloat16, device="cuda")
+    x[:, 0] = 1
+    choice = torch.zeros(rows, 1, dtype=torch.int32, device="cuda")
+    offsets = torch.empty(2, dtype=torch.int32, device="cuda")
+    order, place = (torch.zeros(rows, 1, dtype=torch.int32, device="cuda") for _ in range(2))
+    kk.moe_arrange(choice, rows, 1, offsets, order, place)
+    outs, old = [], kk.moe_tcgen05_rows
+    try:
+        for kk.moe_tcgen05_rows in (0, 1 << 30):
+            outs.append(torch.full((rows, n_out), 9.0, dtype=torch.bfloat16, device="cuda"))
+            kk.moe_grouped_linear(x, w, offsets, order, None, outs[-1], 1, True, True, act, 2000.0, 1.0, gathered=torch.empty_like(x))
+    finally:
+        kk.moe_tcgen05_rows = old
+    kk.raise_on_status()
+    z64 = z.double().cuda()
+    ref = torch.where(z64 < -88.72, 0.0, z64 / (1 + torch.exp(-z64)) * (1024 + (act == 2)))
+    # one rounding to bfloat16, whose 8 bits make half a unit up to 2^-8 of a value, behind a 32-bit gate (some units of 2^-24)
+    for out in outs:
+        assert ((out.double() - ref).abs() <= (2 ** -8 + 1e-6) * ref.abs()).all()

@@ -49,3 +49,17 @@ def test_gated_add(dtype, limit, rows, cols, shift, both):
     K().gated_add_f32(a, f if both else None, g, b1, b2 if both else None, stream, copy)
     assert (stream.double() - ref).abs().max().item() <= 1e-6 * max(1.0, ref.abs().max().item())
     assert (copy.double() - ref).abs().max().item() <= limit * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_gated_add_through_gates_that_are_almost_shut(shift):
+    """Denominators 1 + e^-z up to the largest 32-bit number: the quotient is that of a division (infinite ones give zero)."""
+    z = torch.tensor([-60.0, -87.0, -87.3, -87.4, -87.5, -88.0, -88.5, -88.7, -89.0, -200.0], dtype=torch.float64).repeat(4)
+    a = torch.tensor([1.0, -3.0, 1e30, -3e38], dtype=torch.float32).repeat_interleave(10)
+    g, a = (torch.cat([torch.zeros(shift), v.float()]).cuda()[shift:].view(1, 40) for v in (z, a))  # (shift: off the 16-byte border)
+    stream = torch.zeros(1, 40, device="cuda")
+    K().gated_add_f32(a, None, g, torch.zeros(40, device="cuda"), None, stream)
+    z64 = g.double()
+    ref = torch.where(z64 < -88.72, 0.0, a.double() / (1 + torch.exp(-z64)))
+    # a 32-bit exponential (2 units) and a quotient (2 more), 2^-24 each; results under 2^-126 by its smallest steps
+    assert ((stream.double() - ref).abs() <= 4e-7 * ref.abs() + 3e-45).all()

@@ -93,12 +93,14 @@ __device__ __forceinline__ float act_gelu_tanh(float g) {
 }
 
 // g / (1 + e^-z) without a branch, so that a thread's elements run beside one another (a division's slow path keeps them in
-// series): a reciprocal and one step of Newton's method; from 2^126 on the denominator counts as infinite.  gelu_tanh is this with
-// z = 2 sqrt(2 / pi) (g + 0.044715 g^3), since (1 + tanh v) / 2 = 1 / (1 + e^-2v).
+// series): a reciprocal and one step of Newton's method, of a quarter of both sides where the denominator is beyond what the
+// fast quotient takes (2^126).  gelu_tanh is this with z = 2 sqrt(2 / pi) (g + 0.044715 g^3), since (1 + tanh v) / 2 =
+// 1 / (1 + e^-2v).
 __device__ __forceinline__ float gate_flat(float g, float z) {
-  const float y = 1.f + expf(-z), r = __fdividef(1.f, y), q = g * r;
-  const float s = fabsf(g) <= 3.4028234e38f ? fmaf(fmaf(-q, y, g), r, q) : q;
-  return y < 8.5e37f ? s : (y == y ? g * 0.f : y);
+  const float whole = 1.f + expf(-z), part = whole < 8.5e37f ? 1.f : 0.25f;
+  const float y = whole * part, x = g * part, r = __fdividef(1.f, y), q = x * r;
+  const float s = fabsf(g) <= 3.4028234e38f ? fmaf(fmaf(-q, y, x), r, q) : q;
+  return whole <= 3.4028234e38f ? s : (whole == whole ? g * 0.f : whole);
 }
 __device__ __forceinline__ float act_gelu_tanh_flat(float g) {
   return gate_flat(g, 1.5957691216057308f * (g + 0.044715f * g * g * g));
