@@ -47,9 +47,19 @@ __device__ __forceinline__ void ms_store(const MsParams& p, int at, int col, flo
   p.out[(size_t)at * p.n_out + col] = __float2bfloat16_rn(y);
 }
 
+// A result that goes to several places.  (Not inlined: sixteen copies of it in the tail of every unit made the kernel's code eight
+// times as long.)
+__device__ __noinline__ void ms_store_many(const MsParams& p, int lo, int n_e, int token, int col, float r, float up) {
+#pragma unroll 1
+  for (int q = 0; q < n_e; ++q) {
+    const int pair = p.sorted[lo + q];
+    if (pair / p.top == token) ms_store(p, lo + q, col, r, up, p.pair_weight != nullptr ? p.pair_weight[pair] : 1.f);
+  }
+}
+
 template <int NT>
 __global__ void __launch_bounds__(LS_THREADS, 2)
-moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const MsParams p) {
+moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ MsParams p) {
   constexpr int X_BOX_BYTES = 8 * NT * 128;  // 8 NT rows x 64 k
   constexpr int STAGE_BYTES = LS_W_STAGE_BYTES + 4 * X_BOX_BYTES;
   extern __shared__ unsigned char ms_smem_raw[];
@@ -221,10 +231,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
             if (many_s == 0) {
               if (place_s[m] >= 0) ms_store(p, place_s[m], col, r[i], up[i], scale_s[m]);
             } else {
-              for (int q = 0; q < n_e; ++q) {
-                const int pair = p.sorted[lo + q];
-                if (pair / p.top == m) ms_store(p, lo + q, col, r[i], up[i], p.pair_weight != nullptr ? p.pair_weight[pair] : 1.f);
-              }
+              ms_store_many(p, lo, n_e, m, col, r[i], up[i]);
             }
           }
         }
