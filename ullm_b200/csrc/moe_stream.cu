@@ -162,8 +162,11 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
             if (p.pair_weight != nullptr) scale_s[col] = p.pair_weight[pair];
           }
         }
-        const bool twice = __popc(__match_any_sync(0xffffffffu, col)) > 1 || n_e > 32;
-        const bool many = __any_sync(0xffffffffu, twice);
+        bool many = n_e > 32;
+        if (p.from_tokens) {  // (as many tokens as places, unless one comes twice)
+          const unsigned seen = __reduce_or_sync(0xffffffffu, col < MS_MAX_TOKENS ? 1u << col : 0u);
+          many |= __popc(seen) != __popc(__ballot_sync(0xffffffffu, col < MS_MAX_TOKENS));
+        }
         if (lane == 0) many_s = many ? 1 : 0;  // (some token's result goes to several places)
       }
       float acc[NT][4];
