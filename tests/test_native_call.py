@@ -1,0 +1,111 @@
+"""The calls from Python into the compiled library (csrc/native_call.cpp): arguments as the launchers get them, tensors checked as
+the Python check does; on a GPU the library's product as `torch.mm` forms it."""
+
+import ctypes
+
+import pytest
+import torch
+
+from ullm_b200.csrc import launchers, ops
+from ullm_b200.csrc.build import load_native
+
+
+@pytest.fixture(scope="module")
+def native():
+    module = load_native()
+    module.set_slow_need(ops._checked)
+    return module
+
+
+def test_arguments_arrive_as_ctypes_passes_them(native):
+    """Each kind of argument, past the registers too, in the order and width of a launcher's declaration."""
+    seen = []
+    kinds = {launchers.P: ctypes.c_void_p, launchers.I: ctypes.c_int, launchers.F: ctypes.c_float, launchers.LL: ctypes.c_longlong}
+    name = "ullm_window_attention"  # the longest mixed list
+    types = launchers.LAUNCHERS[name]
+    target = ctypes.CFUNCTYPE(ctypes.c_int, *[kinds[t] for t in types])(lambda *a: seen.append(a) or -7)
+    fn = native.bind(name, ctypes.cast(target, ctypes.c_void_p).value)
+    t = torch.zeros(5)
+    given = [{"P": 1 << 40 | i, "I": -i, "F": 0.1 * i, "LL": -(1 << 40) - i}[k] for i, k in enumerate(types)]
+    pointers = [i for i, k in enumerate(types) if k == "P"]
+    given[pointers[0]], given[pointers[1]], given[types.index("I")] = None, t, (1 << 32) + 3  # (an int is cut to 32 bits)
+    assert fn(*given) == -7
+    want = list(given)
+    want[pointers[1]], want[types.index("I")] = t.data_ptr(), 3
+    want = [ctypes.c_float(w).value if k == "F" else w for w, k in zip(want, types)]
+    assert list(seen[0]) == want
+    for wrong in (given[:-1], given + [0], ["x", *given[1:]], [1.5, *given[1:]]):
+        with pytest.raises(TypeError):
+            fn(*wrong)
+    with pytest.raises(TypeError):
+        fn(*given[:-1], last=0)
+    with pytest.raises(KeyError):
+        native.bind("ullm_no_such_launcher", 1)
+
+
+def test_addresses_and_checks(native):
+    t = torch.zeros(4, 6)
+    assert native.ptr(None) is None and native.ptr(t[1:]) == t.data_ptr() + 24
+    for args, kw in (((t, "x"), {}), ((t, "x", torch.float32), {}), ((t, "x"), {"dtype": torch.int32, "contiguous": False})):
+        with pytest.raises(ops.KernelError, match="x is on cpu"):
+            native.need(*args, **kw)
+    with pytest.raises(AttributeError):
+        native.need(None, "x")
+    with pytest.raises(TypeError):
+        native.need(t)
+
+
+def test_every_entry_of_the_table_is_in_the_library(native):
+    from ullm_b200.csrc.build import build
+
+    dll = ctypes.CDLL(build(verbose=False))
+    for name in (*launchers.LAUNCHERS, *launchers.QUERIES):
+        native.bind(name, ctypes.cast(getattr(dll, name), ctypes.c_void_p).value)
+
+
+@pytest.mark.gpu
+@pytest.mark.needs_cuda
+def test_checks_on_the_device(native):
+    t = torch.zeros(4, 6, device="cuda")
+    assert native.need(t, "x") is None and native.need(t, "x", torch.float32, False) is None
+    assert native.need(t[:, 1:], "x", torch.float32, contiguous=False) is None
+    with pytest.raises(ops.KernelError, match="dtype"):
+        native.need(t, "x", torch.bfloat16)
+    with pytest.raises(ops.KernelError, match="contiguous"):
+        native.need(t[:, 1:], "x", dtype=torch.float32)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        assert native.stream() == side.cuda_stream
+    assert native.stream() == torch.cuda.current_stream().cuda_stream
+
+
+@pytest.mark.gpu
+@pytest.mark.needs_cuda
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("M,N,K", [(2, 2, 2), (17, 8, 7), (33, 1000, 129), (511, 4096, 1024), (1426, 1024, 3072), (2048, 8, 2048)])
+def test_the_product_is_torchs(native, M, N, K, wide):
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    w = torch.randn(N, K, device="cuda").bfloat16()
+    out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float32 if wide else torch.bfloat16)
+    assert native.mm(x, w, out) is True
+    want = torch.mm(x, w.t(), out_dtype=torch.float32) if wide else torch.mm(x, w.t())
+    assert torch.equal(out, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.needs_cuda
+def test_what_the_product_leaves_to_torch(native):
+    x, w = torch.zeros(4, 8, device="cuda").bfloat16(), torch.zeros(6, 8, device="cuda").bfloat16()
+    out = torch.ones(4, 6, device="cuda").bfloat16()
+    for a, b, c in ((x[:1], w, out[:1]), (x[:, 1:], w[:, 1:], out), (x, w[:, ::2], out), (x.float(), w, out), (x, w.half(), out),
+                    (x, w, out.t().contiguous().t()), (x, w, out.half()), (x[:0], w, out[:0]), (x[:, :0], w[:, :0], out), (x.cpu(), w, out),
+                    (x[None], w, out), (x, w[:5], out)):
+        assert native.mm(a, b, c) is False
+    before = torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction
+    torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
+    try:
+        assert native.mm(x, w, out) is False
+    finally:
+        torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = before
+    assert torch.equal(out, torch.ones_like(out))

@@ -1,6 +1,7 @@
 """Compiles the CUDA sources of this folder for sm_100a into one shared
 library and finds it again.  Plain nvcc, no torch headers: a file compiles in
-seconds.  The library lies in `<this folder>/build/` (or, if that cannot be
+seconds.  (native_call.cpp, the calls from Python into that library, is an
+extension module of its own, built by g++ with torch's headers.)  The library lies in `<this folder>/build/` (or, if that cannot be
 written, in $ULLM_B200_BUILD_DIR or a per-user temporary folder) next to a
 stamp of the sources' hash; it is rebuilt when a source or a flag changes.
 """
@@ -8,10 +9,13 @@ stamp of the sources' hash; it is rebuilt when a source or a flag changes.
 from __future__ import annotations
 
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -19,6 +23,8 @@ from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_NAME = "libullm_b200.so"
+NATIVE_NAME = "ullm_b200_native.so"
+NATIVE_FLAGS = ["-O2", "-std=c++17", "-fPIC"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 
@@ -70,17 +76,18 @@ def _writable_dir() -> str:
     raise RuntimeError("no writable folder for the compiled kernels (set ULLM_B200_BUILD_DIR)")
 
 
-def find_built() -> str | None:
-    want = source_hash()
+def _candidates() -> list[str]:
     cands = [os.environ.get("ULLM_B200_BUILD_DIR"), os.path.join(HERE, "build")]
     try:
         cands.append(os.path.join(tempfile.gettempdir(), f"ullm_b200_build_{os.getuid()}"))
     except AttributeError:
         pass
-    for d in cands:
-        if not d:
-            continue
-        lib, stamp = os.path.join(d, LIB_NAME), os.path.join(d, "stamp")
+    return [d for d in cands if d]
+
+
+def _find(name: str, stamp_name: str, want: str) -> str | None:
+    for d in _candidates():
+        lib, stamp = os.path.join(d, name), os.path.join(d, stamp_name)
         if os.path.isfile(lib) and os.path.isfile(stamp):
             with open(stamp) as f:
                 if f.read().strip() == want:
@@ -88,9 +95,71 @@ def find_built() -> str | None:
     return None
 
 
+def find_built() -> str | None:
+    return _find(LIB_NAME, "stamp", source_hash())
+
+
+def native_hash() -> str:
+    import torch
+
+    h = hashlib.sha256()
+    for f in ("native_call.cpp", "launchers.py"):
+        with open(os.path.join(HERE, f), "rb") as fh:
+            h.update(fh.read())
+    h.update(f"{torch.__version__} {sys.version} {NATIVE_FLAGS}".encode())
+    return h.hexdigest()[:16]
+
+
+def build_native(verbose: bool = True, force: bool = False) -> str:
+    """The path of an up-to-date extension module of native_call.cpp, compiling if needed (ten seconds)."""
+    import torch
+
+    from .launchers import call_table
+
+    want = native_hash()
+    if not force:
+        lib = _find(NATIVE_NAME, "native_stamp", want)
+        if lib:
+            return lib
+    out_dir = _writable_dir()
+    home = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    with tempfile.TemporaryDirectory(dir=out_dir) as work:
+        with open(os.path.join(work, "native_table.inc"), "w") as f:
+            f.write(call_table())
+        tmp = os.path.join(work, NATIVE_NAME)
+        cmd = [os.environ.get("CXX", "g++"), *NATIVE_FLAGS, "-shared", "-I", work, "-I", os.path.join(home, "include"),
+               "-I", os.path.join(home, "include", "torch", "csrc", "api", "include"), "-I", sysconfig.get_paths()["include"],
+               "-I", cuda, os.path.join(HERE, "native_call.cpp"), "-o", tmp, "-L", os.path.join(home, "lib"), "-lc10", "-lc10_cuda",
+               "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+        if verbose:
+            print(f"[ullm_b200 build] compiling native_call.cpp into {out_dir}", file=sys.stderr, flush=True)
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed on native_call.cpp:\n{r.stdout}\n{r.stderr}")
+        lib = os.path.join(out_dir, NATIVE_NAME)
+        os.replace(tmp, lib)
+    with open(os.path.join(out_dir, "native_stamp"), "w") as f:
+        f.write(want)
+    return lib
+
+
+def load_native():
+    """The extension module of native_call.cpp."""
+    name = NATIVE_NAME.split(".")[0]
+    if name not in sys.modules:
+        path = build_native()
+        spec = importlib.util.spec_from_file_location(name, path, loader=importlib.machinery.ExtensionFileLoader(name, path))
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        sys.modules[name] = module
+    return sys.modules[name]
+
+
 def build(verbose: bool = True, force: bool = False) -> str:
     """Returns the path of an up-to-date library, compiling if needed.  Prints
     a line per file and a heartbeat every few seconds while nvcc runs."""
+    build_native(verbose, force)
     if not force:
         lib = find_built()
         if lib:

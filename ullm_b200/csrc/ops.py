@@ -1,5 +1,5 @@
-"""Python face of the compiled kernels: loads the shared library with ctypes
-and wraps each extern "C" launcher in a method that checks devices, dtypes,
+"""Python face of the compiled kernels: loads the shared library, binds its
+functions through native_call.cpp and wraps each extern "C" launcher in a method that checks devices, dtypes,
 shapes and contiguity before passing raw pointers and the current CUDA stream.
 
 There is no CPU path here: a tensor that is not on a CUDA device is an error,
@@ -15,7 +15,8 @@ from typing import NamedTuple
 
 import torch
 
-from .build import build
+from .build import build, load_native
+from .launchers import LAUNCHERS, QUERIES
 
 _DT = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
 _ERRORS = {
@@ -51,23 +52,7 @@ def check_attention_sizes(num_heads: int, num_kv_heads: int, head_dim: int, rota
         raise ValueError(f"rotary_dim={rotary_dim} must be even and at most head_dim={head_dim}")
 
 
-def _ptr(t: torch.Tensor | None) -> int | None:
-    return None if t is None else t.data_ptr()  # (a declared c_void_p argument takes an int or None as it is)
-
-
-# The current stream's handle as an int.  `torch.cuda.current_stream()` builds a Stream object and looks the device up through
-# the environment: 5 us a launch here, a quarter of a prompt step's host time at Qwen3-0.6B sizes; the raw query is 0.2 us.
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-_current_device = getattr(torch._C, "_cuda_getDevice", None)
-
-
-def _stream() -> int:
-    if _raw_stream is None or _current_device is None:
-        return torch.cuda.current_stream().cuda_stream
-    return _raw_stream(_current_device())
-
-
-def _need(t: torch.Tensor, name: str, dtype=None, contiguous: bool = True) -> None:
+def _checked(t: torch.Tensor, name: str, dtype=None, contiguous: bool = True) -> None:
     if t.is_cuda and (dtype is None or t.dtype == dtype) and (not contiguous or t.is_contiguous()):
         return
     if not t.is_cuda:
@@ -76,6 +61,10 @@ def _need(t: torch.Tensor, name: str, dtype=None, contiguous: bool = True) -> No
         raise KernelError(f"{name} has dtype {t.dtype}, expected {dtype}")
     if contiguous and not t.is_contiguous():
         raise KernelError(f"{name} must be contiguous")
+
+
+# the native forms (native_call.cpp), set when the library is loaded
+_ptr = _need = _stream = _native = None
 
 
 def _timed(group: str, nbytes=None, skipped=None):
@@ -142,13 +131,28 @@ def _weight_bytes(x, weight, *rest):
     return weight.numel() * weight.element_size()
 
 
+class _Library:
+    """The compiled library: its launchers and queries as calls of native_call.cpp, any other function through ctypes."""
+
+    def __init__(self, path: str):
+        global _ptr, _need, _stream, _native
+        self._dll = ctypes.CDLL(path)
+        _native = load_native()
+        _native.set_slow_need(_checked)
+        _ptr, _need, _stream = _native.ptr, _native.need, _native.stream
+        for name in (*LAUNCHERS, *QUERIES):
+            setattr(self, name, _native.bind(name, ctypes.cast(getattr(self._dll, name), c_void_p).value))
+
+    def __getattr__(self, name):
+        return getattr(self._dll, name)
+
+
 class Kernels:
     def __init__(self, lib_path: str | None = None):
         if not torch.cuda.is_available():
             raise KernelError("no CUDA device: this engine has no CPU path")
         self.lib_path = lib_path or build()
-        self.lib = ctypes.CDLL(self.lib_path)
-        self._declare()
+        self._declare(self.lib_path)
         self.status = torch.zeros(4, dtype=torch.int32, device="cuda")
         self.sm_count = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
         self._f32_out_mm = None
@@ -282,213 +286,11 @@ class Kernels:
         # 71 us against 70 us for the separate kernels at 8 rows, 77 against 70 at 16: no gain yet.
         self.fused_tail_rows = int(get("ULLM_B200_FUSED_TAIL_ROWS", "0"))
 
-    # -- ctypes signatures --------------------------------------------------
-    def _declare(self) -> None:
-        L = self.lib
-        P, I, F, LL = c_void_p, c_int, c_float, c_longlong
-        sig = {
-            "ullm_embedding": [I, P, P, P, I, I, I, P, P, P, P, P],
-            "ullm_gather_rows": [I, P, P, P, I, I, I, P, P],
-            "ullm_add_rmsnorm": [I, P, P, P, P, I, I, F, P],
-            "ullm_act_mul": [I, I, P, P, I, I, P],
-            "ullm_cast_bf16_f32": [P, P, LL, P],
-            "ullm_qk_norm_rope_store": [I, P, I, I, I, I, P, P, F, P, P, I, I, P, P, P, P, LL, P, P],
-            "ullm_qk_norm_in_place": [I, P, I, I, I, I, P, P, F, P, P],
-            "ullm_paged_attention_generic": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_attention_plain": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_attention_plain_supported": [I, I, I, I],
-            "ullm_decode_attention": [P, LL, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, I, LL, P, P],
-            "ullm_decode_attention_balanced": [P, LL, P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_decode_attention_fused": [P, LL, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, I, LL, P, P, F, P, P, I,
-                                            P, P, P, P],
-            "ullm_prefill_attention": [P, LL, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_prefill_attention_kept": [P, LL, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, LL, P, P, I],
-            "ullm_decode_attention_kept": [P, LL, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, I, LL, P, P, I],
-            "ullm_decode_attention_capped": [P, LL, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, I, LL, P, P, I, F],
-            "ullm_decode_attention_parts": [P, LL, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, I, LL, P, P, I],
-            "ullm_prefill_attention_ex": [P, LL, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, LL, P, P, I, F, P],
-            "ullm_prefill_attention_tcgen05": [P, LL, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_prefill_attention_pair": [P, LL, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_prefill_attention_pair_capped": [P, LL, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, LL, P, P, F],
-            "ullm_prefill_attention_pair_parts": [P, LL, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_prefill_attention_pair_biased": [P, LL, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, LL, P, P, P, I, P, LL],
-            "ullm_decode_attention_biased": [P, LL, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, I, LL, P, P, P, I, P, LL],
-            "ullm_linear_tcgen05": [P, P, P, P, I, I, I, I, I, P, LL, P, I, P, P],
-            "ullm_linear_skinny": [P, P, P, P, I, I, I, I, I, P],
-            "ullm_linear_stream": [P, P, P, P, P, I, I, I, I, I, P, P],
-            "ullm_linear_stream_norm": [P, P, P, P, P, I, I, I, I, I, P, P, P, P, I, I, F, P, P],
-            "ullm_layer_tail_fused": [P, P, P, P, P, P, P, P, F, I, I, I, I, I, P, P, P, P],
-            "ullm_linear_f32_split": [P, P, P, P, P, I, I, I, P, P],
-            "ullm_linear_tcgen05_large": [P, P, P, P, I, I, I, I, I, I, P, P],
-            "ullm_decode_attention_tcgen05": [P, LL, P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_lt_linear": [P, P, P, I, I, I, I, P, LL, I, P, LL, P],
-            "ullm_paged_attention_generic_ex": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, LL, P, P, I, I],
-            "ullm_qk_norm_rope_store_ex": [I, P, I, I, I, I, P, P, F, P, P, I, I, P, P, P, P, LL, P, P, I, I],
-            "ullm_act_mul_clamped": [I, P, P, I, I, F, F, P],
-            "ullm_embed_scaled": [I, P, P, P, P, I, I, I, F, P, P, P, P, P, P, P, P, I, LL, LL, P, LL, I, P],
-            "ullm_norm_scale_add": [I, P, P, P, P, I, I, F, F, P],
-            "ullm_norm_scale_add_norm": [I, P, P, P, I, I, F, F, P, F, P, P],
-            "ullm_rmsnorm_rows_f32": [I, P, P, P, P, I, I, I, F, P, P],
-            "ullm_cast_rows_f32": [I, P, P, LL, P],
-            "ullm_mlstm_recurrence": [I, P, LL, I, I, I, P, P, P, P, LL, P, P, P, P, I, I, I, I, F, F, I, P, P, I, P],
-            "ullm_mlstm_chunk": [P, LL, I, I, I, P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, F, F, I, I, P, P],
-            "ullm_mlstm_chunk_supported": [I, I, I],
-            "ullm_mlstm_out_gate": [I, P, P, LL, P, P, I, I, I, F, P],
-            "ullm_gated_add_f32": [I, P, P, P, LL, P, P, P, P, I, I, P],
-            "ullm_side_gate_mul": [I, P, P, P, LL, I, P, I, I, I, P, P, P, P, P],
-            "ullm_softcap_f32": [P, LL, F, P],
-            "ullm_qkv_prepare": [I, P, LL, I, I, I, I, I, P, I, P, LL, P, P, P, I, P, P, I, P, P, I, I, F, I, P, P, P, P,
-                                 P, LL, P, P, P, F, I],
-            "ullm_qkv_conv_prepare": [I, P, LL, I, I, I, I, I, P, I, P, LL, P, P, P, I, P, P, P, F, P, P, P, LL, P, P, F, I, I, P],
-            "ullm_conv_state_update": [I, P, LL, I, I, P, LL, P, P, P, I, I, P],
-            "ullm_paged_attention_generic_ex2": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, LL, P, P, I, I,
-                                                 F, P],
-            "ullm_mix_heads": [I, P, P, P, I, I, I, I, P],
-            "ullm_latent_attention": [P, LL, P, LL, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, LL, P, P],
-            "ullm_latent_attention_supported": [I, I, I, I, I],
-            "ullm_window_attention": [P, LL, P, LL, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, LL, P, P, P, I, P, P,
-                                      P, I, LL, P, LL, F, I, P, I, P, I],
-            "ullm_paged_attention_generic_ex3": [I, P, LL, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, F, LL, P, P, I, I,
-                                                 F, P, I, I, P, P, P, I, LL, P, LL, F, LL, I, P, I],
-            "ullm_norm_add_norm": [I, P, P, P, I, I, F, F, I, P, P, P, F, I, I, P, P, P, P],
-            "ullm_pair_norm_add_norm": [I, P, P, P, P, I, I, F, F, P, P, P, F, I, P, P, P, P, F, F, P],
-            "ullm_act_rows": [I, I, P, LL, P, LL, I, I, P],
-            "ullm_relu2": [I, P, P, LL, P],
-            "ullm_scale_f32": [P, LL, F, P],
-            "ullm_ssd_prepare": [I, P, LL, I, I, I, I, P, I, P, P, P, P, LL, I, P, P, P, I, P, P, P, I, P, P],
-            "ullm_ssd_recurrence": [I, P, LL, I, I, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, P, P, LL, I],
-            "ullm_ssd_chunk": [P, LL, I, I, P, P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, P, P, LL],
-            "ullm_ssd_chunk_short": [P, LL, I, I, P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, P, P, LL],
-            "ullm_ssd_gate_norm": [I, P, P, LL, P, P, I, I, I, F, P, I],
-            "ullm_norm_rows": [I, P, P, P, P, I, I, I, F, I, P, P, P, P],
-            "ullm_xielu": [I, P, P, LL, P, P],
-            "ullm_kv_shared_prepare": [I, P, LL, I, I, I, P, P, F, P, P, P, LL, P, P],
-            "ullm_pool_blocks": [I, P, P, P, P, I, I, LL, P, P, I, I, P, LL, P, P, I, I, P, P],
-            "ullm_latent_prepare": [I, P, P, P, P, I, I, I, I, I, I, P, F, P, P, P, P, LL, P, P, I, LL, LL],
-            "ullm_qkv_rows_prepare": [I, P, LL, P, I, I, I, I, I, P, P, F, P, I, I, P, P, I, P, P, P, LL, P, P],
-            "ullm_concat_rows_f32": [I, P, P, P, I, I, I, P],
-            "ullm_sigmoid_gate": [I, P, P, LL, I, I, P],
-            "ullm_mingru": [I, P, LL, I, I, I, P, P, P, LL, P, P, P, P, LL, F, I, I, I, P, P],
-            "ullm_gla_recurrence": [I, P, LL, I, I, I, P, LL, P, F, F, P, LL, P, P, P, P, I, I, I, I, I, I, P, P, P, I],
-            "ullm_ssd_step": [I, P, LL, I, I, P, P, P, P, LL, P, P, P, I, I, I, I, I, I, P, P, LL, I],
-            "ullm_gla_step": [I, P, LL, I, I, I, P, LL, P, F, F, P, LL, P, P, P, I, I, I, I, I, P, P, P],
-            "ullm_gla_decay": [P, LL, P, F, I, I, P],
-            "ullm_gla_chunk": [P, LL, I, I, I, P, LL, P, F, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, P, P],
-            "ullm_token_shift_mix": [I, P, LL, P, I, I, P, P, LL, I, P, P, P, I, I, P, P],
-            "ullm_low_rank_decay": [I, P, LL, I, I, P, P, P, I, I, I, P],
-            "ullm_linear_stream_grouped": [P, P, P, I, I, I, I, I, P, P],
-            "ullm_head_norm_gate": [I, P, P, LL, P, P, I, I, I, F, I, I, P],
-            "ullm_moe_route": [P, LL, P, P, P, I, I, I, I, I, I, I, F, I, P],
-            "ullm_moe_arrange": [P, I, I, P, P, P, P],
-            "ullm_moe_grouped_linear": [I, P, LL, P, LL, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P],
-            "ullm_moe_stream": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, P],
-            "ullm_moe_grouped_tcgen05": [P, LL, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, P],
-            "ullm_moe_combine": [I, P, P, P, P, I, I, I, P, I, P, LL, P, P, LL, P],
-            "ullm_moe_combine_add_norm": [I, P, P, P, I, I, I, P, I, P, LL, P, P, LL, P, P, P, F, P, P, P, P, P, F],
-            "ullm_argmax": [P, LL, I, I, P, P],
-            "ullm_sample": [P, LL, I, I, P, P, P, P, P, P, P, P, P, P],
-        }
-        for name, args in sig.items():
-            fn = getattr(L, name)
-            fn.argtypes = args
-            fn.restype = c_int
-        L.ullm_mingru_chunk.argtypes = []
-        L.ullm_mingru_chunk.restype = c_int
-        L.ullm_moe_force_plain.argtypes = [I]
-        L.ullm_moe_force_plain.restype = None
-        L.ullm_mlstm_supported.argtypes = [I, I, I]
-        L.ullm_mlstm_supported.restype = c_int
-        L.ullm_mlstm_state_floats.argtypes = [I, I, I]
-        L.ullm_mlstm_state_floats.restype = c_longlong
-        L.ullm_mlstm_chunk_floats.argtypes = [I, I, I, I, I, I]
-        L.ullm_mlstm_chunk_floats.restype = c_longlong
-        L.ullm_gla_supported.argtypes = [I, I, I]
-        L.ullm_gla_supported.restype = c_int
-        L.ullm_gla_state_floats.argtypes = [I, I, I]
-        L.ullm_gla_state_floats.restype = c_longlong
-        L.ullm_gla_chunk_v_tile.argtypes = [I, I]
-        L.ullm_gla_chunk_v_tile.restype = c_int
-        L.ullm_gla_chunk_per_sm.argtypes = [I, I]
-        L.ullm_gla_chunk_per_sm.restype = c_int
-        L.ullm_gla_chunk_supported.argtypes = [I, I, I]
-        L.ullm_gla_chunk_supported.restype = c_int
-        L.ullm_gla_chunk_tiles.argtypes = [I, I]
-        L.ullm_gla_chunk_tiles.restype = c_int
-        L.ullm_gla_chunk_floats.argtypes = [I, I, I]
-        L.ullm_gla_chunk_floats.restype = c_longlong
-        L.ullm_ssd_supported.argtypes = [I, I, I, I, I]
-        L.ullm_ssd_supported.restype = c_int
-        L.ullm_ssd_chunk_supported.argtypes = [I, I, I, I]
-        L.ullm_ssd_chunk_supported.restype = c_int
-        L.ullm_ssd_chunk_short_pays.argtypes = [I, I, I, I, I, I]
-        L.ullm_ssd_chunk_short_pays.restype = c_int
-        L.ullm_ssd_chunk_scratch.argtypes = [I, I, I, I, I, I]
-        L.ullm_ssd_chunk_scratch.restype = c_longlong
-        L.ullm_ssd_chunk_tokens.argtypes = []
-        L.ullm_ssd_chunk_tokens.restype = c_int
-        L.ullm_wait_selftest.argtypes = [I, P, P, P]
-        L.ullm_wait_selftest.restype = c_int
-        L.ullm_decode_attention_supported.argtypes = [I, I, I]
-        L.ullm_decode_attention_supported.restype = c_int
-        L.ullm_decode_attention_balanced_supported.argtypes = [I, I, I, I, I]
-        L.ullm_decode_attention_balanced_supported.restype = c_int
-        L.ullm_linear_f32_split_columns.argtypes = [I, I]
-        L.ullm_linear_f32_split_columns.restype = c_int
-        L.ullm_linear_f32_split_terms.argtypes = [I, I]
-        L.ullm_linear_f32_split_terms.restype = c_longlong
-        L.ullm_decode_attention_balanced_scratch_floats.argtypes = [I, I]
-        L.ullm_decode_attention_balanced_scratch_floats.restype = c_longlong
-        L.ullm_decode_attention_tcgen05_supported.argtypes = [I, I, I, I, I]
-        L.ullm_decode_attention_tcgen05_supported.restype = c_int
-        L.ullm_decode_attention_tcgen05_scratch_floats.argtypes = [I]
-        L.ullm_decode_attention_tcgen05_scratch_floats.restype = c_longlong
-        L.ullm_decode_attention_cluster_merge.argtypes = [I]
-        L.ullm_decode_attention_cluster_merge.restype = None
-        L.ullm_decode_attention_last_used_cluster.argtypes = []
-        L.ullm_decode_attention_last_used_cluster.restype = c_int
-        L.ullm_sample_force_one_block.argtypes = [I]
-        L.ullm_sample_force_one_block.restype = None
-        L.ullm_sample_last_used_cluster.argtypes = []
-        L.ullm_sample_last_used_cluster.restype = c_int
-        L.ullm_lt_available.argtypes = []
-        L.ullm_lt_available.restype = c_int
-        L.ullm_lt_last_choice.argtypes = [P, P, P, P]
-        L.ullm_lt_last_choice.restype = None
-        L.ullm_window_attention_supported.argtypes = [I, I, I, I, I, I]
-        L.ullm_window_attention_supported.restype = c_int
-        L.ullm_prefill_attention_supported.argtypes = [I, I, I]
-        L.ullm_prefill_attention_supported.restype = c_int
-        L.ullm_prefill_attention_tcgen05_supported.argtypes = [I, I, I, I]
-        L.ullm_prefill_attention_tcgen05_supported.restype = c_int
-        L.ullm_prefill_attention_tcgen05_blocks_per_sm.restype = c_int
-        L.ullm_prefill_attention_pair_supported.argtypes = [I, I, I, I]
-        L.ullm_prefill_attention_pair_supported.restype = c_int
-        L.ullm_set_pdl.argtypes = [I]
-        L.ullm_set_pdl.restype = None
-        L.ullm_linear_tcgen05_supported.argtypes = [I, I, I]
-        L.ullm_linear_tcgen05_supported.restype = c_int
-        L.ullm_linear_tcgen05_blocks.restype = c_int
-        L.ullm_linear_tcgen05_large_supported.argtypes = [I, I, I]
-        L.ullm_linear_tcgen05_large_supported.restype = c_int
-        L.ullm_linear_skinny_supported.argtypes = [I, I, I]
-        L.ullm_linear_skinny_supported.restype = c_int
-        L.ullm_layer_tail_fused_supported.argtypes = [I, I, I, I]
-        L.ullm_layer_tail_fused_supported.restype = c_int
-        L.ullm_layer_tail_fused_scratch_floats.argtypes = [I]
-        L.ullm_layer_tail_fused_scratch_floats.restype = c_longlong
-        L.ullm_layer_tail_fused_counters.argtypes = [I]
-        L.ullm_layer_tail_fused_counters.restype = c_longlong
-        L.ullm_layer_tail_fused_last_grid.restype = c_int
-        L.ullm_linear_stream_supported.argtypes = [I, I, I]
-        L.ullm_linear_stream_supported.restype = c_int
-        L.ullm_linear_stream_sq_floats.argtypes = [I]
-        L.ullm_linear_stream_sq_floats.restype = c_longlong
-        L.ullm_linear_stream_blocks_per_sm.argtypes = [I]
-        L.ullm_linear_stream_blocks_per_sm.restype = None
-        L.ullm_linear_stream_smem_kb.argtypes = [I]
-        L.ullm_linear_stream_smem_kb.restype = None
-        L.ullm_linear_stream_ksplit_max.argtypes = [I]
-        L.ullm_linear_stream_ksplit_max.restype = None
+    def _declare(self, path: str) -> None:
+        """`self.lib`: the library's functions, called through native_call.cpp (everything else of it through ctypes)."""
+        self.lib = _Library(path)
+        self.lib.ullm_lt_last_choice.argtypes = [c_void_p] * 4
+        self.lib.ullm_lt_last_choice.restype = None
 
     def _check(self, code: int, what: str) -> None:
         self.launches += 1
@@ -781,7 +583,7 @@ class Kernels:
             return out
         if bias is not None:
             torch.addmm(bias, x, weight.t(), out=out)
-        else:
+        elif not _native.mm(x, weight, out):
             torch.mm(x, weight.t(), out=out)
         return out
 
@@ -853,6 +655,8 @@ class Kernels:
         if self._own_linear(x, weight, out):
             return out
         if self._lt_takes(x.shape[0], weight) and self.lt_linear(x, weight, out):
+            return out
+        if _native.mm(x, weight, out):
             return out
         if self._f32_out_mm is None:
             try:
@@ -2384,12 +2188,13 @@ class Kernels:
 
     def _decode_rows(self, qkv, out, k_pages, v_pages, block_table, req_slots, kv_len, num_q, num_kv, head_dim,
                      page_size, window, scale, num_pages, ragged, ctx, fuse=None, keep_first: int = 0,
-                     softcap: float = 0.0, parts=None, dist_bias=None, head_gate=None) -> None:
-        """Decode attention of T one-token rows (row i belongs to request row i): streams the pages once.
+                     softcap: float = 0.0, parts=None, dist_bias=None, head_gate=None, rows: int | None = None) -> None:
+        """Decode attention of the first `rows` rows (default: all), one token each (row i belongs to request row i): streams
+        the pages once.
         `keep_first` > 0 (with a window), `softcap` > 0 (capped scores) or `parts` (every head's weights on every
         kv head's values, 32-bit [T, num_q * num_kv * head_dim]; `out` unused), `dist_bias` or `head_gate`: the per-request
         split kernel, the one that takes them."""
-        T = qkv.shape[0]
+        T = qkv.shape[0] if rows is None else rows
         choice = self._decode_choice(T, ragged, num_q, num_kv, head_dim, page_size, qkv.stride(0))
         if keep_first > 0 or softcap > 0 or parts is not None or dist_bias is not None or head_gate is not None:
             choice = "split"
@@ -2651,9 +2456,10 @@ class Kernels:
         if decode_ok and self.mixed_decode_rows > 0 and getattr(ctx, "cu_q_host", None) is not None:
             n_dec, ragged_head = self._decoded_head(ctx)
         if n_dec:
-            self._decode_rows(qkv[:n_dec], out[:n_dec], k_pages, v_pages, block_table, req_slots[:n_dec], kv_len[:n_dec],
-                              num_q, num_kv, head_dim, page_size, window, scale, num_pages, ragged_head, ctx)
-            req_slots, cu_q, kv_len = req_slots[n_dec:], cu_q[n_dec:], kv_len[n_dec:]
+            self._decode_rows(qkv, out, k_pages, v_pages, block_table, req_slots, kv_len, num_q, num_kv, head_dim, page_size,
+                              window, scale, num_pages, ragged_head, ctx, rows=n_dec)
+        # (int32 arrays in one piece, `_need` above: the entries behind the first n_dec by their address)
+        behind = tuple(_ptr(t) + 4 * n_dec for t in (req_slots, cu_q, kv_len))
         num_requests = (ctx.num_requests - n_dec) if ctx is not None else 0
         pair = single = False
         if ctx is not None and qkv.dtype == torch.bfloat16 and self.use_tcgen05_attention and qkv.stride(0) % head_dim == 0:
@@ -2665,7 +2471,7 @@ class Kernels:
             self.prefill_attention_kernel = "pair" if pair else "single"
             self._check(entry(
                 _ptr(qkv), qkv.stride(0), _ptr(out), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
-                block_table.shape[1], _ptr(req_slots), _ptr(cu_q), _ptr(kv_len), T, num_requests, num_q, num_kv,
+                block_table.shape[1], *behind, T, num_requests, num_q, num_kv,
                 head_dim, page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream()),
                 f"prefill_attention_tcgen05 (head_dim {head_dim})")
             self.attention_path = "prefill_tcgen05"
@@ -2675,7 +2481,7 @@ class Kernels:
                 and self.lib.ullm_prefill_attention_supported(head_dim, num_q, num_kv)):
             self._check(self.lib.ullm_prefill_attention(
                 _ptr(qkv), qkv.stride(0), _ptr(out), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
-                block_table.shape[1], _ptr(req_slots), _ptr(cu_q), _ptr(kv_len), T, num_requests, num_q, num_kv,
+                block_table.shape[1], *behind, T, num_requests, num_q, num_kv,
                 head_dim, page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream()),
                 f"prefill_attention (head_dim {head_dim})")
             self.attention_path = "prefill"

@@ -172,9 +172,10 @@ class RoutedExperts(FeedForward):
         rows = ws.tokens("moe.rows", T * top, self.H, x.dtype) if top == 1 else ws.get("moe.rows", T * top, self.H, x.dtype, reserve=ws.max_tokens * top)
         on_input = self.weight_on == "input"
         # (a choice at or beyond E, an expert that passes its input, gets no place: `moe_arrange` skips it)
-        K.moe_grouped_linear(x, self.w_gate_up[:E], offsets, order, weight if on_input else None, act, top, True, self.gated,
+        w_gate_up, w_down = (self.w_gate_up, self.w_down) if self.w_down.shape[0] == E else (self.w_gate_up[:E], self.w_down[:E])
+        K.moe_grouped_linear(x, w_gate_up, offsets, order, weight if on_input else None, act, top, True, self.gated,
                              self.act_code, self.limit, self.alpha, **({"gathered": rows} if x.is_cuda else {}))
-        K.moe_grouped_linear(act, self.w_down[:E], offsets, order, None, rows, top, False, False)
+        K.moe_grouped_linear(act, w_down, offsets, order, None, rows, top, False, False)
         shared = None
         if self.shared is not None and not always:
             shared = (self.shared.forward(x, ctx), logits[:, self.R:self.R + 1] if self.shared_gate else None)
