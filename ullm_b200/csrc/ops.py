@@ -173,13 +173,6 @@ class Kernels:
         self.attention_path = None  # which attention kernel the last call chose (tests read it)
         self.launches = 0  # hand-written kernels launched (graph replays add what they captured)
 
-    def begin_step(self, rows: int, dtype) -> None:
-        """Called by the step function before a step's kernels are launched (or recorded into a CUDA graph): with
-        the automatic policy, programmatic dependent launch is on for exactly the steps whose products are all the
-        stream kernel (bfloat16, at most `stream_all_rows` rows), and off otherwise."""
-        if self.pdl_mode == "auto":
-            self.set_pdl(bool(dtype == torch.bfloat16 and self.small_m_mode == "auto" and rows <= self.stream_all_rows))
-
     # -- switches -----------------------------------------------------------
     SWITCHES = ("ULLM_B200_PDL", "ULLM_B200_DECODE_SPLIT_TARGET", "ULLM_B200_TC_ATTN", "ULLM_B200_DECODE_CLUSTER",
                 "ULLM_B200_FUSE_DECODE_ROPE", "ULLM_B200_MIXED_DECODE_ROWS", "ULLM_B200_DECODE_TC",
@@ -195,13 +188,12 @@ class Kernels:
         """Sets every kernel choice from `env` (a mapping; the process environment at start-up): a switch that is
         not in it takes its default.  All switches are optional; the defaults are what was measured fastest."""
         get = env.get
-        # programmatic dependent launch for every kernel of the library: "auto" (the default) for the steps whose
-        # products are all the stream kernel (see `begin_step`), where its ring fills with weights while the kernel
-        # in front drains (Qwen3-8B sizes, batch 1: 3.60 -> 3.38 ms per step); "1" always, "0" never (with the
-        # library's products in between it costs 1 to 2 %: waiting blocks hold SM slots and gain nothing)
-        mode = get("ULLM_B200_PDL", "auto")
-        self.pdl_mode = {"1": True, "0": False}.get(mode, "auto")
-        self.set_pdl(self.pdl_mode is True)
+        # programmatic dependent launch for every kernel of the library ("0": never): a kernel's launch and set-up, and where it
+        # can its first weights, run beside the tail of the kernel in front, which takes most of the 2 us between two launches.
+        # us per step, off and on: Qwen3-8B sizes decode of 1 3,600 and 3,380 (the ring of the products fills early), prompt of
+        # 2,048 26,540 and 25,990, decode of 64 5,916 and 5,914; Qwen3-0.6B mixed step of 1,426 tokens 3,965 and 3,592, float32
+        # prompts 9,282 and 8,519; prompts of the other designs 1 to 5 % less
+        self.set_pdl(get("ULLM_B200_PDL", "1") != "0")
         # blocks the per-request decode attention aims for when it splits the requests' key ranges
         self.decode_split_target = int(get("ULLM_B200_DECODE_SPLIT_TARGET", "400"))
         # prompt attention on the tcgen05 tensor cores (head size 128); 0: the mma.sync kernel
