@@ -145,7 +145,6 @@ decode_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const
   __shared__ uint32_t tmem_slot;
   __shared__ float s_red[2][4][GP], s_lsum[4][GP];
   __shared__ int s_abort;
-  pdl_launch_dependents();
   pdl_wait();
   unsigned char* smem = (unsigned char*)(((uintptr_t)dtc_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* p_s = smem + DTC_STAGES * DTC_STAGE_BYTES;
@@ -204,6 +203,7 @@ decode_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const
                  "r"(DTC_TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -54,7 +54,6 @@ __global__ void __launch_bounds__(LA_THREADS, 1)
 latent_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const LaParams p) {
   // (no static shared memory, so that the dynamic region starts on a 1024-byte boundary; if it did not, the block would leave)
   extern __shared__ __align__(16) unsigned char la_raw[];
-  pdl_launch_dependents();
   if ((tp_smem(la_raw) & 1023u) != 0) {
     if (threadIdx.x == 0) ullm_report(p.status, ULLM_STATUS_TIMEOUT, 60, (int)(tp_smem(la_raw) & 1023u));
     return;
@@ -121,6 +120,7 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tp_smem(&tmem_slot)), "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -85,7 +85,6 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
   // No static shared memory: the tiles need a 1024-byte boundary (128-byte swizzle), and the dynamic region of a
   // block without static shared memory starts on one.  If it ever did not, the block says so and leaves.
   extern __shared__ __align__(16) unsigned char tp_raw[];
-  pdl_launch_dependents();
   if ((tp_smem(tp_raw) & 1023u) != 0) {
     if (threadIdx.x == 0) ullm_report(p.status, ULLM_STATUS_TIMEOUT, 20, (int)(tp_smem(tp_raw) & 1023u));
     return;
@@ -174,6 +173,7 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                  "r"(TP_TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -194,7 +194,6 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   // The tiles need a 1024-byte boundary (128-byte swizzle); the dynamic region of a block that has no static
   // shared memory starts on one.  If it ever did not, the block says so and leaves.
   extern __shared__ __align__(16) unsigned char ta_raw[];
-  pdl_launch_dependents();
   if ((ta_smem(ta_raw) & 1023u) != 0) {
     if (threadIdx.x == 0) ullm_report(p.status, ULLM_STATUS_TIMEOUT, 10, (int)(ta_smem(ta_raw) & 1023u));
     return;
@@ -273,6 +272,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ta_smem(&tmem_slot)), "r"(256)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -185,7 +185,9 @@ __device__ __forceinline__ void store_vec32(float* p, const float (&v)[VEC]) {
 //                             this one are running (its blocks then wait in their own pdl_wait)
 //   pdl_wait();               blocks until the previous kernel in the stream has completed and its
 //                             writes are visible; nothing that depends on it may be touched before
-// so that launch latency and per-block set-up of a kernel overlap with the tail of the one before it.
+// so that launch latency and per-block set-up of a kernel overlap with the tail of the one before it.  A kernel that allocates tensor
+// memory calls the first only when it has it: blocks of several kernels may be resident, and one that waits for its turn must not
+// hold what one in front of it still needs.
 // A kernel may do work that does not depend on its predecessor (reading weights) before pdl_wait().
 // Launches carry the attribute only while ullm_set_pdl(1) is in force; without it both calls are no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -98,7 +98,6 @@ __global__ void __launch_bounds__(FS_THREADS, 1) linear_f32_split_kernel(const _
   extern __shared__ unsigned char fs_smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[FS_STAGES], empty_bar[FS_STAGES], acc_full[FS_SUMS], acc_empty[FS_SUMS];
   __shared__ uint32_t tmem_slot;
-  pdl_launch_dependents();
   unsigned char* tiles = (unsigned char*)(((uintptr_t)fs_smem_raw + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (p.M + FS_BM - 1) / FS_BM;
@@ -119,6 +118,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) linear_f32_split_kernel(const _
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(lin_smem(&tmem_slot)), "r"(TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -87,7 +87,6 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   __shared__ __align__(8) uint64_t full_bar[LIN_MAX_STAGES], empty_bar[LIN_MAX_STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int last_flag, wait_flag[2];
-  pdl_launch_dependents();
   unsigned char* tiles = (unsigned char*)(((uintptr_t)lin_smem_raw + 1023) & ~(uintptr_t)1023);
   const int b_bytes = p.m_pad * 128;                         // one half of the activations' tile (a multiple of 2 KB)
   const int stage_bytes = 2 * LIN_A_HALF + 2 * b_bytes;
@@ -126,6 +125,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                  "r"(tmem_cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -85,7 +85,6 @@ linear_tcgen05_large_kernel(const __grid_constant__ CUtensorMap map_x, const __g
   __shared__ __align__(8) uint64_t full_bar[LG_STAGES], empty_bar[LG_STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int wait_flag[2];
-  pdl_launch_dependents();
   unsigned char* tiles = (unsigned char*)(((uintptr_t)lg_smem_raw + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long num_tiles = (long long)p.m_tiles * p.n_tiles;
@@ -107,6 +106,7 @@ linear_tcgen05_large_kernel(const __grid_constant__ CUtensorMap map_x, const __g
                  "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -262,7 +262,6 @@ linear_tcgen05_large2_kernel(const __grid_constant__ CUtensorMap map_x, const __
   __shared__ __align__(8) uint64_t full_bar[LG2_STAGES], empty_bar[LG2_STAGES], acc_full, acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int wait_flag[2];
-  pdl_launch_dependents();
   unsigned char* tiles = (unsigned char*)(((uintptr_t)lg_smem_raw + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long num_tiles = (long long)p.m_tiles * p.n_tiles;
@@ -283,6 +282,7 @@ linear_tcgen05_large2_kernel(const __grid_constant__ CUtensorMap map_x, const __
                  "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

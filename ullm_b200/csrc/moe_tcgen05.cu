@@ -97,7 +97,6 @@ moe_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
   __shared__ uint32_t tmem_base_slot;
   __shared__ int wait_flag[2];
   __shared__ int first_s[MT_MAX_EXPERTS + 1];  // row tiles in front of every expert
-  pdl_launch_dependents();
   unsigned char* tiles = (unsigned char*)(((uintptr_t)mt_smem_raw + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -116,6 +115,7 @@ moe_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(lin_smem(&tmem_base_slot)), "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
   }
   pdl_wait();
   if (warp == 0) {  // running count of row tiles, 32 experts at a time
