@@ -1,5 +1,5 @@
 """32-bit attention by row tiles (csrc/attention_plain.cu) against the plain reference and against the general kernel, at the
-edges of its tiles: rows of a tile (32, shared by the query heads of a kv head), 64 keys, windows and stretches that begin inside
+edges of its tiles: rows of a tile (32, shared by the query heads of a kv head), 32 keys of two groups, windows and stretches that begin inside
 a tile, single tokens beside prompt portions, padding rows."""
 
 import pytest
@@ -48,7 +48,8 @@ def run(c, Hq, Hkv, D, page, window, scale, on=True):
 @pytest.mark.parametrize("Hq,Hkv,D", [(4, 4, 64), (4, 2, 128), (12, 4, 64), (8, 2, 128), (5, 1, 64), (16, 2, 128), (32, 1, 64)])
 @pytest.mark.parametrize("window", [0, 33, -64])
 @pytest.mark.parametrize("q_lens,kv_lens", [
-    ([1, 31, 32, 33], [64, 31, 32, 97]), ([65, 1, 2], [65, 129, 66]), ([1, 1, 1], [1, 33, 260]), ([17], [81])])
+    ([1, 31, 32, 33], [64, 31, 32, 97]), ([65, 1, 2], [65, 129, 66]), ([1, 1, 1], [1, 33, 260]), ([17], [81]),
+    ([2, 40], [193, 223])])
 def test_row_tiles_match_the_reference_and_the_general_kernel(dtype, Hq, Hkv, D, window, q_lens, kv_lens):
     scale, page = D ** -0.5, 16
     c = case(dtype, Hq, Hkv, D, page, q_lens, kv_lens)

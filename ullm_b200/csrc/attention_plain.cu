@@ -4,13 +4,16 @@
 //
 // The general kernel gives a warp one (token, head): each lane walks a key of its own (rows 512 bytes apart), a key is read
 // once per query row, and a dot product is one serial chain of head_dim multiply-adds.  At Qwen3-0.6B sizes that took 749 us
-// per layer for prompts of 170 + 341 tokens and 589 us for 8 decoded tokens with 300 to 700 keys; these two take 76 and 29 us:
+// per layer for prompts of 170 + 341 tokens and 589 us for 8 decoded tokens with 300 to 700 keys; these two take 69 and 29 us:
 //
 //   * rows of prompt portions (requests that bring more than one token): a block owns PT_ROWS (token, query head) rows of ONE
-//     kv head and walks the keys 64 at a time, K and V staged in shared memory once for all rows.  A thread forms 4 rows x 4
-//     keys of the scores and 4 rows x 8 columns of the output from 16-byte reads: 64 multiply-adds per 8 reads, so the
-//     multiply-add pipe binds it, not shared memory.  32 rows and not 64: at the prompt lengths of a step (hundreds of tokens)
-//     the longest row tile sets the time, and half a tile's rows are half its time.
+//     kv head.  Two groups of 128 threads walk the keys, 32 at a time and in turn, each with K and V of its tile in shared memory
+//     and with maxima, sums and outputs of its own, which meet at the end: one loads while the other multiplies, and the longest
+//     row tile, which sets the time at the prompt lengths of a step (hundreds of tokens), is walked in half the turns.  A thread
+//     forms 4 rows x 2 keys of the scores and 4 rows x 8 columns of the output from 16-byte reads.  One group with tiles of 64 keys:
+//     prompts of 170 + 341 tokens 81 us, 100 tokens 30, 500 108, 2,048 861; two of 32: 69, 24, 91, 749 (16 query heads of 128).
+//     32 rows and not 64: half a tile's rows are half its time.  What is left: the busiest SM is active 1.7 times as long as the
+//     average one, and issues an instruction in 42 % of its clocks.
 //   * decoded tokens (requests that bring one): a block of 8 warps owns (request, kv head); eight lanes share a key, so a
 //     warp reads whole 128-byte lines of four keys at a time, and the 32 groups of eight lanes keep running maxima and sums
 //     of their own, which meet in shared memory at the end.  Bound by the latency of its loads: a step has only requests x
@@ -18,8 +21,10 @@
 #include "common.cuh"
 
 #define PT_ROWS 32
-#define PT_KEYS 64
-#define PT_THREADS 128
+#define PT_KEYS 32                         // keys of a tile
+#define PT_GROUPS 2                        // groups of threads with tiles of their own
+#define PT_GROUP_THREADS 128
+#define PT_THREADS (PT_GROUPS * PT_GROUP_THREADS)
 #define PT_PAD 4  // floats between rows of K, V and Q beyond head_dim: neighbouring rows start 4 banks apart
 #define PT_PS (PT_KEYS + 4)
 
@@ -57,7 +62,7 @@ __device__ __forceinline__ bool pl_odd(const float4& v) {
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(PT_THREADS)
+__global__ void __launch_bounds__(PT_THREADS, 2)
 plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T* __restrict__ out,
                               const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                               const int* __restrict__ block_table, int max_pages, const int* __restrict__ req_slots,
@@ -67,11 +72,14 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
   constexpr int ST = D + PT_PAD;
   constexpr int CV = D / 64;  // groups of four output columns a thread owns
   extern __shared__ __align__(16) float pl_smem[];
-  float* qs = pl_smem;                    // [PT_ROWS][ST]
-  float* ks = qs + PT_ROWS * ST;          // [PT_KEYS][ST]
-  float* vs = ks + PT_KEYS * ST;          // [PT_KEYS][ST]
-  float* ps = vs + PT_KEYS * ST;          // [PT_ROWS][PT_PS]
-  __shared__ long long slot_s[PT_KEYS];
+  const int tid = threadIdx.x, group = tid / PT_GROUP_THREADS, gt = tid % PT_GROUP_THREADS, tx = gt & 15, ty = gt >> 4;
+  float* qs = pl_smem;                                                             // [PT_ROWS][ST]
+  float* ks = qs + PT_ROWS * ST + group * (2 * PT_KEYS * ST + PT_ROWS * PT_PS);    // [PT_KEYS][ST], a group's own
+  float* vs = ks + PT_KEYS * ST;                                                   // [PT_KEYS][ST]
+  float* ps = vs + PT_KEYS * ST;                                                   // [PT_ROWS][PT_PS]
+  __shared__ long long slot_all[PT_GROUPS][PT_KEYS];
+  __shared__ float m_s[PT_ROWS], l_s[PT_ROWS];                                     // of the second group, at the end
+  long long* slot_s = slot_all[group];
   pdl_launch_dependents();
   pdl_wait();
   const int gq = num_q / num_kv, per = PT_ROWS / gq;  // query heads per kv head; tokens of a row tile
@@ -89,7 +97,7 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
     tile -= tiles;
   }
   if (r >= requests) return;
-  const int kh = blockIdx.y, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int kh = blockIdx.y;
   const int row0 = tile * per, rows = min(per, n - row0) * gq;  // row i: token row0 + i / gq, query head i % gq
   const int kvl = kv_len[r];
   const int pos0 = kvl - n + row0;
@@ -118,6 +126,7 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
   const int* bt = block_table + (long long)req_slots[r] * max_pages;
   const long long kv_row = (long long)num_kv * D;
   const int last = pos0 + (rows - 1) / gq;
+  auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(PT_GROUP_THREADS) : "memory"); };
   // A weight of zero must not meet a value that a row does not see and that is infinite or NaN: where an output is not finite, the
   // tile's rows run once more, and each adds up only what it sees.
   bool odd = false;
@@ -130,21 +139,22 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
 #pragma unroll
       for (int c = 0; c < CV; ++c) o[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (int base = max(0, first_seen(pos0, window)); base <= last; base += PT_KEYS) {
-      __syncthreads();  // (the tile before has been read; Q is in place)
-      if (tid < PT_KEYS) {
-        const int key = base + tid;
+    __syncthreads();  // Q is in place; what the groups left to one another has been read
+    for (int base = max(0, first_seen(pos0, window)) + group * PT_KEYS; base <= last; base += PT_GROUPS * PT_KEYS) {
+      group_sync();  // (the tile before has been read)
+      if (gt < PT_KEYS) {
+        const int key = base + gt;
         long long slot = -1;
         if (key <= last) {
           const int page = bt[key / page_size];
           if (page < 0 || page >= num_pages) ullm_report(status, ULLM_STATUS_PAGE, t0 + row0, page);
           else slot = (long long)page * page_size + key % page_size;
         }
-        slot_s[tid] = slot;
+        slot_s[gt] = slot;
       }
-      __syncthreads();
+      group_sync();
 #pragma unroll 4
-      for (int i = tid; i < PT_KEYS * (D / 4); i += PT_THREADS) {
+      for (int i = gt; i < PT_KEYS * (D / 4); i += PT_GROUP_THREADS) {
         const int key = i / (D / 4), e = (i - key * (D / 4)) * 4;
         const long long slot = slot_s[key];
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
@@ -156,51 +166,45 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
         *reinterpret_cast<float4*>(ks + key * ST + e) = a;
         *reinterpret_cast<float4*>(vs + key * ST + e) = b;
       }
-      __syncthreads();
-      // scores of rows 4 ty .. + 3 against keys tx, tx + 16, tx + 32, tx + 48
-      float s[4][4];
+      group_sync();
+      // scores of rows 4 ty .. + 3 against keys tx, tx + 16
+      float s[4][2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+      for (int i = 0; i < 4; ++i) s[i][0] = s[i][1] = 0.f;
 #pragma unroll 4
       for (int e = 0; e < D; e += 4) {
-        float4 a[4], b[4];
+        float4 a[4], b[2];
 #pragma unroll
         for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(qs + (ty * 4 + i) * ST + e);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * ST + e);
+        for (int j = 0; j < 2; ++j) b[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * ST + e);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) s[i][j] = pl_dot(a[i], b[j], s[i][j]);
+          for (int j = 0; j < 2; ++j) s[i][j] = pl_dot(a[i], b[j], s[i][j]);
       }
-      bool there[4];
+      bool there[2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) there[j] = slot_s[tx + 16 * j] >= 0;
+      for (int j = 0; j < 2; ++j) there[j] = slot_s[tx + 16 * j] >= 0;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float top = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < 2; ++j) {
           const int key = base + tx + 16 * j;
           s[i][j] = (there[j] && key >= first[i] && key <= pos[i]) ? s[i][j] * scale : -INFINITY;
-          top = fmaxf(top, s[i][j]);
         }
+        float top = fmaxf(s[i][0], s[i][1]);
 #pragma unroll
         for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
         const float m2 = fmaxf(m[i], top);
         const float keep = m2 == -INFINITY ? 1.f : expf(m[i] - m2);  // (no key seen yet: nothing to rescale)
-        float sum = 0.f;
+        l[i] *= keep;  // (the sum of this lane's own keys)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < 2; ++j) {
           const float p = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m2);
           ps[(ty * 4 + i) * PT_PS + tx + 16 * j] = p;
-          sum += p;
+          l[i] += p;
         }
-#pragma unroll
-        for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-        l[i] = l[i] * keep + sum;
         m[i] = m2;
 #pragma unroll
         for (int c = 0; c < CV; ++c) o[i][c].x *= keep, o[i][c].y *= keep, o[i][c].z *= keep, o[i][c].w *= keep;
@@ -244,23 +248,46 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
     }
     bool bad = false;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int x = 8; x > 0; x >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], x);
 #pragma unroll
       for (int c = 0; c < CV; ++c) bad |= pl_odd(o[i][c]);
+    }
     if (odd || !__syncthreads_or(bad)) break;
     odd = true;
   }
+  // the groups meet: the second one's rows lie in its tile of keys
+  if (group == 1) {
+    group_sync();  // (its last tile has been read)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (tx == 0) m_s[ty * 4 + i] = m[i], l_s[ty * 4 + i] = l[i];
+#pragma unroll
+      for (int c = 0; c < CV; ++c) *reinterpret_cast<float4*>(ks + (ty * 4 + i) * ST + c * 64 + tx * 4) = o[i][c];
+    }
+  }
+  __syncthreads();
+  if (group == 1) return;
+  const float* rest = ks + 2 * PT_KEYS * ST + PT_ROWS * PT_PS;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int row = ty * 4 + i;
     if (row >= rows) continue;
-    const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
+    // (a group that saw no key of the row has a maximum of -infinity, and adds nothing)
+    const float m2 = fmaxf(m[i], m_s[row]);
+    const float f0 = m[i] == -INFINITY ? 0.f : expf(m[i] - m2), f1 = m_s[row] == -INFINITY ? 0.f : expf(m_s[row] - m2);
+    const float sum = l[i] * f0 + l_s[row] * f1;
+    const float inv = sum > 0.f ? 1.f / sum : 0.f;
     const bool padding = token_req[t0 + row0 + row / gq] < 0;
     T* dst = out + (long long)(t0 + row0 + row / gq) * num_q * D + (long long)(kh * gq + row % gq) * D + tx * 4;
 #pragma unroll
-    for (int c = 0; c < CV; ++c)
-      pl_store4(dst + c * 64, padding ? make_float4(0.f, 0.f, 0.f, 0.f)
-                                      : make_float4(o[i][c].x * inv, o[i][c].y * inv, o[i][c].z * inv, o[i][c].w * inv));
+    for (int c = 0; c < CV; ++c) {
+      const float4 b = *reinterpret_cast<const float4*>(rest + row * ST + c * 64 + tx * 4);
+      const float4 v = make_float4((o[i][c].x * f0 + b.x * f1) * inv, (o[i][c].y * f0 + b.y * f1) * inv,
+                                   (o[i][c].z * f0 + b.z * f1) * inv, (o[i][c].w * f0 + b.w * f1) * inv);
+      pl_store4(dst + c * 64, padding ? make_float4(0.f, 0.f, 0.f, 0.f) : v);
+    }
   }
 }
 
@@ -406,7 +433,7 @@ static int plain_launch(const void* q, long long q_row_stride, void* out, const 
   const int gq = num_q / num_kv;
   if (longest != 1 || tokens != requests) {  // (as many rows as requests alone says nothing: a request may bring none)
     constexpr int ST = D + PT_PAD;
-    constexpr size_t smem = ((size_t)(PT_ROWS + 2 * PT_KEYS) * ST + (size_t)PT_ROWS * PT_PS) * sizeof(float);
+    constexpr size_t smem = ((size_t)(PT_ROWS + PT_GROUPS * 2 * PT_KEYS) * ST + (size_t)PT_GROUPS * PT_ROWS * PT_PS) * sizeof(float);
     static bool allowed = false;
     if (!allowed) {
       if (cudaFuncSetAttribute(plain_attention_prompt_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=

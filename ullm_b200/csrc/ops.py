@@ -2482,7 +2482,7 @@ class Kernels:
             raise KernelError("paged_attention: a step's decode rows were split off but no prompt kernel takes the rest")
         self.attention_path = "generic"
         # 32-bit arithmetic at head sizes 64 and 128 (float32, float16): keys staged once for many rows; the kernel of one warp
-        # per row stays for every other size (per layer at Qwen3-0.6B sizes, prompts of 170 + 341 tokens: 76 against 749 us)
+        # per row stays for every other size (per layer at Qwen3-0.6B sizes, prompts of 170 + 341 tokens: 69 against 749 us)
         # (prompts of up to 16 tokens stay with that kernel while its warps, one per row, fit the chip: 2 / 8 / 17 tokens, 16 query heads
         # of 128: 6.9 / 9.6 / 13.7 us there, 13.5 / 14.0 / 15.0 by tiles of 64 keys; 16 prompts of 8 tokens, 16 / 32 heads: 14.4 /
         # 24.0 and 19.8 / 19.9)
