@@ -56,6 +56,7 @@ struct DecFuse {
   // longer distance) and a gate per head ([batch][num_q], row stride gate_stride): out *= sigmoid(gate); null: none
   const float* dist_bias;
   int dist_len;
+  bool beside;  // see decode_core.cuh (the kernel's BESIDE)
   const __nv_bfloat16* gate;
   long long gate_stride;
 };
@@ -78,7 +79,8 @@ __device__ __forceinline__ float dec_tanh(float x) {
 
 // CL: the splits of a (request, kv head) pair are the blocks of one thread-block cluster (at most 8) and merge
 // their partials through distributed shared memory; no scratch arrays, no second kernel.
-template <int D, bool CL>
+// BESIDE: see decode_core.cuh.  (A constant: with the wait under a condition the loads behind it were moved in front of it.)
+template <int D, bool CL, bool BESIDE = false>
 __global__ void __launch_bounds__(DEC_WARPS * 32)
 decode_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_row_stride,
                         const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
@@ -185,7 +187,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_row_str
       }
     }
   }
-  pdl_wait();
+  if constexpr (!BESIDE) pdl_wait();
 
   // ---- Q fragments (A operand), rows >= group are zero -------------------------------
   unsigned qa[KSTEPS][4];
@@ -540,6 +542,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_row_str
     }
     cluster.sync();  // no block leaves while a peer may still read its partial
   }
+  if constexpr (BESIDE) pdl_wait();
 }
 
 // out[b, h, :] = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M)
@@ -586,7 +589,7 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
   else out[bh * D + d] = __float2bfloat16_rn(val * dec_head_gate(gate, gate_stride, bh / num_q, (int)(bh % num_q)));
 }
 
-static int g_decode_attr_set[2] = {0, 0};
+static int g_decode_attr_set[2][2] = {};  // [head size][beside]
 static int g_decode_cluster = 1;  // 1: splits of 2 to 8 merge inside a cluster; 0: always scratch arrays + merge kernel
 
 // 0 switches the cluster form off (tests and measurements compare the two).
@@ -602,17 +605,14 @@ static int launch_decode(int which, const void* q, long long q_row_stride, const
                          float scale, int num_splits, long long num_pages, int* status, cudaStream_t st,
                          const DecFuse& fu) {
   using S = DecodeSmem<D>;
-  if (!g_decode_attr_set[which]) {
-    if (cudaFuncSetAttribute(decode_attention_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(decode_attention_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES) !=
-            cudaSuccess)
-      return ULLM_ERR_LAUNCH;
-    cudaFuncSetAttribute(decode_attention_kernel<D, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(decode_attention_kernel<D, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
-    g_decode_attr_set[which] = 1;
+  const auto clustered = fu.beside ? decode_attention_kernel<D, true, true> : decode_attention_kernel<D, true, false>;
+  const auto plain = fu.beside ? decode_attention_kernel<D, false, true> : decode_attention_kernel<D, false, false>;
+  if (!g_decode_attr_set[which][fu.beside]) {
+    for (auto kernel : {clustered, plain}) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES) != cudaSuccess) return ULLM_ERR_LAUNCH;
+      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    }
+    g_decode_attr_set[which][fu.beside] = 1;
   }
   const int o_rep = fu.parts != nullptr ? num_kv : 1;
   dim3 grid(num_splits, num_kv * o_rep, batch);
@@ -632,7 +632,7 @@ static int launch_decode(int which, const void* q, long long q_row_stride, const
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_ullm_pdl ? 2 : 1;
-    if (cudaLaunchKernelEx(&cfg, decode_attention_kernel<D, true>, (const __nv_bfloat16*)q, q_row_stride,
+    if (cudaLaunchKernelEx(&cfg, clustered, (const __nv_bfloat16*)q, q_row_stride,
                            (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, block_table, max_pages, req_slots,
                            kv_len, (__nv_bfloat16*)out, part_o, part_ml, num_q, num_kv, page_size, window,
                            scale * 1.4426950408889634f, num_pages, status, fu) == cudaSuccess) {
@@ -642,7 +642,7 @@ static int launch_decode(int which, const void* q, long long q_row_stride, const
     cudaGetLastError();
     g_decode_cluster = -1;  // this device does not take the cluster launch: scratch arrays and merge kernel from now on
   }
-  int rc = ullm_launch_kernel(decode_attention_kernel<D, false>, grid, dim3(DEC_WARPS * 32), (size_t)S::BYTES, st,
+  int rc = ullm_launch_kernel(plain, grid, dim3(DEC_WARPS * 32), (size_t)S::BYTES, st,
       (const __nv_bfloat16*)q, q_row_stride, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, block_table,
       max_pages, req_slots, kv_len, (__nv_bfloat16*)out, part_o, part_ml, num_q, num_kv, page_size, window,
       scale * 1.4426950408889634f, num_pages, status, fu);
@@ -692,6 +692,19 @@ extern "C" int ullm_decode_attention(const void* q, long long q_row_stride, cons
                                      int page_size, int window, float scale, int num_splits, long long num_pages,
                                      int* status, void* stream) {
   DecFuse fu = {};
+  return decode_attention_impl(q, q_row_stride, k_cache, v_cache, block_table, max_pages, req_slots, kv_len, out, scratch,
+                               batch, num_q, num_kv, head_dim, page_size, window, scale, num_splits, num_pages, status,
+                               stream, fu);
+}
+
+// Behind the prompt attention of the same step's other rows, and beside it (see decode_core.cuh).
+extern "C" int ullm_decode_attention_beside(const void* q, long long q_row_stride, const void* k_cache, const void* v_cache,
+                                            const int* block_table, int max_pages, const int* req_slots,
+                                            const int* kv_len, void* out, float* scratch, int batch, int num_q,
+                                            int num_kv, int head_dim, int page_size, int window, float scale,
+                                            int num_splits, long long num_pages, int* status, void* stream) {
+  DecFuse fu = {};
+  fu.beside = true;
   return decode_attention_impl(q, q_row_stride, k_cache, v_cache, block_table, max_pages, req_slots, kv_len, out, scratch,
                                batch, num_q, num_kv, head_dim, page_size, window, scale, num_splits, num_pages, status,
                                stream, fu);

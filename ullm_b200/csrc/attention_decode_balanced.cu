@@ -92,14 +92,10 @@ struct DecbCursor {
 };
 
 template <int D>
-__global__ void __launch_bounds__(DECB_WARPS * 32, DECB_STAGES >= 4 ? 1 : 3)
-decode_attention_balanced_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                                 const DecbParams p) {
+__device__ __forceinline__ void decb_block(const CUtensorMap& map_k, const CUtensorMap& map_v, const DecbParams& p) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ int s_pre[DECB_MAX_BATCH + 1], s_lo[DECB_MAX_BATCH], s_end[DECB_MAX_BATCH], s_slot[DECB_MAX_BATCH];
   __shared__ __align__(8) uint64_t s_full[DECB_WARPS][DECB_STAGES];
-  pdl_launch_dependents();
-  pdl_wait();
   constexpr int HALVES = D / 64;            // 64-element halves of a row
   constexpr int KSTEPS = D / 16;            // k-steps of the score product
   constexpr int NT_O = D / 8;               // n-tiles of the output
@@ -441,6 +437,16 @@ decode_attention_balanced_kernel(const __grid_constant__ CUtensorMap map_k, cons
   }
 }
 
+template <int D, bool BESIDE>
+__global__ void __launch_bounds__(DECB_WARPS * 32, DECB_STAGES >= 4 ? 1 : 3)
+decode_attention_balanced_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                                 const DecbParams p) {
+  pdl_launch_dependents();
+  if constexpr (!BESIDE) pdl_wait();
+  decb_block<D>(map_k, map_v, p);
+  if constexpr (BESIDE) pdl_wait();  // (see decode_core.cuh)
+}
+
 static int g_decb_blocks[2] = {0, 0};
 
 // dynamic shared memory of a block: the warps' rings, and room to align them to 1024 bytes
@@ -453,15 +459,14 @@ template <int D>
 static int decb_blocks(int which) {
   if (g_decb_blocks[which] == 0) {
     constexpr int SMEM = decb_smem_bytes(D);
-    if (cudaFuncSetAttribute(decode_attention_balanced_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             SMEM) != cudaSuccess)
-      return 0;
-    cudaFuncSetAttribute(decode_attention_balanced_kernel<D>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
+    for (auto kernel : {decode_attention_balanced_kernel<D, false>, decode_attention_balanced_kernel<D, true>}) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return 0;
+      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    }
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_attention_balanced_kernel<D>, DECB_WARPS * 32,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_attention_balanced_kernel<D, false>, DECB_WARPS * 32,
                                                       SMEM) != cudaSuccess ||
         sms <= 0 || per_sm <= 0)
       return 0;
@@ -494,7 +499,7 @@ extern "C" int ullm_decode_attention_balanced(const void* q, long long q_row_str
                                               const int* req_slots, const int* kv_len, void* out, float* part,
                                               int* prefix, int* flags, int batch, int num_q, int num_kv, int head_dim,
                                               int page_size, int window, float scale, long long num_pages, int* status,
-                                              void* stream) {
+                                              void* stream, int beside) {
   cudaStream_t st = (cudaStream_t)stream;
   if (batch < 0 || num_q <= 0 || num_kv <= 0 || page_size <= 0 || max_pages <= 0) return ULLM_ERR_BAD_SIZE;
   if (!ullm_decode_attention_balanced_supported(head_dim, num_q, num_kv, batch, page_size)) return ULLM_ERR_UNSUPPORTED;
@@ -534,13 +539,15 @@ extern "C" int ullm_decode_attention_balanced(const void* q, long long q_row_str
     return ULLM_ERR_LAUNCH;
   int rc;
   if (head_dim == 64) {
-    rc = ullm_launch_kernel(decode_attention_balanced_kernel<64>, dim3(blocks), dim3(DECB_WARPS * 32),
+    rc = ullm_launch_kernel(beside ? decode_attention_balanced_kernel<64, true> : decode_attention_balanced_kernel<64, false>,
+                            dim3(blocks), dim3(DECB_WARPS * 32),
                             (size_t)decb_smem_bytes(64), st, map_k, map_v, p);
     if (rc == ULLM_OK)
       rc = ullm_launch_kernel(decode_balanced_merge_kernel<64>, dim3(batch * num_kv), dim3(DECB_MERGE_THREADS), 0, st,
                               (const float*)part, (const int*)prefix, flags, (__nv_bfloat16*)out, batch, num_q, num_kv, warps, DECB_MIN_TILES);
   } else {
-    rc = ullm_launch_kernel(decode_attention_balanced_kernel<128>, dim3(blocks), dim3(DECB_WARPS * 32),
+    rc = ullm_launch_kernel(beside ? decode_attention_balanced_kernel<128, true> : decode_attention_balanced_kernel<128, false>,
+                            dim3(blocks), dim3(DECB_WARPS * 32),
                             (size_t)decb_smem_bytes(128), st, map_k, map_v, p);
     if (rc == ULLM_OK)
       rc = ullm_launch_kernel(decode_balanced_merge_kernel<128>, dim3(batch * num_kv), dim3(DECB_MERGE_THREADS), 0, st,

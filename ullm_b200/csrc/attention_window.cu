@@ -61,6 +61,7 @@ struct WinArgs {
   int gate_heads;  // the gate has one number per head
   const float* dist_bias;  // [num_q][dist_len] or null
   int dist_len;
+  int beside;  // see decode_core.cuh (not with a distance bias, which waits as always)
   int ksplit;  // the column groups of a row group share the steps of Q K^T (needs the exchange buffer)
 };
 
@@ -122,10 +123,8 @@ static inline long long win_exchange_bytes(int dv) {
 // steps of Q K^T become constants and the loops unroll); DKT = 0: both are read from the arguments.
 // BIAS: with a distance bias.
 template <int DVW, int CW, int RW, int DKT, bool BIAS>
-__global__ void __launch_bounds__(RW * CW * 32, CW == 1 ? 3 : 1) window_attention_kernel(const WinArgs a) {
+__device__ __forceinline__ void window_block(const WinArgs& a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  pdl_launch_dependents();
-  pdl_wait();
   constexpr int NT_S = WIN_N / 8, NT_O = DVW / 8, THREADS = RW * CW * 32, WIN_M = RW * 16;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rw = warp % RW, cw = warp / RW;
@@ -540,6 +539,14 @@ __global__ void __launch_bounds__(RW * CW * 32, CW == 1 ? 3 : 1) window_attentio
   }
 }
 
+template <int DVW, int CW, int RW, int DKT, bool BIAS, bool BESIDE>
+__global__ void __launch_bounds__(RW * CW * 32, CW == 1 ? 3 : 1) window_attention_kernel(const WinArgs a) {
+  pdl_launch_dependents();
+  if constexpr (!BESIDE) pdl_wait();
+  window_block<DVW, CW, RW, DKT, BIAS>(a);
+  if constexpr (BESIDE) pdl_wait();  // (see decode_core.cuh)
+}
+
 // One block per (token, head): the splits' accumulators, weighted by 2^(m_s - max m), over the weighted sums;
 // then the scale, the gate and the one rounding.
 __global__ void __launch_bounds__(128) window_merge_kernel(const WinArgs a) {
@@ -584,7 +591,7 @@ __global__ void __launch_bounds__(128) window_merge_kernel(const WinArgs a) {
 #define WIN_SMEM_LIMIT (227 * 1024)
 #define WIN_MAX_SPLITS 64
 
-template <int DVW, int CW, int RW, int DKT, bool BIAS>
+template <int DVW, int CW, int RW, int DKT, bool BIAS, bool BESIDE>
 static int launch_window_as(WinArgs a, int tokens, long long smem, cudaStream_t st) {
   if (BIAS) smem += win_bias_bytes(a.num_q / a.num_kv);
   if (CW > 1 && smem + win_exchange_bytes(a.dv) <= WIN_SMEM_LIMIT) {
@@ -593,10 +600,10 @@ static int launch_window_as(WinArgs a, int tokens, long long smem, cudaStream_t 
   }
   static long long attr_bytes = 0;  // (one per instantiation) the largest size the attribute was set for
   if (smem > attr_bytes) {
-    if (cudaFuncSetAttribute(window_attention_kernel<DVW, CW, RW, DKT, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    if (cudaFuncSetAttribute(window_attention_kernel<DVW, CW, RW, DKT, BIAS, BESIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
       return ULLM_ERR_LAUNCH;
-    cudaFuncSetAttribute(window_attention_kernel<DVW, CW, RW, DKT, BIAS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(window_attention_kernel<DVW, CW, RW, DKT, BIAS, BESIDE>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
     attr_bytes = smem;
   }
@@ -604,7 +611,7 @@ static int launch_window_as(WinArgs a, int tokens, long long smem, cudaStream_t 
   // at most ceil(tokens / tpt) + num_requests token tiles exist, however the tokens are spread
   const long long blocks = ((long long)(tokens + tpt - 1) / tpt + a.num_requests) * a.num_kv;
   if (blocks > 0x7fffffffLL) return ULLM_ERR_BAD_SIZE;
-  const int rc = ullm_launch_kernel(window_attention_kernel<DVW, CW, RW, DKT, BIAS>, dim3((unsigned)blocks, (unsigned)a.nsplit),
+  const int rc = ullm_launch_kernel(window_attention_kernel<DVW, CW, RW, DKT, BIAS, BESIDE>, dim3((unsigned)blocks, (unsigned)a.nsplit),
                                     dim3(RW * CW * 32), (size_t)smem, st, a);
   if (rc != ULLM_OK || a.nsplit <= 1) return rc;
   return ullm_launch_kernel(window_merge_kernel, dim3((unsigned)((long long)tokens * a.num_q)), dim3(128), 0, st, a);
@@ -612,8 +619,9 @@ static int launch_window_as(WinArgs a, int tokens, long long smem, cudaStream_t 
 
 template <int DVW, int CW, int RW, int DKT = 0>
 static int launch_window(const WinArgs& a, int tokens, long long smem, cudaStream_t st) {
-  if (a.dist_bias != nullptr) return launch_window_as<DVW, CW, RW, DKT, true>(a, tokens, smem, st);
-  return launch_window_as<DVW, CW, RW, DKT, false>(a, tokens, smem, st);
+  if (a.dist_bias != nullptr) return launch_window_as<DVW, CW, RW, DKT, true, false>(a, tokens, smem, st);
+  if (a.beside) return launch_window_as<DVW, CW, RW, DKT, false, true>(a, tokens, smem, st);
+  return launch_window_as<DVW, CW, RW, DKT, false, false>(a, tokens, smem, st);
 }
 
 // Sizes this kernel takes (bfloat16): key rows and values multiples of 16, values up to 512, at most 64 query
@@ -640,7 +648,7 @@ extern "C" int ullm_window_attention(const void* q, long long q_row_stride, void
                                      int pool, const void* pk, const void* pv, const int* p_block_table,
                                      int p_max_pages, long long p_num_pages, const void* gate, long long gate_stride,
                                      float out_scale, int nsplit, float* parts, int gate_heads, const float* dist_bias,
-                                     int dist_len) {
+                                     int dist_len, int beside) {
   cudaStream_t st = (cudaStream_t)stream;
   if (tokens < 0 || num_requests <= 0 || page_size <= 0 || max_pages <= 0 || pool < 0)
     return ULLM_ERR_BAD_SIZE;
@@ -693,6 +701,7 @@ extern "C" int ullm_window_attention(const void* q, long long q_row_stride, void
   a.gate_heads = gate_heads;
   a.dist_bias = dist_bias;
   a.dist_len = dist_len;
+  a.beside = beside;
   const long long smem = win_smem_bytes(dk, dv, v_cache != nullptr);
   // the sizes of the usual head shapes (64, 128; latents of 384 + 64 and 512 + 64) as constants
   if (dk == 64 && dv == 64) return launch_window<64, 1, 4, 64>(a, tokens, smem, st);

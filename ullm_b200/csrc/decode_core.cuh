@@ -6,6 +6,10 @@
 
 #include "common.cuh"
 
+// `beside` (attention_decode.cu, attention_decode_balanced.cu, attention_window.cu): the kernel in front in the stream is the prompt
+// attention of the same step's other rows, which nothing here reads, so the two run side by side.  A prompt attention kernel lets its
+// dependents start only behind its own griddepcontrol.wait: whatever came before it, the rows and pages that this kernel reads
+// among it, is complete by then.  The wait stands at this kernel's end instead, so that its end still is the end of both.
 #define DEC_WARPS 4
 #define DEC_TILE 16   // keys per warp iteration
 #define DEC_STAGES 3

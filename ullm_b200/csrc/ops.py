@@ -1130,7 +1130,7 @@ class Kernels:
     def windowed_attention(self, q, out, k_pages, v_pages, block_table, req_slots, cu_q, kv_len, token_req, num_q: int,
                            num_kv: int, head_dim: int, v_dim: int, page_size: int, window: int, scale: float, *,
                            slopes=None, pool: int = 0, pooled=None, gate=None, out_scale: float = 1.0, dist_bias=None,
-                           num_requests: int | None = None, workspace=None, ctx=None):
+                           num_requests: int | None = None, workspace=None, ctx=None, beside: bool = False):
         """Windowed attention (`window` as in `paged_attention`) with its further options: in bfloat16, at sizes `ullm_window_attention_supported`
         takes and with `num_requests` (the batch rows that `cu_q` describes) given, the tensor-core kernel of
         csrc/attention_window.cu; otherwise (32-bit storage, other sizes) the general kernel.  With a `workspace`
@@ -1141,7 +1141,7 @@ class Kernels:
         (row stride free): out *= sigmoid(gate); a gate [T, num_q] has one number per head.  `dist_bias` (float32
         [num_q, n]): score(i, j) += dist_bias[h][min(i - j, n - 1)]; with the step's `ctx` such calls take the split decode
         kernel (steps of single tokens, heads of 64 or 128) and the tcgen05 prompt kernel (heads of 128) where they can.  `out` [T, num_q x v_dim] may be a column range of
-        wider rows."""
+        wider rows.  `beside` as in `_decode_rows`."""
         _need(q, "q", contiguous=False)
         _need(out, "out", q.dtype, contiguous=False)
         _need(k_pages, "k_pages", q.dtype)
@@ -1230,7 +1230,7 @@ class Kernels:
                         self.windowed_attention(
                             q[:n_dec], out[:n_dec], k_pages, None, block_table, req_slots[:n_dec], cu_q[:n_dec + 1],
                             kv_len[:n_dec], token_req[:n_dec], num_q, num_kv, head_dim, v_dim, page_size, window, scale,
-                            num_requests=n_dec, workspace=workspace)
+                            num_requests=n_dec, workspace=workspace, beside=True)
                     return
         p_pages = pk.numel() // (page_size * num_kv * head_dim) if pk is not None else 0
         if (self.window_attention_tc and q.dtype == torch.bfloat16 and num_requests and q.stride(0) % 8 == 0
@@ -1250,7 +1250,7 @@ class Kernels:
                 head_dim, v_dim, page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream(),
                 _ptr(slopes), int(pool), _ptr(pk), _ptr(pv), _ptr(pbt), pbt.shape[1] if pbt is not None else 0, p_pages,
                 _ptr(gate), gate.stride(0) if gate is not None else 0, float(out_scale), splits, _ptr(parts), gate_heads,
-                _ptr(dist_bias), bias_len),
+                _ptr(dist_bias), bias_len, int(beside)),
                 f"window_attention (key rows {head_dim}, values {v_dim}, pool {pool})")
             return
         self.attention_path = "generic"
@@ -2180,9 +2180,9 @@ class Kernels:
 
     def _decode_rows(self, qkv, out, k_pages, v_pages, block_table, req_slots, kv_len, num_q, num_kv, head_dim,
                      page_size, window, scale, num_pages, ragged, ctx, fuse=None, keep_first: int = 0,
-                     softcap: float = 0.0, parts=None, dist_bias=None, head_gate=None, rows: int | None = None) -> None:
+                     softcap: float = 0.0, parts=None, dist_bias=None, head_gate=None, rows: int | None = None, beside: bool = False) -> None:
         """Decode attention of the first `rows` rows (default: all), one token each (row i belongs to request row i): streams
-        the pages once.
+        the pages once.  `beside`: the launch in front is a tcgen05 prompt attention of other rows, and the kernel runs beside it.
         `keep_first` > 0 (with a window), `softcap` > 0 (capped scores) or `parts` (every head's weights on every
         kv head's values, 32-bit [T, num_q * num_kv * head_dim]; `out` unused), `dist_bias` or `head_gate`: the per-request
         split kernel, the one that takes them."""
@@ -2211,7 +2211,7 @@ class Kernels:
             self._check(fn(
                 _ptr(qkv), qkv.stride(0), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.shape[1],
                 _ptr(req_slots), _ptr(kv_len), _ptr(out), _ptr(part), _ptr(prefix), _ptr(flags), T, num_q, num_kv, head_dim,
-                page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream()),
+                page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream(), *(() if tc else (int(beside),))),
                 f"decode_attention_{'tcgen05' if tc else 'balanced'} (head_dim {head_dim})")
             self.launches += 1  # the merge of the shared pairs
             self.attention_path = "decode_tcgen05" if tc else "decode_balanced"
@@ -2279,7 +2279,7 @@ class Kernels:
                 int(window), float(scale), splits, num_pages, _ptr(self.status), _stream(), int(keep_first)),
                 f"decode_attention (head_dim {head_dim}, first {keep_first} kept)")
         else:
-            self._check(self.lib.ullm_decode_attention(
+            self._check((self.lib.ullm_decode_attention_beside if beside else self.lib.ullm_decode_attention)(
                 _ptr(qkv), qkv.stride(0), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), block_table.shape[1],
                 _ptr(req_slots), _ptr(kv_len), _ptr(out), _ptr(scratch), T, num_q, num_kv, head_dim, page_size,
                 int(window), float(scale), splits, num_pages, _ptr(self.status), _stream()),
@@ -2447,9 +2447,11 @@ class Kernels:
         n_dec = 0
         if decode_ok and self.mixed_decode_rows > 0 and getattr(ctx, "cu_q_host", None) is not None:
             n_dec, ragged_head = self._decoded_head(ctx)
-        if n_dec:
-            self._decode_rows(qkv, out, k_pages, v_pages, block_table, req_slots, kv_len, num_q, num_kv, head_dim, page_size,
-                              window, scale, num_pages, ragged_head, ctx, rows=n_dec)
+        def decoded(beside: bool) -> None:
+            if n_dec:
+                self._decode_rows(qkv, out, k_pages, v_pages, block_table, req_slots, kv_len, num_q, num_kv, head_dim, page_size,
+                                  window, scale, num_pages, ragged_head, ctx, rows=n_dec, beside=beside)
+
         # (int32 arrays in one piece, `_need` above: the entries behind the first n_dec by their address)
         behind = tuple(_ptr(t) + 4 * n_dec for t in (req_slots, cu_q, kv_len))
         num_requests = (ctx.num_requests - n_dec) if ctx is not None else 0
@@ -2466,9 +2468,13 @@ class Kernels:
                 block_table.shape[1], *behind, T, num_requests, num_q, num_kv,
                 head_dim, page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream()),
                 f"prefill_attention_tcgen05 (head_dim {head_dim})")
+            # (behind the prompt kernel and beside it: 23 rows and prompts of 1,403 tokens, 16 heads, 45 us from the first to the
+            # merge; one after the other 52.  Latent rows, 12 beside prompts of 1,500: 77 and 88)
+            decoded(True)
             self.attention_path = "prefill_tcgen05"
             self.tcgen05_attention_blocks_per_sm = self.lib.ullm_prefill_attention_tcgen05_blocks_per_sm()
             return
+        decoded(False)
         if (ctx is not None and qkv.dtype == torch.bfloat16
                 and self.lib.ullm_prefill_attention_supported(head_dim, num_q, num_kv)):
             self._check(self.lib.ullm_prefill_attention(
