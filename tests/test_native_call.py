@@ -109,3 +109,51 @@ def test_what_the_product_leaves_to_torch(native):
     finally:
         torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = before
     assert torch.equal(out, torch.ones_like(out))
+
+
+def recorded(native, fn, calls):
+    native.record()
+    try:
+        for c in calls:
+            fn(*c)
+    finally:
+        tape = native.recorded()
+    return tape
+
+
+def test_lists_of_launches_run_with_other_tensors(native):
+    """A list runs with the addresses inside one layer's tensors moved to another's and everything else as it was; layers whose
+    lists differ in any other way, and launches that answer an error, are not alike."""
+    seen = []
+    target = ctypes.CFUNCTYPE(ctypes.c_int, *[{"P": ctypes.c_void_p, "I": ctypes.c_int, "F": ctypes.c_float, "LL": ctypes.c_longlong}[t]
+                                              for t in launchers.LAUNCHERS["ullm_add_rmsnorm"]])(lambda *a: seen.append(a) or 0)
+    fn = native.bind("ullm_add_rmsnorm", ctypes.cast(target, ctypes.c_void_p).value)
+    a, b, c = ((torch.zeros(8, 4), torch.zeros(3)) for _ in range(3))
+    step = torch.zeros(100)
+
+    def launch(layer, rows=7, eps=0.25, other=step):
+        return [(1, other, layer[0].data_ptr() + 20, None, layer[1], rows, -1, eps, 5), (0, layer[0], other, layer[1], None, rows, 2, 1.5, None)]
+
+    ta, tb = recorded(native, fn, launch(a)), recorded(native, fn, launch(b))
+    assert native.alike(ta, a, tb, b)
+    seen.clear()
+    assert native.replay(tb, c) == 0
+    want = [tuple(x.data_ptr() if isinstance(x, torch.Tensor) else x for x in call) for call in launch(c)]
+    assert seen == want
+    for other in (launch(b, rows=8), launch(b, eps=0.5), launch(b)[:1], launch(b, other=torch.zeros(100)), launch((b[1], b[0]))):
+        assert not native.alike(ta, a, recorded(native, fn, other), b)
+    assert not native.alike(ta, a, tb, (b[0], torch.zeros(4)))
+    assert not native.alike(ta, a, tb, b[:1])
+    with pytest.raises(ValueError):
+        native.replay(recorded(native, fn, launch(b)), c)  # (not compared)
+    with pytest.raises(ValueError):
+        native.replay(tb, (c[0][:1], c[1]))
+    native.record()
+    fn(*launch(a)[0])
+    native.unlisted()
+    assert native.recorded() is None
+    native.record()
+    assert native.recorded() is None  # (nothing ran)
+    failing = ctypes.CFUNCTYPE(ctypes.c_int, *[ctypes.c_longlong] * 6)(lambda *x: 4)
+    bad = native.bind("ullm_argmax", ctypes.cast(failing, ctypes.c_void_p).value)
+    assert recorded(native, bad, [(None, 1, 2, 3, None, None)]) is None

@@ -10,6 +10,11 @@
 //   mm        out = x . w^T in bfloat16 by the vendor library, called as `torch.mm` calls it (the same handle, workspace, stream,
 //             algorithm and math mode), without the dispatcher's 4 us; False for what only `torch.mm` should decide
 //
+//   record / recorded / alike / replay
+//             the launches of a layer as a list, and the same list run for another layer of the same make: two layers are recorded as
+//             they launch, `alike` finds every argument equal but for addresses inside the layers' own tensors, and `replay` runs the
+//             list with those addresses moved to a third layer's.  A list lives as long as the step that recorded it.
+//
 // The table of argument types is generated from launchers.py when this file is compiled.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -22,6 +27,7 @@
 #include <cstring>
 #include <tuple>
 #include <utility>
+#include <vector>
 
 namespace {
 
@@ -68,12 +74,78 @@ bool take(PyObject* o, float* v) {
   return true;
 }
 
-using Call = PyObject* (*)(void*, PyObject* const*, Py_ssize_t);
+// ---- lists of launches ----------------------------------------------------------------------------------------------------------
+constexpr int MAX_ARGS = 48;
+struct Value {
+  unsigned long long bits = 0;
+  bool address = false;
+};
+Value value(void* p) { return {reinterpret_cast<unsigned long long>(p), true}; }
+Value value(int i) { return {static_cast<unsigned long long>(static_cast<long long>(i)), false}; }
+Value value(long long i) { return {static_cast<unsigned long long>(i), false}; }
+Value value(float f) {
+  unsigned u;
+  std::memcpy(&u, &f, 4);
+  return {u, false};
+}
+void back(unsigned long long bits, void** v) { *v = reinterpret_cast<void*>(bits); }
+void back(unsigned long long bits, int* v) { *v = static_cast<int>(bits); }
+void back(unsigned long long bits, long long* v) { *v = static_cast<long long>(bits); }
+void back(unsigned long long bits, float* v) {
+  const unsigned u = static_cast<unsigned>(bits);
+  std::memcpy(v, &u, 4);
+}
+using Again = long long (*)(void*, const unsigned long long*);
+struct Launch {
+  Again again;
+  void* fn;
+  int n;
+  Value v[MAX_ARGS];
+};
+struct Moved {  // argument `arg` of launch `launch` lies `offset` bytes into tensor `tensor` of the layer
+  int launch, arg, tensor;
+  unsigned long long offset;
+};
+struct Tape {
+  PyObject_HEAD
+  std::vector<Launch>* launches;
+  std::vector<Moved>* moved;  // null: not compared yet
+  bool whole;                 // nothing ran that is not in the list
+};
+thread_local Tape* recording = nullptr;
 
 template <class R, class... A, std::size_t... N>
+long long again_as(void* fn, const unsigned long long* bits, std::index_sequence<N...>) {
+  std::tuple<A...> v;
+  (back(bits[N], &std::get<N>(v)), ...);
+  if constexpr (std::is_void_v<R>) {
+    reinterpret_cast<R (*)(A...)>(fn)(std::get<N>(v)...);
+    return 0;
+  } else {
+    return static_cast<long long>(reinterpret_cast<R (*)(A...)>(fn)(std::get<N>(v)...));
+  }
+}
+template <class R, class... A>
+long long again(void* fn, const unsigned long long* bits) {
+  return again_as<R, A...>(fn, bits, std::index_sequence_for<A...>{});
+}
+template <class... A>
+void note(Again how, void* fn, const A&... args) {
+  static_assert(sizeof...(A) <= MAX_ARGS, "a launcher's arguments fit the list");
+  Launch l = {how, fn, static_cast<int>(sizeof...(A)), {}};
+  int i = 0;
+  ((l.v[i++] = value(args)), ...);
+  recording->launches->push_back(l);
+}
+
+using Call = PyObject* (*)(void*, PyObject* const*, Py_ssize_t);
+
+// LISTED: launches and settings, not questions
+template <bool LISTED, class R, class... A, std::size_t... N>
 PyObject* invoke(void* fn, PyObject* const* args, std::index_sequence<N...>) {
   std::tuple<A...> v;
   if (!(take(args[N], &std::get<N>(v)) && ...)) return nullptr;
+  if (LISTED && recording != nullptr) note(again<R, A...>, fn, std::get<N>(v)...);
   if constexpr (std::is_void_v<R>) {
     Py_BEGIN_ALLOW_THREADS
     reinterpret_cast<R (*)(A...)>(fn)(std::get<N>(v)...);
@@ -84,16 +156,17 @@ PyObject* invoke(void* fn, PyObject* const* args, std::index_sequence<N...>) {
     Py_BEGIN_ALLOW_THREADS
     r = reinterpret_cast<R (*)(A...)>(fn)(std::get<N>(v)...);
     Py_END_ALLOW_THREADS
+    if (LISTED && recording != nullptr && r != 0) recording->whole = false;  // (what follows depends on it)
     return PyLong_FromLongLong(r);
   }
 }
-template <class R, class... A>
+template <bool LISTED, class R, class... A>
 PyObject* call(void* fn, PyObject* const* args, Py_ssize_t n) {
   if (n != static_cast<Py_ssize_t>(sizeof...(A))) {
     PyErr_Format(PyExc_TypeError, "this launcher takes %zd arguments (%zd given)", static_cast<Py_ssize_t>(sizeof...(A)), n);
     return nullptr;
   }
-  return invoke<R, A...>(fn, args, std::index_sequence_for<A...>{});
+  return invoke<LISTED, R, A...>(fn, args, std::index_sequence_for<A...>{});
 }
 
 using P = void*;
@@ -199,7 +272,14 @@ PyObject* need(PyObject*, PyObject* const* args, Py_ssize_t n, PyObject* kwnames
   return PyObject_Vectorcall(slow_need, args, n, kwnames);
 }
 
-// mm(x, w, out): out [M, N] (bfloat16 or float32) = x [M, K] . w [N, K]^T in bfloat16
+// out [M, N] (bfloat16, or float32 where `wide`) = x [M, K] . w [N, K]^T, on the current stream; the library's status
+int product(void* x, void* w, void* out, int M, int N, int K, int wide) {
+  const float one = 1.f, zero = 0.f;
+  return cublasGemmEx(at::cuda::getCurrentCUDABlasHandle(), CUBLAS_OP_T, CUBLAS_OP_N, N, M, K, &one, w, CUDA_R_16BF, K, x, CUDA_R_16BF,
+                      K, &zero, out, wide ? CUDA_R_32F : CUDA_R_16BF, N, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
+}
+
+// mm(x, w, out): the product, False for what only `torch.mm` should decide
 PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 3 || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1]) || !THPVariable_Check(args[2])) {
     PyErr_SetString(PyExc_TypeError, "mm(x, w, out): three tensors");
@@ -219,26 +299,161 @@ PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (context.allowBF16ReductionCuBLAS() != at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK ||
       context.deterministicAlgorithms())
     Py_RETURN_FALSE;
-  cublasStatus_t rc;
+  void *px = x.data_ptr(), *pw = w.data_ptr(), *po = out.data_ptr();
+  const int m = static_cast<int>(M), nn = static_cast<int>(N), k = static_cast<int>(K), f = wide ? 1 : 0;
+  if (recording != nullptr)
+    note(again<int, void*, void*, void*, int, int, int, int>, reinterpret_cast<void*>(product), px, pw, po, m, nn, k, f);
+  int rc = 0;
+  const char* thrown = nullptr;
+  Py_BEGIN_ALLOW_THREADS
   try {
-    cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
-    const float one = 1.f, zero = 0.f;
-    Py_BEGIN_ALLOW_THREADS
-    rc = cublasGemmEx(handle, CUBLAS_OP_T, CUBLAS_OP_N, static_cast<int>(N), static_cast<int>(M), static_cast<int>(K), &one,
-                      w.data_ptr(), CUDA_R_16BF, static_cast<int>(K), x.data_ptr(), CUDA_R_16BF, static_cast<int>(K), &zero,
-                      out.data_ptr(), wide ? CUDA_R_32F : CUDA_R_16BF, static_cast<int>(N), CUBLAS_COMPUTE_32F,
-                      CUBLAS_GEMM_DEFAULT_TENSOR_OP);
-    Py_END_ALLOW_THREADS
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
+    rc = product(px, pw, po, m, nn, k, f);
+  } catch (const std::exception&) {
+    thrown = "mm: the library's handle could not be had";
   }
-  if (rc != CUBLAS_STATUS_SUCCESS) {
-    PyErr_Format(PyExc_RuntimeError, "cublasGemmEx (%lld x %lld . %lld x %lld) answered %d", static_cast<long long>(M),
-                 static_cast<long long>(K), static_cast<long long>(N), static_cast<long long>(K), static_cast<int>(rc));
+  Py_END_ALLOW_THREADS
+  if (thrown != nullptr || rc != 0) {
+    if (recording != nullptr) recording->whole = false;
+    if (thrown != nullptr) PyErr_SetString(PyExc_RuntimeError, thrown);
+    else PyErr_Format(PyExc_RuntimeError, "cublasGemmEx (%d x %d . %d x %d) answered %d", m, k, nn, k, rc);
     return nullptr;
   }
   Py_RETURN_TRUE;
+}
+
+// ---- record, compare, run again ---------------------------------------------------------------------------------------------------
+PyTypeObject TapeType = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyObject* record(PyObject*, PyObject*) {
+  Tape* t = PyObject_New(Tape, &TapeType);
+  if (t == nullptr) return nullptr;
+  t->launches = new std::vector<Launch>;
+  t->launches->reserve(32);
+  t->moved = nullptr;
+  t->whole = true;
+  Py_XDECREF(reinterpret_cast<PyObject*>(recording));
+  recording = t;
+  Py_RETURN_NONE;
+}
+// work that is not in the list is about to run
+PyObject* unlisted(PyObject*, PyObject*) {
+  if (recording != nullptr) recording->whole = false;
+  Py_RETURN_NONE;
+}
+// ends the recording: the list, or None where something ran beside it
+PyObject* recorded(PyObject*, PyObject*) {
+  Tape* t = recording;
+  recording = nullptr;
+  if (t == nullptr) Py_RETURN_NONE;
+  if (!t->whole || t->launches->empty()) {
+    Py_DECREF(reinterpret_cast<PyObject*>(t));
+    Py_RETURN_NONE;
+  }
+  return reinterpret_cast<PyObject*>(t);
+}
+
+struct Span {
+  unsigned long long at, bytes;
+};
+bool spans(PyObject* tensors, std::vector<Span>* out) {
+  if (!PyTuple_Check(tensors)) {
+    PyErr_SetString(PyExc_TypeError, "a layer's tensors are a tuple");
+    return false;
+  }
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(tensors); ++i) {
+    PyObject* o = PyTuple_GET_ITEM(tensors, i);
+    if (!THPVariable_Check(o)) {
+      PyErr_SetString(PyExc_TypeError, "a layer's tensors are tensors");
+      return false;
+    }
+    const at::Tensor& t = THPVariable_Unpack(o);
+    out->push_back({reinterpret_cast<unsigned long long>(t.data_ptr()), t.is_contiguous() ? static_cast<unsigned long long>(t.nbytes()) : 0});
+  }
+  return true;
+}
+bool is_tape(PyObject* o) {
+  if (Py_TYPE(o) == &TapeType) return true;
+  PyErr_SetString(PyExc_TypeError, "not a recorded list");
+  return false;
+}
+
+// alike(a, a's tensors, b, b's tensors): whether b's list is a's with the addresses moved; b can then be replayed
+PyObject* alike(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 4) {
+    PyErr_SetString(PyExc_TypeError, "alike(a, tensors of a, b, tensors of b)");
+    return nullptr;
+  }
+  if (!is_tape(args[0]) || !is_tape(args[2])) return nullptr;
+  Tape *a = reinterpret_cast<Tape*>(args[0]), *b = reinterpret_cast<Tape*>(args[2]);
+  std::vector<Span> sa, sb;
+  if (!spans(args[1], &sa) || !spans(args[3], &sb)) return nullptr;
+  if (sa.size() != sb.size() || a->launches->size() != b->launches->size()) Py_RETURN_FALSE;
+  for (size_t i = 0; i < sa.size(); ++i)
+    if (sa[i].bytes != sb[i].bytes || sa[i].bytes == 0) Py_RETURN_FALSE;
+  std::vector<Moved> moved;
+  for (size_t l = 0; l < a->launches->size(); ++l) {
+    const Launch &x = (*a->launches)[l], &y = (*b->launches)[l];
+    if (x.fn != y.fn || x.again != y.again || x.n != y.n) Py_RETURN_FALSE;
+    for (int i = 0; i < x.n; ++i) {
+      int tensor = -1;
+      if (y.v[i].address)
+        for (size_t t = 0; t < sb.size() && tensor < 0; ++t)
+          if (y.v[i].bits >= sb[t].at && y.v[i].bits < sb[t].at + sb[t].bytes) tensor = static_cast<int>(t);
+      if (tensor < 0) {
+        if (x.v[i].bits != y.v[i].bits) Py_RETURN_FALSE;  // (what differs has to lie in a tensor of the layer's)
+        continue;
+      }
+      const unsigned long long offset = y.v[i].bits - sb[tensor].at;
+      if (x.v[i].bits != sa[tensor].at + offset) Py_RETURN_FALSE;
+      moved.push_back({static_cast<int>(l), i, tensor, offset});
+    }
+  }
+  delete b->moved;
+  b->moved = new std::vector<Moved>(std::move(moved));
+  Py_RETURN_TRUE;
+}
+
+// replay(list, tensors of another layer): runs it there; the first launch's code that is not 0, else 0
+PyObject* replay(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 2) {
+    PyErr_SetString(PyExc_TypeError, "replay(list, tensors)");
+    return nullptr;
+  }
+  if (!is_tape(args[0])) return nullptr;
+  Tape* t = reinterpret_cast<Tape*>(args[0]);
+  if (t->moved == nullptr) {
+    PyErr_SetString(PyExc_ValueError, "replay: a list that has not been compared");
+    return nullptr;
+  }
+  std::vector<Span> to;
+  if (!spans(args[1], &to)) return nullptr;
+  for (const Moved& m : *t->moved)
+    if (m.tensor >= static_cast<int>(to.size()) || m.offset >= to[m.tensor].bytes) {
+      PyErr_SetString(PyExc_ValueError, "replay: tensors of another make");
+      return nullptr;
+    }
+  long long code = 0;
+  const char* thrown = nullptr;
+  Py_BEGIN_ALLOW_THREADS
+  try {
+    size_t at = 0;
+    for (size_t l = 0; l < t->launches->size() && code == 0; ++l) {
+      const Launch& launch = (*t->launches)[l];
+      unsigned long long bits[MAX_ARGS];
+      for (int i = 0; i < launch.n; ++i) bits[i] = launch.v[i].bits;
+      for (; at < t->moved->size() && (*t->moved)[at].launch == static_cast<int>(l); ++at)
+        bits[(*t->moved)[at].arg] = to[(*t->moved)[at].tensor].at + (*t->moved)[at].offset;
+      code = launch.again(launch.fn, bits);
+    }
+  } catch (const std::exception&) {
+    thrown = "replay: the library's handle could not be had";
+  }
+  Py_END_ALLOW_THREADS
+  if (thrown != nullptr) {
+    PyErr_SetString(PyExc_RuntimeError, thrown);
+    return nullptr;
+  }
+  return PyLong_FromLongLong(code);
 }
 
 PyMethodDef methods[] = {
@@ -248,6 +463,11 @@ PyMethodDef methods[] = {
     {"stream", stream, METH_NOARGS, "the current stream's handle on the current device"},
     {"set_slow_need", set_slow_need, METH_O, "the check that `need` falls back to"},
     {"mm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(mm)), METH_FASTCALL, "a bfloat16 product by the vendor library"},
+    {"record", record, METH_NOARGS, "begins a list of this thread's launches"},
+    {"unlisted", unlisted, METH_NOARGS, "work that the list cannot hold is about to run"},
+    {"recorded", recorded, METH_NOARGS, "the list, or None"},
+    {"alike", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(alike)), METH_FASTCALL, "whether two lists differ by their tensors alone"},
+    {"replay", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(replay)), METH_FASTCALL, "runs a list with other tensors"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "ullm_b200_native", nullptr, -1, methods};
@@ -261,6 +481,14 @@ PyMODINIT_FUNC PyInit_ullm_b200_native() {
   LauncherType.tp_vectorcall_offset = offsetof(Launcher, vectorcall);
   LauncherType.tp_call = PyVectorcall_Call;
   LauncherType.tp_dealloc = [](PyObject* o) { PyObject_Free(o); };
-  if (PyType_Ready(&LauncherType) < 0) return nullptr;
+  TapeType.tp_name = "ullm_b200_native.Tape";
+  TapeType.tp_basicsize = sizeof(Tape);
+  TapeType.tp_flags = Py_TPFLAGS_DEFAULT;
+  TapeType.tp_dealloc = [](PyObject* o) {
+    delete reinterpret_cast<Tape*>(o)->launches;
+    delete reinterpret_cast<Tape*>(o)->moved;
+    PyObject_Free(o);
+  };
+  if (PyType_Ready(&LauncherType) < 0 || PyType_Ready(&TapeType) < 0) return nullptr;
   return PyModule_Create(&module);
 }

@@ -171,7 +171,38 @@ class Kernels:
         # group costs inside a step, by the difference; the step's results are wrong while this is set
         self.skip_groups: frozenset = frozenset()
         self.attention_path = None  # which attention kernel the last call chose (tests read it)
+        self.listed_layers = 0  # layers that ran from a list of launches
         self.launches = 0  # hand-written kernels launched (graph replays add what they captured)
+
+    # -- a layer's launches as a list ----------------------------------------
+    # Host time of a prompt or mixed step is its launches, some 300 at Qwen3-0.6B sizes, 9 us each through Python; layers of the same
+    # make launch the same kernels with other tensors, so two of them are recorded as they launch and the rest run from the list
+    # (native_call.cpp): 3 us a launch.  See `DecoderModel.forward_hidden`.
+    layer_lists = True
+
+    def lists_apply(self) -> bool:
+        return self.layer_lists and self.timer is None and not self.skip_groups
+
+    def record_launches(self, run):
+        """(what `run` returns, the list of what it launched or None)."""
+        before = self.launches
+        _native.record()
+        try:
+            done = run()
+        finally:
+            tape = _native.recorded()
+        return done, None if tape is None else (tape, self.launches - before)
+
+    def lists_alike(self, a, tensors_a, b, tensors_b) -> bool:
+        """True when list b is list a but for addresses inside the layers' tensors; b can then be run for another layer."""
+        return a is not None and b is not None and a[1] == b[1] and _native.alike(a[0], tensors_a, b[0], tensors_b)
+
+    def run_list(self, listed, tensors) -> None:
+        code = _native.replay(listed[0], tensors)
+        if code != 0:
+            raise KernelError(f"a layer's launches: {_ERRORS.get(code, f'error {code}')}")
+        self.launches += listed[1]
+        self.listed_layers += 1
 
     # -- switches -----------------------------------------------------------
     SWITCHES = ("ULLM_B200_PDL", "ULLM_B200_DECODE_SPLIT_TARGET", "ULLM_B200_TC_ATTN", "ULLM_B200_DECODE_CLUSTER",
@@ -514,6 +545,7 @@ class Kernels:
         key = (M, N, K, out_f32)
         flush = None
         if tune and key not in self._lt_tuned and not torch.cuda.is_current_stream_capturing():
+            _native.unlisted()
             try:
                 flush = torch.zeros(256 << 20, dtype=torch.uint8, device="cuda")  # larger than L2; gone after this call
             except torch.cuda.OutOfMemoryError:
@@ -573,9 +605,12 @@ class Kernels:
             return out
         if x.dtype == torch.float32 and self._split_pays(x, weight) and self.linear_f32_split(x, weight, out, bias):
             return out
+        if bias is None and _native.mm(x, weight, out):
+            return out
+        _native.unlisted()
         if bias is not None:
             torch.addmm(bias, x, weight.t(), out=out)
-        elif not _native.mm(x, weight, out):
+        else:
             torch.mm(x, weight.t(), out=out)
         return out
 
@@ -608,6 +643,7 @@ class Kernels:
                 or (bias is not None and (bias.dtype != torch.float32 or bias.shape != (N,) or not bias.is_contiguous()))):
             return False
         # (of the caller's stream, not a kept buffer: products on two streams may run side by side)
+        _native.unlisted()
         terms = torch.empty(int(self.lib.ullm_linear_f32_split_terms(M, K)), dtype=torch.bfloat16, device=x.device)
         code = self.lib.ullm_linear_f32_split(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), _ptr(terms), M, N, K, _ptr(self.status),
                                               _stream())
@@ -642,6 +678,7 @@ class Kernels:
         _need(out, "out", torch.float32)
         if x.dtype == torch.float32:
             if not (self._split_pays(x, weight) and self.linear_f32_split(x, weight, out)):
+                _native.unlisted()
                 torch.mm(x, weight.t(), out=out)
             return out
         if self._own_linear(x, weight, out):
@@ -650,6 +687,7 @@ class Kernels:
             return out
         if _native.mm(x, weight, out):
             return out
+        _native.unlisted()
         if self._f32_out_mm is None:
             try:
                 torch.mm(x[:1], weight[:8].t(), out_dtype=torch.float32)

@@ -304,6 +304,11 @@ class PagedAttention(Mixer, SharesInput):
     def _ragged(ctx) -> bool:
         return bool(ctx.decode_only and is_ragged(ctx.num_live_requests, ctx.max_kv_len, ctx.sum_kv_len))
 
+    def launches_only(self):
+        return (type(self) is PagedAttention and not self.general and self.own_kv
+                and not (self.position is not None and self.position.transforms_qk())
+                and all(n is None or n.launches_only() for n in (self.q_norm, self.k_norm)))
+
     def output_projection(self):
         return self.tensors[self.names["o"]], self.w_o_bias
 

@@ -130,6 +130,12 @@ class Part:
                 out[key] = max(out.get(key, 0), size)
         return out
 
+    def launches_only(self) -> bool:
+        """True when `forward` in a step that is no decode step does nothing on the device but call the compiled launchers, leaves
+        nothing behind that a later part reads, and takes what differs between two parts of equal specs from their tensors
+        (`all_tensors`, the position encoding's tables) and caches alone: a layer of such parts can run from another one's list of launches."""
+        return False
+
     # -- walking a tree of parts ------------------------------------------
     def all_decls(self, prefix: str = "") -> dict[str, ParamDecl]:
         out = {prefix + n: d for n, d in self.param_decls().items()}

@@ -46,6 +46,9 @@ class PreNormResidualBlock(Block):
 
     takes_next_norm = True  # `forward` accepts the norm that the next block (or nobody) will apply first
 
+    def launches_only(self):
+        return type(self) is PreNormResidualBlock and all(p.launches_only() for p in self.subparts().values())
+
     def accepts_folded_norm(self) -> bool:
         """True when this block can start from an operand r * w and the rows' sums of squares that the block
         before left (instead of norming r itself): an RMSNorm in front of a mixer whose first step is a product."""

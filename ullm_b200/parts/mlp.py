@@ -50,6 +50,9 @@ class GatedMLP(FeedForward):
             return None  # (the fused kernels know silu and gelu only)
         return self.w_gate_up, self.tensors[self.names["down"]], _ACTIVATIONS[self.activation]
 
+    def launches_only(self):
+        return True
+
     def activation_elems(self):
         return 3 * self.intermediate_size + self.hidden_size  # gate | up, their product, the output
 

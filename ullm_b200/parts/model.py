@@ -8,6 +8,8 @@ context and one LayerCache per schedule entry.
 
 from __future__ import annotations
 
+import dataclasses
+
 import torch
 
 from ..config.specs import ModelSpec
@@ -15,6 +17,17 @@ from ..csrc import kernels
 from .base import ParamDecl, Part
 from .embedding import OutputHead, PairTable, TokenEmbedding, TokenSideTable
 from .registry import build_block, build_norm, build_position_encoding
+
+
+def _same(a, b) -> bool:
+    """Whether two specs are equal in every field (also in those that their own comparison leaves out)."""
+    if a is b:
+        return True
+    if type(a) is not type(b):
+        return False
+    if dataclasses.is_dataclass(a):
+        return all(_same(getattr(a, f.name), getattr(b, f.name)) for f in dataclasses.fields(a))
+    return a == b
 
 
 class DecoderModel(Part):
@@ -58,6 +71,7 @@ class DecoderModel(Part):
         self._graph_key_mixers = list(seen.values())
         self.dtype: torch.dtype | None = None
         self.device = None
+        self._alike: bool | None = None  # see `_layers_alike`
 
     def subparts(self):
         s = {self.spec.embedding_name: self.embedding}
@@ -102,6 +116,7 @@ class DecoderModel(Part):
         biases in `dtype`, norm weights in float32."""
         self.dtype = dtype
         self.device = torch.device(device)
+        self._alike = None
 
         def make(name, decl):
             dt = torch.float32 if decl.role in ("norm", "bias32") else dtype
@@ -110,6 +125,23 @@ class DecoderModel(Part):
         self.materialize_all(make)
 
     # -- one step -----------------------------------------------------------
+    def _layers_alike(self) -> bool:
+        """True when all layers behind the first are of one make and each runs once, nothing is added between them, and there are
+        enough of them for a list of launches."""
+        if self._alike is None:
+            order = [e.layer for e in self.schedule]
+            specs = [self.spec.layers[i] for i in order[1:]]
+            self._alike = (len(specs) >= 4 and len(set(order)) == len(order) and self.blocks[order[1]].launches_only()
+                           and not any(e.add_input or e.add_vector is not None or e.project_input or e.cache_of is not None
+                                       for e in self.schedule)
+                           and all(_same(specs[0], s) for s in specs[1:]))
+        return self._alike
+
+    def _layer_tensors(self, i: int, caches) -> tuple:
+        c, block = caches[i], self.blocks[self.schedule[i].layer]
+        position = block.mixer.position
+        return (*block.all_tensors().values(), *(position.tables().values() if position is not None else ()), *(t for t in (c.k_pages, c.v_pages) if t is not None))
+
     def forward_hidden(self, ctx, caches):
         """Runs the blocks over the step's tokens.  Returns (y, residual): what the last block left to be added
         (or None) and the residual stream, before the final norm."""
@@ -139,8 +171,24 @@ class DecoderModel(Part):
             x0.copy_(x)
         residual = None
         n = len(self.schedule)
+        # Layers of one make launch the same kernels with other tensors: layers 1 and 2 are recorded as they launch, and where their
+        # lists differ by the layers' tensors alone the rest run from the second one's.  A list does not outlive the step.
+        K = kernels()
+        listing = (not ctx.decode_only and self._layers_alike() and getattr(K, "lists_apply", bool)()
+                   and all(c.group is caches[1].group and c.writes and c.state is None and c.aux is None for c in caches[1:n]))
+        first = listed = None
         for i, e in enumerate(self.schedule):
             block = self.blocks[e.layer]
+            if listing and i in (1, 2):
+                (x, residual), tape = K.record_launches(lambda: block.forward(x, residual, ctx, caches[i]))
+                if i == 1:
+                    first = tape
+                elif K.lists_alike(first, self._layer_tensors(1, caches), tape, self._layer_tensors(2, caches)):
+                    listed = tape
+                continue
+            if listed is not None:
+                K.run_list(listed, self._layer_tensors(i, caches))
+                continue
             if e.project_input:
                 self._project_stream(residual if residual is not None else x, x0, ctx)
             if e.add_input or e.add_vector is not None:

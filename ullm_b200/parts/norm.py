@@ -40,6 +40,9 @@ class RMSNorm(Norm):
             return self._one_plus
         return self.tensors[self.param]
 
+    def launches_only(self):
+        return not self.around_zero  # (its weights lie in a tensor of their own then)
+
     def rms_params(self):
         return self.weight, self.eps
 
