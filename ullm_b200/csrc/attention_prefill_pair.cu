@@ -27,6 +27,9 @@
 // a page past the request's length are zeroed in shared memory before V is used (they may hold anything).  Every
 // load is issued by the block that uses it.
 //
+// With a window that keeps a request's first positions (KEEP), the key tiles that hold them and lie in front of the window's are
+// walked first; what else such a tile holds is masked, and its values are cleared as those past the length are.
+//
 // A learned bias per head and distance (BIAS) is added to the scores as they are read: element by element where distances
 // differ, as one number per row in key tiles that lie wholly beyond the last distinct distance.
 //
@@ -73,12 +76,13 @@ struct TpParams {
   long long gate_stride;
   int dist_len;
   float inv_scale;
+  int keep_first;  // KEEP: the positions below it stay visible beside the window
 };
 
 // tanh by one exponential and one division of the hardware's units: 1 - 2 / (e^(2x) + 1)
 __device__ __forceinline__ float tp_tanh(float x) { return 1.f - __fdividef(2.f, tp_ex2(x * 2.8853900817779268f) + 1.f); }
 
-template <bool CAP, bool PARTS, bool BIAS>
+template <bool CAP, bool PARTS, bool BIAS, bool KEEP>
 __global__ void __launch_bounds__(TP_THREADS, 1)
 prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                               const __grid_constant__ CUtensorMap map_v, const TpParams p) {
@@ -147,8 +151,10 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
   const int key_lo = first_seen(p0, p.window);
   const int k_start = key_lo / TP_KEYS * TP_KEYS;
   // key tiles each query tile walks (tile 1 sees later keys: tiles1 >= tiles0 when it has rows)
-  const int tiles0 = (p0 + ntok0 - 1 - k_start) / TP_KEYS + 1;
-  const int tiles1 = ntok1 > 0 ? (p0 + ntok_all - 1 - k_start) / TP_KEYS + 1 : 0;
+  const int front = KEEP ? min(k_start / TP_KEYS, (p.keep_first + TP_KEYS - 1) / TP_KEYS) : 0;  // tiles of kept positions alone
+  const int tiles0 = front + (p0 + ntok0 - 1 - k_start) / TP_KEYS + 1;
+  const int tiles1 = ntok1 > 0 ? front + (p0 + ntok_all - 1 - k_start) / TP_KEYS + 1 : 0;
+  auto first_key = [&](int t) { return KEEP && t < front ? t * TP_KEYS : k_start + (t - front) * TP_KEYS; };
   const int tiles = max(tiles0, tiles1);
   const int* bt = p.block_table + (long long)p.req_slots[r] * p.max_pages;
   const int pages_per_tile = TP_KEYS / p.page_size;
@@ -192,7 +198,7 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
       }
     }
     auto page_of = [&](int t) -> int {  // lane pg: the page that holds the pg-th page of key tile t
-      const int key = k_start + t * TP_KEYS + lane * p.page_size;
+      const int key = first_key(t) + lane * p.page_size;
       int page = -1;
       if (lane < pages_per_tile && key < kvl) {
         // a tile may begin before the first key any row can see; pages there may have been given back
@@ -355,7 +361,7 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < tiles_i && ok; ++j) {
-      const int key0 = k_start + j * TP_KEYS;
+      const int key0 = first_key(j);
       if (!tp_mbar_wait(&s_full[i], j & 1)) {
         if (lane == 0) ullm_report(p.status, ULLM_STATUS_TIMEOUT, 28 + i, j);
         ok = false;
@@ -409,7 +415,7 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
 #pragma unroll
         for (int k = 0; k < TP_KEYS; ++k) {
           const int key = key0 + k;
-          if (!(key <= pos && key >= lo)) sr[k] = 0xff800000u;  // -inf
+          if (!(key <= pos && (key >= lo || (KEEP && key < p.keep_first)))) sr[k] = 0xff800000u;  // -inf
         }
       }
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -443,17 +449,23 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
       l = l * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
       // the last key tile may hold slots past the request's length: whatever they contain must not reach O.
       // The first warp group that works on this tile clears them (its P.V product is issued first).
-      if (key0 + TP_KEYS > kvl && (i == 0 || j >= tiles0)) {
+      // (So are the values between the kept positions and the block's window, which none of its rows sees.)
+      const int end = KEEP && j < front ? p.keep_first : kvl;
+      const int gap = KEEP && j == front && key0 < key_lo ? key_lo : 0;  // the window's first tile: cleared from the kept ones up to here
+      if ((key0 + TP_KEYS > end || gap > max(key0, p.keep_first)) && (i == 0 || j >= tiles0)) {
         if (!tp_mbar_wait(&full[j & 1], (j >> 1) & 1)) {
           if (lane == 0) ullm_report(p.status, ULLM_STATUS_TIMEOUT, 30 + i, j);
           ok = false;
         } else {
           unsigned char* v_t = pair_s + (j & 1) * 2 * TP_TILE_KV;
-          const int first_bad = max(0, kvl - key0);
-          for (int x = row; x < (TP_KEYS - first_bad) * 16; x += 128) {
-            const int key = first_bad + x / 16, ch = x % 16;  // 16 chunks of 16 bytes per key: 8 per half
-            *reinterpret_cast<uint4*>(v_t + (ch >> 3) * (TP_TILE_KV / 2) + key * 128 + (ch & 7) * 16) = make_uint4(0, 0, 0, 0);
-          }
+          auto clear = [&](int from, int to) {  // rows of the tile
+            for (int x = row; x < (to - from) * 16; x += 128) {
+              const int key = from + x / 16, ch = x % 16;  // 16 chunks of 16 bytes per key: 8 per half
+              *reinterpret_cast<uint4*>(v_t + (ch >> 3) * (TP_TILE_KV / 2) + key * 128 + (ch & 7) * 16) = make_uint4(0, 0, 0, 0);
+            }
+          };
+          clear(max(0, end - key0), TP_KEYS);
+          if (KEEP) clear(max(0, p.keep_first - key0), gap - key0);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
       }
@@ -576,13 +588,13 @@ extern "C" int ullm_prefill_attention_pair_supported(int head_dim, int num_q, in
   return page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128;
 }
 
-template <bool CAP, bool PARTS, bool BIAS = false>
+template <bool CAP, bool PARTS, bool BIAS = false, bool KEEP = false>
 static int tp_launch(const void* q, long long q_row_stride, void* out, const void* k_cache, const void* v_cache,
                      const int* block_table, int max_pages, const int* req_slots, const int* cu_q, const int* kv_len,
                      int tokens, int num_requests, int num_q, int num_kv, int head_dim, int page_size, int window,
                      float scale, long long num_pages, int* status, void* stream, float softcap, float* parts,
                      const float* dist_bias = nullptr, int dist_len = 0, const void* gate = nullptr,
-                     long long gate_stride = 0) {
+                     long long gate_stride = 0, int keep_first = 0) {
   cudaStream_t st = (cudaStream_t)stream;
   if (tokens < 0 || num_requests <= 0 || max_pages <= 0) return ULLM_ERR_BAD_SIZE;
   if (CAP && !(softcap > 0.f)) return ULLM_ERR_BAD_SIZE;
@@ -600,7 +612,7 @@ static int tp_launch(const void* q, long long q_row_stride, void* out, const voi
     return ULLM_ERR_LAUNCH;
   static int attr_set = 0;  // (one flag per instantiation)
   if (!attr_set) {
-    if (cudaFuncSetAttribute(prefill_attention_pair_kernel<CAP, PARTS, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(prefill_attention_pair_kernel<CAP, PARTS, BIAS, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              TP_SMEM) != cudaSuccess)
       return ULLM_ERR_LAUNCH;
     attr_set = 1;
@@ -628,9 +640,10 @@ static int tp_launch(const void* q, long long q_row_stride, void* out, const voi
   p.gate = (const __nv_bfloat16*)gate;
   p.gate_stride = gate_stride;
   p.inv_scale = 1.f / scale;
+  p.keep_first = keep_first;
   const int tpb = 2 * (TP_ROWS / G);
   dim3 grid(((tokens + tpb - 1) / tpb + num_requests) * num_kv * (PARTS ? num_kv : 1));
-  return ullm_launch_kernel(prefill_attention_pair_kernel<CAP, PARTS, BIAS>, grid, dim3(TP_THREADS), (size_t)TP_SMEM, st, mq, mk,
+  return ullm_launch_kernel(prefill_attention_pair_kernel<CAP, PARTS, BIAS, KEEP>, grid, dim3(TP_THREADS), (size_t)TP_SMEM, st, mq, mk,
                             mv, p);
 }
 
@@ -642,6 +655,19 @@ extern "C" int ullm_prefill_attention_pair(const void* q, long long q_row_stride
   return tp_launch<false, false>(q, q_row_stride, out, k_cache, v_cache, block_table, max_pages, req_slots, cu_q,
                                  kv_len, tokens, num_requests, num_q, num_kv, head_dim, page_size, window, scale,
                                  num_pages, status, stream, 0.f, nullptr);
+}
+
+// With a window that keeps the first `keep_first` positions of every request visible.
+extern "C" int ullm_prefill_attention_pair_kept(const void* q, long long q_row_stride, void* out, const void* k_cache,
+                                                const void* v_cache, const int* block_table, int max_pages,
+                                                const int* req_slots, const int* cu_q, const int* kv_len, int tokens,
+                                                int num_requests, int num_q, int num_kv, int head_dim, int page_size,
+                                                int window, float scale, long long num_pages, int* status, void* stream,
+                                                int keep_first) {
+  if (keep_first <= 0 || window <= 0) return ULLM_ERR_BAD_SIZE;
+  return tp_launch<false, false, false, true>(q, q_row_stride, out, k_cache, v_cache, block_table, max_pages, req_slots, cu_q,
+                                              kv_len, tokens, num_requests, num_q, num_kv, head_dim, page_size, window, scale,
+                                              num_pages, status, stream, 0.f, nullptr, nullptr, 0, nullptr, 0, keep_first);
 }
 
 // With capped scores, s <- softcap * tanh(s * scale / softcap).

@@ -251,6 +251,10 @@ class Kernels:
         self.state_step_on = get("ULLM_B200_STATE_STEP", "1") != "0"
         # rows from which a step with distance biases (heads of 128) takes the tcgen05 prompt kernel
         self.pair_biased_rows = int(get("ULLM_B200_PAIR_BIASED_ROWS", "128"))
+        # rows of prompt portions from which a window that keeps first positions (heads of 128) takes the tcgen05 prompt kernel: all
+        # of them (us there and on the mma.sync kernel, 16 heads, window 1,024: 2,048 tokens 39 and 74, 300 18 and 26, 64 15 and 15,
+        # 24 12 and 14; 17 behind 1,783 36 and 70)
+        self.kept_pair_rows = 1
         self.window_attention_tc = get("ULLM_B200_WINDOW_ATTN_TC", "1") != "0"
         # rows per expert, on average, from which the routed experts' products of more than 16 tokens run on the tcgen05 kernel: at
         # 4 rows it takes 44 + 24 us for mma.sync's 45 + 34 (16 experts, gated 1,024 x 2,048), at 2 rows 162 + 90 for 213 + 132 (32
@@ -2450,6 +2454,23 @@ class Kernels:
             if ctx.decode_only and T == ctx.num_requests:
                 self._decode_rows(qkv, out, k_pages, v_pages, block_table, req_slots, kv_len, num_q, num_kv, head_dim,
                                   page_size, window, scale, num_pages, False, ctx, None, keep_first)
+                return
+            n_dec, _ragged = self._decoded_head(ctx) if getattr(ctx, "cu_q_host", None) is not None else (0, False)
+            if (T - n_dec >= self.kept_pair_rows and window > 0 and self.use_tcgen05_attention and self.tc_attention_mode != "single"
+                    and qkv.stride(0) % head_dim == 0
+                    and self.lib.ullm_prefill_attention_pair_supported(head_dim, num_q, num_kv, page_size)):
+                # the tcgen05 kernel for the portions, and the split decode kernel for the one-token entries in front of them
+                behind = tuple(_ptr(t) + 4 * n_dec for t in (req_slots, cu_q, kv_len))
+                self._check(self.lib.ullm_prefill_attention_pair_kept(
+                    _ptr(qkv), qkv.stride(0), _ptr(out), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
+                    block_table.shape[1], *behind, T, ctx.num_requests - n_dec, num_q, num_kv, head_dim, page_size, int(window),
+                    float(scale), num_pages, _ptr(self.status), _stream(), int(keep_first)),
+                    f"prefill_attention_pair (head_dim {head_dim}, first {keep_first} kept)")
+                if n_dec:
+                    self._decode_rows(qkv, out, k_pages, v_pages, block_table, req_slots, kv_len, num_q, num_kv, head_dim,
+                                      page_size, window, scale, num_pages, False, ctx, None, keep_first, rows=n_dec)
+                self.prefill_attention_kernel = "pair"
+                self.attention_path = "prefill_tcgen05"
                 return
             self._check(self.lib.ullm_prefill_attention_kept(
                 _ptr(qkv), qkv.stride(0), _ptr(out), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
