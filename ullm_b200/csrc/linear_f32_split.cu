@@ -26,7 +26,9 @@
 
 #define FS_BM 128
 #define FS_BK 64
-#define FS_THREADS (17 * 32)
+#define FS_ISSUERS 2
+#define FS_FETCH 4  // k blocks of w that are asked for into L2 beyond those in registers
+#define FS_THREADS ((16 + FS_ISSUERS) * 32)
 #define FS_A_BYTES (FS_BM * 128)  // one term of x
 
 // two neighbouring floats in one 64-bit register, the low one first, for the instructions that work on both
@@ -124,6 +126,16 @@ __global__ void __launch_bounds__(FS_THREADS, 1) linear_f32_split_kernel(const _
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_d = tmem_slot;
+  // w into L2 some k blocks before a thread loads it: its registers hold one or two blocks, too few for the way from memory
+  auto fetch = [&](int kb) {
+    if (kb >= k_blocks) return;
+    for (int i = threadIdx.x; i < BN * 2; i += 256) {
+      const long long row = n0 + (i >> 1), col = (long long)kb * FS_BK + (i & 1) * 32;
+      if (row < p.N && col < p.K) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + row * p.K + col));
+    }
+  };
+  if (warp < 8)
+    for (int kb = 0; kb < AHEAD + FS_FETCH; ++kb) fetch(kb);
   pdl_wait();
 
   if (warp < 8) {
@@ -179,6 +191,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) linear_f32_split_kernel(const _
           *reinterpret_cast<uint2*>(d + 2 * B_BYTES) = l;
         }
         if (kb + AHEAD < k_blocks) load(rb[q], kb + AHEAD);
+        fetch(kb + AHEAD + FS_FETCH);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(&full_bar[s]);
@@ -189,50 +202,43 @@ __global__ void __launch_bounds__(FS_THREADS, 1) linear_f32_split_kernel(const _
     if (threadIdx.x == 0)  // (a block that gives up does not leave copies behind that are still on their way)
       for (int kb = issued > FS_STAGES ? issued - FS_STAGES : 0; kb < issued; ++kb)
         mbar_wait(&full_bar[kb % FS_STAGES], (kb / FS_STAGES) & 1);
-  } else if (warp == 16) {
-    // ---- products (a thread of its own: it stands still while the tensor core's queue is full) ---------------------------------
-    if (lane == 0) {
-      auto idesc = [](int columns) {
-        return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(columns >> 3) << 17) | ((uint32_t)(FS_BM >> 4) << 24);
-      };
-      const uint64_t desc0 = umma_desc(tiles);
-      const uint32_t desc_hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
-      int s = 0, buf = 0;
-      uint32_t phase = 0, acc_phase = 1;
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait(&full_bar[s], phase) || !mbar_wait(&acc_empty[buf], acc_phase)) {
-          ullm_report(p.status, ULLM_STATUS_TIMEOUT, 62, kb);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d = tmem_d + (uint32_t)(buf * SUM_COLS);
-        const uint32_t a = lo0 + (uint32_t)((s * STAGE) >> 4), b = a + (3 * FS_A_BYTES >> 4);
-        constexpr uint32_t A1 = FS_A_BYTES >> 4, B1 = B_BYTES >> 4;
-        if (JOINED) {  // columns 0: h h; BN: h m + m h; 2 BN: h l + m m + l h
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (k == 0) umma_bf16_lo<-1>(d, a, b, desc_hi, idesc(3 * BN), 0u);
-            else umma_bf16_lo<1>(d, a + 2 * k, b + 2 * k, desc_hi, idesc(3 * BN));
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma_bf16_lo<1>(d + BN, a + A1 + 2 * k, b + 2 * k, desc_hi, idesc(2 * BN));
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma_bf16_lo<1>(d + 2 * BN, a + 2 * A1 + 2 * k, b + 2 * k, desc_hi, idesc(BN));
-        } else {
-          const uint32_t ta[6] = {2 * A1, 0, A1, A1, 0, 0}, tb[6] = {0, 2 * B1, B1, 0, B1, 0};  // l h, h l, m m, m h, h m, h h
-#pragma unroll
-          for (int t = 0; t < 6; ++t)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              if (t == 0 && k == 0) umma_bf16_lo<-1>(d, a + ta[t], b + tb[t], desc_hi, idesc(BN), 0u);
-              else umma_bf16_lo<1>(d, a + ta[t] + 2 * k, b + tb[t] + 2 * k, desc_hi, idesc(BN));
-            }
-        }
-        umma_commit(&empty_bar[s]);
-        umma_commit(&acc_full[buf]);
-        if (++s == FS_STAGES) s = 0, phase ^= 1;
-        if (++buf == FS_SUMS) buf = 0, acc_phase ^= 1;
+  } else if (warp >= 16) {
+    // ---- products: two warps take the k blocks in turn, each block with a stage and a block sum of its own, so that one's waits and
+    // commits pass while the other's products run (a warp stands still while the tensor core's queue is full) --------------------------
+    // (Neither mistakes a barrier's parity: its last block but one was full, or drained, at a time when the stage's, or the sum's, use
+    // before last had been; FS_ISSUERS is no more than the stages and the sums.)
+    static_assert(FS_ISSUERS <= FS_STAGES && FS_ISSUERS <= FS_SUMS, "a wait's parity is not mistaken");
+    auto idesc = [](int columns) {
+      return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(columns >> 3) << 17) | ((uint32_t)(FS_BM >> 4) << 24);
+    };
+    const uint64_t desc0 = umma_desc(tiles);
+    const uint32_t lead = elect_one();
+    for (int kb = warp - 16; kb < k_blocks; kb += FS_ISSUERS) {
+      const int s = kb % FS_STAGES, buf = kb % FS_SUMS;
+      if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], kb / FS_STAGES & 1) && mbar_wait(&acc_empty[buf], (kb / FS_SUMS & 1) ^ 1))) {
+        if (lane == 0) ullm_report(p.status, ULLM_STATUS_TIMEOUT, 62, kb);
+        break;
       }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t d = tmem_d + (uint32_t)(buf * SUM_COLS);
+      const uint64_t a = desc0 + (uint64_t)((s * STAGE) >> 4), b = a + (3 * FS_A_BYTES >> 4);
+      constexpr uint32_t A1 = FS_A_BYTES >> 4, B1 = B_BYTES >> 4;
+      if (JOINED) {  // columns 0: h h; BN: h m + m h; 2 BN: h l + m m + l h
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_bf16_warp(lead, d, a + 2 * k, b + 2 * k, idesc(3 * BN), k > 0 ? 1u : 0u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_bf16_warp(lead, d + BN, a + A1 + 2 * k, b + 2 * k, idesc(2 * BN), 1u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_bf16_warp(lead, d + 2 * BN, a + 2 * A1 + 2 * k, b + 2 * k, idesc(BN), 1u);
+      } else {
+        const uint32_t ta[6] = {2 * A1, 0, A1, A1, 0, 0}, tb[6] = {0, 2 * B1, B1, 0, B1, 0};  // l h, h l, m m, m h, h m, h h
+#pragma unroll
+        for (int t = 0; t < 6; ++t)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_bf16_warp(lead, d, a + ta[t] + 2 * k, b + tb[t] + 2 * k, idesc(BN), t > 0 || k > 0 ? 1u : 0u);
+      }
+      umma_commit_warp(lead, lin_smem(&empty_bar[s]));
+      umma_commit_warp(lead, lin_smem(&acc_full[buf]));
     }
   } else {
     // ---- sums ------------------------------------------------------------------------------------------------------------

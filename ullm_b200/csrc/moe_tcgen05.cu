@@ -174,42 +174,37 @@ moe_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
       for (int i = issued > MT_STAGES ? issued - MT_STAGES : 0; i < issued; ++i) mbar_wait(&full_bar[i % MT_STAGES], (i / MT_STAGES) & 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---- MMAs ------------------------------------------------------------------------------------------------
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MT_BN >> 3) << 17) | ((uint32_t)(MT_BM >> 4) << 24);
-      const uint64_t desc0 = umma_desc(tiles);
-      const uint32_t desc_hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
-      const uint32_t full0 = lin_smem(&full_bar[0]), empty0 = lin_smem(&empty_bar[0]);
-      uint32_t a_lo = lo0, full_s = full0, empty_s = empty0;
-      int s = 0, it = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
-        const int buf = it & 1;
-        if (!mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1)) {
-          ullm_report(p.status, ULLM_STATUS_TIMEOUT, 54, it);
+    // ---- MMAs (the whole warp, see `umma_bf16_warp`) -----------------------------------------------------------------------
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MT_BN >> 3) << 17) | ((uint32_t)(MT_BM >> 4) << 24);
+    const uint64_t a0 = umma_desc(tiles);
+    const uint32_t full0 = lin_smem(&full_bar[0]), empty0 = lin_smem(&empty_bar[0]), lead = elect_one();
+    int s = 0, it = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
+      const int buf = it & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1))) {
+        if (lane == 0) ullm_report(p.status, ULLM_STATUS_TIMEOUT, 54, it);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t d = tmem_d + (uint32_t)(buf * MT_BN);
+      for (int kb = 0; kb < p.k_blocks; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait_addr(full0 + 8 * s, phase))) {
+          if (lane == 0) ullm_report(p.status, ULLM_STATUS_TIMEOUT, 52, kb);
+          ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d = tmem_d + (uint32_t)(buf * MT_BN);
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!mbar_wait_addr(full_s, phase)) {
-            ullm_report(p.status, ULLM_STATUS_TIMEOUT, 52, kb);
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t b_lo = a_lo + (MT_A_BYTES >> 4);
-          umma_bf16_lo<-1>(d, a_lo, b_lo, desc_hi, idesc, kb > 0 ? 1u : 0u);
-          umma_bf16_lo<1>(d, a_lo + 2, b_lo + 2, desc_hi, idesc);
-          umma_bf16_lo<1>(d, a_lo + 4, b_lo + 4, desc_hi, idesc);
-          umma_bf16_lo<1>(d, a_lo + 6, b_lo + 6, desc_hi, idesc);
-          umma_commit_addr(empty_s);
-          a_lo += (MT_STAGE_BYTES >> 4), full_s += 8, empty_s += 8;
-          if (++s == MT_STAGES) s = 0, phase ^= 1, a_lo = lo0, full_s = full0, empty_s = empty0;
-        }
-        if (ok) umma_commit(&acc_full[buf]);
+        const uint64_t a = a0 + (uint64_t)(s * (MT_STAGE_BYTES >> 4)), b = a + (MT_A_BYTES >> 4);
+        umma_bf16_warp(lead, d, a, b, idesc, kb > 0 ? 1u : 0u);
+        umma_bf16_warp(lead, d, a + 2, b + 2, idesc, 1u);
+        umma_bf16_warp(lead, d, a + 4, b + 4, idesc, 1u);
+        umma_bf16_warp(lead, d, a + 6, b + 6, idesc, 1u);
+        umma_commit_warp(lead, empty0 + 8 * s);
+        if (++s == MT_STAGES) s = 0, phase ^= 1;
       }
+      if (ok) umma_commit_warp(lead, lin_smem(&acc_full[buf]));
     }
   } else {
     // ---- results: a thread owns one place of the tile -----------------------------------------------------------------

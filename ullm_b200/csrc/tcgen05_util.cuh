@@ -143,6 +143,30 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(lin_smem(bar)) : "memory");
 }
 
+// ---- MMAs issued by a whole warp -------------------------------------------------------------------------------------------------
+// The warp runs the issuing loop together and one lane's predicate (`lead`, of elect_one) guards the instructions: what they take
+// (addresses, descriptors) is then known to be the same in all lanes and stays in uniform registers.  By one lane in a branch of its own each
+// value is moved there for every instruction, 58 clocks an MMA.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t lead;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(lead));
+  return lead;
+}
+__device__ __forceinline__ void umma_bf16_warp(uint32_t lead, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.b32 p, %5, 0;\n setp.ne.b32 q, %0, 0;\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %4, p;\n}\n"
+      ::"r"(lead), "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_warp(uint32_t lead, uint32_t bar_smem) {
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.b32 q, %0, 0;\n"
+      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%1];\n}\n"
+      ::"r"(lead), "r"(bar_smem)
+      : "memory");
+}
+
 // ---------------------------------------------------------------------------------------------
 // host side: tensor maps
 // ---------------------------------------------------------------------------------------------
