@@ -7,16 +7,18 @@
 // k block of 64 run in tensor memory, smallest products first, and are then added to float32 registers by ordinary rounded
 // additions: the tensor core's own additions do not round to nearest, and over a whole row of K that would show.
 //
-// What bounds it: the issue slots that splitting takes (22 instructions for four values), and behind them shared memory (288 KB per
-// k block of 128 x 128 results: 2,250 cycles, for 1,536 of the tensor pipe).  So x is split once, by a kernel of its own, into three
-// planes that TMA brings; w, which is read by few blocks each, is split on the way in.  The library's float32 product is bound by its
-// multiply-add instructions.  Measured with cold caches, against the library: 511 rows, 4,096 columns of k 1,024 48 us for 92;
-// 6,144 of 1,024 67 for 150; 1,024 of 3,072 54 for 90; 24,576 of 4,096 595 for 1,784; 64 rows, 4,096 of 4,096 64 for 115.  Errors
-// against 64 bits there: 1.0e-7 to 2.6e-7, the library's 5.7e-7 to 2.0e-6.
+// What bounds it: the products themselves, 12 or 24 per k block, and the splitting of w (22 instructions for four values) and shared
+// memory close behind (288 KB per k block of 128 x 128 results: 2,250 cycles, for 1,536 of the tensor pipe).  So x is split once, by a
+// kernel of its own, into three planes that TMA brings; w, which is read by few blocks each, is split on the way in.  The library's
+// float32 product is bound by its multiply-add instructions.  Measured with cold caches, against the library: 511 rows, 4,096 columns of
+// k 1,024 33 us for 92; 6,144 of 1,024 54 for 150; 1,024 of 3,072 40 for 90; 100 rows, 6,144 of 1,024 23.  Errors against 64 bits there:
+// 1.0e-7 to 1.5e-7, the library's 5.7e-7 to 2.0e-6.
 //
-// Warps 0..7 load rows of w (one or two k blocks ahead, in registers), split them and store the terms in K-major 128-byte-swizzled
-// tiles; a thread of warp 0 asks for the planes of x; a thread of warp 16 issues the products; warps 8..15 add the block sums up, a
-// quarter of the rows and half of the columns each.  Two or three stages, two or four block sums in tensor memory.  BN from 32 to 128, so that the tiles fill the SMs.
+// Warps 0..7 load rows of w (one or two k blocks ahead, in registers; four more are asked for into L2: 31.7 and 29.7 us for 511 x 1,024 x
+// 2,048), split them and store the terms in K-major 128-byte-swizzled tiles; a thread of warp 0 asks for the planes of x; warps 16 and 17
+// issue the products, a k block each in turn (one thread for all of them paced everything, 1,500 clocks a k block of 32 columns: 52 us for
+// 511 x 1,024 x 3,072); warps 8..15 add the block sums up, a quarter of the rows and half of the columns each.  Two or three stages, two
+// or four block sums in tensor memory.  BN from 32 to 128, so that the tiles fill the SMs.
 //
 // Infinities, NaN, operands from 2^104 on and sums from 2^80 on (which the factor takes to infinity) turn a sum into an infinity or
 // NaN that float32 may not show: such a result is formed again with multiply-adds from the rows themselves.
@@ -283,24 +285,32 @@ __global__ void __launch_bounds__(FS_THREADS, 1) linear_f32_split_kernel(const _
     const int row = m0 + quarter * 32 + lane;
     if (ok && row < p.M) {
       float* dst = p.out + (long long)row * p.N + n0 + c0;
+      unsigned long long odd = 0;  // the columns whose sum is infinite or NaN
 #pragma unroll
       for (int c = 0; c < HALF; c += 4) {
         const int col = n0 + c0 + c;
-        if (col >= p.N) break;  // (N is a multiple of 4)
-        float v[4];
+        if (col < p.N) {  // (N is a multiple of 4)
+          float v[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          v[i] = acc[c + i] * FS_DOWN;
-          if (!(fabsf(acc[c + i]) <= 3.4028234e38f)) {
-            const float* xr = p.x + (long long)row * p.K;
-            const float* wr = p.w + (long long)(col + i) * p.K;
-            float sum = 0.f;
-            for (int k = 0; k < p.K; ++k) sum = fmaf(xr[k], wr[k], sum);
-            v[i] = sum;
+          for (int i = 0; i < 4; ++i) {
+            v[i] = acc[c + i] * FS_DOWN;
+            if (!(fabsf(acc[c + i]) <= 3.4028234e38f)) odd |= 1ull << (c + i);
+            if (p.bias != nullptr) v[i] += __ldg(p.bias + col + i);
           }
-          if (p.bias != nullptr) v[i] += __ldg(p.bias + col + i);
+          *reinterpret_cast<float4*>(dst + c) = make_float4(v[0], v[1], v[2], v[3]);
         }
-        *reinterpret_cast<float4*>(dst + c) = make_float4(v[0], v[1], v[2], v[3]);
+      }
+      // (In a loop of its own: beside every result, unrolled, it was 20 us of code to fetch on the way past, at 128 columns.)
+#pragma unroll 1
+      while (odd != 0) {
+        const int c = __ffsll(odd) - 1, col = n0 + c0 + c;
+        odd &= odd - 1;
+        const float *xr = p.x + (long long)row * p.K, *wr = p.w + (long long)col * p.K;
+        float sum = 0.f;
+#pragma unroll 1
+        for (int k = 0; k < p.K; ++k) sum = fmaf(xr[k], wr[k], sum);
+        if (p.bias != nullptr) sum += __ldg(p.bias + col);
+        dst[c] = sum;
       }
     }
   }
@@ -328,8 +338,9 @@ static int fs_go(const CUtensorMap& x_map, const FsParams& p, long long tiles, c
   return ullm_launch_kernel(linear_f32_split_kernel<BN>, dim3((unsigned)tiles), dim3(FS_THREADS), (size_t)smem, st, x_map, p);
 }
 
-// Columns per tile by (waves of tiles) x (ns of a k block, measured: 511 rows, 1,024 columns of k 3,072 in tiles of 32, 64, 96 and
-// 128: 54, 58, 79, 91 us in one wave each); the wider tile where both agree.  0: the device's SM count cannot be read.
+// Columns per tile by (waves of tiles) x (ns of a k block, measured: 511 rows, 1,024 columns of k 1,024 to 4,096 in tiles of 32, 64,
+// 96 and 128: 19.5 to 50, 23.5 to 61, 27.7 to 81, 31.7 to 85 us in one wave each); the wider tile where both agree.  0: the device's SM
+// count cannot be read.
 extern "C" int ullm_linear_f32_split_columns(int M, int N) {
   static int sms = 0;
   if (sms == 0) {
@@ -338,7 +349,7 @@ extern "C" int ullm_linear_f32_split_columns(int M, int N) {
       return 0;
     sms = n;
   }
-  const double ns[4] = {950., 1050., 1450., 1700.};
+  const double ns[4] = {640., 770., 950., 1070.};
   int best = 0;
   double least = 0.;
   for (int bn = 128; bn >= 32; bn -= 32) {
