@@ -4,16 +4,18 @@
 //
 // The general kernel gives a warp one (token, head): each lane walks a key of its own (rows 512 bytes apart), a key is read
 // once per query row, and a dot product is one serial chain of head_dim multiply-adds.  At Qwen3-0.6B sizes that took 749 us
-// per layer for prompts of 170 + 341 tokens and 589 us for 8 decoded tokens with 300 to 700 keys; these two take 69 and 29 us:
+// per layer for prompts of 170 + 341 tokens and 589 us for 8 decoded tokens with 300 to 700 keys; these two take 51 and 29 us:
 //
 //   * rows of prompt portions (requests that bring more than one token): a block owns PT_ROWS (token, query head) rows of ONE
 //     kv head.  Two groups of 128 threads walk the keys, 32 at a time and in turn, each with K and V of its tile in shared memory
 //     and with maxima, sums and outputs of its own, which meet at the end: one loads while the other multiplies, and the longest
 //     row tile, which sets the time at the prompt lengths of a step (hundreds of tokens), is walked in half the turns.  A thread
 //     forms 4 rows x 2 keys of the scores and 4 rows x 8 columns of the output from 16-byte reads.  One group with tiles of 64 keys:
-//     prompts of 170 + 341 tokens 81 us, 100 tokens 30, 500 108, 2,048 861; two of 32: 69, 24, 91, 749 (16 query heads of 128).
-//     32 rows and not 64: half a tile's rows are half its time.  What is left: the busiest SM is active 1.7 times as long as the
-//     average one, and issues an instruction in 42 % of its clocks.
+//     prompts of 170 + 341 tokens 81 us, 100 tokens 30, 500 108, 2,048 861; two of 32: 69, 24, 91, 749 (16 query heads of 128); with
+//     K and V of the next tile on their way (cp.async; K behind the scores, V behind the outputs) 67, 24, 87, 710; with two multiply-
+//     adds an instruction (fma.rn.f32x2: even and odd channels of a score sum up apart) 63, 22, 81, 650; with the kv heads of a row
+//     tile as neighbours in the grid, the row tiles of most keys first, so that an SM gets a long one and a short one 51, 22, 71, 552.
+//     32 rows and not 64: half a tile's rows are half its time.
 //   * decoded tokens (requests that bring one): a block of 8 warps owns (request, kv head); eight lanes share a key, so a
 //     warp reads whole 128-byte lines of four keys at a time, and the 32 groups of eight lanes keep running maxima and sums
 //     of their own, which meet in shared memory at the end.  Bound by the latency of its loads: a step has only requests x
@@ -56,6 +58,37 @@ __device__ __forceinline__ void pl_axpy(float p, const float4& v, float4& o) {
   o.w = fmaf(p, v.w, o.w);
 }
 
+// four neighbouring elements into shared memory, as 32-bit values: 32-bit ones arrive behind the thread's back (pl_wait), others at once.
+// None of them read: zeros.
+// pairs of neighbouring 32-bit values, multiplied and added two at a time
+struct __align__(16) pl_four { unsigned long long lo, hi; };
+__device__ __forceinline__ void pl_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pl_twice(float x) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
+  return v;
+}
+__device__ __forceinline__ void pl_axpy2(unsigned long long p, const pl_four& v, float4& o) {
+  unsigned long long lo, hi;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(lo) : "f"(o.x), "f"(o.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(hi) : "f"(o.z), "f"(o.w));
+  pl_fma2(lo, p, v.lo);
+  pl_fma2(hi, p, v.hi);
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(lo));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(o.z), "=f"(o.w) : "l"(hi));
+}
+__device__ __forceinline__ void pl_bring(float* dst, const float* src, bool there) {
+  const unsigned at = (unsigned)__cvta_generic_to_shared(dst), bytes = there ? 16u : 0u;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void pl_bring(float* dst, const __half* src, bool there) {
+  *reinterpret_cast<float4*>(dst) = there ? pl_load4(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ void pl_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void pl_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // whether one of them is infinite or NaN
 __device__ __forceinline__ bool pl_odd(const float4& v) {
   return fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, v.w * 0.f))) != 0.f;  // (a zero times either is NaN)
@@ -77,14 +110,13 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
   float* ks = qs + PT_ROWS * ST + group * (2 * PT_KEYS * ST + PT_ROWS * PT_PS);    // [PT_KEYS][ST], a group's own
   float* vs = ks + PT_KEYS * ST;                                                   // [PT_KEYS][ST]
   float* ps = vs + PT_KEYS * ST;                                                   // [PT_ROWS][PT_PS]
-  __shared__ long long slot_all[PT_GROUPS][PT_KEYS];
+  __shared__ long long slot_all[PT_GROUPS][2][PT_KEYS];                            // of a tile and of the one behind it
   __shared__ float m_s[PT_ROWS], l_s[PT_ROWS];                                     // of the second group, at the end
-  long long* slot_s = slot_all[group];
   pdl_launch_dependents();
   pdl_wait();
   const int gq = num_q / num_kv, per = PT_ROWS / gq;  // query heads per kv head; tokens of a row tile
   // which request and which of its row tiles (requests of one token are the other kernel's, requests of none have no rows)
-  int r = 0, tile = blockIdx.x, t0 = 0, n = 0;
+  int r = 0, tile = blockIdx.x / num_kv, t0 = 0, n = 0;
   for (; r < requests; ++r) {
     t0 = cu_q[r];
     n = cu_q[r + 1] - t0;
@@ -97,7 +129,7 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
     tile -= tiles;
   }
   if (r >= requests) return;
-  const int kh = blockIdx.y;
+  const int kh = blockIdx.x % num_kv;
   const int row0 = tile * per, rows = min(per, n - row0) * gq;  // row i: token row0 + i / gq, query head i % gq
   const int kvl = kv_len[r];
   const int pos0 = kvl - n + row0;
@@ -127,6 +159,25 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
   const long long kv_row = (long long)num_kv * D;
   const int last = pos0 + (rows - 1) / gq;
   auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(PT_GROUP_THREADS) : "memory"); };
+  auto look_up = [&](int base, int buf) {  // where the keys of a tile lie; -1: none
+    if (gt >= PT_KEYS) return;
+    const int key = base + gt;
+    long long slot = -1;
+    if (key <= last) {
+      const int page = bt[key / page_size];
+      if (page < 0 || page >= num_pages) ullm_report(status, ULLM_STATUS_PAGE, t0 + row0, page);
+      else slot = (long long)page * page_size + key % page_size;
+    }
+    slot_all[group][buf][gt] = slot;
+  };
+  auto bring = [&](float* dst, const T* cache, int buf) {
+#pragma unroll 4
+    for (int i = gt; i < PT_KEYS * (D / 4); i += PT_GROUP_THREADS) {
+      const int key = i / (D / 4), e = (i - key * (D / 4)) * 4;
+      const long long slot = slot_all[group][buf][key];
+      pl_bring(dst + key * ST + e, cache + (slot >= 0 ? slot : 0) * kv_row + (long long)kh * D + e, slot >= 0);
+    }
+  };
   // A weight of zero must not meet a value that a row does not see and that is infinite or NaN: where an output is not finite, the
   // tile's rows run once more, and each adds up only what it sees.
   bool odd = false;
@@ -140,48 +191,49 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
       for (int c = 0; c < CV; ++c) o[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();  // Q is in place; what the groups left to one another has been read
-    for (int base = max(0, first_seen(pos0, window)) + group * PT_KEYS; base <= last; base += PT_GROUPS * PT_KEYS) {
-      group_sync();  // (the tile before has been read)
-      if (gt < PT_KEYS) {
-        const int key = base + gt;
-        long long slot = -1;
-        if (key <= last) {
-          const int page = bt[key / page_size];
-          if (page < 0 || page >= num_pages) ullm_report(status, ULLM_STATUS_PAGE, t0 + row0, page);
-          else slot = (long long)page * page_size + key % page_size;
-        }
-        slot_s[gt] = slot;
-      }
-      group_sync();
-#pragma unroll 4
-      for (int i = gt; i < PT_KEYS * (D / 4); i += PT_GROUP_THREADS) {
-        const int key = i / (D / 4), e = (i - key * (D / 4)) * 4;
-        const long long slot = slot_s[key];
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-        if (slot >= 0) {
-          const long long at = slot * kv_row + (long long)kh * D + e;
-          a = pl_load4(k_cache + at);
-          b = pl_load4(v_cache + at);
-        }
-        *reinterpret_cast<float4*>(ks + key * ST + e) = a;
-        *reinterpret_cast<float4*>(vs + key * ST + e) = b;
-      }
-      group_sync();
+    int turn = 0;
+    const int start = max(0, first_seen(pos0, window)) + group * PT_KEYS;
+    look_up(start, 0);
+    group_sync();
+    bring(ks, k_cache, 0);
+    pl_commit();
+    bring(vs, v_cache, 0);
+    pl_commit();
+    look_up(start + PT_GROUPS * PT_KEYS, 1);
+#pragma unroll 1
+    for (int base = start; base <= last; base += PT_GROUPS * PT_KEYS, turn ^= 1) {
+      const long long* slot_s = slot_all[group][turn];
+      pl_wait<1>();
+      group_sync();  // K is there, and the places of the keys behind
       // scores of rows 4 ty .. + 3 against keys tx, tx + 16
       float s[4][2];
+      {
+        unsigned long long w[4][2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) s[i][0] = s[i][1] = 0.f;
+        for (int i = 0; i < 4; ++i) w[i][0] = w[i][1] = 0ull;
 #pragma unroll 4
-      for (int e = 0; e < D; e += 4) {
-        float4 a[4], b[2];
+        for (int e = 0; e < D; e += 4) {
+          pl_four a[4], b[2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(qs + (ty * 4 + i) * ST + e);
+          for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const pl_four*>(qs + (ty * 4 + i) * ST + e);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) b[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * ST + e);
+          for (int j = 0; j < 2; ++j) b[j] = *reinterpret_cast<const pl_four*>(ks + (tx + 16 * j) * ST + e);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              pl_fma2(w[i][j], a[i].lo, b[j].lo);
+              pl_fma2(w[i][j], a[i].hi, b[j].hi);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 2; ++j) s[i][j] = pl_dot(a[i], b[j], s[i][j]);
+          for (int j = 0; j < 2; ++j) {
+            float x, y;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(w[i][j]));
+            s[i][j] = x + y;
+          }
       }
       bool there[2];
 #pragma unroll
@@ -209,7 +261,10 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
 #pragma unroll
         for (int c = 0; c < CV; ++c) o[i][c].x *= keep, o[i][c].y *= keep, o[i][c].z *= keep, o[i][c].w *= keep;
       }
-      __syncwarp();  // (a row's weights are written and read by the 16 lanes that own the row)
+      pl_wait<0>();
+      group_sync();  // V is there, K has been read  (a row's weights are written and read by the 16 lanes that own the row)
+      bring(ks, k_cache, turn ^ 1);
+      pl_commit();
       if (odd) {  // each row adds up the keys that it sees
 #pragma unroll 1
         for (int key = 0; key < PT_KEYS; ++key) {
@@ -222,9 +277,7 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
             for (int c = 0; c < CV; ++c) pl_axpy(p, *reinterpret_cast<const float4*>(vs + key * ST + c * 64 + tx * 4), o[i][c]);
           }
         }
-        __syncwarp();
-        continue;
-      }
+      } else {
 #pragma unroll 2
       for (int key = 0; key < PT_KEYS; key += 4) {
         float4 p[4];
@@ -233,19 +286,24 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
 #pragma unroll
         for (int c = 0; c < CV; ++c) {
           const float* vp = vs + key * ST + c * 64 + tx * 4;
-          const float4 v0 = *reinterpret_cast<const float4*>(vp), v1 = *reinterpret_cast<const float4*>(vp + ST),
-                       v2 = *reinterpret_cast<const float4*>(vp + 2 * ST), v3 = *reinterpret_cast<const float4*>(vp + 3 * ST);
+          const pl_four v0 = *reinterpret_cast<const pl_four*>(vp), v1 = *reinterpret_cast<const pl_four*>(vp + ST),
+                        v2 = *reinterpret_cast<const pl_four*>(vp + 2 * ST), v3 = *reinterpret_cast<const pl_four*>(vp + 3 * ST);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            pl_axpy(p[i].x, v0, o[i][c]);
-            pl_axpy(p[i].y, v1, o[i][c]);
-            pl_axpy(p[i].z, v2, o[i][c]);
-            pl_axpy(p[i].w, v3, o[i][c]);
+            pl_axpy2(pl_twice(p[i].x), v0, o[i][c]);
+            pl_axpy2(pl_twice(p[i].y), v1, o[i][c]);
+            pl_axpy2(pl_twice(p[i].z), v2, o[i][c]);
+            pl_axpy2(pl_twice(p[i].w), v3, o[i][c]);
           }
         }
       }
-      __syncwarp();
+      }
+      group_sync();  // V has been read
+      bring(vs, v_cache, turn ^ 1);
+      pl_commit();
+      look_up(base + 2 * PT_GROUPS * PT_KEYS, turn);
     }
+    pl_wait<0>();  // (the tile behind the last one: zeros)
     bool bad = false;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -445,8 +503,8 @@ static int plain_launch(const void* q, long long q_row_stride, void* out, const 
     }
     const int per = PT_ROWS / gq;
     const long long tiles = tokens / per + requests;
-    if (tiles > 0x7fffffffLL) return ULLM_ERR_BAD_SIZE;
-    const int rc = ullm_launch_kernel(plain_attention_prompt_kernel<T, D>, dim3((int)tiles, num_kv), dim3(PT_THREADS), smem, st,
+    if (tiles * num_kv > 0x7fffffffLL) return ULLM_ERR_BAD_SIZE;
+    const int rc = ullm_launch_kernel(plain_attention_prompt_kernel<T, D>, dim3((int)(tiles * num_kv)), dim3(PT_THREADS), smem, st,
                                       (const T*)q, q_row_stride, (T*)out, (const T*)k_cache, (const T*)v_cache, block_table,
                                       max_pages, req_slots, cu_q, kv_len, token_req, requests, num_q, num_kv, page_size, window,
                                       scale, num_pages, status);

@@ -2,12 +2,12 @@
 // generation tensor cores:  out[p] = f(W_e . (s_p * x[row(p)])) for every place p of every expert e.
 //
 // Bound by the tensor cores: at 2,048 tokens with 2 of 16 experts of 1,024 x 2,048 each (gated) the two products are 52 GFLOP,
-// 31 us at the card's rate; measured with cold caches 69 + 37 us (512 tokens 46 + 25, bound by the 201 MB of matrices; 32 experts
-// of 2,048 x 4,096: 214 + 114).  The mma.sync kernel of moe.cu takes 140 + 88 us there: tiles of 64 x 64 read both operands from
+// 31 us at the card's rate; measured with cold caches 58 + 33 us (69 + 37 with the MMAs issued by a lane in a branch of its own, whose
+// descriptors take 58 clocks an instruction to uniform registers; 512 tokens then 46 + 25, bound by the 201 MB of matrices).  The mma.sync kernel of moe.cu takes 140 + 88 us there: tiles of 64 x 64 read both operands from
 // shared memory once per 64 columns, and its warps spend their issue slots on ldmatrix.
 //
 // A persistent kernel, one block per SM, built as linear_tcgen05_large.cu: warp 0 loads, warp 1 issues the MMAs (M = 128,
-// N = 256, K = 16; one thread), warps 2..5 drain the accumulators; four stages of 48 KB; two accumulators in tensor memory, so
+// N = 256, K = 16; the whole warp, one lane elected), warps 2..5 drain the accumulators; four stages of 48 KB; two accumulators in tensor memory, so
 // that a tile's activation and stores run behind the next tile's products.  What is different:
 //
 //   * a tile is 128 places of ONE expert x 256 rows of its matrix (gated: 128 gate rows and the same 128 rows of up, a

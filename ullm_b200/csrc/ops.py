@@ -636,7 +636,7 @@ class Kernels:
         """out = x @ weight.T (+ bias) in float32 on the tensor cores, every operand as three bfloat16 terms
         (csrc/linear_f32_split.cu).  False for what the kernel does not take and where the library's product is as fast
         (nothing has run): up to 16 rows, and fewer than 2^16 results, whose tiles leave most SMs idle (1,024 columns of
-        k 2,048: 32 rows 38 us for 26, 64 rows 38 for 57; 511 x 64 results 40 for 26, 2,048 x 64 44 for 58); very many columns
+        k 2,048: 32 rows 28 us for 26, 64 rows 28 for 56; 511 x 64 results 28 for 26, 2,048 x 64 33 for 58); very many columns
         at few rows, where a tile's start is a fifth of its time (151,936 columns of k 1,024: 32 rows 278 us for 261, 48 rows
         279 for 386)."""
         M, K = x.shape
@@ -2547,7 +2547,7 @@ class Kernels:
             raise KernelError("paged_attention: a step's decode rows were split off but no prompt kernel takes the rest")
         self.attention_path = "generic"
         # 32-bit arithmetic at head sizes 64 and 128 (float32, float16): keys staged once for many rows; the kernel of one warp
-        # per row stays for every other size (per layer at Qwen3-0.6B sizes, prompts of 170 + 341 tokens: 69 against 749 us)
+        # per row stays for every other size (per layer at Qwen3-0.6B sizes, prompts of 170 + 341 tokens: 51 against 749 us)
         # (prompts of up to 16 tokens stay with that kernel while its warps, one per row, fit the chip: 2 / 8 / 17 tokens, 16 query heads
         # of 128: 6.9 / 9.6 / 13.7 us there, 13.5 / 14.0 / 15.0 by tiles of 64 keys; 16 prompts of 8 tokens, 16 / 32 heads: 14.4 /
         # 24.0 and 19.8 / 19.9)
