@@ -11,7 +11,7 @@
 // memory close behind (288 KB per k block of 128 x 128 results: 2,250 cycles, for 1,536 of the tensor pipe).  So x is split once, by a
 // kernel of its own, into three planes that TMA brings; w, which is read by few blocks each, is split on the way in.  The library's
 // float32 product is bound by its multiply-add instructions.  Measured with cold caches, against the library: 511 rows, 4,096 columns of
-// k 1,024 33 us for 92; 6,144 of 1,024 54 for 150; 1,024 of 3,072 40 for 90; 100 rows, 6,144 of 1,024 23.  Errors against 64 bits there:
+// k 1,024 34 us for 92; 6,144 of 1,024 54 for 150; 1,024 of 3,072 42 for 90; 100 rows, 6,144 of 1,024 24.  Errors against 64 bits there:
 // 1.0e-7 to 1.5e-7, the library's 5.7e-7 to 2.0e-6.
 //
 // Warps 0..7 load rows of w (one or two k blocks ahead, in registers; four more are asked for into L2: 31.7 and 29.7 us for 511 x 1,024 x
@@ -24,6 +24,7 @@
 // NaN that float32 may not show: such a result is formed again with multiply-adds from the rows themselves.
 //
 // Every wait on an mbarrier is bounded (ULLM_STATUS_TIMEOUT in the status word, then the role leaves, and the others after it).
+#include "ring_turns.h"
 #include "tcgen05_util.cuh"
 
 #define FS_BM 128
@@ -207,9 +208,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1) linear_f32_split_kernel(const _
   } else if (warp >= 16) {
     // ---- products: two warps take the k blocks in turn, each block with a stage and a block sum of its own, so that one's waits and
     // commits pass while the other's products run (a warp stands still while the tensor core's queue is full) --------------------------
-    // (Neither mistakes a barrier's parity: its last block but one was full, or drained, at a time when the stage's, or the sum's, use
-    // before last had been; FS_ISSUERS is no more than the stages and the sums.)
-    static_assert(FS_ISSUERS <= FS_STAGES && FS_ISSUERS <= FS_SUMS, "a wait's parity is not mistaken");
+    // (How neither takes an old use of a stage or a sum for the present one: ring_turns.h.)
+    static_assert(FS_ISSUERS <= FS_STAGES && FS_ISSUERS <= FS_SUMS, "what ring_issue_turn asks for");
     auto idesc = [](int columns) {
       return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(columns >> 3) << 17) | ((uint32_t)(FS_BM >> 4) << 24);
     };
@@ -217,7 +217,10 @@ __global__ void __launch_bounds__(FS_THREADS, 1) linear_f32_split_kernel(const _
     const uint32_t lead = elect_one();
     for (int kb = warp - 16; kb < k_blocks; kb += FS_ISSUERS) {
       const int s = kb % FS_STAGES, buf = kb % FS_SUMS;
-      if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], kb / FS_STAGES & 1) && mbar_wait(&acc_empty[buf], (kb / FS_SUMS & 1) ^ 1))) {
+      const bool turn = ring_issue_turn(kb, FS_STAGES, FS_SUMS, [&](RingBarrier which, int i, unsigned parity) {
+        return mbar_wait(which == RING_STAGE_EMPTY ? &empty_bar[i] : which == RING_STAGE_FULL ? &full_bar[i] : &acc_empty[i], parity);
+      });
+      if (!__all_sync(0xffffffffu, turn)) {
         if (lane == 0) ullm_report(p.status, ULLM_STATUS_TIMEOUT, 62, kb);
         break;
       }
