@@ -427,11 +427,16 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
       // until then P is at most 256 (exact in bf16 range, sums in 32-bit), and O and l, which share the
       // reference, need no rescaling.  The result O / l does not depend on the reference.
       const float m_cand = fmaxf(m, row_max * p.scale_log2);
-      const float m_new = (m == -INFINITY || m_cand - m > 8.f) ? m_cand : m;
+      // (KEEP: the reference is the maximum itself, as in the mma.sync kernel, which took these rows before.  The weight of the largest
+      // score is then 1, which bfloat16 holds exactly; with the slack it is rounded, and errors against 64 bits were 1.02 to 1.21 times
+      // that kernel's.  With the maximum they are 1.004 times, its tiles being half as long, and with sums of the rounded weights
+      // 0.997.  2,048 tokens, 16 heads, window 1,024: 39 us with the slack, 41 with the maximum, 43 with both; that kernel 74.)
+      const float m_new = (KEEP || m == -INFINITY || m_cand - m > 8.f) ? m_cand : m;
       const float m_use = m_new == -INFINITY ? 0.f : m_new;
       const float alpha = m == -INFINITY ? 1.f : tp_ex2(m - m_use);  // (no key seen yet: O and l are still zero)
       m = m_new;
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      unsigned long long rounded[2] = {0ull, 0ull};  // KEEP: two sums in each
       const float neg_m = BIAS ? fmaf(add, p.scale_log2, -m_use) : -m_use;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -440,11 +445,21 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
         for (int k = 0; k < 32; ++k) {
           const float a = tp_ex2(fmaf(__uint_as_float(sr[h * 64 + 2 * k]), p.scale_log2, neg_m));
           const float b = tp_ex2(fmaf(__uint_as_float(sr[h * 64 + 2 * k + 1]), p.scale_log2, neg_m));
-          sum[(2 * k) & 3] += a;
-          sum[(2 * k + 1) & 3] += b;
           pk[k] = tp_pack_bf16(a, b);
+          if constexpr (KEEP) {  // the sum of the rounded weights, which then add up to one
+            unsigned long long w;
+            asm("mov.b64 %0, {%1, %2};" : "=l"(w) : "r"(pk[k] << 16), "r"(pk[k] & 0xffff0000u));
+            asm("add.rn.f32x2 %0, %0, %1;" : "+l"(rounded[k & 1]) : "l"(w));
+          } else {
+            sum[(2 * k) & 3] += a;
+            sum[(2 * k + 1) & 3] += b;
+          }
         }
         tp_tmem_st32_nowait(tmem_s + h * 32, pk);  // keys 64 h .. 64 h + 63 of this row
+      }
+      if constexpr (KEEP) {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(sum[0]), "=f"(sum[1]) : "l"(rounded[0]));
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(sum[2]), "=f"(sum[3]) : "l"(rounded[1]));
       }
       l = l * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
       // the last key tile may hold slots past the request's length: whatever they contain must not reach O.
@@ -472,14 +487,26 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
       if (ok && j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
         // O shares the reference point.  P.V of the tile before is in it: this tile's scores were issued behind
         // that product, and their completion was awaited above.  Rescale this warp's rows.
+        if constexpr (KEEP) {  // (in most tiles, so in wide pieces)
 #pragma unroll 1
-        for (int c = 0; c < TP_D / 8; ++c) {
-          uint32_t v[8];
-          tp_tmem_ld8_nowait(tmem_o + c * 8, v);
-          tp_tmem_ld_wait();
+          for (int c = 0; c < TP_D / 32; ++c) {
+            uint32_t v[32];
+            tp_tmem_ld32_nowait(tmem_o + c * 32, v);
+            tp_tmem_ld_wait();
 #pragma unroll
-          for (int k = 0; k < 8; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * alpha);
-          tp_tmem_st8_nowait(tmem_o + c * 8, v);
+            for (int k = 0; k < 32; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * alpha);
+            tp_tmem_st32_nowait(tmem_o + c * 32, v);
+          }
+        } else {
+#pragma unroll 1
+          for (int c = 0; c < TP_D / 8; ++c) {
+            uint32_t v[8];
+            tp_tmem_ld8_nowait(tmem_o + c * 8, v);
+            tp_tmem_ld_wait();
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * alpha);
+            tp_tmem_st8_nowait(tmem_o + c * 8, v);
+          }
         }
       }
       tp_tmem_st_wait();

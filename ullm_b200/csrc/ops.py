@@ -251,9 +251,10 @@ class Kernels:
         self.state_step_on = get("ULLM_B200_STATE_STEP", "1") != "0"
         # rows from which a step with distance biases (heads of 128) takes the tcgen05 prompt kernel
         self.pair_biased_rows = int(get("ULLM_B200_PAIR_BIASED_ROWS", "128"))
-        # rows of prompt portions from which a window that keeps first positions (heads of 128) takes the tcgen05 prompt kernel: all
-        # of them (us there and on the mma.sync kernel, 16 heads, window 1,024: 2,048 tokens 39 and 74, 300 18 and 26, 64 15 and 15,
-        # 24 12 and 14; 17 behind 1,783 36 and 70)
+        # rows of prompt portions from which a window that keeps first positions (heads of 128) takes the tcgen05 prompt kernel: every
+        # prompt does (us there and on the mma.sync kernel, 16 heads, window 1,024: 2,048 tokens 43 and 74, 300 18 and 27, 64 14 and 16,
+        # 24 12 and 14; 17 behind 1,783 39 and 70).  The mma.sync kernel takes the page sizes and head groups which that one does not
+        # and every size under ULLM_B200_TC_ATTN=0 or "single"; the tests reach it by a larger number here.
         self.kept_pair_rows = 1
         self.window_attention_tc = get("ULLM_B200_WINDOW_ATTN_TC", "1") != "0"
         # rows per expert, on average, from which the routed experts' products of more than 16 tokens run on the tcgen05 kernel: at
