@@ -2225,7 +2225,8 @@ class Kernels:
                      page_size, window, scale, num_pages, ragged, ctx, fuse=None, keep_first: int = 0,
                      softcap: float = 0.0, parts=None, dist_bias=None, head_gate=None, rows: int | None = None, beside: bool = False) -> None:
         """Decode attention of the first `rows` rows (default: all), one token each (row i belongs to request row i): streams
-        the pages once.  `beside`: the launch in front is a tcgen05 prompt attention of other rows, and the kernel runs beside it.
+        the pages once.  `beside`: the launch in front is a tcgen05 prompt attention of other rows, and the kernel runs beside it;
+        nothing may be enqueued between the two (what it reads or writes would not be waited for).
         `keep_first` > 0 (with a window), `softcap` > 0 (capped scores) or `parts` (every head's weights on every
         kv head's values, 32-bit [T, num_q * num_kv * head_dim]; `out` unused), `dist_bias` or `head_gate`: the per-request
         split kernel, the one that takes them."""
@@ -2249,6 +2250,7 @@ class Kernels:
                 self._decb[key] = (torch.empty(n, dtype=torch.float32, device="cuda"),
                                    torch.zeros(513, dtype=torch.int32, device="cuda"),
                                    torch.zeros(512 * num_q, dtype=torch.int32, device="cuda"))
+                beside = False  # (the fills stand behind the prompt kernel, and the kernel writes what they fill)
             part, prefix, flags = self._decb[key]
             fn = self.lib.ullm_decode_attention_tcgen05 if tc else self.lib.ullm_decode_attention_balanced
             self._check(fn(
