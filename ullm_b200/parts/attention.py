@@ -304,10 +304,19 @@ class PagedAttention(Mixer, SharesInput):
     def _ragged(ctx) -> bool:
         return bool(ctx.decode_only and is_ragged(ctx.num_live_requests, ctx.max_kv_len, ctx.sum_kv_len))
 
-    def launches_only(self):
-        return (type(self) is PagedAttention and not self.general and self.own_kv
-                and not (self.position is not None and self.position.transforms_qk())
-                and all(n is None or n.launches_only() for n in (self.q_norm, self.k_norm)))
+    def launch_tensors(self):
+        if (not self.runs_as_written(PagedAttention) or self.general or not self.own_kv
+                or (self.position is not None and self.position.transforms_qk())):
+            return None
+        found = [self.w_qkv, self.tensors[self.names["o"]], *(b for b in (self.b_qkv, self.w_o_bias) if b is not None)]
+        for norm in (self.q_norm, self.k_norm):
+            tensors = norm.launch_tensors() if norm is not None else ()
+            if tensors is None:
+                return None
+            found += tensors
+        if self.position is not None:
+            found += self.position.tables().values()
+        return tuple(found)
 
     def output_projection(self):
         return self.tensors[self.names["o"]], self.w_o_bias
@@ -488,3 +497,5 @@ class PagedAttention(Mixer, SharesInput):
             **({} if plain else {"v_dim": self.value_dim, "keep_first": self.keep_first if self.window else 0}),
         )
         return self._project(attn, ctx, project_output, out)
+
+    written_forward = forward

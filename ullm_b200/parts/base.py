@@ -130,11 +130,20 @@ class Part:
                 out[key] = max(out.get(key, 0), size)
         return out
 
-    def launches_only(self) -> bool:
-        """True when `forward` in a step that is no decode step does nothing on the device but call the compiled launchers, leaves
-        nothing behind that a later part reads, and takes what differs between two parts of equal specs from their tensors
-        (`all_tensors`, the position encoding's tables) and caches alone: a layer of such parts can run from another one's list of launches."""
-        return False
+    # `forward` as the class that answers `launch_tensors` wrote it (see `runs_as_written`)
+    written_forward: Callable | None = None
+
+    def runs_as_written(self, cls: type) -> bool:
+        """Whether this is a `cls` itself whose `forward` is the one written there: a subclass may do more, and so may a `forward` that
+        was put in its place, on the part or on the class."""
+        return type(self) is cls and getattr(self.forward, "__func__", None) is cls.written_forward
+
+    def launch_tensors(self) -> tuple[torch.Tensor, ...] | None:
+        """None, unless `forward` in a step that is no decode step does nothing on the device but call the compiled launchers, leaves
+        nothing behind that a later part reads, and takes what differs between two parts of equal specs from tensors and caches alone:
+        then those tensors.  A layer of such parts can run from another one's list of launches, with these tensors in place of the
+        other's; nothing of its Python runs then, so this is asked of every layer in every step."""
+        return None
 
     # -- walking a tree of parts ------------------------------------------
     def all_decls(self, prefix: str = "") -> dict[str, ParamDecl]:

@@ -46,8 +46,16 @@ class PreNormResidualBlock(Block):
 
     takes_next_norm = True  # `forward` accepts the norm that the next block (or nobody) will apply first
 
-    def launches_only(self):
-        return type(self) is PreNormResidualBlock and all(p.launches_only() for p in self.subparts().values())
+    def launch_tensors(self):
+        if not self.runs_as_written(PreNormResidualBlock):
+            return None
+        found = []
+        for part in (self.mixer_norm, self.mixer, self.feed_forward_norm, self.feed_forward):
+            tensors = part.launch_tensors() if part is not None else None
+            if tensors is None:
+                return None
+            found += tensors
+        return tuple(found)
 
     def accepts_folded_norm(self) -> bool:
         """True when this block can start from an operand r * w and the rows' sums of squares that the block
@@ -124,6 +132,8 @@ class PreNormResidualBlock(Block):
         self.feed_forward_norm.forward(a, residual, out=h)
         y = self.feed_forward.forward(h, ctx)
         return y, residual
+
+    written_forward = forward
 
     def _fusable_chain(self, rows: int, residual):
         """The same parts as `_fusable_tail` needs, when the step's products are all the stream kernel."""

@@ -50,8 +50,8 @@ class GatedMLP(FeedForward):
             return None  # (the fused kernels know silu and gelu only)
         return self.w_gate_up, self.tensors[self.names["down"]], _ACTIVATIONS[self.activation]
 
-    def launches_only(self):
-        return True
+    def launch_tensors(self):
+        return (self.w_gate_up, self.tensors[self.names["down"]]) if self.runs_as_written(GatedMLP) else None
 
     def activation_elems(self):
         return 3 * self.intermediate_size + self.hidden_size  # gate | up, their product, the output
@@ -69,6 +69,8 @@ class GatedMLP(FeedForward):
         out = ctx.workspace.tokens("ffn.out", T, self.hidden_size, x.dtype)
         linear(act, self.tensors[self.names["down"]], out)
         return out
+
+    written_forward = forward
 
 
 @register_feed_forward("dense_mlp")

@@ -27,6 +27,10 @@ def _same(a, b) -> bool:
         return False
     if dataclasses.is_dataclass(a):
         return all(_same(getattr(a, f.name), getattr(b, f.name)) for f in dataclasses.fields(a))
+    if isinstance(a, dict):
+        return list(a) == list(b) and all(_same(x, b[k]) for k, x in a.items())
+    if isinstance(a, (list, tuple)):
+        return len(a) == len(b) and all(map(_same, a, b))
     return a == b
 
 
@@ -131,16 +135,16 @@ class DecoderModel(Part):
         if self._alike is None:
             order = [e.layer for e in self.schedule]
             specs = [self.spec.layers[i] for i in order[1:]]
-            self._alike = (len(specs) >= 4 and len(set(order)) == len(order) and self.blocks[order[1]].launches_only()
+            self._alike = (len(specs) >= 4 and len(set(order)) == len(order)
                            and not any(e.add_input or e.add_vector is not None or e.project_input or e.cache_of is not None
                                        for e in self.schedule)
                            and all(_same(specs[0], s) for s in specs[1:]))
         return self._alike
 
-    def _layer_tensors(self, i: int, caches) -> tuple:
-        c, block = caches[i], self.blocks[self.schedule[i].layer]
-        position = block.mixer.position
-        return (*block.all_tensors().values(), *(position.tables().values() if position is not None else ()), *(t for t in (c.k_pages, c.v_pages) if t is not None))
+    def _launch_tensors(self, i: int, caches) -> tuple | None:
+        """What layer i's launches take of its own (`Part.launch_tensors`, its pages), or None when it has to run itself."""
+        c, tensors = caches[i], self.blocks[self.schedule[i].layer].launch_tensors()
+        return None if tensors is None else (*tensors, *(t for t in (c.k_pages, c.v_pages) if t is not None))
 
     def forward_hidden(self, ctx, caches):
         """Runs the blocks over the step's tokens.  Returns (y, residual): what the last block left to be added
@@ -179,16 +183,19 @@ class DecoderModel(Part):
         first = listed = None
         for i, e in enumerate(self.schedule):
             block = self.blocks[e.layer]
-            if listing and i in (1, 2):
-                (x, residual), tape = K.record_launches(lambda: block.forward(x, residual, ctx, caches[i]))
-                if i == 1:
-                    first = tape
-                elif K.lists_alike(first, self._layer_tensors(1, caches), tape, self._layer_tensors(2, caches)):
-                    listed = tape
-                continue
-            if listed is not None:
-                K.run_list(listed, self._layer_tensors(i, caches))
-                continue
+            if listing and i > 0:
+                own = self._launch_tensors(i, caches)
+                if own is not None and i < 3:
+                    (x, residual), tape = K.record_launches(lambda: block.forward(x, residual, ctx, caches[i]))
+                    if i == 1:
+                        first = tape, own
+                    elif K.lists_alike(*first, tape, own):
+                        listed = tape
+                    continue
+                if own is not None and listed is not None:
+                    K.run_list(listed, own)
+                    continue
+                listing = False  # (what this layer leaves need not lie where a list takes it from)
             if e.project_input:
                 self._project_stream(residual if residual is not None else x, x0, ctx)
             if e.add_input or e.add_vector is not None:

@@ -40,8 +40,8 @@ class RMSNorm(Norm):
             return self._one_plus
         return self.tensors[self.param]
 
-    def launches_only(self):
-        return not self.around_zero  # (its weights lie in a tensor of their own then)
+    def launch_tensors(self):
+        return (self.weight,) if self.runs_as_written(RMSNorm) and not self.around_zero else None
 
     def rms_params(self):
         return self.weight, self.eps
@@ -65,6 +65,8 @@ class RMSNorm(Norm):
             out = x
         kernels().add_rmsnorm(x, residual, self.weight, self.eps, out)
         return out
+
+    written_forward = forward
 
 
 @register_norm("layernorm")
