@@ -31,6 +31,7 @@ class Listing(CpuKernels):
 
     def run_list(self, listed, tensors):
         self.listed += 1
+        return True
 
 
 CONFIG = dict(architectures=["Qwen3ForCausalLM"], num_hidden_layers=6, hidden_size=64, num_attention_heads=2, num_key_value_heads=1,
@@ -107,3 +108,12 @@ def test_specs_differ_in_fields_that_their_comparison_leaves_out():
 
     assert _same([S(1, 2)], [S(1, 2)]) and not _same([S(1, 2)], [S(1, 3)])
     assert not _same({"x": (S(1, 2),)}, {"x": (S(1, 3),)}) and not _same({"x": 1}, {"y": 1})
+
+
+def test_a_list_that_is_refused_leaves_the_layer_to_itself(monkeypatch):
+    monkeypatch.setattr(Listing, "run_list", lambda self, listed, tensors: False)
+    called = []
+    forward = GatedMLP.forward
+    monkeypatch.setattr(GatedMLP, "forward", lambda self, *a, **kw: called.append(self) or forward(self, *a, **kw))
+    monkeypatch.setattr(GatedMLP, "written_forward", GatedMLP.forward)
+    assert run() == 0 and len(called) == 6

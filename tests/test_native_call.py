@@ -157,3 +157,20 @@ def test_lists_of_launches_run_with_other_tensors(native):
     failing = ctypes.CFUNCTYPE(ctypes.c_int, *[ctypes.c_longlong] * 6)(lambda *x: 4)
     bad = native.bind("ullm_argmax", ctypes.cast(failing, ctypes.c_void_p).value)
     assert recorded(native, bad, [(None, 1, 2, 3, None, None)]) is None
+
+
+def test_a_list_refuses_tensors_of_other_sizes(native):
+    """The launches take sizes and types from the recorded layer: a shorter tensor would be read past its end, also where the recorded
+    address is its first."""
+    seen = []
+    target = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_float, ctypes.c_void_p)(lambda *a: seen.append(a) or 0)
+    fn = native.bind("ullm_softcap_f32", ctypes.cast(target, ctypes.c_void_p).value)
+    a, b, c = ((torch.zeros(8),) for _ in range(3))
+    ta, tb = (recorded(native, fn, [(t[0], 8, 1.0, None)]) for t in (a, b))
+    assert native.alike(ta, a, tb, b)
+    seen.clear()
+    for other in ((c[0][:7],), (torch.zeros(9),), (torch.zeros(8, 2)[:, 0],), (), (c[0], c[0]), (c[0].view(torch.int32),)):
+        with pytest.raises(ValueError):
+            native.replay(tb, other)
+    assert not seen
+    assert native.replay(tb, c) == 0 and seen[0][0] == c[0].data_ptr()

@@ -106,11 +106,17 @@ struct Moved {  // argument `arg` of launch `launch` lies `offset` bytes into te
   int launch, arg, tensor;
   unsigned long long offset;
 };
+struct Span {  // a layer's tensor; `bytes` 0: not in one piece
+  unsigned long long at, bytes;
+  int type, device;
+  bool like(const Span& o) const { return bytes == o.bytes && type == o.type && device == o.device; }
+};
 struct Tape {
   PyObject_HEAD
   std::vector<Launch>* launches;
-  std::vector<Moved>* moved;  // null: not compared yet
-  bool whole;                 // nothing ran that is not in the list
+  std::vector<Moved>* moved;               // null: not compared yet
+  std::vector<Span>* make;                 // of the compared layers' tensors: how long they are, and of what
+  bool whole;                              // nothing ran that is not in the list
 };
 thread_local Tape* recording = nullptr;
 
@@ -330,6 +336,7 @@ PyObject* record(PyObject*, PyObject*) {
   t->launches = new std::vector<Launch>;
   t->launches->reserve(32);
   t->moved = nullptr;
+  t->make = nullptr;
   t->whole = true;
   Py_XDECREF(reinterpret_cast<PyObject*>(recording));
   recording = t;
@@ -352,9 +359,6 @@ PyObject* recorded(PyObject*, PyObject*) {
   return reinterpret_cast<PyObject*>(t);
 }
 
-struct Span {
-  unsigned long long at, bytes;
-};
 bool spans(PyObject* tensors, std::vector<Span>* out) {
   if (!PyTuple_Check(tensors)) {
     PyErr_SetString(PyExc_TypeError, "a layer's tensors are a tuple");
@@ -367,7 +371,8 @@ bool spans(PyObject* tensors, std::vector<Span>* out) {
       return false;
     }
     const at::Tensor& t = THPVariable_Unpack(o);
-    out->push_back({reinterpret_cast<unsigned long long>(t.data_ptr()), t.is_contiguous() ? static_cast<unsigned long long>(t.nbytes()) : 0});
+    out->push_back({reinterpret_cast<unsigned long long>(t.data_ptr()), t.is_contiguous() ? static_cast<unsigned long long>(t.nbytes()) : 0,
+                    static_cast<int>(t.scalar_type()), t.is_cuda() ? t.get_device() : -1});
   }
   return true;
 }
@@ -389,7 +394,7 @@ PyObject* alike(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (!spans(args[1], &sa) || !spans(args[3], &sb)) return nullptr;
   if (sa.size() != sb.size() || a->launches->size() != b->launches->size()) Py_RETURN_FALSE;
   for (size_t i = 0; i < sa.size(); ++i)
-    if (sa[i].bytes != sb[i].bytes || sa[i].bytes == 0) Py_RETURN_FALSE;
+    if (!sa[i].like(sb[i]) || sa[i].bytes == 0) Py_RETURN_FALSE;
   std::vector<Moved> moved;
   for (size_t l = 0; l < a->launches->size(); ++l) {
     const Launch &x = (*a->launches)[l], &y = (*b->launches)[l];
@@ -409,7 +414,9 @@ PyObject* alike(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
   }
   delete b->moved;
+  delete b->make;
   b->moved = new std::vector<Moved>(std::move(moved));
+  b->make = new std::vector<Span>(std::move(sb));
   Py_RETURN_TRUE;
 }
 
@@ -427,11 +434,12 @@ PyObject* replay(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   std::vector<Span> to;
   if (!spans(args[1], &to)) return nullptr;
-  for (const Moved& m : *t->moved)
-    if (m.tensor >= static_cast<int>(to.size()) || m.offset >= to[m.tensor].bytes) {
-      PyErr_SetString(PyExc_ValueError, "replay: tensors of another make");
-      return nullptr;
-    }
+  bool same = to.size() == t->make->size();  // (the launches take sizes and types from the layer that was recorded)
+  for (size_t i = 0; same && i < to.size(); ++i) same = to[i].like((*t->make)[i]);
+  if (!same) {
+    PyErr_SetString(PyExc_ValueError, "replay: tensors of another make");
+    return nullptr;
+  }
   long long code = 0;
   const char* thrown = nullptr;
   Py_BEGIN_ALLOW_THREADS
@@ -487,6 +495,7 @@ PyMODINIT_FUNC PyInit_ullm_b200_native() {
   TapeType.tp_dealloc = [](PyObject* o) {
     delete reinterpret_cast<Tape*>(o)->launches;
     delete reinterpret_cast<Tape*>(o)->moved;
+    delete reinterpret_cast<Tape*>(o)->make;
     PyObject_Free(o);
   };
   if (PyType_Ready(&LauncherType) < 0 || PyType_Ready(&TapeType) < 0) return nullptr;

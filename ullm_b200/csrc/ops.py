@@ -197,12 +197,17 @@ class Kernels:
         """True when list b is list a but for addresses inside the layers' tensors; b can then be run for another layer."""
         return a is not None and b is not None and a[1] == b[1] and _native.alike(a[0], tensors_a, b[0], tensors_b)
 
-    def run_list(self, listed, tensors) -> None:
-        code = _native.replay(listed[0], tensors)
+    def run_list(self, listed, tensors) -> bool:
+        """Runs the list with these tensors; False (nothing ran) where their sizes are not the recorded layer's."""
+        try:
+            code = _native.replay(listed[0], tensors)
+        except ValueError:
+            return False
         if code != 0:
             raise KernelError(f"a layer's launches: {_ERRORS.get(code, f'error {code}')}")
         self.launches += listed[1]
         self.listed_layers += 1
+        return True
 
     # -- switches -----------------------------------------------------------
     SWITCHES = ("ULLM_B200_PDL", "ULLM_B200_DECODE_SPLIT_TARGET", "ULLM_B200_TC_ATTN", "ULLM_B200_DECODE_CLUSTER",

@@ -192,8 +192,7 @@ class DecoderModel(Part):
                     elif K.lists_alike(*first, tape, own):
                         listed = tape
                     continue
-                if own is not None and listed is not None:
-                    K.run_list(listed, own)
+                if own is not None and listed is not None and K.run_list(listed, own):
                     continue
                 listing = False  # (what this layer leaves need not lie where a list takes it from)
             if e.project_input:
