@@ -174,3 +174,26 @@ def test_a_list_refuses_tensors_of_other_sizes(native):
             native.replay(tb, other)
     assert not seen
     assert native.replay(tb, c) == 0 and seen[0][0] == c[0].data_ptr()
+
+
+def test_a_tensor_without_storage_is_an_exception(native):
+    """As `Tensor.data_ptr` says it, from every way in."""
+    t = torch.zeros(2, 2).to_sparse()
+    never = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_float, ctypes.c_void_p)(lambda *a: pytest.fail("called"))
+    fn = native.bind("ullm_softcap_f32", ctypes.cast(never, ctypes.c_void_p).value)
+    with pytest.raises(RuntimeError, match="doesn't have storage"):
+        native.ptr(t)
+    with pytest.raises(RuntimeError, match="doesn't have storage"):
+        fn(t, 4, 1.0, None)
+
+
+def test_lists_of_tensors_without_storage_are_an_exception(native):
+    quiet = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_float, ctypes.c_void_p)(lambda *a: 0)
+    fn = native.bind("ullm_softcap_f32", ctypes.cast(quiet, ctypes.c_void_p).value)
+    a, b, t = torch.zeros(3), torch.zeros(3), torch.zeros(2, 2).to_sparse()
+    ta, tb = (recorded(native, fn, [(x, 3, 1.0, None)]) for x in (a, b))
+    with pytest.raises(RuntimeError, match="doesn't have storage"):
+        native.alike(ta, (a, t), tb, (b, t))
+    assert native.alike(ta, (a,), tb, (b,))
+    with pytest.raises(RuntimeError, match="doesn't have storage"):
+        native.replay(tb, (t,))

@@ -22,14 +22,28 @@
 #include <ATen/Context.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstring>
+#include <exception>
 #include <tuple>
 #include <utility>
 #include <vector>
 
 namespace {
+
+// What a function called from Python answers where C++ threw (a tensor without storage, the library's handle): Python's exception for it.
+PyObject* thrown(const std::exception_ptr& e = std::current_exception()) {
+  try {
+    std::rethrow_exception(e);
+  } catch (const std::exception&) {
+    torch::translate_exception_to_python(e);
+  } catch (...) {
+    PyErr_SetString(PyExc_RuntimeError, "an unknown C++ exception");
+  }
+  return nullptr;
+}
 
 bool take(PyObject* o, void** v) {
   if (o == Py_None) {
@@ -148,7 +162,7 @@ using Call = PyObject* (*)(void*, PyObject* const*, Py_ssize_t);
 
 // LISTED: launches and settings, not questions
 template <bool LISTED, class R, class... A, std::size_t... N>
-PyObject* invoke(void* fn, PyObject* const* args, std::index_sequence<N...>) {
+PyObject* invoke(void* fn, PyObject* const* args, std::index_sequence<N...>) try {
   std::tuple<A...> v;
   if (!(take(args[N], &std::get<N>(v)) && ...)) return nullptr;
   if (LISTED && recording != nullptr) note(again<R, A...>, fn, std::get<N>(v)...);
@@ -165,6 +179,8 @@ PyObject* invoke(void* fn, PyObject* const* args, std::index_sequence<N...>) {
     if (LISTED && recording != nullptr && r != 0) recording->whole = false;  // (what follows depends on it)
     return PyLong_FromLongLong(r);
   }
+} catch (...) {
+  return thrown();  // (of the arguments: a launcher throws nothing)
 }
 template <bool LISTED, class R, class... A>
 PyObject* call(void* fn, PyObject* const* args, Py_ssize_t n) {
@@ -232,19 +248,18 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return nullptr;
 }
 
-PyObject* ptr(PyObject*, PyObject* o) {
+PyObject* ptr(PyObject*, PyObject* o) try {
   if (o == Py_None) Py_RETURN_NONE;
   if (!THPVariable_Check(o)) return PyObject_CallMethod(o, "data_ptr", nullptr);
   return PyLong_FromVoidPtr(THPVariable_Unpack(o).data_ptr());
+} catch (...) {
+  return thrown();
 }
 
-PyObject* stream(PyObject*, PyObject*) {
-  try {
-    return PyLong_FromVoidPtr(at::cuda::getCurrentCUDAStream().stream());
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+PyObject* stream(PyObject*, PyObject*) try {
+  return PyLong_FromVoidPtr(at::cuda::getCurrentCUDAStream().stream());
+} catch (...) {
+  return thrown();
 }
 
 PyObject* set_slow_need(PyObject*, PyObject* o) {
@@ -254,7 +269,7 @@ PyObject* set_slow_need(PyObject*, PyObject* o) {
 }
 
 // need(tensor, name, dtype=None, contiguous=True)
-PyObject* need(PyObject*, PyObject* const* args, Py_ssize_t n, PyObject* kwnames) {
+PyObject* need(PyObject*, PyObject* const* args, Py_ssize_t n, PyObject* kwnames) try {
   const Py_ssize_t named = kwnames == nullptr ? 0 : PyTuple_GET_SIZE(kwnames);
   if (n >= 2 && n + named <= 4 && THPVariable_Check(args[0])) {
     PyObject* dtype = n > 2 ? args[2] : Py_None;
@@ -276,6 +291,8 @@ PyObject* need(PyObject*, PyObject* const* args, Py_ssize_t n, PyObject* kwnames
     }
   }
   return PyObject_Vectorcall(slow_need, args, n, kwnames);
+} catch (...) {
+  return thrown();
 }
 
 // out [M, N] (bfloat16, or float32 where `wide`) = x [M, K] . w [N, K]^T, on the current stream; the library's status
@@ -286,7 +303,7 @@ int product(void* x, void* w, void* out, int M, int N, int K, int wide) {
 }
 
 // mm(x, w, out): the product, False for what only `torch.mm` should decide
-PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) try {
   if (n != 3 || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1]) || !THPVariable_Check(args[2])) {
     PyErr_SetString(PyExc_TypeError, "mm(x, w, out): three tensors");
     return nullptr;
@@ -310,21 +327,23 @@ PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (recording != nullptr)
     note(again<int, void*, void*, void*, int, int, int, int>, reinterpret_cast<void*>(product), px, pw, po, m, nn, k, f);
   int rc = 0;
-  const char* thrown = nullptr;
+  std::exception_ptr failed;
   Py_BEGIN_ALLOW_THREADS
   try {
     rc = product(px, pw, po, m, nn, k, f);
-  } catch (const std::exception&) {
-    thrown = "mm: the library's handle could not be had";
+  } catch (...) {
+    failed = std::current_exception();
   }
   Py_END_ALLOW_THREADS
-  if (thrown != nullptr || rc != 0) {
+  if (failed || rc != 0) {
     if (recording != nullptr) recording->whole = false;
-    if (thrown != nullptr) PyErr_SetString(PyExc_RuntimeError, thrown);
-    else PyErr_Format(PyExc_RuntimeError, "cublasGemmEx (%d x %d . %d x %d) answered %d", m, k, nn, k, rc);
+    if (failed) return thrown(failed);
+    PyErr_Format(PyExc_RuntimeError, "cublasGemmEx (%d x %d . %d x %d) answered %d", m, k, nn, k, rc);
     return nullptr;
   }
   Py_RETURN_TRUE;
+} catch (...) {
+  return thrown();
 }
 
 // ---- record, compare, run again ---------------------------------------------------------------------------------------------------
@@ -383,7 +402,7 @@ bool is_tape(PyObject* o) {
 }
 
 // alike(a, a's tensors, b, b's tensors): whether b's list is a's with the addresses moved; b can then be replayed
-PyObject* alike(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* alike(PyObject*, PyObject* const* args, Py_ssize_t n) try {
   if (n != 4) {
     PyErr_SetString(PyExc_TypeError, "alike(a, tensors of a, b, tensors of b)");
     return nullptr;
@@ -418,10 +437,12 @@ PyObject* alike(PyObject*, PyObject* const* args, Py_ssize_t n) {
   b->moved = new std::vector<Moved>(std::move(moved));
   b->make = new std::vector<Span>(std::move(sb));
   Py_RETURN_TRUE;
+} catch (...) {
+  return thrown();
 }
 
 // replay(list, tensors of another layer): runs it there; the first launch's code that is not 0, else 0
-PyObject* replay(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* replay(PyObject*, PyObject* const* args, Py_ssize_t n) try {
   if (n != 2) {
     PyErr_SetString(PyExc_TypeError, "replay(list, tensors)");
     return nullptr;
@@ -441,7 +462,7 @@ PyObject* replay(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return nullptr;
   }
   long long code = 0;
-  const char* thrown = nullptr;
+  std::exception_ptr failed;
   Py_BEGIN_ALLOW_THREADS
   try {
     size_t at = 0;
@@ -453,15 +474,14 @@ PyObject* replay(PyObject*, PyObject* const* args, Py_ssize_t n) {
         bits[(*t->moved)[at].arg] = to[(*t->moved)[at].tensor].at + (*t->moved)[at].offset;
       code = launch.again(launch.fn, bits);
     }
-  } catch (const std::exception&) {
-    thrown = "replay: the library's handle could not be had";
+  } catch (...) {
+    failed = std::current_exception();
   }
   Py_END_ALLOW_THREADS
-  if (thrown != nullptr) {
-    PyErr_SetString(PyExc_RuntimeError, thrown);
-    return nullptr;
-  }
+  if (failed) return thrown(failed);
   return PyLong_FromLongLong(code);
+} catch (...) {
+  return thrown();
 }
 
 PyMethodDef methods[] = {
