@@ -197,3 +197,60 @@ def test_lists_of_tensors_without_storage_are_an_exception(native):
     assert native.alike(ta, (a,), tb, (b,))
     with pytest.raises(RuntimeError, match="doesn't have storage"):
         native.replay(tb, (t,))
+
+
+@pytest.mark.gpu
+@pytest.mark.needs_cuda
+def test_the_product_is_torchs_where_somebody_watches_or_chooses(native):
+    """Profilers, modes and subclasses see `torch.mm`; another preferred library and tunable operations decide in it."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Sub(torch.Tensor):
+        pass
+
+    x, w = torch.randn(4, 8, device="cuda").bfloat16(), torch.randn(6, 8, device="cuda").bfloat16()
+    out = torch.ones(4, 6, device="cuda").bfloat16()
+    with Function():
+        assert native.mm(x, w, out) is False
+    with Dispatch():
+        assert native.mm(x, w, out) is False
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]):
+        assert native.mm(x, w, out) is False
+    assert native.mm(x.as_subclass(Sub), w, out) is False and native.mm(x, torch.nn.Parameter(w), out) is False
+    before = torch.backends.cuda.preferred_blas_library()
+    torch.backends.cuda.preferred_blas_library("cublaslt")
+    try:
+        assert native.mm(x, w, out) is False
+    finally:
+        torch.backends.cuda.preferred_blas_library(before)
+    torch.cuda.tunable.enable(True)
+    try:
+        assert native.mm(x, w, out) is False
+    finally:
+        torch.cuda.tunable.enable(False)
+    assert torch.equal(out, torch.ones_like(out))
+    assert native.mm(x, torch.nn.Parameter(w, requires_grad=False), out) is True
+
+
+@pytest.mark.gpu
+@pytest.mark.needs_cuda
+def test_a_profiler_sees_the_products_of_the_engine():
+    from ullm_b200.csrc import kernels
+
+    K = kernels()
+    x, w = torch.randn(400, 2048, device="cuda").bfloat16(), torch.randn(4096, 2048, device="cuda").bfloat16()
+    out = torch.empty(400, 4096, device="cuda").bfloat16()
+    K.linear(x, w, out)
+    want = out.clone()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as seen:
+        K.linear(x, w, out)
+    assert any(e.key == "aten::mm" for e in seen.key_averages()) and torch.equal(out, want)

@@ -20,7 +20,11 @@
 #include <Python.h>
 
 #include <ATen/Context.h>
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/tunable/Tunable.h>
+#include <ATen/record_function.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -302,6 +306,22 @@ int product(void* x, void* w, void* out, int M, int N, int K, int wide) {
                       K, &zero, out, wide ? CUDA_R_32F : CUDA_R_16BF, N, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
 }
 
+// Whether `torch.mm` would be this product and nothing besides: nobody watches or replaces torch's operations (profilers, dispatch and
+// function modes, subclasses, transforms), and no setting picks another library or algorithm.
+bool plain(PyObject* o) {
+  if (!THPVariable_CheckExact(o)) return false;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return t.has_storage() && !t.key_set().has(c10::DispatchKey::Python) && !t.requires_grad() && !t._fw_grad(0).defined();
+}
+bool as_torch_does() {
+  if (at::hasCallbacks() || c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled()) return false;
+  at::Context& context = at::globalContext();
+  const at::BlasBackend library = context.blasPreferredBackend();
+  return (library == at::BlasBackend::Default || library == at::BlasBackend::Cublas) &&
+         context.allowBF16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK &&
+         !context.deterministicAlgorithms() && !at::cuda::tunable::getTuningContext()->IsTunableOpEnabled();
+}
+
 // mm(x, w, out): the product, False for what only `torch.mm` should decide
 PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) try {
   if (n != 3 || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1]) || !THPVariable_Check(args[2])) {
@@ -309,18 +329,14 @@ PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) try {
     return nullptr;
   }
   const at::Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]), &out = THPVariable_Unpack(args[2]);
+  if (!plain(args[0]) || !plain(args[1]) || !plain(args[2])) Py_RETURN_FALSE;
   if (x.dim() != 2 || w.dim() != 2 || out.dim() != 2 || !x.is_cuda() || !w.is_cuda() || !out.is_cuda()) Py_RETURN_FALSE;
   const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
   const bool wide = out.scalar_type() == at::kFloat;
   if (M < 2 || N < 2 || K < 2 || M > INT_MAX || N > INT_MAX || K > INT_MAX || w.size(1) != K || out.size(0) != M || out.size(1) != N ||
       x.scalar_type() != at::kBFloat16 || w.scalar_type() != at::kBFloat16 || !(wide || out.scalar_type() == at::kBFloat16) ||
       !x.is_contiguous() || !w.is_contiguous() || !out.is_contiguous() || x.get_device() != w.get_device() ||
-      x.get_device() != out.get_device() || x.get_device() != at::cuda::current_device() || x.requires_grad() || w.requires_grad() ||
-      out.requires_grad())
-    Py_RETURN_FALSE;
-  at::Context& context = at::globalContext();
-  if (context.allowBF16ReductionCuBLAS() != at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK ||
-      context.deterministicAlgorithms())
+      x.get_device() != out.get_device() || x.get_device() != at::cuda::current_device() || !as_torch_does())
     Py_RETURN_FALSE;
   void *px = x.data_ptr(), *pw = w.data_ptr(), *po = out.data_ptr();
   const int m = static_cast<int>(M), nn = static_cast<int>(N), k = static_cast<int>(K), f = wide ? 1 : 0;
