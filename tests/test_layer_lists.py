@@ -1,12 +1,14 @@
 """Which layers may run from another layer's list of launches: those of the parts as they are written, and no others (no GPU: the lists
 themselves are a stand-in's)."""
 
+from types import SimpleNamespace
+
 import pytest
 
 from cpu_kernels import CpuKernels
 from helpers import random_ids
 from ullm_b200 import csrc
-from ullm_b200.csrc import set_kernels
+from ullm_b200.csrc import ops, set_kernels
 from ullm_b200.parts.mlp import GatedMLP
 from ullm_b200.parts.model import _same
 from ullm_b200.parts.norm import RMSNorm
@@ -117,3 +119,12 @@ def test_a_list_that_is_refused_leaves_the_layer_to_itself(monkeypatch):
     monkeypatch.setattr(GatedMLP, "forward", lambda self, *a, **kw: called.append(self) or forward(self, *a, **kw))
     monkeypatch.setattr(GatedMLP, "written_forward", GatedMLP.forward)
     assert run() == 0 and len(called) == 6
+
+
+@pytest.mark.parametrize("code,says", [(4, ops._ERRORS[4]), (-7, "cublasGemmEx answered 7"), (99, "error 99")])
+def test_a_list_that_fails_says_whose_error_it_was(monkeypatch, code, says):
+    monkeypatch.setattr(ops, "_native", SimpleNamespace(replay=lambda tape, tensors: code))
+    k = ops.Kernels.__new__(ops.Kernels)
+    with pytest.raises(ops.KernelError) as e:
+        k.run_list(("list", 3), ())
+    assert says in str(e.value)

@@ -306,6 +306,9 @@ int product(void* x, void* w, void* out, int M, int N, int K, int wide) {
                       K, &zero, out, wide ? CUDA_R_32F : CUDA_R_16BF, N, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
 }
 
+// As a list runs it: a launcher's codes are 0 and above, the library's status counts down from there.
+int listed_product(void* x, void* w, void* out, int M, int N, int K, int wide) { return -product(x, w, out, M, N, K, wide); }
+
 // Whether `torch.mm` would be this product and nothing besides: nobody watches or replaces torch's operations (profilers, dispatch and
 // function modes, subclasses, transforms), and no setting picks another library or algorithm.
 bool plain(PyObject* o) {
@@ -341,7 +344,7 @@ PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) try {
   void *px = x.data_ptr(), *pw = w.data_ptr(), *po = out.data_ptr();
   const int m = static_cast<int>(M), nn = static_cast<int>(N), k = static_cast<int>(K), f = wide ? 1 : 0;
   if (recording != nullptr)
-    note(again<int, void*, void*, void*, int, int, int, int>, reinterpret_cast<void*>(product), px, pw, po, m, nn, k, f);
+    note(again<int, void*, void*, void*, int, int, int, int>, reinterpret_cast<void*>(listed_product), px, pw, po, m, nn, k, f);
   int rc = 0;
   std::exception_ptr failed;
   Py_BEGIN_ALLOW_THREADS
@@ -457,7 +460,8 @@ PyObject* alike(PyObject*, PyObject* const* args, Py_ssize_t n) try {
   return thrown();
 }
 
-// replay(list, tensors of another layer): runs it there; the first launch's code that is not 0, else 0
+// replay(list, tensors of another layer): runs it there; the first launch's code that is not 0 (below it: the library's status,
+// negated), else 0
 PyObject* replay(PyObject*, PyObject* const* args, Py_ssize_t n) try {
   if (n != 2) {
     PyErr_SetString(PyExc_TypeError, "replay(list, tensors)");

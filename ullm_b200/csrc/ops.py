@@ -204,7 +204,7 @@ class Kernels:
         except ValueError:
             return False
         if code != 0:
-            raise KernelError(f"a layer's launches: {_ERRORS.get(code, f'error {code}')}")
+            raise KernelError(f"a layer's launches: {_ERRORS.get(code, f'error {code}') if code > 0 else f'cublasGemmEx answered {-code}'}")
         self.launches += listed[1]
         self.listed_layers += 1
         return True
