@@ -254,3 +254,52 @@ def test_a_profiler_sees_the_products_of_the_engine():
     with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as seen:
         K.linear(x, w, out)
     assert any(e.key == "aten::mm" for e in seen.key_averages()) and torch.equal(out, want)
+
+
+def test_without_headers_the_library_is_called_through_ctypes(monkeypatch):
+    """Where the extension module cannot be built, the kernels run all the same: a warning, the same arguments, nothing listed."""
+    from ullm_b200.csrc import build as b
+
+    def missing(*a, **kw):
+        raise RuntimeError("g++ failed on native_call.cpp: Python.h: No such file or directory")
+
+    monkeypatch.setattr(b, "load_native", missing)
+    monkeypatch.setattr(b, "build_native", missing)
+    assert b.build(verbose=False).endswith(b.LIB_NAME)
+    with pytest.warns(UserWarning, match="Python.h"):
+        plain = b.calls()
+    plain.set_slow_need(ops._checked)
+    seen = []
+    target = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_float, ctypes.c_void_p)(lambda *a: seen.append(a) or 3)
+    fn = plain.bind("ullm_softcap_f32", ctypes.cast(target, ctypes.c_void_p).value)
+    t = torch.zeros(3)
+    assert fn(t, 1 << 40, 0.5, None) == 3 and fn(plain.ptr(t), 1, 0.5, 1 << 41) == 3
+    assert seen == [(t.data_ptr(), 1 << 40, 0.5, None), (t.data_ptr(), 1, 0.5, 1 << 41)]
+    assert plain.mm(t, t, t) is False and plain.record() is None and plain.unlisted() is None and plain.recorded() is None
+    with pytest.raises(ops.KernelError, match="x is on cpu"):
+        plain.need(t, "x")
+    for wrong in ((t, 1, 0.5), ("x", 1, 0.5, None)):
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            fn(*wrong)
+
+
+@pytest.mark.gpu
+@pytest.mark.needs_cuda
+def test_a_kernel_called_through_ctypes(monkeypatch):
+    from ullm_b200.csrc import build as b
+    from ullm_b200.csrc.plain_call import PlainCalls
+
+    x = torch.randn(5, 64, device="cuda").bfloat16()
+    w, want = torch.rand(64, device="cuda"), torch.empty(5, 64, device="cuda").bfloat16()
+    names = ("_native", "_ptr", "_need", "_stream")
+    for n in names:
+        monkeypatch.setattr(ops, n, getattr(ops, n))  # (put back afterwards)
+    ops.Kernels().add_rmsnorm(x, None, w, 1e-6, want)
+    monkeypatch.setattr(ops, "calls", PlainCalls)
+    k, out = ops.Kernels(), torch.empty_like(want)
+    assert isinstance(ops._native, PlainCalls)
+    k.add_rmsnorm(x, None, w, 1e-6, out)
+    product = torch.empty(5, 64, device="cuda").bfloat16()
+    k.linear(x, torch.eye(64, device="cuda").bfloat16(), product)
+    k.raise_on_status()
+    assert torch.equal(out, want) and torch.equal(product, x)

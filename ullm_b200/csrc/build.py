@@ -19,6 +19,7 @@ import sysconfig
 import tempfile
 import threading
 import time
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -144,6 +145,17 @@ def build_native(verbose: bool = True, force: bool = False) -> str:
     return lib
 
 
+def calls():
+    """The calls into the library: the extension module of native_call.cpp, or ctypes where that cannot be built or loaded."""
+    try:
+        return load_native()
+    except (RuntimeError, OSError, ImportError) as e:
+        from .plain_call import PlainCalls
+
+        warnings.warn(f"the kernels are called through ctypes, which is slower: native_call.cpp could not be used ({e})")
+        return PlainCalls()
+
+
 def load_native():
     """The extension module of native_call.cpp."""
     name = NATIVE_NAME.split(".")[0]
@@ -159,7 +171,10 @@ def load_native():
 def build(verbose: bool = True, force: bool = False) -> str:
     """Returns the path of an up-to-date library, compiling if needed.  Prints
     a line per file and a heartbeat every few seconds while nvcc runs."""
-    build_native(verbose, force)
+    try:
+        build_native(verbose, force)
+    except (RuntimeError, OSError) as e:  # (see `calls`)
+        print(f"[ullm_b200 build] native_call.cpp was not built: {e}", file=sys.stderr, flush=True)
     if not force:
         lib = find_built()
         if lib:

@@ -15,7 +15,7 @@ from typing import NamedTuple
 
 import torch
 
-from .build import build, load_native
+from .build import build, calls
 from .launchers import LAUNCHERS, QUERIES
 
 _DT = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
@@ -137,7 +137,7 @@ class _Library:
     def __init__(self, path: str):
         global _ptr, _need, _stream, _native
         self._dll = ctypes.CDLL(path)
-        _native = load_native()
+        _native = calls()
         _native.set_slow_need(_checked)
         _ptr, _need, _stream = _native.ptr, _native.need, _native.stream
         for name in (*LAUNCHERS, *QUERIES):
