@@ -15,6 +15,7 @@ __global__ void __launch_bounds__(64) wait_selftest_kernel(int limit, int* statu
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tmem_base_slot;
   __shared__ int gave_up;
+  pdl_wait();  // (it has nothing to read; but a kernel behind it takes its end for the end of all in front)
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     gave_up = 0;
