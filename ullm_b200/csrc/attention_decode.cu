@@ -82,10 +82,10 @@ __device__ __forceinline__ float dec_tanh(float x) {
 // BESIDE: see decode_core.cuh.  (A constant: with the wait under a condition the loads behind it were moved in front of it.)
 template <int D, bool CL, bool BESIDE = false>
 __global__ void __launch_bounds__(DEC_WARPS * 32)
-decode_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_row_stride,
-                        const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
-                        const int* __restrict__ block_table, int max_pages, const int* __restrict__ req_slots,
-                        const int* __restrict__ kv_len, __nv_bfloat16* __restrict__ out, float* __restrict__ part_o,
+decode_attention_kernel(const __nv_bfloat16* q, long long q_row_stride,
+                        const __nv_bfloat16* k_cache, const __nv_bfloat16* v_cache,
+                        const int* block_table, int max_pages, const int* req_slots,
+                        const int* kv_len, __nv_bfloat16* __restrict__ out, float* __restrict__ part_o,
                         float* __restrict__ part_ml, int num_q, int num_kv, int page_size, int window,
                         float scale_log2, long long num_pages, int* status, const DecFuse fu) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -547,9 +547,9 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_row_str
 
 // out[b, h, :] = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M)
 template <int D>
-__global__ void decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+__global__ void decode_merge_kernel(const float* part_o, const float* part_ml,
                                     __nv_bfloat16* __restrict__ out, int num_splits, float* __restrict__ out_f32,
-                                    const __nv_bfloat16* __restrict__ gate, long long gate_stride, int num_q) {
+                                    const __nv_bfloat16* gate, long long gate_stride, int num_q) {
   pdl_launch_dependents();
   pdl_wait();
   const long long bh = blockIdx.x;

@@ -63,12 +63,12 @@ struct AttExtras {
 };
 
 template <typename T, int OREGS>
-__global__ void paged_attention_generic_kernel(const T* __restrict__ q, long long q_row_stride, T* __restrict__ out,
-                                               const T* __restrict__ k_cache, const T* __restrict__ v_cache,
-                                               const int* __restrict__ block_table, int max_pages,
-                                               const int* __restrict__ req_slots,
-                                               const int* __restrict__ cu_q, const int* __restrict__ kv_len,
-                                               const int* __restrict__ token_req, int tokens, int num_q, int num_kv,
+__global__ void paged_attention_generic_kernel(const T* q, long long q_row_stride, T* __restrict__ out,
+                                               const T* k_cache, const T* v_cache,
+                                               const int* block_table, int max_pages,
+                                               const int* req_slots,
+                                               const int* cu_q, const int* kv_len,
+                                               const int* token_req, int tokens, int num_q, int num_kv,
                                                int head_dim, int page_size, int window, float scale,
                                                long long num_pages, int* status, int v_dim, int keep_first,
                                                float softcap, int v_rep, float* __restrict__ out_f32, AttExtras ex) {
@@ -195,7 +195,7 @@ __global__ void paged_attention_generic_kernel(const T* __restrict__ q, long lon
 // reads its column of the parts once and finishes the GQ heads of that kv head together; the mixer lies in shared
 // memory.  GQ = 0: any group size, one head at a time.
 template <typename T, int GQ>
-__global__ void mix_heads_kernel(const float* __restrict__ part, const float* __restrict__ mix, T* __restrict__ out,
+__global__ void mix_heads_kernel(const float* part, const float* __restrict__ mix, T* __restrict__ out,
                                  long long total, int num_q, int num_kv, int v_dim, int in_smem) {
   extern __shared__ float mix_smem[];  // [num_q][num_q], unless the mixer is too large for it
   pdl_launch_dependents();

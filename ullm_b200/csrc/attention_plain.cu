@@ -96,10 +96,10 @@ __device__ __forceinline__ bool pl_odd(const float4& v) {
 
 template <typename T, int D>
 __global__ void __launch_bounds__(PT_THREADS, 2)
-plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T* __restrict__ out,
-                              const T* __restrict__ k_cache, const T* __restrict__ v_cache,
-                              const int* __restrict__ block_table, int max_pages, const int* __restrict__ req_slots,
-                              const int* __restrict__ cu_q, const int* __restrict__ kv_len, const int* __restrict__ token_req,
+plain_attention_prompt_kernel(const T* q, long long q_row_stride, T* __restrict__ out,
+                              const T* k_cache, const T* v_cache,
+                              const int* block_table, int max_pages, const int* req_slots,
+                              const int* cu_q, const int* kv_len, const int* token_req,
                               int requests, int num_q, int num_kv, int page_size, int window, float scale,
                               long long num_pages, int* status) {
   constexpr int ST = D + PT_PAD;
@@ -355,10 +355,10 @@ plain_attention_prompt_kernel(const T* __restrict__ q, long long q_row_stride, T
 // GQ query heads of a kv head at a time (grid z counts them)
 template <typename T, int D, int GQ>
 __global__ void __launch_bounds__(PD_WARPS * 32)
-plain_attention_decode_kernel(const T* __restrict__ q, long long q_row_stride, T* __restrict__ out,
-                              const T* __restrict__ k_cache, const T* __restrict__ v_cache,
-                              const int* __restrict__ block_table, int max_pages, const int* __restrict__ req_slots,
-                              const int* __restrict__ cu_q, const int* __restrict__ kv_len, const int* __restrict__ token_req,
+plain_attention_decode_kernel(const T* q, long long q_row_stride, T* __restrict__ out,
+                              const T* k_cache, const T* v_cache,
+                              const int* block_table, int max_pages, const int* req_slots,
+                              const int* cu_q, const int* kv_len, const int* token_req,
                               int tokens, int requests, int num_q, int num_kv, int page_size, int window, float scale,
                               long long num_pages, int* status) {
   constexpr int P = D / 32;           // pieces of four channels a lane holds: 4 (lane % 8) + 32 i

@@ -83,10 +83,10 @@ __device__ __forceinline__ float pre_tanh(float x) {
 // [token][head][value head][D] (what mixing the weights across heads needs); `out` is not written.
 template <int D, bool CAP, bool PARTS>
 __global__ void __launch_bounds__(PRE_WARPS * 32, 2)
-prefill_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_row_stride, __nv_bfloat16* __restrict__ out,
-                         const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
-                         const int* __restrict__ block_table, int max_pages, const int* __restrict__ req_slots,
-                         const int* __restrict__ cu_q, const int* __restrict__ kv_len, int num_requests, int num_q,
+prefill_attention_kernel(const __nv_bfloat16* q, long long q_row_stride, __nv_bfloat16* __restrict__ out,
+                         const __nv_bfloat16* k_cache, const __nv_bfloat16* v_cache,
+                         const int* block_table, int max_pages, const int* req_slots,
+                         const int* cu_q, const int* kv_len, int num_requests, int num_q,
                          int num_kv, int page_size, int window, float scale_log2, long long num_pages, int* status,
                          int keep_first, float cap_pre, float* __restrict__ parts) {
   extern __shared__ __align__(128) unsigned char smem[];

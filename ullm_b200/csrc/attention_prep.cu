@@ -26,16 +26,16 @@
 #define PREP_MAX_TAPS 32
 
 template <typename T>
-__global__ void qkv_prepare_kernel(const T* __restrict__ qkv, long long row_stride, int tokens, int num_q, int num_kv,
+__global__ void qkv_prepare_kernel(const T* qkv, long long row_stride, int tokens, int num_q, int num_kv,
                                    int head_dim, int v_dim, const T* __restrict__ conv_w, int taps,
-                                   const float* __restrict__ conv_state, long long state_stride,
-                                   const int* __restrict__ cu_q, const int* __restrict__ token_req,
-                                   const int* __restrict__ req_slots, int num_state_slots,
-                                   const int* __restrict__ positions, const float* __restrict__ inv_freq,
+                                   const float* conv_state, long long state_stride,
+                                   const int* cu_q, const int* token_req,
+                                   const int* req_slots, int num_state_slots,
+                                   const int* positions, const float* __restrict__ inv_freq,
                                    int rotary_dim, const float* __restrict__ q_w, const float* __restrict__ k_w,
                                    int norm_first, int norm_last, float eps, int vmix_mode,
-                                   const float* __restrict__ vmix_lambda, T* __restrict__ v_first,
-                                   const int* __restrict__ slot_mapping, T* __restrict__ k_cache,
+                                   const float* __restrict__ vmix_lambda, T* v_first,
+                                   const int* slot_mapping, T* __restrict__ k_cache,
                                    T* __restrict__ v_cache, long long num_slots, T* __restrict__ q_out, int* status,
                                    float temp_coef, int temp_every) {
   __shared__ float buf[PREP_WARPS][PREP_MAX_DIM];
@@ -153,10 +153,10 @@ __global__ void qkv_prepare_kernel(const T* __restrict__ qkv, long long row_stri
 // and cosines are formed once, in shared memory, for all heads; a thread then moves 8 + 8 elements of a head's rotated part
 // (dimensions i .. i + 7 and their partners) or 8 elements that only pass, in 16-byte pieces (`VEC` elements each).
 template <typename T, int VEC>
-__global__ void qkv_rotate_store_kernel(const T* __restrict__ qkv, long long row_stride, int num_q, int num_kv,
-                                        int head_dim, int v_dim, const int* __restrict__ positions,
+__global__ void qkv_rotate_store_kernel(const T* qkv, long long row_stride, int num_q, int num_kv,
+                                        int head_dim, int v_dim, const int* positions,
                                         const float* __restrict__ inv_freq, int rotary_dim,
-                                        const int* __restrict__ slot_mapping, T* __restrict__ k_cache,
+                                        const int* slot_mapping, T* __restrict__ k_cache,
                                         T* __restrict__ v_cache, long long num_slots, T* __restrict__ q_out, int* status) {
   extern __shared__ __align__(16) float rot_sm[];  // [half] cosines, [half] sines
   pdl_launch_dependents();
@@ -222,11 +222,11 @@ __global__ void qkv_rotate_store_kernel(const T* __restrict__ qkv, long long row
 // channel is then the only reader of its memory and moves it on itself.
 template <typename T, int VEC, int TAPS, int TOK>
 __global__ void __launch_bounds__(128)
-qkv_conv_prepare_kernel(const T* __restrict__ qkv, long long row_stride, int tokens, int num_q, int num_kv, int head_dim,
-                        int v_dim, const T* __restrict__ conv_w, float* __restrict__ conv_state, long long state_stride,
-                        const int* __restrict__ cu_q, const int* __restrict__ token_req, const int* __restrict__ req_slots,
-                        int num_state_slots, const int* __restrict__ positions, const float* __restrict__ q_w,
-                        const float* __restrict__ k_w, float eps, const int* __restrict__ slot_mapping,
+qkv_conv_prepare_kernel(const T* qkv, long long row_stride, int tokens, int num_q, int num_kv, int head_dim,
+                        int v_dim, const T* __restrict__ conv_w, float* conv_state, long long state_stride,
+                        const int* cu_q, const int* token_req, const int* req_slots,
+                        int num_state_slots, const int* positions, const float* __restrict__ q_w,
+                        const float* __restrict__ k_w, float eps, const int* slot_mapping,
                         T* __restrict__ k_cache, T* __restrict__ v_cache, long long num_slots, T* __restrict__ q_out,
                         int* status, float temp_coef, int temp_every, int single) {
   pdl_launch_dependents();
@@ -330,10 +330,10 @@ qkv_conv_prepare_kernel(const T* __restrict__ qkv, long long row_stride, int tok
 // per (request, channel); rows are moved in ascending order, so a request that brought fewer than taps - 1 tokens
 // shifts its old rows down before it appends (row s takes old row s + n: always a row not yet written).
 template <typename T>
-__global__ void conv_state_update_kernel(const T* __restrict__ qkv, long long row_stride, int row_width, int taps,
-                                         float* __restrict__ conv_state, long long state_stride,
-                                         const int* __restrict__ cu_q, const int* __restrict__ token_req,
-                                         const int* __restrict__ req_slots, int num_state_slots, int requests) {
+__global__ void conv_state_update_kernel(const T* qkv, long long row_stride, int row_width, int taps,
+                                         float* conv_state, long long state_stride,
+                                         const int* cu_q, const int* token_req,
+                                         const int* req_slots, int num_state_slots, int requests) {
   pdl_launch_dependents();
   pdl_wait();
   const int r = blockIdx.y;

@@ -25,9 +25,9 @@
 
 // One block per token.  qk: [tokens][stride], q in columns 0 .. q_size-1, k in q_size .. q_size + kv_size - 1.
 template <typename T>
-__global__ void kv_shared_prepare_kernel(T* __restrict__ qk, long long stride, int q_size, int kv_size,
+__global__ void kv_shared_prepare_kernel(T* qk, long long stride, int q_size, int kv_size,
                                          const float* __restrict__ wq, const float* __restrict__ wk, float eps,
-                                         const int* __restrict__ slot_mapping, T* __restrict__ k_pages,
+                                         const int* slot_mapping, T* __restrict__ k_pages,
                                          T* __restrict__ v_pages, long long num_slots, int* status) {
   __shared__ float scratch[33];
   pdl_launch_dependents();
@@ -76,11 +76,11 @@ __global__ void kv_shared_prepare_kernel(T* __restrict__ qk, long long stride, i
 // One block per token; a token whose pooled slot is -1 completes no block.  The block's positions are
 // pos - pool + 1 .. pos of the token's request, found through the request's row of the block table.
 template <typename T>
-__global__ void pool_blocks_kernel(const int* __restrict__ positions, const int* __restrict__ token_req,
-                                   const int* __restrict__ req_slots, const int* __restrict__ block_table,
-                                   int max_pages, int page_size, long long num_pages, const T* __restrict__ k_pages,
-                                   const T* __restrict__ v_pages, int row, int v_row,
-                                   const int* __restrict__ pool_slots, long long num_pool_slots,
+__global__ void pool_blocks_kernel(const int* positions, const int* token_req,
+                                   const int* req_slots, const int* block_table,
+                                   int max_pages, int page_size, long long num_pages, const T* k_pages,
+                                   const T* v_pages, int row, int v_row,
+                                   const int* pool_slots, long long num_pool_slots,
                                    T* __restrict__ pk_pages, T* __restrict__ pv_pages, int pool, int* status) {
   pdl_launch_dependents();
   pdl_wait();
@@ -148,12 +148,12 @@ __global__ void pool_blocks_kernel(const int* __restrict__ positions, const int*
 // [heads][tokens][rank] (q_h W_uk,h; null: already in q_out), dkv [tokens][rank + rot] (rows `dkv_stride` apart);
 // q_out [tokens][heads][rank + rot]; key pages [*][rank + rot].
 template <typename T>
-__global__ void latent_prepare_kernel(const T* __restrict__ q_full, long long q_stride, const T* __restrict__ q_lat,
-                                      const T* __restrict__ dkv, long long dkv_stride, T* __restrict__ q_out,
+__global__ void latent_prepare_kernel(const T* q_full, long long q_stride, const T* q_lat,
+                                      const T* dkv, long long dkv_stride, T* __restrict__ q_out,
                                       int tokens, int heads,
                                       int dim, int rot, int rank, int rot_dims, int interleaved,
                                       const float* __restrict__ w_c, float eps, const float* __restrict__ inv_freq,
-                                      const int* __restrict__ positions, const int* __restrict__ slot_mapping,
+                                      const int* positions, const int* slot_mapping,
                                       T* __restrict__ k_pages, long long num_slots, int* status) {
   __shared__ float scratch[33];
   pdl_launch_dependents();
@@ -220,12 +220,12 @@ __global__ void latent_prepare_kernel(const T* __restrict__ q_full, long long q_
 // One block per token.  qkv [tokens][stride]: q (num_q heads of head_dim) | k (num_kv heads of head_dim) | v (num_kv
 // heads of v_dim) as projected; q_out [tokens][num_q * head_dim].
 template <typename T>
-__global__ void qkv_rows_prepare_kernel(const T* __restrict__ qkv, long long stride, T* __restrict__ q_out, int num_q,
+__global__ void qkv_rows_prepare_kernel(const T* qkv, long long stride, T* __restrict__ q_out, int num_q,
                                         int num_kv, int head_dim, int v_dim, const float* __restrict__ wq,
                                         const float* __restrict__ wk, float eps, const float* __restrict__ inv_freq,
-                                        int rot_dims, int interleaved, const int* __restrict__ positions,
+                                        int rot_dims, int interleaved, const int* positions,
                                         const float* __restrict__ q_head_scale, int v_unit,
-                                        const int* __restrict__ slot_mapping, T* __restrict__ k_pages,
+                                        const int* slot_mapping, T* __restrict__ k_pages,
                                         T* __restrict__ v_pages, long long num_slots, int* status) {
   __shared__ float scratch[33];
   __shared__ float cs_s[ROWS_MAX_ROT / 2], sn_s[ROWS_MAX_ROT / 2];
@@ -320,13 +320,13 @@ __device__ __forceinline__ void store_pair(__half* p, float a, float b) {
 // (a rotation of neighbours then needs no second read; paired stores).  Needs an even head size; `row` holds
 // q | k | v.
 template <typename T>
-__global__ void qkv_rows_prepare_staged_kernel(const T* __restrict__ qkv, long long stride, T* __restrict__ q_out,
+__global__ void qkv_rows_prepare_staged_kernel(const T* qkv, long long stride, T* __restrict__ q_out,
                                                int num_q, int num_kv, int head_dim, int v_dim,
                                                const float* __restrict__ wq, const float* __restrict__ wk, float eps,
                                                const float* __restrict__ inv_freq, int rot_dims, int interleaved,
-                                               const int* __restrict__ positions,
+                                               const int* positions,
                                                const float* __restrict__ q_head_scale, int v_unit,
-                                               const int* __restrict__ slot_mapping, T* __restrict__ k_pages,
+                                               const int* slot_mapping, T* __restrict__ k_pages,
                                                T* __restrict__ v_pages, long long num_slots, int wide, int* status) {
   extern __shared__ __align__(16) float prep_row[];
   __shared__ float scratch2[64];

@@ -189,6 +189,10 @@ __device__ __forceinline__ void store_vec32(float* p, const float (&v)[VEC]) {
 // memory calls the first only when it has it: blocks of several kernels may be resident, and one that waits for its turn must not
 // hold what one in front of it still needs.
 // A kernel may do work that does not depend on its predecessor (reading weights) before pdl_wait().
+// What a kernel of the same step may have written is read through pointers WITHOUT __restrict__, and never by __ldg or ld.global.nc: all of
+// them tell the compiler that the data does not change while this kernel runs, so that it may load before pdl_wait(), memory clobber or
+// not (with the wait under a condition it did, in attention_decode.cu).  Weights and tables, which no step writes, keep __restrict__, and
+// so do results that the kernel writes and does not read: no load of an input then has to wait for a store of a result.
 // Launches carry the attribute only while ullm_set_pdl(1) is in force; without it both calls are no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -23,7 +23,7 @@ __host__ __device__ __forceinline__ long long decb_ranges(long long total_tiles,
 #define DECB_MERGE_LANES 4
 template <int D>
 __global__ void __launch_bounds__(DECB_MERGE_THREADS)
-decode_balanced_merge_kernel(const float* __restrict__ part, const int* __restrict__ prefix, int* __restrict__ flags,
+decode_balanced_merge_kernel(const float* part, const int* prefix, int* flags,
                              __nv_bfloat16* __restrict__ out, int batch, int num_q, int num_kv, long long warps, int min_tiles) {
   constexpr int PER = D / 4;                                             // threads that hold one row of D
   constexpr int HEADS = DECB_MERGE_THREADS / PER / DECB_MERGE_LANES;     // heads at a time

@@ -13,10 +13,10 @@ extern "C" void ullm_set_pdl(int on) { g_ullm_pdl = on ? 1 : 0; }
 // row copies: out[r, :] = src[index[r], :]
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void gather_rows_kernel(const int* __restrict__ index, const T* __restrict__ src, T* __restrict__ out,
+__global__ void gather_rows_kernel(const int* index, const T* src, T* __restrict__ out,
                                    int rows, int cols, long long src_stride, long long out_stride, int src_rows,
-                                   int status_code, int* status, const int* __restrict__ last_tokens,
-                                   const int* __restrict__ token_req, const int* __restrict__ req_slots) {
+                                   int status_code, int* status, const int* last_tokens,
+                                   const int* token_req, const int* req_slots) {
   pdl_launch_dependents();
   pdl_wait();
   const int r = blockIdx.x;
@@ -282,7 +282,7 @@ extern "C" int ullm_add_rmsnorm(int dtype, const void* x, void* residual, const 
 // ---------------------------------------------------------------------------
 
 template <typename T, int ACT>
-__global__ void act_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, long long rows, int inter) {
+__global__ void act_mul_kernel(const T* gu, T* __restrict__ out, long long rows, int inter) {
   pdl_launch_dependents();
   pdl_wait();
   const long long n = rows * inter;
@@ -300,7 +300,7 @@ __global__ void act_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, lo
 // up of both before anything else (no division per element, four loads in flight per thread).
 template <int ACT>
 __global__ void __launch_bounds__(256)
-act_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long rows,
+act_mul_bf16x8_kernel(const __nv_bfloat16* gu, __nv_bfloat16* __restrict__ out, long long rows,
                       int inter) {
   pdl_launch_dependents();
   pdl_wait();
@@ -375,7 +375,7 @@ extern "C" int ullm_act_mul(int dtype, int act, const void* gate_up, void* out, 
 // ---------------------------------------------------------------------------
 // bf16 -> f32 cast of a contiguous array (logits for the sampler and the host)
 // ---------------------------------------------------------------------------
-__global__ void cast_bf16_f32_kernel(const __nv_bfloat16* __restrict__ in, float* __restrict__ out, long long n) {
+__global__ void cast_bf16_f32_kernel(const __nv_bfloat16* in, float* __restrict__ out, long long n) {
   pdl_launch_dependents();
   pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -398,7 +398,7 @@ extern "C" int ullm_cast_bf16_f32(const void* in, float* out, long long n, void*
 // a time, 31 us in 16-byte pieces; 101 MB are 15 us at the copy rate)
 // ---------------------------------------------------------------------------
 template <typename T, int VEC>
-__global__ void act_mul_clamped_kernel(const T* __restrict__ gu, T* __restrict__ out, long long pieces, int per_row,
+__global__ void act_mul_clamped_kernel(const T* gu, T* __restrict__ out, long long pieces, int per_row,
                                        float limit, float alpha) {
   pdl_launch_dependents();
   pdl_wait();

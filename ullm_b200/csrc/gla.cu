@@ -29,7 +29,7 @@ __device__ __forceinline__ float gla_log_sigmoid(float x) { return fminf(x, 0.f)
 
 // z (32-bit, rows `stride` apart) <- exp(logsigmoid(z + bias) / tau) in place: the decays, evaluated once per
 // token and channel in front of the recurrence, whose blocks would otherwise each evaluate them again.
-__global__ void gla_decay_kernel(float* __restrict__ z, long long stride, const float* __restrict__ bias, int cols,
+__global__ void gla_decay_kernel(float* z, long long stride, const float* __restrict__ bias, int cols,
                                  long long total, float inv_tau) {
   pdl_launch_dependents();
   pdl_wait();
@@ -48,10 +48,10 @@ __global__ void gla_decay_kernel(float* __restrict__ z, long long stride, const 
 // BONUS: the form with the bonus `u` [heads * dim] for the current token.
 template <typename T, int RPT, int CPT, bool BONUS>
 __global__ void __launch_bounds__(2 * GLA_THREADS)
-gla_recurrence_kernel(const T* __restrict__ qkv, long long row_stride, int q_off, int k_off, int v_off,
-                      const float* __restrict__ decay, long long decay_stride, float q_scale,
-                      float* __restrict__ state, long long state_stride, const int* __restrict__ cu_q,
-                      const int* __restrict__ req_slots, const int* __restrict__ token_req, float* __restrict__ out,
+gla_recurrence_kernel(const T* qkv, long long row_stride, int q_off, int k_off, int v_off,
+                      const float* decay, long long decay_stride, float q_scale,
+                      float* state, long long state_stride, const int* cu_q,
+                      const int* req_slots, const int* token_req, float* __restrict__ out,
                       int heads, int dim, int vdim, int rs, int chunk, int num_slots, int* status,
                       const float* __restrict__ bonus, int most_tokens) {
   extern __shared__ __align__(16) float sm[];

@@ -103,9 +103,9 @@ __device__ __forceinline__ void gch_load_v(__nv_bfloat16* v_s, const __nv_bfloat
 // fold[(tile * heads + head)][vdim][dim] = sum_s v_s (W(s, Q) k_s)^T;  total[(tile * heads + head)][dim] = W(0, Q)
 template <int NT>
 __global__ void __launch_bounds__(GCH_THREADS)
-gla_fold_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int k_off, int v_off,
-                const float* __restrict__ decay, long long decay_stride, const int* __restrict__ cu_q,
-                const int* __restrict__ token_req, int requests, int least, int heads, int dim, int vdim,
+gla_fold_kernel(const __nv_bfloat16* qkv, long long row_stride, int k_off, int v_off,
+                const float* decay, long long decay_stride, const int* cu_q,
+                const int* token_req, int requests, int least, int heads, int dim, int vdim,
                 float* __restrict__ fold, float* __restrict__ total) {
   extern __shared__ __align__(16) unsigned char gch_smem[];
   pdl_launch_dependents();
@@ -192,9 +192,9 @@ gla_fold_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int
 // fold <- the state in front of every chunk, as pairs of key channels: with PAIRS (two rounded values, two rounded rests), the
 // operands that `gla_out` needs in two terms, else as it is; state <- the state behind the last.  Two neighbouring key channels per thread.
 template <bool PAIRS>
-__global__ void gla_scan_kernel(float* __restrict__ fold, const float* __restrict__ total, float* __restrict__ state,
-                                long long state_stride, const int* __restrict__ cu_q, const int* __restrict__ req_slots,
-                                const int* __restrict__ token_req, int least, int heads, int dim, int vdim,
+__global__ void gla_scan_kernel(float* fold, const float* total, float* state,
+                                long long state_stride, const int* cu_q, const int* req_slots,
+                                const int* token_req, int least, int heads, int dim, int vdim,
                                 int num_slots, int* status) {
   pdl_launch_dependents();
   pdl_wait();
@@ -249,10 +249,10 @@ __global__ void gla_scan_kernel(float* __restrict__ fold, const float* __restric
 // (chunk, head, v_tile value columns): see `gch_v_tile`.
 template <bool BONUS>
 __global__ void __launch_bounds__(GCH_THREADS, 3)
-gla_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int q_off, int k_off, int v_off,
-               const float* __restrict__ decay, long long decay_stride, const float* __restrict__ bonus, float q_scale,
-               const int* __restrict__ cu_q, const int* __restrict__ token_req, int requests, int least, int heads, int dim,
-               int vdim, int v_tile, const float* __restrict__ fold, float* __restrict__ out) {
+gla_out_kernel(const __nv_bfloat16* qkv, long long row_stride, int q_off, int k_off, int v_off,
+               const float* decay, long long decay_stride, const float* __restrict__ bonus, float q_scale,
+               const int* cu_q, const int* token_req, int requests, int least, int heads, int dim,
+               int vdim, int v_tile, const float* fold, float* __restrict__ out) {
   constexpr int NT = BONUS ? 2 : 3;  // terms of a 32-bit operand
   extern __shared__ __align__(16) unsigned char gch_smem[];
   pdl_launch_dependents();

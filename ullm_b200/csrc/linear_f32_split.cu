@@ -64,7 +64,7 @@ __device__ __forceinline__ void fs_split(const float4& v, uint2& h, uint2& m, ui
 }
 
 // x [M][K] as three planes of bfloat16 terms [3][M][stride]; four values per thread
-__global__ void f32_terms_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ terms, int M, int K, int stride) {
+__global__ void f32_terms_kernel(const float* x, __nv_bfloat16* __restrict__ terms, int M, int K, int stride) {
   pdl_launch_dependents();
   pdl_wait();
   const int per_row = K / 4;
@@ -73,7 +73,7 @@ __global__ void f32_terms_kernel(const float* __restrict__ x, __nv_bfloat16* __r
     const long long row = i / per_row;
     const int c = (int)(i - row * per_row) * 4;
     uint2 h, m, l;
-    fs_split(__ldg(reinterpret_cast<const float4*>(x + row * K + c)), h, m, l);
+    fs_split(*reinterpret_cast<const float4*>(x + row * K + c), h, m, l);
     __nv_bfloat16* d = terms + row * stride + c;
     *reinterpret_cast<uint2*>(d) = h;
     *reinterpret_cast<uint2*>(d + plane) = m;

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(SK_THREADS) linear_skinny_kernel(const SkParam
       const bool in = c + u < c_end && k < p.K;
 #pragma unroll
       for (int n = 0; n < NT; ++n)
-        b[u][n] = in && xok[n] ? __ldg(reinterpret_cast<const uint4*>(xrow[n] + (long long)(c + u) * 32))
+        b[u][n] = in && xok[n] ? *reinterpret_cast<const uint4*>(xrow[n] + (long long)(c + u) * 32)
                                : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll

@@ -26,10 +26,10 @@ __device__ __forceinline__ void mg_gates(float a, float x, float bz, float bx, f
 }
 
 template <typename T>
-__global__ void mingru_walk_kernel(const float* __restrict__ azg, long long stride, int a_off, int x_off, int g_off,
+__global__ void mingru_walk_kernel(const float* azg, long long stride, int a_off, int x_off, int g_off,
                                    const float* __restrict__ bz, const float* __restrict__ bx,
-                                   float* __restrict__ state, long long state_stride, const int* __restrict__ cu_q,
-                                   const int* __restrict__ req_slots, const int* __restrict__ token_req,
+                                   float* state, long long state_stride, const int* cu_q,
+                                   const int* req_slots, const int* token_req,
                                    T* __restrict__ out, long long out_stride, float out_scale, int width) {
   pdl_launch_dependents();
   pdl_wait();
@@ -59,9 +59,9 @@ __global__ void mingru_walk_kernel(const float* __restrict__ azg, long long stri
 // chunk k of the step covers rows k * MG_CHUNK .. of the flat batch, cut at request borders by `chunk_req` /
 // `chunk_first` / `chunk_last` computed here from cu_q: a chunk never spans two requests because the grid is
 // (channels, chunks per request, requests) and a chunk beyond the request's length does nothing.
-__global__ void mingru_fold_kernel(const float* __restrict__ azg, long long stride, int a_off, int x_off,
+__global__ void mingru_fold_kernel(const float* azg, long long stride, int a_off, int x_off,
                                    const float* __restrict__ bz, const float* __restrict__ bx,
-                                   const int* __restrict__ cu_q, const int* __restrict__ token_req,
+                                   const int* cu_q, const int* token_req,
                                    float* __restrict__ fold_a, float* __restrict__ fold_b, int max_chunks, int width) {
   pdl_launch_dependents();
   pdl_wait();
@@ -85,9 +85,9 @@ __global__ void mingru_fold_kernel(const float* __restrict__ azg, long long stri
 }
 
 // the state at the start of every chunk (left in fold_b's place), and the request's state behind the step
-__global__ void mingru_carry_kernel(float* __restrict__ fold_a, float* __restrict__ fold_b,
-                                    float* __restrict__ state, long long state_stride, const int* __restrict__ cu_q,
-                                    const int* __restrict__ req_slots, const int* __restrict__ token_req,
+__global__ void mingru_carry_kernel(float* fold_a, float* fold_b,
+                                    float* state, long long state_stride, const int* cu_q,
+                                    const int* req_slots, const int* token_req,
                                     int max_chunks, int width) {
   pdl_launch_dependents();
   pdl_wait();
@@ -109,10 +109,10 @@ __global__ void mingru_carry_kernel(float* __restrict__ fold_a, float* __restric
 }
 
 template <typename T>
-__global__ void mingru_replay_kernel(const float* __restrict__ azg, long long stride, int a_off, int x_off, int g_off,
+__global__ void mingru_replay_kernel(const float* azg, long long stride, int a_off, int x_off, int g_off,
                                      const float* __restrict__ bz, const float* __restrict__ bx,
-                                     const float* __restrict__ start, const int* __restrict__ cu_q,
-                                     const int* __restrict__ token_req, T* __restrict__ out, long long out_stride,
+                                     const float* start, const int* cu_q,
+                                     const int* token_req, T* __restrict__ out, long long out_stride,
                                      float out_scale, int max_chunks, int width) {
   pdl_launch_dependents();
   pdl_wait();

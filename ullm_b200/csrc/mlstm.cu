@@ -46,13 +46,13 @@ constexpr int mlstm_blocks() {
 }
 template <typename T, int RPT, int RS, int CPT>
 __global__ void __launch_bounds__(2 * MLSTM_THREADS, mlstm_blocks<T, RPT, RS, CPT>())
-mlstm_recurrence_kernel(const T* __restrict__ qkv, long long row_stride, int q_off, int k_off, int v_off,
-                        const float* __restrict__ gates, const float* __restrict__ bias_i,
-                        const float* __restrict__ bias_f, float* __restrict__ state, long long state_stride,
-                        const int* __restrict__ cu_q, const int* __restrict__ req_slots,
-                        const int* __restrict__ token_req, float* __restrict__ out, int heads, int dim, int vdim,
+mlstm_recurrence_kernel(const T* qkv, long long row_stride, int q_off, int k_off, int v_off,
+                        const float* gates, const float* __restrict__ bias_i,
+                        const float* __restrict__ bias_f, float* state, long long state_stride,
+                        const int* cu_q, const int* req_slots,
+                        const int* token_req, float* __restrict__ out, int heads, int dim, int vdim,
                         int rs_arg, int chunk, float q_scale, float cap, int num_slots, int* status, int most_tokens,
-                        int* __restrict__ arrived) {
+                        int* arrived) {
   constexpr bool FULL = RS != 0;
   const int rs = FULL ? RS : rs_arg;
   // Threads 0 .. 127 run the recurrence; threads 128 .. 255 stage the next chunk of tokens (q, k, the tile's v,
@@ -329,7 +329,7 @@ mlstm_recurrence_kernel(const T* __restrict__ qkv, long long row_stride, int q_o
 
 // out[t, h, :] = o[t, h, :] / sqrt(mean(o[t, h, :]^2) + eps) * w[h, :] * sigmoid(g[t, h, :]); one warp per (token, head).
 template <typename T>
-__global__ void mlstm_out_gate_kernel(const float* __restrict__ o, const T* __restrict__ g, long long g_stride,
+__global__ void mlstm_out_gate_kernel(const float* o, const T* g, long long g_stride,
                                       const float* __restrict__ w, T* __restrict__ out, long long units, int heads,
                                       int vdim, float eps, int w_per_head, int silu) {
   pdl_launch_dependents();
@@ -354,7 +354,7 @@ __global__ void mlstm_out_gate_kernel(const float* __restrict__ o, const T* __re
 
 // The same in 16-byte pieces: LPH lanes (a power of two) share a head of VEC * LPH columns.
 template <typename T, int VEC>
-__global__ void head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ g, long long g_stride,
+__global__ void head_norm_gate_vec_kernel(const float* o, const T* g, long long g_stride,
                                           const float* __restrict__ w, T* __restrict__ out, long long pieces, int heads,
                                           int lph, float eps, int w_per_head, int silu) {
   pdl_launch_dependents();

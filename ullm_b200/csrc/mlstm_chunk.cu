@@ -125,9 +125,9 @@ __device__ __forceinline__ float mch_log_sigmoid(float x) { return fminf(x, 0.f)
 
 // One block per (head, request); a warp takes a chunk at a time, a lane two neighbouring tokens.
 __global__ void __launch_bounds__(MCH_THREADS)
-mlstm_chunk_gates_kernel(const float* __restrict__ gates, const float* __restrict__ bias_i, const float* __restrict__ bias_f,
-                         float cap, float* __restrict__ state, long long state_stride, long long m_off,
-                         const int* __restrict__ cu_q, const int* __restrict__ req_slots, const int* __restrict__ token_req,
+mlstm_chunk_gates_kernel(const float* gates, const float* __restrict__ bias_i, const float* __restrict__ bias_f,
+                         float cap, float* state, long long state_stride, long long m_off,
+                         const int* cu_q, const int* req_slots, const int* token_req,
                          int tokens, int least, int heads, int num_slots, MchScratch sc, int* status) {
   extern __shared__ __align__(16) unsigned char mch_smem[];
   pdl_launch_dependents();
@@ -235,8 +235,8 @@ __device__ __forceinline__ void mch_load(__nv_bfloat16* dst, const __nv_bfloat16
 
 // fold[tile, head] = sum_s v_s (to_state_s k_s)^T, and behind it sum_s to_state_s k_s
 __global__ void __launch_bounds__(MCH_THREADS)
-mlstm_chunk_fold_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int k_off, int v_off,
-                        const int* __restrict__ cu_q, const int* __restrict__ token_req, int requests, int tokens, int least,
+mlstm_chunk_fold_kernel(const __nv_bfloat16* qkv, long long row_stride, int k_off, int v_off,
+                        const int* cu_q, const int* token_req, int requests, int tokens, int least,
                         int heads, int dim, int vdim, MchScratch sc) {
   extern __shared__ __align__(16) unsigned char mch_smem[];
   __shared__ float to_s[MCH_Q];
@@ -289,8 +289,8 @@ mlstm_chunk_fold_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_str
 }
 
 // fold <- the state in front of every chunk; state <- the state behind the last.  Two neighbouring key channels per thread.
-__global__ void mlstm_chunk_scan_kernel(float* __restrict__ state, long long state_stride, const int* __restrict__ cu_q,
-                                        const int* __restrict__ req_slots, const int* __restrict__ token_req, int least,
+__global__ void mlstm_chunk_scan_kernel(float* state, long long state_stride, const int* cu_q,
+                                        const int* req_slots, const int* token_req, int least,
                                         int heads, int dim, int vdim, int num_slots, MchScratch sc) {
   pdl_launch_dependents();
   pdl_wait();
@@ -334,8 +334,8 @@ __global__ void mlstm_chunk_scan_kernel(float* __restrict__ state, long long sta
 // 16 value columns at a time, transposed (rows value columns, columns tokens), so that each part of the state is split into its
 // terms by one warp only.
 __global__ void __launch_bounds__(MCH_THREADS, 2)
-mlstm_chunk_out_kernel(const __nv_bfloat16* __restrict__ qkv, long long row_stride, int q_off, int k_off, int v_off,
-                       float q_scale, const int* __restrict__ cu_q, const int* __restrict__ token_req, int requests, int tokens,
+mlstm_chunk_out_kernel(const __nv_bfloat16* qkv, long long row_stride, int q_off, int k_off, int v_off,
+                       float q_scale, const int* cu_q, const int* token_req, int requests, int tokens,
                        int least, int heads, int dim, int vdim, MchScratch sc, float* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char mch_smem[];
   __shared__ double row_s[MCH_Q], col_s[MCH_Q];

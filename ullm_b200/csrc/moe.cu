@@ -29,7 +29,7 @@
 
 #define MOE_MAX_TOP 32
 
-__global__ void moe_route_kernel(const float* __restrict__ logits, long long logits_stride,
+__global__ void moe_route_kernel(const float* logits, long long logits_stride,
                                  const float* __restrict__ correction, int* __restrict__ choice,
                                  float* __restrict__ weight, int tokens, int experts, int top, int softmax_scores,
                                  int renormalize, int groups, int keep, float scale, int always) {
@@ -140,8 +140,8 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long log
 }
 
 // One block.  counts in shared memory (experts <= 1024).
-__global__ void moe_arrange_kernel(const int* __restrict__ choice, int pairs, int experts, int* __restrict__ offsets,
-                                   int* __restrict__ sorted, int* __restrict__ place) {
+__global__ void moe_arrange_kernel(const int* choice, int pairs, int experts, int* offsets,
+                                   int* sorted, int* place) {
   __shared__ int count[1024];
   __shared__ int cursor[1024];
   pdl_launch_dependents();
@@ -183,9 +183,9 @@ __global__ void moe_arrange_kernel(const int* __restrict__ choice, int pairs, in
 
 template <typename T, bool GATED>
 __global__ void __launch_bounds__(MOE_THREADS)
-moe_grouped_linear_kernel(const T* __restrict__ x, long long x_stride, const T* __restrict__ weights,
-                          long long expert_stride, const int* __restrict__ offsets, const int* __restrict__ sorted,
-                          const float* __restrict__ pair_weight, T* __restrict__ out, int experts, int top,
+moe_grouped_linear_kernel(const T* x, long long x_stride, const T* __restrict__ weights,
+                          long long expert_stride, const int* offsets, const int* sorted,
+                          const float* pair_weight, T* __restrict__ out, int experts, int top,
                           int rows_from_pairs, int n_out, int k_dim, int act, float limit, float alpha) {
   __shared__ float As[MOE_BK][MOE_BM + 1];
   __shared__ float Bs[GATED ? 2 : 1][MOE_BK][MOE_BN + 1];
@@ -315,10 +315,10 @@ __device__ __forceinline__ void moe_mma(float (&c)[4], const unsigned (&a)[4], u
 
 template <bool GATED, int STAGES>
 __global__ void __launch_bounds__(MMA_THREADS)
-moe_grouped_mma_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride,
+moe_grouped_mma_kernel(const __nv_bfloat16* x, long long x_stride,
                        const __nv_bfloat16* __restrict__ weights, long long expert_stride,
-                       const int* __restrict__ offsets, const int* __restrict__ sorted,
-                       const float* __restrict__ pair_weight, __nv_bfloat16* __restrict__ out, int experts, int top,
+                       const int* offsets, const int* sorted,
+                       const float* pair_weight, __nv_bfloat16* __restrict__ out, int experts, int top,
                        int rows_from_pairs, int n_out, int k_dim, int act, float limit, float alpha) {
   constexpr int NB = GATED ? 2 : 1;
   constexpr int TILE = MMA_BM * MMA_BK * 2;  // bytes of one 64 x 64 tile
@@ -443,11 +443,11 @@ moe_grouped_mma_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride,
 
 // A block: one token x (blockDim.x * VEC) columns (blockIdx.y counts the column ranges); a thread: VEC columns.
 template <typename T, int VEC>
-__global__ void moe_combine_kernel(const T* __restrict__ rows, const int* __restrict__ place,
-                                   const float* __restrict__ pair_weight, T* __restrict__ y, int top, int cols,
-                                   const int* __restrict__ choice, int experts, const T* __restrict__ x,
-                                   long long x_stride, const T* __restrict__ shared_rows,
-                                   const float* __restrict__ shared_gate, long long gate_stride) {
+__global__ void moe_combine_kernel(const T* rows, const int* place,
+                                   const float* pair_weight, T* __restrict__ y, int top, int cols,
+                                   const int* choice, int experts, const T* x,
+                                   long long x_stride, const T* shared_rows,
+                                   const float* shared_gate, long long gate_stride) {
   pdl_launch_dependents();
   pdl_wait();
   const long long t = blockIdx.x;
@@ -489,12 +489,12 @@ __global__ void moe_combine_kernel(const T* __restrict__ rows, const int* __rest
 // row as it is, rounded.  With an outer norm `wo`: stream[t] += scale * wo * y[t] / sqrt(mean(y[t]^2) + eps_o).  One block per token; the sum never leaves 32-bit.  `x` (the passing experts' input) and `out` may be the
 // same rows: a block reads its token's row of x before the barrier and writes its row of out behind it.
 template <typename T, int VEC>
-__global__ void moe_combine_add_norm_kernel(const T* __restrict__ rows, const int* __restrict__ place,
-                                            const float* __restrict__ pair_weight, int top, int cols,
-                                            const int* __restrict__ choice, int experts, const T* x,
-                                            long long x_stride, const T* __restrict__ shared_rows,
-                                            const float* __restrict__ shared_gate, long long gate_stride,
-                                            float* __restrict__ stream, const float* __restrict__ scale,
+__global__ void moe_combine_add_norm_kernel(const T* rows, const int* place,
+                                            const float* pair_weight, int top, int cols,
+                                            const int* choice, int experts, const T* x,
+                                            long long x_stride, const T* shared_rows,
+                                            const float* shared_gate, long long gate_stride,
+                                            float* stream, const float* __restrict__ scale,
                                             const float* __restrict__ w2, float eps2, T* out,
                                             const float* __restrict__ alpha2, const float* __restrict__ b2,
                                             const float* __restrict__ wo, float eps_o) {

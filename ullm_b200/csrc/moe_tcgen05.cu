@@ -270,8 +270,8 @@ static bool mt_map(CUtensorMap* m, const void* ptr, long long cols, long long ro
 }
 
 // out[p] = x[sorted[p] / top] for every place p that belongs to an expert, 16 bytes at a time
-__global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, long long x_stride, const int* __restrict__ sorted,
-                                       const int* __restrict__ offsets, int experts, int top, uint4* __restrict__ out,
+__global__ void moe_gather_rows_kernel(const uint4* x, long long x_stride, const int* sorted,
+                                       const int* offsets, int experts, int top, uint4* __restrict__ out,
                                        int pieces) {
   pdl_launch_dependents();
   pdl_wait();

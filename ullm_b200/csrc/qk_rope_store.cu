@@ -19,8 +19,8 @@ template <typename T>
 __global__ void qk_norm_rope_store_kernel(T* qkv, int tokens, int num_q, int num_kv, int head_dim,
                                           const float* __restrict__ q_w, const float* __restrict__ k_w, float eps,
                                           const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                          int rotary_dim, int max_positions, const int* __restrict__ positions,
-                                          const int* __restrict__ slot_mapping, T* k_cache, T* v_cache,
+                                          int rotary_dim, int max_positions, const int* positions,
+                                          const int* slot_mapping, T* k_cache, T* v_cache,
                                           long long num_slots, int* status, int k_in_place, int v_dim,
                                           int kv_in_row) {
   // v_dim: head size of the values; kv_in_row 0: a row holds the query heads only (the keys and values are
@@ -110,8 +110,8 @@ template <int D, int QKV_STEPS>
 __global__ void __launch_bounds__(256)
 qk_norm_rope_store_bf16_kernel(__nv_bfloat16* qkv, int tokens, int num_q, int num_kv, const float* __restrict__ q_w,
                                const float* __restrict__ k_w, float eps, const float* __restrict__ cos_t,
-                               const float* __restrict__ sin_t, int max_positions, const int* __restrict__ positions,
-                               const int* __restrict__ slot_mapping, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache,
+                               const float* __restrict__ sin_t, int max_positions, const int* positions,
+                               const int* slot_mapping, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache,
                                long long num_slots, int* status) {
   constexpr int LW = D / 8;                  // lanes of a row
   constexpr int ROWS = 32 / LW;              // rows of a warp, side by side

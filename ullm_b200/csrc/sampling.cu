@@ -44,7 +44,7 @@ __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
   return a;
 }
 
-__device__ ArgMax block_argmax(const float* __restrict__ row, int n, float inv_t, ArgMax* sh) {
+__device__ ArgMax block_argmax(const float* row, int n, float inv_t, ArgMax* sh) {
   ArgMax best = {-INFINITY, 0x7fffffff};
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     ArgMax c = {row[i] * inv_t, i};
@@ -90,10 +90,10 @@ __device__ unsigned long long block_sum_u64(unsigned long long v, unsigned long 
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_kernel(const float* __restrict__ logits, long long row_stride, int vocab, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
-              const float* __restrict__ uniform, int* __restrict__ out, float* __restrict__ probs_out,
-              const int* __restrict__ row_slots, int* __restrict__ last_tokens) {
+sample_kernel(const float* logits, long long row_stride, int vocab, const float* temperature,
+              const int* top_k, const float* top_p, const float* min_p,
+              const float* uniform, int* __restrict__ out, float* probs_out,
+              const int* row_slots, int* last_tokens) {
   __shared__ ArgMax sh_arg[33];
   __shared__ unsigned long long sh_u64[33];
   __shared__ unsigned long long hist_mass[256];
@@ -272,7 +272,7 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int vocab,
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-argmax_kernel(const float* __restrict__ logits, long long row_stride, int vocab, int* __restrict__ out) {
+argmax_kernel(const float* logits, long long row_stride, int vocab, int* __restrict__ out) {
   __shared__ ArgMax sh_arg[33];
   pdl_launch_dependents();
   pdl_wait();
@@ -403,11 +403,11 @@ __device__ __forceinline__ int sc_find_digit(const T* tot, T bound, T start, T* 
 }
 
 __global__ void __launch_bounds__(SC_THREADS)
-sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, int vocab, int slice,
-                      const float* __restrict__ temperature, const int* __restrict__ top_k,
-                      const float* __restrict__ top_p, const float* __restrict__ min_p,
-                      const float* __restrict__ uniform, int* __restrict__ out, float* __restrict__ probs_out,
-                      const int* __restrict__ row_slots, int* __restrict__ last_tokens) {
+sample_cluster_kernel(const float* logits, long long row_stride, int vocab, int slice,
+                      const float* temperature, const int* top_k,
+                      const float* top_p, const float* min_p,
+                      const float* uniform, int* __restrict__ out, float* probs_out,
+                      const int* row_slots, int* last_tokens) {
   extern __shared__ __align__(16) unsigned char sc_raw[];
   __shared__ ScShared sh;
   pdl_launch_dependents();
@@ -439,7 +439,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
 #pragma unroll
       for (int u = 0; u < SC_UNROLL; ++u) {
         const int i = i0 + u * SC_THREADS;
-        v[u] = i < n4 ? __ldg(src + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        v[u] = i < n4 ? src[i] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
       }
 #pragma unroll
       for (int u = 0; u < SC_UNROLL; ++u) {
@@ -464,7 +464,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
 #pragma unroll
       for (int u = 0; u < SC_UNROLL; ++u) {
         const int i = i0 + u * SC_THREADS;
-        v[u] = i < n ? __ldg(row + begin + i) : -INFINITY;
+        v[u] = i < n ? row[begin + i] : -INFINITY;
       }
 #pragma unroll
       for (int u = 0; u < SC_UNROLL; ++u) {

@@ -43,9 +43,9 @@ __device__ __forceinline__ float row_rstd(const float* row, int cols, bool cente
 }
 
 template <typename TA, typename TO>
-__global__ void norm_add_norm_kernel(const TA* __restrict__ a, float* __restrict__ stream,
+__global__ void norm_add_norm_kernel(const TA* a, float* stream,
                                      const float* __restrict__ w, int cols, float eps, float mult, int center,
-                                     const float* __restrict__ extra_rows, const float* __restrict__ extra_vec,
+                                     const float* extra_rows, const float* __restrict__ extra_vec,
                                      const float* __restrict__ w2, float eps2, int center2, TO* __restrict__ out,
                                      const float* __restrict__ alpha2, const float* __restrict__ b2) {
   extern __shared__ float sn_smem[];  // [cols] the operand's row, then [cols] the stream's row
@@ -122,8 +122,8 @@ __device__ __forceinline__ float piece_rstd(const float (&v)[8], bool on, int co
 }
 
 template <typename TA, typename TO>
-__global__ void norm_add_norm_piece_kernel(const TA* __restrict__ a, float* __restrict__ stream, const float* __restrict__ w, int cols,
-                                           float eps, float mult, int center, const float* __restrict__ extra_rows,
+__global__ void norm_add_norm_piece_kernel(const TA* a, float* stream, const float* __restrict__ w, int cols,
+                                           float eps, float mult, int center, const float* extra_rows,
                                            const float* __restrict__ extra_vec, const float* __restrict__ w2, float eps2, int center2,
                                            TO* __restrict__ out, const float* __restrict__ alpha2, const float* __restrict__ b2) {
   __shared__ float scratch[33];
@@ -175,9 +175,9 @@ __global__ void norm_add_norm_piece_kernel(const TA* __restrict__ a, float* __re
 // to the stream; then the norm that reads the stream next.  One block per row; VEC neighbouring columns per thread and
 // turn (16-byte pieces where the rows allow), both sums of squares in one set of barriers.
 template <typename T, int VEC>
-__global__ void pair_norm_add_norm_kernel(const T* __restrict__ a, const T* __restrict__ b,
+__global__ void pair_norm_add_norm_kernel(const T* a, const T* b,
                                           const float* __restrict__ wa, const float* __restrict__ wb, int cols,
-                                          float eps, float mult, float* __restrict__ stream, T* __restrict__ rows_out,
+                                          float eps, float mult, float* stream, T* __restrict__ rows_out,
                                           const float* __restrict__ w2, float eps2, int kind2,
                                           const float* __restrict__ alpha2, const float* __restrict__ b2,
                                           T* __restrict__ out, const float* __restrict__ wo, float eps_o, float mult_o) {
@@ -284,7 +284,7 @@ __global__ void pair_norm_add_norm_kernel(const T* __restrict__ a, const T* __re
 }
 
 template <typename TO>
-__global__ void norm_rows_kernel(const float* __restrict__ stream, const int* __restrict__ rows,
+__global__ void norm_rows_kernel(const float* stream, const int* rows,
                                  const float* __restrict__ w, TO* __restrict__ out, int cols, int src_rows, float eps,
                                  int center, int* status, const float* __restrict__ alpha,
                                  const float* __restrict__ b) {
@@ -318,7 +318,7 @@ __device__ __forceinline__ float softplus_f32(float v) { return log1pf(expf(-fab
 // VEC neighbouring elements per thread and turn: bound by the bytes moved (67 MB at 2,048 x 8,192: 43 us one element at a time,
 // 33 us in 16-byte pieces, with cold caches)
 template <typename T, int VEC>
-__global__ void xielu_kernel(const T* __restrict__ in, T* __restrict__ out, long long n,
+__global__ void xielu_kernel(const T* in, T* __restrict__ out, long long n,
                              const float* __restrict__ pq) {
   pdl_launch_dependents();
   pdl_wait();

@@ -35,12 +35,12 @@ __device__ __forceinline__ float ssd_softplus(float v) { return fmaxf(v, 0.f) + 
 // channels' (blockIdx.x >= channel_blocks) do the step sizes.  `single`: every request of the step has one token; the
 // thread that convolves a channel is then the only reader of its memory and moves it on itself.
 template <typename T, int VEC, int TAPS, int TOK>
-__global__ void ssd_prepare_kernel(const T* __restrict__ u, long long row_stride, int xbc_off, int dt_off, int channels,
+__global__ void ssd_prepare_kernel(const T* u, long long row_stride, int xbc_off, int dt_off, int channels,
                                    int heads, const T* __restrict__ conv_w, int taps_rt,
                                    const float* __restrict__ conv_b, const float* __restrict__ dt_bias,
-                                   const float* __restrict__ a_log, float* __restrict__ conv_state,
-                                   long long state_stride, int num_slots, const int* __restrict__ cu_q,
-                                   const int* __restrict__ token_req, const int* __restrict__ req_slots, int tokens,
+                                   const float* __restrict__ a_log, float* conv_state,
+                                   long long state_stride, int num_slots, const int* cu_q,
+                                   const int* token_req, const int* req_slots, int tokens,
                                    T* __restrict__ xbc, float* __restrict__ dt, float* __restrict__ log_decay,
                                    int channel_blocks, int single, int* status) {
   pdl_launch_dependents();
@@ -156,10 +156,10 @@ __global__ void ssd_prepare_kernel(const T* __restrict__ u, long long row_stride
 // has no bounds checks: the padded rows of S stay zero.  CPT: neighbouring columns a thread holds.
 template <typename T, int RPT, int CPT>
 __global__ void __launch_bounds__(2 * SSD_THREADS)
-ssd_recurrence_kernel(const T* __restrict__ xbc, long long row_stride, int b_off, int c_off,
-                      const float* __restrict__ dt, const float* __restrict__ log_decay, const float* __restrict__ d_skip,
-                      float* __restrict__ state, long long state_stride, const int* __restrict__ cu_q,
-                      const int* __restrict__ req_slots, const int* __restrict__ token_req, float* __restrict__ out,
+ssd_recurrence_kernel(const T* xbc, long long row_stride, int b_off, int c_off,
+                      const float* dt, const float* log_decay, const float* __restrict__ d_skip,
+                      float* state, long long state_stride, const int* cu_q,
+                      const int* req_slots, const int* token_req, float* __restrict__ out,
                       int heads, int n_state, int pdim, int per_group, int rs, int chunk, int num_slots, int most_tokens,
                       int* status, long long dt_stride, int silu_in) {
   extern __shared__ __align__(16) float sm[];
@@ -354,7 +354,7 @@ ssd_recurrence_kernel(const T* __restrict__ xbc, long long row_stride, int b_off
 
 // One block per (token, part): g = y silu(z) waits in shared memory for the part's sum of squares.
 template <typename T, int VEC>
-__global__ void ssd_gate_norm_kernel(const float* __restrict__ y, const T* __restrict__ z, long long z_stride,
+__global__ void ssd_gate_norm_kernel(const float* y, const T* z, long long z_stride,
                                      const float* __restrict__ w, T* __restrict__ out, int inner, int part_size,
                                      float eps, int gate_behind) {
   extern __shared__ __align__(16) float sm[];

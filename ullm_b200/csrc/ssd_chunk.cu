@@ -53,9 +53,9 @@ __device__ __forceinline__ int ssc_find(int tile, const int* cu_q, int requests,
 // scores[(group * tokens + t) * SSC_Q + s] = C_t . B_s for the tokens s <= t of t's chunk (others: undefined).  The blocks
 // behind the groups' (blockIdx.y == groups) form the heads' running sums and weights, a warp per head at a time.
 __global__ void __launch_bounds__(SSC_THREADS)
-ssd_scores_kernel(const __nv_bfloat16* __restrict__ xbc, long long row_stride, int b_off, int c_off, int n_state, int groups,
-                  const float* __restrict__ dt, const float* __restrict__ log_decay, long long dt_stride, int heads,
-                  const int* __restrict__ cu_q, const int* __restrict__ token_req, int requests, int tokens, int least,
+ssd_scores_kernel(const __nv_bfloat16* xbc, long long row_stride, int b_off, int c_off, int n_state, int groups,
+                  const float* dt, const float* log_decay, long long dt_stride, int heads,
+                  const int* cu_q, const int* token_req, int requests, int tokens, int least,
                   float* __restrict__ scores, SscScratch sc) {
   extern __shared__ __align__(16) unsigned char sc_smem[];
   pdl_launch_dependents();
@@ -143,9 +143,9 @@ ssd_scores_kernel(const __nv_bfloat16* __restrict__ xbc, long long row_stride, i
 // cp.async.  What a chunk adds is summed apart from S: its tensor instructions do not wait for the chunk before it.
 template <int NT, int DEPTH>
 __global__ void __launch_bounds__(SSC_THREADS)
-ssd_walk_kernel(const __nv_bfloat16* __restrict__ xbc, long long row_stride, int b_off, float* __restrict__ state,
-                long long state_stride, const int* __restrict__ cu_q, const int* __restrict__ req_slots,
-                const int* __restrict__ token_req, int heads, int pdim, int per_group, int tokens, int num_slots, int least,
+ssd_walk_kernel(const __nv_bfloat16* xbc, long long row_stride, int b_off, float* state,
+                long long state_stride, const int* cu_q, const int* req_slots,
+                const int* token_req, int heads, int pdim, int per_group, int tokens, int num_slots, int least,
                 SscScratch sc, int* status) {
   constexpr int N = 32 * NT, NW = N / 4;  // NW: a warp's columns of S^T
   constexpr int RS = N * 2 + 16, XS = SSC_PT * 2 + 16;  // bytes between rows of B and of x
@@ -263,9 +263,9 @@ ssd_walk_kernel(const __nv_bfloat16* __restrict__ xbc, long long row_stride, int
 // transposed (rows columns of S, columns tokens): every part of the state is split into its terms by one warp only, and is
 // used for all the chunk's tokens from registers.
 __global__ void __launch_bounds__(SSC_OUT_WARPS * 32, 2)
-ssd_out_kernel(const __nv_bfloat16* __restrict__ xbc, long long row_stride, int c_off, const float* __restrict__ d_skip,
-               const float* __restrict__ scores, const int* __restrict__ cu_q, const int* __restrict__ req_slots,
-               const int* __restrict__ token_req, float* __restrict__ out, int requests, int heads, int n_state, int pdim,
+ssd_out_kernel(const __nv_bfloat16* xbc, long long row_stride, int c_off, const float* __restrict__ d_skip,
+               const float* scores, const int* cu_q, const int* req_slots,
+               const int* token_req, float* __restrict__ out, int requests, int heads, int n_state, int pdim,
                int per_group, int tokens, int num_slots, int least, SscScratch sc) {
   constexpr int THREADS = SSC_OUT_WARPS * 32, COLS = SSC_OUT_WARPS * SSC_PT;
   constexpr int XS = COLS * 2 + 16;  // bytes between rows of x

@@ -17,8 +17,8 @@ extern "C" int ullm_ssd_chunk_supported(int heads, int n_state, int pdim, int gr
 // scores[(group * tokens + t) * SSC_Q + s] = C_t . B_s for the tokens s <= t of t's chunk (others: undefined).  Chunks
 // are counted from a request's first token of the step; requests of at most `least` tokens are left out.
 __global__ void __launch_bounds__(SSC_THREADS)
-ssd_short_scores_kernel(const __nv_bfloat16* __restrict__ xbc, long long row_stride, int b_off, int c_off, int n_state,
-                  const int* __restrict__ cu_q, const int* __restrict__ token_req, int requests, int tokens, int least,
+ssd_short_scores_kernel(const __nv_bfloat16* xbc, long long row_stride, int b_off, int c_off, int n_state,
+                  const int* cu_q, const int* token_req, int requests, int tokens, int least,
                   float* __restrict__ scores) {
   extern __shared__ __align__(16) unsigned char sc_smem[];
   pdl_launch_dependents();
@@ -88,10 +88,10 @@ ssd_short_scores_kernel(const __nv_bfloat16* __restrict__ xbc, long long row_str
 // one, where two do not fit, a second barrier stands in front of their renewal).
 template <int PT, int NT, int SB>
 __global__ void __launch_bounds__(2 * SSC_THREADS)
-ssd_short_kernel(const __nv_bfloat16* __restrict__ xbc, long long row_stride, int b_off, int c_off,
-                 const float* __restrict__ dt, const float* __restrict__ log_decay, const float* __restrict__ d_skip,
-                 const float* __restrict__ scores, float* __restrict__ state, long long state_stride,
-                 const int* __restrict__ cu_q, const int* __restrict__ req_slots, const int* __restrict__ token_req,
+ssd_short_kernel(const __nv_bfloat16* xbc, long long row_stride, int b_off, int c_off,
+                 const float* dt, const float* log_decay, const float* __restrict__ d_skip,
+                 const float* scores, float* state, long long state_stride,
+                 const int* cu_q, const int* req_slots, const int* token_req,
                  float* __restrict__ out, int heads, int pdim, int per_group, int tokens, int num_slots, int least,
                  int* status, long long dt_stride) {
   constexpr int N = 32 * NT, NW = N / 4;      // a warp's columns of S^T

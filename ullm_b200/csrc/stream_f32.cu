@@ -38,11 +38,11 @@ struct PairEmbedding {
 };
 
 template <typename T, typename TAB, int VEC>
-__global__ void embed_scaled_kernel(const int* __restrict__ ids, const TAB* __restrict__ table,
-                                    float* __restrict__ stream, T* __restrict__ copy, int hidden, int vocab,
+__global__ void embed_scaled_kernel(const int* ids, const TAB* __restrict__ table,
+                                    float* stream, T* __restrict__ copy, int hidden, int vocab,
                                     float scale, const float* __restrict__ inv_freq,
-                                    const int* __restrict__ positions, const int* __restrict__ last_tokens,
-                                    const int* __restrict__ token_req, const int* __restrict__ req_slots,
+                                    const int* positions, const int* last_tokens,
+                                    const int* token_req, const int* req_slots,
                                     int* status, PairEmbedding pe) {
   pdl_launch_dependents();
   pdl_wait();
@@ -104,7 +104,7 @@ __global__ void embed_scaled_kernel(const int* __restrict__ ids, const TAB* __re
 }
 
 template <typename T>
-__global__ void norm_scale_add_kernel(const T* __restrict__ a, float* __restrict__ stream,
+__global__ void norm_scale_add_kernel(const T* a, float* stream,
                                       const float* __restrict__ w, T* __restrict__ copy, int cols, float eps,
                                       float mult) {
   __shared__ float scratch[33];
@@ -127,7 +127,7 @@ __global__ void norm_scale_add_kernel(const T* __restrict__ a, float* __restrict
 
 // The same in 16-byte pieces: ITEMS pieces of VEC columns per thread, which wait in registers between the sum and the update.
 template <typename T, int VEC, int ITEMS>
-__global__ void norm_scale_add_vec_kernel(const T* __restrict__ a, float* __restrict__ stream,
+__global__ void norm_scale_add_vec_kernel(const T* a, float* stream,
                                           const float* __restrict__ w, T* __restrict__ copy, int cols, float eps,
                                           float mult) {
   __shared__ float scratch[33];
@@ -191,7 +191,7 @@ static bool norm_scale_add_vec(const void* a, float* stream, const float* w, voi
 // for s = the stream's new row, which waits in shared memory (`cols` floats) between the two sums: the stream is
 // neither written and read again nor normed by a kernel of its own.
 template <typename T>
-__global__ void norm_scale_add_norm_kernel(const T* __restrict__ a, float* __restrict__ stream,
+__global__ void norm_scale_add_norm_kernel(const T* a, float* stream,
                                            const float* __restrict__ w, int cols, float eps, float mult,
                                            const float* __restrict__ w2, float eps2, T* __restrict__ out) {
   extern __shared__ float row_s[];
@@ -217,7 +217,7 @@ __global__ void norm_scale_add_norm_kernel(const T* __restrict__ a, float* __res
 }
 
 template <typename T>
-__global__ void rmsnorm_rows_f32_kernel(const float* __restrict__ stream, const int* __restrict__ rows,
+__global__ void rmsnorm_rows_f32_kernel(const float* stream, const int* rows,
                                         const float* __restrict__ w, T* __restrict__ out, int cols, int src_rows,
                                         float eps, int* status) {
   __shared__ float scratch[33];
@@ -239,7 +239,7 @@ __global__ void rmsnorm_rows_f32_kernel(const float* __restrict__ stream, const 
 }
 
 template <typename T>
-__global__ void cast_rows_f32_kernel(const float* __restrict__ in, T* __restrict__ out, long long n) {
+__global__ void cast_rows_f32_kernel(const float* in, T* __restrict__ out, long long n) {
   pdl_launch_dependents();
   pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -247,7 +247,7 @@ __global__ void cast_rows_f32_kernel(const float* __restrict__ in, T* __restrict
 }
 
 template <typename T>
-__global__ void concat_rows_f32_kernel(const float* __restrict__ a, const float* __restrict__ b, T* __restrict__ out,
+__global__ void concat_rows_f32_kernel(const float* a, const float* b, T* __restrict__ out,
                                        int cols_a, int cols_b) {
   pdl_launch_dependents();
   pdl_wait();
@@ -258,7 +258,7 @@ __global__ void concat_rows_f32_kernel(const float* __restrict__ a, const float*
 }
 
 template <typename T>
-__global__ void sigmoid_gate_kernel(T* __restrict__ a, const T* __restrict__ g, long long g_stride, int cols) {
+__global__ void sigmoid_gate_kernel(T* a, const T* g, long long g_stride, int cols) {
   pdl_launch_dependents();
   pdl_wait();
   const long long t = blockIdx.x;
@@ -274,9 +274,9 @@ __global__ void sigmoid_gate_kernel(T* __restrict__ a, const T* __restrict__ g, 
 // VEC neighbouring columns per thread and turn (two sub-layers of 2,048 x 2,048 in bfloat16, 92 MB with cold caches: 40 us one
 // column at a time, 23 us in 16-byte pieces, in a step 29 and 13 us; 8 rows 12.4 and 8.2 us).
 template <typename T, int VEC>
-__global__ void gated_add_f32_kernel(const T* __restrict__ a, const T* __restrict__ f, const float* __restrict__ g,
+__global__ void gated_add_f32_kernel(const T* a, const T* f, const float* g,
                                      long long g_stride, const float* __restrict__ b1, const float* __restrict__ b2,
-                                     float* __restrict__ stream, T* __restrict__ copy, int cols) {
+                                     float* stream, T* __restrict__ copy, int cols) {
   pdl_launch_dependents();
   pdl_wait();
   const long long base = (long long)blockIdx.x * cols;
@@ -308,10 +308,10 @@ __global__ void gated_add_f32_kernel(const T* __restrict__ a, const T* __restric
 // a layer reads `cols` columns from `offset` on) gated by a projection of the stream.  An id of -1 is the token
 // the request sampled last, as in the embedding kernels.
 template <typename T>
-__global__ void side_gate_mul_kernel(const T* __restrict__ s, const int* __restrict__ ids, const T* __restrict__ table,
+__global__ void side_gate_mul_kernel(const T* s, const int* ids, const T* __restrict__ table,
                                      long long table_stride, int offset, T* __restrict__ out, int cols, int vocab,
-                                     const int* __restrict__ last_tokens, const int* __restrict__ token_req,
-                                     const int* __restrict__ req_slots, int* status) {
+                                     const int* last_tokens, const int* token_req,
+                                     const int* req_slots, int* status) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
@@ -329,7 +329,7 @@ __global__ void side_gate_mul_kernel(const T* __restrict__ s, const int* __restr
   }
 }
 
-__global__ void softcap_f32_kernel(float* __restrict__ x, long long n, float cap) {
+__global__ void softcap_f32_kernel(float* x, long long n, float cap) {
   pdl_launch_dependents();
   pdl_wait();
   const float inv = 1.f / cap;
@@ -337,7 +337,7 @@ __global__ void softcap_f32_kernel(float* __restrict__ x, long long n, float cap
     x[i] = cap * tanhf(x[i] * inv);
 }
 
-__global__ void scale_f32_kernel(float* __restrict__ x, long long n, float factor) {
+__global__ void scale_f32_kernel(float* x, long long n, float factor) {
   pdl_launch_dependents();
   pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)

@@ -12,10 +12,10 @@
 #define TSH_MAX_MIXES 16
 
 template <typename T, int VEC>
-__global__ void token_shift_mix_kernel(const T* __restrict__ h, long long h_stride, const float* __restrict__ mu, int mixes,
-                                       int width, T* __restrict__ out, float* __restrict__ state, long long state_stride,
-                                       int num_slots, const int* __restrict__ cu_q, const int* __restrict__ token_req,
-                                       const int* __restrict__ req_slots, int tokens, int single, int* status) {
+__global__ void token_shift_mix_kernel(const T* h, long long h_stride, const float* __restrict__ mu, int mixes,
+                                       int width, T* __restrict__ out, float* state, long long state_stride,
+                                       int num_slots, const int* cu_q, const int* token_req,
+                                       const int* req_slots, int tokens, int single, int* status) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.y;
@@ -57,7 +57,7 @@ __global__ void token_shift_mix_kernel(const T* __restrict__ h, long long h_stri
 
 template <typename T, int TOK>  // TOK tokens per block, TOK / LRD_TG per thread
 __global__ void __launch_bounds__(LRD_C * LRD_TG)
-low_rank_decay_kernel(const T* __restrict__ a, long long a_stride, int tokens, int rank, const T* __restrict__ w2,
+low_rank_decay_kernel(const T* a, long long a_stride, int tokens, int rank, const T* __restrict__ w2,
                       const float* __restrict__ w0, float* __restrict__ out, int out_stride, int channels, int log_out) {
   constexpr int PER = TOK / LRD_TG;
   __shared__ float w_s[LRD_C][LRD_R + 1];
@@ -109,7 +109,7 @@ __device__ __forceinline__ void lrm_mma(float (&c)[4], const unsigned (&a)[4], u
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __global__ void __launch_bounds__(128)
-low_rank_decay_mma_kernel(const __nv_bfloat16* __restrict__ a, long long a_stride, int tokens, int rank,
+low_rank_decay_mma_kernel(const __nv_bfloat16* a, long long a_stride, int tokens, int rank,
                           const __nv_bfloat16* __restrict__ w2, const float* __restrict__ w0, float* __restrict__ out,
                           int out_stride, int channels, int log_out) {
   pdl_launch_dependents();
