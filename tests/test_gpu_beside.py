@@ -36,12 +36,21 @@ def batch(q_lens, kv_lens, page, key_dim, kv_heads):
     return ctx, bt.cuda(), i32(cu), i32(kv_lens), i32([r for r, q in enumerate(q_lens) for _ in range(q)]), i32(range(len(q_lens))), pages
 
 
-@pytest.mark.parametrize("q_lens,kv_lens", [([1] * 4 + [200], [700, 650, 690, 700, 200]), ([1] * 9 + [33, 300], [9, 40, 2000, 100, 30, 700, 64, 5, 1200, 33, 410]),
-                                           ([1] * 40 + [17], [300 + i for i in range(40)] + [17])])
+@pytest.mark.parametrize("q_lens,kv_lens,kernel", [
+    ([1] * 4 + [200], [700, 650, 690, 700, 200], "decode"),
+    ([1] * 9 + [33, 300], [9, 40, 2000, 100, 30, 700, 64, 5, 1200, 33, 410], "decode_balanced"),
+    ([1] * 40 + [17], [300 + i for i in range(40)] + [17], "decode")])
 @pytest.mark.parametrize("Hq,Hkv", [(16, 8), (8, 1)])
 @pytest.mark.parametrize("window", [0, 128])
-def test_rows_beside_prompts(q_lens, kv_lens, Hq, Hkv, window):
-    kk = K()
+def test_rows_beside_prompts(monkeypatch, q_lens, kv_lens, kernel, Hq, Hkv, window):
+    kk, taken = K(), []
+    rows_of = kk._decode_rows
+
+    def watched(*a, beside=False, **kw):
+        rows_of(*a, beside=beside, **kw)
+        taken.append((kk.attention_path, beside))
+
+    monkeypatch.setattr(kk, "_decode_rows", watched)
     ctx, bt, cu, kl, req, rs, kp = batch(q_lens, kv_lens, 16, 128, Hkv)
     vp = rnd(*kp.shape, seed=4, dtype=torch.bfloat16)
     T = sum(q_lens)
@@ -54,6 +63,7 @@ def test_rows_beside_prompts(q_lens, kv_lens, Hq, Hkv, window):
         out = torch.full((T, Hq * 128), 7.0, dtype=torch.bfloat16, device="cuda")
         kk.qk_norm_in_place(qkv, Hq, Hkv, 128, weight, weight, 1e-6)  # (what the attention reads is written right in front of it)
         kk.paged_attention(qkv, out, kp, vp, bt, rs, cu, kl, req, Hq, Hkv, 128, 16, window, 128 ** -0.5, ctx)
+        assert kk.attention_path == "prefill_tcgen05" and taken.pop() == (kernel, True) and not taken
         return out
 
     on = kk.pdl
@@ -66,8 +76,15 @@ def test_rows_beside_prompts(q_lens, kv_lens, Hq, Hkv, window):
     kk.raise_on_status()
 
 
-def test_latent_rows_beside_prompts():
+def test_latent_rows_beside_prompts(monkeypatch):
     kk, Hq, dk, dv = K(), 16, 448, 384
+    taken, attention = [], kk.windowed_attention
+
+    def watched(*a, **kw):
+        attention(*a, **kw)
+        taken.append((kk.attention_path, kw.get("beside", False)))
+
+    monkeypatch.setattr(kk, "windowed_attention", watched)
     q_lens, kv_lens = [1] * 12 + [900, 600], [60 + 150 * i for i in range(12)] + [900, 600]
     ctx, bt, cu, kl, req, rs, kp = batch(q_lens, kv_lens, 16, dk, 1)
     T = sum(q_lens)
@@ -78,7 +95,9 @@ def test_latent_rows_beside_prompts():
         out = torch.full((T, Hq * dv), 7.0, dtype=torch.bfloat16, device="cuda")
         kk.windowed_attention(q, out, kp, None, bt, rs, cu, kl, req, Hq, 1, dk, dv, 16, 0, 0.07, num_requests=len(q_lens),
                               workspace=ctx.workspace, ctx=ctx)
-        assert kk.attention_path in ("latent_tcgen05", "window_mma")
+        # (the call for the rows ends before the call that it is part of)
+        assert taken == [("window_mma", True), ("latent_tcgen05", False)] and kk.attention_path == "latent_tcgen05"
+        taken.clear()
         return out
 
     on = kk.pdl

@@ -1273,12 +1273,12 @@ class Kernels:
                     head_dim, v_dim, page_size, int(window), float(scale), num_pages, _ptr(self.status), _stream())
                 if code != 4:
                     self._check(code, f"latent_attention (key rows {head_dim}, values {v_dim})")
-                    self.attention_path = "latent_tcgen05"
                     if n_dec:
                         self.windowed_attention(
                             q[:n_dec], out[:n_dec], k_pages, None, block_table, req_slots[:n_dec], cu_q[:n_dec + 1],
                             kv_len[:n_dec], token_req[:n_dec], num_q, num_kv, head_dim, v_dim, page_size, window, scale,
                             num_requests=n_dec, workspace=workspace, beside=True)
+                    self.attention_path = "latent_tcgen05"
                     return
         p_pages = pk.numel() // (page_size * num_kv * head_dim) if pk is not None else 0
         if (self.window_attention_tc and q.dtype == torch.bfloat16 and num_requests and q.stride(0) % 8 == 0
