@@ -120,7 +120,9 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tp_smem(&tmem_slot)), "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
+    // (Only now: a kernel behind this one must not hold tensor memory that this one waits for; and only behind pdl_wait(): decode attention
+    // beside this kernel takes its own start for the end of everything in front of this one.)
+    pdl_launch_dependents();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

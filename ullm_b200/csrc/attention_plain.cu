@@ -58,8 +58,6 @@ __device__ __forceinline__ void pl_axpy(float p, const float4& v, float4& o) {
   o.w = fmaf(p, v.w, o.w);
 }
 
-// four neighbouring elements into shared memory, as 32-bit values: 32-bit ones arrive behind the thread's back (pl_wait), others at once.
-// None of them read: zeros.
 // pairs of neighbouring 32-bit values, multiplied and added two at a time
 struct __align__(16) pl_four { unsigned long long lo, hi; };
 __device__ __forceinline__ void pl_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
@@ -79,6 +77,8 @@ __device__ __forceinline__ void pl_axpy2(unsigned long long p, const pl_four& v,
   asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(lo));
   asm("mov.b64 {%0, %1}, %2;" : "=f"(o.z), "=f"(o.w) : "l"(hi));
 }
+// four neighbouring elements into shared memory, as 32-bit values: 32-bit ones arrive behind the thread's back (pl_wait), others at once.
+// None of them read: zeros.
 __device__ __forceinline__ void pl_bring(float* dst, const float* src, bool there) {
   const unsigned at = (unsigned)__cvta_generic_to_shared(dst), bytes = there ? 16u : 0u;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(src), "r"(bytes) : "memory");
@@ -279,24 +279,24 @@ plain_attention_prompt_kernel(const T* q, long long q_row_stride, T* __restrict_
         }
       } else {
 #pragma unroll 2
-      for (int key = 0; key < PT_KEYS; key += 4) {
-        float4 p[4];
+        for (int key = 0; key < PT_KEYS; key += 4) {
+          float4 p[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(ps + (ty * 4 + i) * PT_PS + key);
+          for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(ps + (ty * 4 + i) * PT_PS + key);
 #pragma unroll
-        for (int c = 0; c < CV; ++c) {
-          const float* vp = vs + key * ST + c * 64 + tx * 4;
-          const pl_four v0 = *reinterpret_cast<const pl_four*>(vp), v1 = *reinterpret_cast<const pl_four*>(vp + ST),
-                        v2 = *reinterpret_cast<const pl_four*>(vp + 2 * ST), v3 = *reinterpret_cast<const pl_four*>(vp + 3 * ST);
+          for (int c = 0; c < CV; ++c) {
+            const float* vp = vs + key * ST + c * 64 + tx * 4;
+            const pl_four v0 = *reinterpret_cast<const pl_four*>(vp), v1 = *reinterpret_cast<const pl_four*>(vp + ST),
+                          v2 = *reinterpret_cast<const pl_four*>(vp + 2 * ST), v3 = *reinterpret_cast<const pl_four*>(vp + 3 * ST);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            pl_axpy2(pl_twice(p[i].x), v0, o[i][c]);
-            pl_axpy2(pl_twice(p[i].y), v1, o[i][c]);
-            pl_axpy2(pl_twice(p[i].z), v2, o[i][c]);
-            pl_axpy2(pl_twice(p[i].w), v3, o[i][c]);
+            for (int i = 0; i < 4; ++i) {
+              pl_axpy2(pl_twice(p[i].x), v0, o[i][c]);
+              pl_axpy2(pl_twice(p[i].y), v1, o[i][c]);
+              pl_axpy2(pl_twice(p[i].z), v2, o[i][c]);
+              pl_axpy2(pl_twice(p[i].w), v3, o[i][c]);
+            }
           }
         }
-      }
       }
       group_sync();  // V has been read
       bring(vs, v_cache, turn ^ 1);

@@ -179,7 +179,9 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
                  "r"(TP_TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    pdl_launch_dependents();  // (only now: a kernel behind this one must not hold tensor memory that this one waits for)
+    // (Only now: a kernel behind this one must not hold tensor memory that this one waits for; and only behind pdl_wait(): decode attention
+    // beside this kernel takes its own start for the end of everything in front of this one.)
+    pdl_launch_dependents();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -185,9 +185,11 @@ __device__ __forceinline__ void store_vec32(float* p, const float (&v)[VEC]) {
 //                             this one are running (its blocks then wait in their own pdl_wait)
 //   pdl_wait();               blocks until the previous kernel in the stream has completed and its
 //                             writes are visible; nothing that depends on it may be touched before
-// so that launch latency and per-block set-up of a kernel overlap with the tail of the one before it.  A kernel that allocates tensor
-// memory calls the first only when it has it: blocks of several kernels may be resident, and one that waits for its turn must not
-// hold what one in front of it still needs.
+// so that launch latency and per-block set-up of a kernel overlap with the tail of the one before it.  Two exceptions:
+// A kernel that allocates tensor memory calls the first only when it has it: blocks of several kernels may be resident, and one that
+// waits for its turn must not hold what one in front of it still needs.  The tcgen05 prompt attention kernels call it behind their own
+// pdl_wait() besides, because decode attention of the same step's other rows may run beside them (decode_core.cuh): that kernel reads
+// q and the pages at once and waits at its end.
 // A kernel may do work that does not depend on its predecessor (reading weights) before pdl_wait().
 // What a kernel of the same step may have written is read through pointers WITHOUT __restrict__, and never by __ldg or ld.global.nc: all of
 // them tell the compiler that the data does not change while this kernel runs, so that it may load before pdl_wait(), memory clobber or

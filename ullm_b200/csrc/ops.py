@@ -1,5 +1,5 @@
 """Python face of the compiled kernels: loads the shared library, binds its
-functions through native_call.cpp and wraps each extern "C" launcher in a method that checks devices, dtypes,
+functions through native_call.cpp (or plain_call.py) and wraps each extern "C" launcher in a method that checks devices, dtypes,
 shapes and contiguity before passing raw pointers and the current CUDA stream.
 
 There is no CPU path here: a tensor that is not on a CUDA device is an error,
@@ -2266,7 +2266,7 @@ class Kernels:
             self.launches += 1  # the merge of the shared pairs
             self.attention_path = "decode_tcgen05" if tc else "decode_balanced"
             return
-        # Up to 8 rows (the steps that run under dependent launch) the splits of a request merge inside a
+        # Up to `stream_all_rows` rows (16, and 8 at least) the splits of a request merge inside a
         # thread-block cluster: no merge kernel stands between the attention and the output projection, whose ring
         # fills meanwhile.  The cluster is the largest power of two that keeps all blocks in one wave of two per
         # SM (8 requests x 8 kv heads: 4 splits, 3.59 ms per step against 3.87 with 7 splits and the merge kernel;
