@@ -15,7 +15,7 @@
 // 1.0e-7 to 1.5e-7, the library's 5.7e-7 to 2.0e-6.
 //
 // Warps 0..7 load rows of w (one or two k blocks ahead, in registers; four more are asked for into L2: 31.7 and 29.7 us for 511 x 1,024 x
-// 2,048), split them and store the terms in K-major 128-byte-swizzled tiles; a thread of warp 0 asks for the planes of x; warps 16 and 17
+// 2,048 when that was brought in, 31.7 with it since the issuing warps wait for their stage), split them and store the terms in K-major 128-byte-swizzled tiles; a thread of warp 0 asks for the planes of x; warps 16 and 17
 // issue the products, a k block each in turn (one thread for all of them paced everything, 1,500 clocks a k block of 32 columns: 52 us for
 // 511 x 1,024 x 3,072); warps 8..15 add the block sums up, a quarter of the rows and half of the columns each.  Two or three stages, two
 // or four block sums in tensor memory.  BN from 32 to 128, so that the tiles fill the SMs.
@@ -342,8 +342,9 @@ static int fs_go(const CUtensorMap& x_map, const FsParams& p, long long tiles, c
 }
 
 // Columns per tile by (waves of tiles) x (ns of a k block, measured: 511 rows, 1,024 columns of k 1,024 to 4,096 in tiles of 32, 64,
-// 96 and 128: 19.5 to 50, 23.5 to 61, 27.7 to 81, 31.7 to 85 us in one wave each); the wider tile where both agree.  0: the device's SM
-// count cannot be read.
+// 96 and 128: 21.5 to 52, 23.5 to 61, 27.7 to 81, 31.7 to 85 us in one wave each, the last three before the issuing warps waited for their
+// stage, which added 2 us to the first and nothing to its slope); the wider tile where both agree.  0: the device's SM count cannot be
+// read.
 extern "C" int ullm_linear_f32_split_columns(int M, int N) {
   static int sms = 0;
   if (sms == 0) {
